@@ -3,7 +3,7 @@ by one) for every kind of model it runs, and a single operator call on host data
 
 A case of a decoder: `context` positions stand in the cache, a prompt of `prompt` tokens is prefilled behind them, then
 `steps` tokens are decoded one at a time.  The tokens are the caller's (a sampler of its own, or a text being scored);
-the greedy next tokens and the logits of the last position come back.  Weights are random, in the formats that a model
+the logits of the last position come back.  Weights are random, in the formats that a model
 file has; dense and MoE stacks hold K-quant blocks, the mixed stacks bf16.
 """
 from __future__ import annotations
@@ -152,7 +152,7 @@ class _Quantised:
         g, self.pool = _gpu_rng(seed), {}
         for t in (Q4_K, Q6_K):
             most = max(r * k // 256 for n, (u, r, k) in (self.shapes | self.globals).items() if u == t and n != "token_embd")
-            self.pool[t] = _blocks(t, most + 65536, g, 0.64 / D ** 0.5)
+            self.pool[t] = _blocks(t, most + 65536, g, 0.45 / D ** 0.5)
         self.pool["token_embd"] = _blocks(Q4_K, V * D // 256, g, 1.0)
         if host:
             self.pool = {t: b.cpu().numpy() for t, b in self.pool.items()}
@@ -294,16 +294,16 @@ def run(state):
     c = state["case"]
     if c["kind"] == "operator":
         return (ops.q4k_gemv if c["type"] == Q4_K else ops.q6k_gemv)(state["w"], c["rows"], c["cols"], state["x"])
-    dec, tokens, pos, ids = state["decoder"], state["tokens"], c["context"], []
+    dec, tokens, pos = state["decoder"], state["tokens"], c["context"]
     if c["prompt"]:
-        ids.append(dec.prefill(tokens[:c["prompt"]], pos))
+        dec.prefill(tokens[:c["prompt"]], pos)
         pos += c["prompt"]
     for t in tokens[c["prompt"]:]:
-        ids.append(dec.step(t, pos))
+        dec.step(t, pos)
         pos += 1
-    # what a step adds to the caches and states shows in the next one's logits; a single token is their argmax, no more
-    out = {"logits": dec.read_logits()}
-    return out | {"next": np.array(ids, np.int64)} if len(ids) > 1 else out
+    # What a step adds to the caches and states shows in the next one's logits.  The greedy tokens stay out: where two
+    # logits nearly tie, another order of a sum picks the other one.
+    return {"logits": dec.read_logits()}
 
 
 # ---- what it cannot do without -------------------------------------------------------------------
@@ -354,13 +354,11 @@ def tolerance(case):
     # Activations are quantised to 8 bits (steps) or rounded to bf16 (prompts): a last-bit change in the order of a sum
     # moves some of them by one step, and later layers more.  Measured with other attention kernels (a step's in chunks
     # instead of in order, a prompt's split over the keys), another epilogue of the gate and up product, and prompts cut
-    # into portions: 2.3e-2, 1.1e-2 and 6e-3 (largest 0.13, 0.05 and 0.025); the operator gave the same bits.  `differ`: the
-    # greedy token where two logits nearly tie, 2 of 17 in one of 25 cases.
+    # into portions, 35 cases: 1.24e-2 with steps, 6e-3 without and for mixed stacks (largest 0.057 and 0.026); the
+    # operator gave the same bits.
     if case["kind"] == "operator":
         return {"rel": 1e-5, "max": 1e-4}
-    n = case["steps"] + (1 if case["prompt"] else 0)
-    rel, most = (0.025, 0.1) if case["kind"] in ("punisun", "dutivik") else (0.09, 0.5) if case["steps"] else (0.045, 0.2)
-    return {"rel": rel, "max": most, "differ": 1.0 / n + 0.25 if n > 1 else 0.0}
+    return {"rel": 0.03, "max": 0.23} if case["kind"] in ("dense", "moe") and case["steps"] else {"rel": 0.024, "max": 0.11}
 
 
 # ---- the same in 64 bits -------------------------------------------------------------------------
@@ -371,8 +369,7 @@ def exact(case, seed):
         x = np.random.default_rng(seed).standard_normal(c["cols"]).astype(np.float32)
         return w @ torch.from_numpy(x).double().cuda()
     tokens = torch.from_numpy(_tokens(c, seed)).cuda()
-    out = {"logits": (_exact_dense if c["kind"] in ("dense", "moe") else _exact_stack)(c, seed, tokens)}
-    return out | {"next": None} if c["steps"] + (1 if c["prompt"] else 0) > 1 else out
+    return {"logits": (_exact_dense if c["kind"] in ("dense", "moe") else _exact_stack)(c, seed, tokens)}
 
 
 def _mix64(z):
