@@ -406,6 +406,7 @@ int prefill_gemm_setup() {
     static bool done = false;
     if (done) return RNB_B200_OK;
     RNB_CU(cudaFuncSetAttribute(prefill_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PG_SMEM));
+    RNB_CU(cudaFuncSetAttribute(prefill_gemm_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PS_SMEM));
     done = true;
     return RNB_B200_OK;
 }

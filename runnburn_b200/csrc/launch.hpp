@@ -11,6 +11,7 @@
 #include "gemv_q5k.cuh"
 #include "moe.cuh"
 #include "prefill_gemm.cuh"
+#include "prefill_gemm_split.cuh"
 #include "q8k.cuh"
 #include "state.hpp"
 
@@ -48,9 +49,9 @@ inline cudaError_t launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, siz
     return e;
 }
 
-// The same launch as one thread-block cluster per grid column: cluster dimensions (1, cluster_y, 1).
+// The same launch in thread-block clusters.
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_k_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, unsigned cluster_y, Args... args) {
+inline cudaError_t launch_k_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, dim3 cluster, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -58,9 +59,9 @@ inline cudaError_t launch_k_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 bl
     cfg.stream = s;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 1;
-    attr[0].val.clusterDim.y = cluster_y;
-    attr[0].val.clusterDim.z = 1;
+    attr[0].val.clusterDim.x = cluster.x;
+    attr[0].val.clusterDim.y = cluster.y;
+    attr[0].val.clusterDim.z = cluster.z;
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
@@ -637,7 +638,7 @@ inline int launch_flash_decode_partials(cudaStream_t s, const float *q, const ui
             m = *merge;
             m.counters = nullptr;
             if (merged) *merged = true;
-            RNB_CU(launch_k_cluster(flash_decode_mma_kernel, dim3(num_kv_heads, n_chunks), dim3(FDM_THREADS), 0, s, (unsigned)n_chunks, q, k, v, kv_len_dev,
+            RNB_CU(launch_k_cluster(flash_decode_mma_kernel, dim3(num_kv_heads, n_chunks), dim3(FDM_THREADS), 0, s, dim3(1, (unsigned)n_chunks), q, k, v, kv_len_dev,
                                     kv_len_host, num_heads, num_kv_heads, scale, partials, dev_error, m));
             return RNB_B200_OK;
         }
@@ -734,6 +735,50 @@ inline int encode_token_map(PgTensorMap *out, const uint16_t *xb, size_t seq, si
     if (r != CUDA_SUCCESS) return fail(RNB_B200_CUDA_ERROR, "cuTensorMapEncodeTiled failed with driver code %d", (int)r);
     return RNB_B200_OK;
 }
+// CTAs along K for a short prompt, 0: the 512-token tiles.  Measured on the matrices of the 8B and 1B shapes, 16 to 512
+// tokens (us, 512-token tiles / this rule):
+//   matrices of their own: 203 tokens 4096 x 4096 55 / 29, 4096 x 14336 251 / 61, q + k + v 77 / 43, 2048 x 8192 147 / 38;
+//     400 tokens 55 / 37, 255 / 112, 77 / 71, 148 / 41.  With 4 to 7, 8 to 31 and more blocks of 256 columns 2, 4 and 8
+//     CTAs were the fastest or within 5 % of it; the count depends on K and the tokens alone, so that a matrix gives the
+//     same bits in every launch that it can be part of.
+//   gate + up: 45 tokens 116 / 67 (14336 x 4096) and 35 / 26 (8192 x 2048), 203 tokens 124 / 93 and 39 / 40, 320 tokens
+//     128 / 159 and 41 / 51 - two token tiles dequantise twice, so longer prompts keep the 512-token tile.  Its row tiles
+//     fill the chip without a cut from 128 on (cut in 2: 119 and 46 at 203 tokens).
+inline int prefill_split_ks(bool pair, int tiles, size_t seq, size_t cols) {
+    const int nb = (int)(cols / 256);
+    if (pair) {
+        if (seq > PS_TOK) return 0;
+        int ks = 1;
+        while (ks * 2 * tiles <= 148 && ks * 2 <= std::min(nb / 2, PS_MAX_KS)) ks *= 2;
+        return ks;
+    }
+    if (seq >= (size_t)PG_TOK) return 0;
+    return nb < 4 ? 1 : nb < 8 ? 2 : nb < 32 ? 4 : PS_MAX_KS;
+}
+// `tiles`: row tiles of all jobs
+inline int launch_prefill_gemm_tiles(cudaStream_t s, const PgJobs &jobs, int tiles, size_t seq, size_t cols, const uint16_t *xb, int *dev_error) {
+    PgTensorMap tmap;
+    const int ks = prefill_split_ks(jobs.j[0].w2 != nullptr, tiles, seq, cols);
+    if (ks == 0) {
+        RNB_TRY(encode_token_map(&tmap, xb, seq, cols));
+        const dim3 grid((unsigned)tiles, (unsigned)((seq + PG_TOK - 1) / PG_TOK));
+        RNB_CU(launch_k(prefill_gemm_kernel, grid, dim3(PG_THREADS), PG_SMEM, s, jobs, tmap, (int)seq, (int)cols, dev_error));
+        return RNB_B200_OK;
+    }
+    PsParams P;
+    const int token_tiles = (int)((seq + PS_TOK - 1) / PS_TOK);
+    P.seq = (int)seq;
+    P.cols = (int)cols;
+    P.ks = ks;
+    P.nt = ((P.seq + token_tiles - 1) / token_tiles + 15) & ~15;
+    P.stages = std::min<int>(PS_MAX_STAGES, (int)(PS_SMEM_STAGES / ((uint32_t)P.nt * 128u + PG_B_BYTES)));
+    P.tmem_cols = 32;
+    while ((int)P.tmem_cols < P.nt) P.tmem_cols *= 2;
+    RNB_TRY(encode_token_map(&tmap, xb, seq, cols, 0, P.nt));
+    const dim3 grid((unsigned)(tiles * ks), (unsigned)token_tiles);
+    RNB_CU(launch_k_cluster(prefill_gemm_split_kernel, grid, dim3(PS_THREADS), PS_SMEM, s, dim3((unsigned)ks), jobs, tmap, P, dev_error));
+    return RNB_B200_OK;
+}
 inline int launch_prefill_gemm_multi(cudaStream_t s, int n, const int *types, const uint8_t *const *w, const size_t *rows, float *const *y,
                                      size_t cols, const float *x, size_t seq, uint16_t *xb, int *dev_error) {
     if (n < 1 || n > PG_MAX_JOBS) return fail(RNB_B200_VALIDATION_FAILED, "prefill matmul takes 1..%d matrices per launch", PG_MAX_JOBS);
@@ -760,11 +805,7 @@ inline int launch_prefill_gemm_multi(cudaStream_t s, int n, const int *types, co
     RNB_TRY(prefill_gemm_setup());
     const size_t ne = seq * cols;
     if (x) RNB_CU(launch_k(f32_to_bf16_kernel, dim3((unsigned)((ne / 8 + 255) / 256)), dim3(256), 0, s, x, xb, ne));
-    PgTensorMap tmap;
-    RNB_TRY(encode_token_map(&tmap, xb, seq, cols));
-    const dim3 grid((unsigned)tiles, (unsigned)((seq + PG_TOK - 1) / PG_TOK));
-    RNB_CU(launch_k(prefill_gemm_kernel, grid, dim3(PG_THREADS), PG_SMEM, s, jobs, tmap, (int)seq, (int)cols, dev_error));
-    return RNB_B200_OK;
+    return launch_prefill_gemm_tiles(s, jobs, tiles, seq, cols, xb, dev_error);
 }
 // gate + up of a token batch with silu(gate) * up in the epilogue: act [seq][rows] bf16, ready to be the token matrix of
 // the down matmul.  `act` must not alias `xb` (other CTAs are still reading tokens when the first tiles finish).
@@ -788,11 +829,7 @@ inline int launch_prefill_gemm_silu(cudaStream_t s, int type, const uint8_t *gat
     RNB_TRY(prefill_gemm_setup());
     const size_t ne = seq * cols;
     if (x) RNB_CU(launch_k(f32_to_bf16_kernel, dim3((unsigned)((ne / 8 + 255) / 256)), dim3(256), 0, s, x, xb, ne));
-    PgTensorMap tmap;
-    RNB_TRY(encode_token_map(&tmap, xb, seq, cols));
-    const dim3 grid((unsigned)tiles, (unsigned)((seq + PG_TOK - 1) / PG_TOK));
-    RNB_CU(launch_k(prefill_gemm_kernel, grid, dim3(PG_THREADS), PG_SMEM, s, jobs, tmap, (int)seq, (int)cols, dev_error));
-    return RNB_B200_OK;
+    return launch_prefill_gemm_tiles(s, jobs, tiles, seq, cols, xb, dev_error);
 }
 inline int launch_prefill_gemm(cudaStream_t s, int type, const uint8_t *w, size_t rows, size_t cols, const float *x, size_t seq,
                                uint16_t *xb, float *y, int *dev_error) {

@@ -1,0 +1,285 @@
+// Prefill matmul for short prompts: the same product as prefill_gemm_kernel (dequantised bf16 weights x bf16 tokens,
+// f32 accumulators in tensor memory), cut so that a few hundred tokens still occupy the chip.
+//
+// A CTA owns 128 weight rows x up to 256 tokens and a part of K; the `ks` CTAs of a thread-block cluster share a tile
+// and add their accumulators over distributed shared memory in rank order (the same bits on every run, whichever CTA
+// adds).  A 512-token tile per CTA leaves 32 CTAs for the 4096 rows of an output projection on 148 SMs, each with a
+// chain of 64 to 224 stages; with K cut in 8 the chain is 8 to 28 stages on 256 CTAs.
+//
+// Two CTAs per SM.  A stage is 64 elements of K: nt tokens x 128 bytes by one tiled TMA copy, and 128 weight rows that
+// eight warps dequantise straight into the operand tile (layouts as in prefill_gemm.cuh).  Weights do not depend on the
+// previous launch: the CTA asks L2 for its whole part of every row and dequantises its first stages before the
+// dependency wait; only the token copies and the stores come after it.  Warps 0-7 dequantise, then reduce and store;
+// warp 8 issues the MMAs, warp 9 the token copies.  Every wait is bounded; after a timeout all threads still meet at
+// the cluster barriers.
+//
+// What bounds it: the dequantising warps' chain of a stage (about 800 cycles per SM and stage at any token count, 40 % of
+// the issue slots, tensor pipe 28 % busy at 203 tokens).  Seven matmuls of an 8B layer at 203 tokens: 226 us, with the
+// 512-token tiles 507 us; of a 1B layer at 45 tokens 84 against 252 us.
+#pragma once
+#include "prefill_gemm.cuh"
+
+namespace rnb {
+
+constexpr int PS_TOK = 256;        // most tokens per CTA
+constexpr int PS_THREADS = 320;
+constexpr int PS_MAX_STAGES = 5;
+constexpr uint32_t PS_SMEM_STAGES = 96 * 1024;   // operand stages; the reduction reuses them
+constexpr size_t PS_SMEM = PS_SMEM_STAGES + 1024;
+constexpr int PS_MAX_KS = 8;
+
+struct PsParams {
+    int seq, cols, nt, stages, ks;   // nt: tokens per CTA (multiple of 16), ks: CTAs along K (the cluster)
+    uint32_t tmem_cols;
+};
+
+__device__ __forceinline__ void ps_mma(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+template <int N>
+__device__ __forceinline__ void ps_tmem_ld(uint32_t taddr, uint32_t (&v)[N]) {
+    static_assert(N == 8 || N == 16, "columns per load");
+    if constexpr (N == 16)
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                     : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
+                       "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+                     : "r"(taddr));
+    else
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                     : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void ps_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t ps_map(uint32_t addr, int rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void ps_st_remote(uint32_t addr, uint32_t v) { asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
+
+// Sums and stores the tile.  A round gives every CTA of the cluster one chunk of 2 * SUB tokens: the others send it
+// their accumulators of that chunk, it adds them in rank order with its own.  Warp w holds the rows of lane quarter
+// w & 3 and the chunk's tokens (w >> 2) * SUB ..; all threads of the CTA come through here (cluster barriers).
+template <int SUB>
+__device__ __forceinline__ void ps_finish(const PgJob &job, const PsParams &P, uint8_t *smem, uint32_t tmem, int kr, int n0, int m0, bool fin) {
+    constexpr int CT = 2 * SUB;                       // tokens per chunk
+    constexpr uint32_t SLOT = CT * PG_ROWS * 4;       // one CTA's accumulators of a chunk: [token][row]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, ks = P.ks;
+    const bool worker = warp < 8, pair = job.w2 != nullptr;
+    const int q = warp & 3, sub = (warp >> 2) & 1, rows = job.rows;
+    const int end = min(P.seq, m0 + P.nt), n_chunks = (end - m0 + CT - 1) / CT;
+    const uint32_t base = smem_u32(smem), mine = (uint32_t)(sub * SUB * PG_ROWS + q * 32 + lane) * 4u;
+    const uint32_t lanes = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(sub * SUB);
+    float *ex = reinterpret_cast<float *>(smem + (size_t)(ks - 1) * SLOT);   // gate / up exchange, two buffers in turn
+    for (int j = 0; j * ks < n_chunks; j++) {
+        if (ks > 1) {
+            if (worker)
+                for (int i = 1; i < ks; i++) {
+                    const int to = (kr + i) % ks, cc = j * ks + to;
+                    if (cc >= n_chunks) continue;
+                    uint32_t v[SUB];
+                    if (fin) ps_tmem_ld<SUB>(lanes + (uint32_t)(cc * CT), v);
+                    const uint32_t dst = ps_map(base + (uint32_t)(kr < to ? kr : kr - 1) * SLOT + mine, to);
+#pragma unroll
+                    for (int t = 0; t < SUB; t++) ps_st_remote(dst + (uint32_t)(t * PG_ROWS * 4), fin ? v[t] : 0u);
+                }
+            ps_cluster_sync();
+        }
+        const int cc = j * ks + kr;
+        if (worker && cc < n_chunks) {
+            uint32_t v[SUB];
+            if (fin) ps_tmem_ld<SUB>(lanes + (uint32_t)(cc * CT), v);
+            float s[SUB];
+#pragma unroll
+            for (int t = 0; t < SUB; t++) {
+                const float own = fin ? __uint_as_float(v[t]) : 0.f;
+                const float *part = reinterpret_cast<const float *>(smem + mine) + t * PG_ROWS;
+                s[t] = kr == 0 ? own : part[0];
+                for (int r = 1; r < ks; r++) s[t] += r == kr ? own : part[(size_t)(r < kr ? r : r - 1) * (SLOT / 4)];
+            }
+            const int tok0 = m0 + cc * CT;
+            if (pair) {
+                // gate rows on lane quarters 0 and 1, the same rows of up on 2 and 3: each warp finishes half of its tokens
+                float *buf = ex + (size_t)(j & 1) * (SLOT / 4);
+#pragma unroll
+                for (int t = 0; t < SUB; t++) buf[(sub * SUB + t) * PG_ROWS + q * 32 + lane] = s[t];
+                asm volatile("bar.sync 1, 256;" ::: "memory");
+                const int row = n0 + (q & 1) * 32 + lane, t_lo = sub * SUB + (q >> 1) * (SUB / 2);
+                if (fin && row < rows) {
+#pragma unroll
+                    for (int t = t_lo; t < t_lo + SUB / 2; t++) {
+                        const float g = buf[t * PG_ROWS + (q & 1) * 32 + lane], u = buf[t * PG_ROWS + 64 + (q & 1) * 32 + lane];
+                        // fast exponential and division: their 2^-21 relative error disappears in the bf16 rounding below
+                        const float a = __fdividef(g, 1.0f + __expf(-g)) * u;
+                        if (tok0 + t < end) job.yb[(size_t)(tok0 + t) * rows + row] = (uint16_t)(pg_pack_bf16(a, 0.f) & 0xffffu);
+                    }
+                }
+            } else if (fin && n0 + q * 32 + lane < rows) {
+                float *dst = job.y + (size_t)(tok0 + sub * SUB) * rows + n0 + q * 32 + lane;
+#pragma unroll
+                for (int t = 0; t < SUB; t++)
+                    if (tok0 + sub * SUB + t < end) dst[(size_t)t * rows] = s[t];
+            }
+        }
+        if (ks > 1 && (j + 1) * ks < n_chunks) ps_cluster_sync();   // the slots are free for the next round
+    }
+}
+
+// grid = (row tiles of all jobs x ks, token tiles), cluster (ks, 1, 1); 320 threads; dynamic shared memory PS_SMEM.
+RNB_GLOBAL void __launch_bounds__(PS_THREADS, 2)
+prefill_gemm_split_kernel(const __grid_constant__ PgJobs jobs, const __grid_constant__ PgTensorMap tmap_x, const PsParams P, int *__restrict__ err_flag) {
+    extern __shared__ __align__(1024) uint8_t pg_smem_raw[];
+    __shared__ __align__(8) uint64_t full[PS_MAX_STAGES], empty[PS_MAX_STAGES], done_bar;
+    __shared__ uint32_t tmem_slot;
+    __shared__ int s_failed;
+    pdl_launch_dependents();
+    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(pg_smem_raw) + 1023) & ~(uintptr_t)1023);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tile = (int)blockIdx.x / P.ks, kr = (int)blockIdx.x - tile * P.ks;
+    int jsel = 0;
+    for (int i = 1; i < jobs.n; i++)
+        if (tile >= jobs.j[i].tile0) jsel = i;
+    const PgJob &job = jobs.j[jsel];
+    const int rows = job.rows, S = P.stages;
+    const bool pair = job.w2 != nullptr, q4 = job.type == TYPE_Q4_K;
+    const uint32_t BLK = q4 ? Q4K_BYTES : Q6K_BYTES, x_bytes = (uint32_t)P.nt * 128u, stage_bytes = x_bytes + PG_B_BYTES;
+    const int n0 = (tile - job.tile0) * (pair ? PG_ROWS / 2 : PG_ROWS), m0 = blockIdx.y * P.nt;
+    const int nb = P.cols >> 8, b0 = nb * kr / P.ks, b1 = nb * (kr + 1) / P.ks, KT = (b1 - b0) * 4;   // this CTA's blocks of K
+    if (tid == 0) {
+        for (int s = 0; s < S; s++) {
+            mbar_init(&full[s], 9);    // one arrival per dequantising warp + the thread that issues the token copies
+            mbar_init(&empty[s], 1);   // tcgen05.commit
+        }
+        mbar_init(&done_bar, 1);
+        mbar_fence_init();
+        s_failed = 0;
+    }
+    __syncthreads();
+    bool ok = true;
+
+    if (warp < 8) {
+        const int row = tid >> 1, h = tid & 1, rr = row & 7;
+        const size_t rb = (size_t)nb * BLK;
+        // rows past the end repeat the last one (never stored)
+        const uint8_t *wr = (pair ? (row < PG_ROWS / 2 ? job.w : job.w2) + (size_t)min(n0 + (row & (PG_ROWS / 2 - 1)), rows - 1) * rb
+                                  : job.w + (size_t)min(n0 + row, rows - 1) * rb) + (size_t)b0 * BLK;
+        for (uint32_t o = 128u * (uint32_t)h; o < (uint32_t)(b1 - b0) * BLK; o += 256u) asm volatile("prefetch.global.L2 [%0];" ::"l"(wr + o));
+        uint8_t *const brow = smem + x_bytes + (row >> 3) * 1024 + rr * 128;
+        int s = 0;
+        uint32_t phase = 0;
+        auto begin = [&]() { return __all_sync(0xffffffffu, mbar_wait_bounded(&empty[s], phase ^ 1u)); };   // warp-uniform: shuffles follow
+        auto end = [&]() {
+            pg_proxy_fence();
+            __syncwarp();
+            if (lane == 0) pg_arrive(&full[s]);
+            if (++s == S) s = 0, phase ^= 1u;
+        };
+        if (q4) {
+            // a whole block (four stages) is fetched while the one before it is used
+            uint2 hh, hn = make_uint2(0u, 0u);
+            uint4 qc[4], qn[4];
+            auto load = [&](const uint8_t *blk, uint2 &hd, uint4 (&qq)[4]) {
+                hd = ldg_nc_u2(blk + 8 * h);
+#pragma unroll
+                for (int g = 0; g < 4; g++) qq[g] = ldg_nc_u4(blk + 16 + 32 * g + 16 * h);
+            };
+            load(wr, hh, qc);
+            for (int b = b0; b < b1 && ok; b++) {
+                wr += BLK;
+                if (b + 1 < b1) load(wr, hn, qn);
+                const uint32_t ox = __shfl_xor_sync(0xffffffffu, hh.x, 1), oy = __shfl_xor_sync(0xffffffffu, hh.y, 1);
+                const uint4 hdr = h ? make_uint4(ox, oy, hh.x, hh.y) : make_uint4(hh.x, hh.y, ox, oy);
+#pragma unroll
+                for (int g = 0; g < 4; g++) {
+                    if (ok) ok = begin();
+                    if (!ok) break;
+                    const uint4 other = pg_pair_exchange(qc[g]);
+                    pg_dequant_q4(hdr, h ? other : qc[g], h ? qc[g] : other, g, h, brow + (uint32_t)s * stage_bytes, rr);
+                    end();
+                }
+                hh = hn;
+#pragma unroll
+                for (int g = 0; g < 4; g++) qc[g] = qn[g];
+            }
+        } else {
+            PgRawQ6 cur, nxt;
+            pg_load_q6(cur, wr, 0, h);
+            for (int hb = 0; hb < 2 * (b1 - b0) && ok; hb++) {   // half blocks of 128 elements, two stages each
+                if (hb + 1 < 2 * (b1 - b0)) pg_load_q6(nxt, wr + (size_t)((hb + 1) >> 1) * BLK, (hb + 1) & 1, h);
+#pragma unroll
+                for (int g = 0; g < 2; g++) {
+                    if (ok) ok = begin();
+                    if (!ok) break;
+                    pg_dequant_q6(cur, g, h, brow + (uint32_t)s * stage_bytes, rr);
+                    end();
+                }
+                cur = nxt;
+            }
+        }
+    } else if (warp == 8) {
+        pdl_wait();   // tensor memory is asked for when no earlier launch can still hold it
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(P.tmem_cols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        __syncwarp();
+        const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(&tmem_slot);
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(P.nt >> 3) << 17) | ((uint32_t)(PG_ROWS >> 4) << 24);
+        int s = 0;
+        uint32_t phase = 0;
+        for (int kt = 0; kt < KT && ok; kt++) {
+            ok = __all_sync(0xffffffffu, mbar_wait_bounded(&full[s], phase));
+            if (!ok) break;
+            pg_fence_after();
+            if (lane == 0) {
+                const uint32_t x_addr = smem_u32(smem + (uint32_t)s * stage_bytes), w_addr = x_addr + x_bytes;
+#pragma unroll
+                for (int k = 0; k < 4; k++)
+                    ps_mma(tmem, pg_smem_desc(w_addr + (uint32_t)k * 32u), pg_smem_desc(x_addr + (uint32_t)k * 32u), idesc, (kt > 0 || k > 0) ? 1u : 0u);
+                pg_commit(&empty[s]);
+            }
+            __syncwarp();
+            if (++s == S) s = 0, phase ^= 1u;
+        }
+        if (ok && lane == 0) pg_commit(&done_bar);
+        __syncwarp();
+    } else if (lane == 0) {
+        pdl_wait();   // the tokens are the previous launch's result
+        int s = 0, issued = 0;
+        uint32_t phase = 0;
+        for (int kt = 0; kt < KT && ok; kt++) {
+            ok = mbar_wait_bounded(&empty[s], phase ^ 1u);
+            if (!ok) break;
+            mbar_arrive_expect_tx(&full[s], x_bytes);
+            pg_tma_2d(smem_u32(smem + (uint32_t)s * stage_bytes), &tmap_x, (b0 * 4 + kt) * PG_K, m0, &full[s]);
+            issued = kt + 1;
+            if (++s == S) s = 0, phase ^= 1u;
+        }
+        // after a failure the copies that were announced must land before the stages are reused
+        for (int kt = max(0, issued - S); kt < issued && !ok; kt++) mbar_wait_bounded(&full[kt % S], (uint32_t)((kt / S) & 1));
+    }
+    if (!ok) s_failed = 1;
+    __syncthreads();   // the accumulators' address; a failure of any role
+    pdl_wait();        // every thread that stores comes after the launches before this one
+    bool fin = s_failed == 0;
+    fin = __all_sync(0xffffffffu, fin && mbar_wait_bounded(&done_bar, 0u));
+    if (!fin) s_failed = 1;
+    pg_fence_after();
+    const uint32_t tmem = tmem_slot;
+    if (P.ks > 1) ps_cluster_sync();   // every CTA's MMAs have read their stages: the slots may be written
+    if (P.ks > 4) ps_finish<8>(job, P, smem, tmem, kr, n0, m0, fin);
+    else ps_finish<16>(job, P, smem, tmem, kr, n0, m0, fin);
+    pg_fence_before();
+    __syncthreads();
+    if (warp == 8) {
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(P.tmem_cols) : "memory");
+        if (lane == 0 && s_failed && err_flag) atomicExch(err_flag, DEV_ERR_GEMM_TIMEOUT);
+    }
+}
+
+}  // namespace rnb

@@ -1,0 +1,53 @@
+"""Prefill matmul of short prompts (K cut over a cluster): token counts at the edges of the tiles, ragged rows, and
+blocks of K that do not divide evenly, against the oracle's weights and the tokens, both rounded once to bf16, in f64.
+
+Bound: f32 accumulation only, a random walk of sqrt(K) * 2^-24 of the dot product's scale sqrt(sum (x w)^2) per
+partial sum (under 1e-5 at K = 14336); 1e-4 of that scale, as for the 512-token tiles."""
+import numpy as np
+import pytest
+
+import oracle as orc
+from synth import Q4_K, Q6_K, quantized, random_blocks
+from test_gpu_prefill_gemm import bf16_round, ops  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("t,rows,cols,seq", [
+    (Q4_K, 128, 256, 1), (Q4_K, 129, 768, 16), (Q6_K, 127, 512, 17), (Q4_K, 200, 1024, 255), (Q6_K, 130, 1280, 256), (Q4_K, 256, 2304, 257),
+    (Q6_K, 100, 2048, 290), (Q4_K, 260, 4096, 33), (Q6_K, 256, 8448, 48), (Q4_K, 128, 14336, 300), (Q6_K, 384, 14336, 511), (Q4_K, 64, 8192, 511),
+])
+def test_short_prompt_matmul(ops, t, rows, cols, seq):
+    rng = np.random.default_rng(rows + 7 * cols + seq)
+    w = quantized(rng, t, rows, cols)[1] if rows * cols < 1 << 20 else random_blocks(rng, t, rows, cols)
+    x = rng.standard_normal((seq, cols)).astype(np.float32)
+    wd = orc.dequantize_matrix(t, w, rows, cols).reshape(rows, cols)
+    fn = ops.q4k_bf16_gemm_batch if t == Q4_K else ops.q6k_bf16_gemm_batch
+    got = fn(w, rows, cols, x).reshape(seq, rows)
+    ref = bf16_round(x).astype(np.float64) @ bf16_round(wd).astype(np.float64).T
+    scale = np.sqrt((x.astype(np.float64) ** 2) @ (wd.astype(np.float64) ** 2).T)
+    assert np.max(np.abs(got - ref) / np.maximum(scale, 1e-30)) <= 1e-4
+    assert np.array_equal(got, fn(w, rows, cols, x).reshape(seq, rows))   # summed in rank order: the same bits each time
+
+
+@pytest.mark.parametrize("t,rows,cols,seq", [(Q4_K, 64, 1024, 16), (Q4_K, 1000, 2048, 45), (Q6_K, 65, 768, 256), (Q4_K, 4096, 1024, 255)])
+def test_short_prompt_gate_up(ops, t, rows, cols, seq):
+    """silu(gate) * up as bf16: half an ulp (2^-8 at most) of the result, plus what f32 sums in another order move g and
+    u by (1e-4 of their scale, as above), relative to the largest result."""
+    import torch
+
+    import runnburn_b200 as r
+    rng = np.random.default_rng(rows + seq)
+    ws = [quantized(rng, t, rows, cols)[1] for _ in range(2)]
+    x = rng.standard_normal((seq, cols)).astype(np.float32)
+    g, u = (bf16_round(x).astype(np.float64) @ bf16_round(orc.dequantize_matrix(t, w, rows, cols).reshape(rows, cols)).astype(np.float64).T for w in ws)
+    ref = g / (1.0 + np.exp(-g)) * u
+    wt, xt = [torch.from_numpy(np.ascontiguousarray(w)).cuda() for w in ws], torch.from_numpy(x).cuda()
+    xb = torch.empty(seq * cols, dtype=torch.int16, device="cuda")
+    act = torch.zeros(seq, rows, dtype=torch.bfloat16, device="cuda")
+    assert r.load().rnb_b200_dev_prefill_gemm_silu(t, wt[0].data_ptr(), wt[1].data_ptr(), rows, cols, xt.data_ptr(), seq, xb.data_ptr(), act.data_ptr(),
+                                                   torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    assert ops.dev_error_flag() == 0
+    got = act.float().cpu().numpy().astype(np.float64)
+    assert np.max(np.abs(got - ref) - 2.0 ** -8 * np.abs(ref)) <= 1e-4 * np.max(np.abs(ref))
