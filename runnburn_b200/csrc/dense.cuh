@@ -3,6 +3,7 @@
 //   dense_gemv_kernel       1..8 tokens, f32 activations: one warp per two rows, weights streamed by
 //                           16-byte loads (the first ones issued before the dependency wait)
 //   dense_gemm_kernel       many tokens, bf16 activations, tcgen05: 128 rows x 256 tokens per CTA
+//   dense_gemm_split_kernel the same for prompts whose tiles do not fill the chip: K cut over a cluster
 //   dense_gemm_simt_kernel  many tokens in true f32 (and bf16 activations whose rows are not
 //                           16-byte aligned, which the tiled copies cannot describe)
 //
@@ -13,6 +14,7 @@
 
 #include "common.cuh"
 #include "prefill_gemm.cuh"
+#include "prefill_gemm_split.cuh"
 
 namespace rnb {
 
@@ -340,6 +342,145 @@ dense_gemm_kernel(const __grid_constant__ DenseGemmJobs jobs, const __grid_const
     __syncthreads();
     if (warp == 1) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256) : "memory");
+        if (lane == 0 && s_failed && err_flag) atomicExch(err_flag, DEV_ERR_GEMM_TIMEOUT);
+    }
+}
+
+// ---- some tokens, tcgen05, K cut over a cluster --------------------------------------------------
+// A tile of 128 rows x nt tokens (a multiple of 16, at most 256) belongs to the ks CTAs of a cluster; each multiplies its
+// part of K and they add their accumulators over distributed shared memory in rank order (ps_reduce).  Fewer tokens leave
+// room for more stages, so that the weights stream.  The first stages' weights are asked for before the dependency wait.
+// What bounds it: the stream of the weights, and the fill and drain of a launch.  An output and down projection of 2048
+// rows gave the 256-token tiles 16 CTAs at 150 tokens; a prompt of 64 tokens through 8 Punisun layers of width 2048 takes
+// 1.46 ms (2.45 with those tiles), one of 150 through 6 Dutivik layers 1.06 ms (1.58).
+// Warp 0 issues the copies, warp 1 the MMAs, warps 2-5 reduce and store.  grid = (row tiles of all jobs x ks, token tiles).
+constexpr int DP_SUB = 16, DP_MAX_STAGES = 5;
+struct DenseSplit {
+    int nt, stages, ks;
+    uint32_t tmem_cols;
+};
+RNB_GLOBAL void __launch_bounds__(DG_THREADS)
+dense_gemm_split_kernel(const __grid_constant__ DenseGemmJobs jobs, const __grid_constant__ DenseMaps maps, const DenseSplit P, int *__restrict__ err_flag) {
+    extern __shared__ __align__(1024) uint8_t dg_smem_raw[];
+    __shared__ __align__(8) uint64_t full[DP_MAX_STAGES], empty[DP_MAX_STAGES], done_bar;
+    __shared__ uint32_t tmem_slot;
+    __shared__ int s_failed;
+    pdl_launch_dependents();
+    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(dg_smem_raw) + 1023) & ~(uintptr_t)1023);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tile = (int)blockIdx.x / P.ks, kr = (int)blockIdx.x - tile * P.ks;
+    int js = 0;
+    for (int i = 1; i < jobs.n; i++)
+        if (tile >= jobs.j[i].tile0) js = i;
+    const DenseGemmJob &job = jobs.j[js];
+    const bool pair = job.pair != 0;
+    const int rows = job.rows, S = P.stages;
+    const int n0 = (tile - job.tile0) * (pair ? DG_ROWS / 2 : DG_ROWS), m0 = blockIdx.y * P.nt, end = min(jobs.seq, m0 + P.nt);
+    const int all = (job.cols + DG_K - 1) / DG_K, k0 = all * kr / P.ks, KT = all * (kr + 1) / P.ks - k0;   // this CTA's stages of K
+    const uint32_t x_bytes = (uint32_t)P.nt * 128u, stage_bytes = x_bytes + DG_W_BYTES;
+    if (tid == 0) {
+        for (int s = 0; s < S; s++) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
+        }
+        mbar_init(&done_bar, 1);
+        mbar_fence_init();
+        s_failed = 0;
+    }
+    __syncthreads();
+    bool ok = true;
+    if (warp == 0) {
+        if (lane == 0) {
+            auto weights = [&](int kt) {
+                const uint32_t dst = smem_u32(smem + (uint32_t)(kt % S) * stage_bytes) + x_bytes;
+                uint64_t *bar = &full[kt % S];
+                mbar_arrive_expect_tx(bar, stage_bytes);
+                pg_tma_2d(dst, &maps.w[js], (k0 + kt) * DG_K, n0, bar);
+                pg_tma_2d(dst + DG_W_BYTES / 2, pair ? &maps.w2[js] : &maps.w[js], (k0 + kt) * DG_K, pair ? n0 : n0 + DG_ROWS / 2, bar);
+            };
+            const int head = min(S, KT);
+            for (int kt = 0; kt < head; kt++) weights(kt);
+            pdl_wait();   // the tokens are the previous launch's result
+            int issued = 0;
+            for (int kt = 0; kt < KT && ok; kt++) {
+                const int s = kt % S;
+                if (kt >= S) {
+                    ok = mbar_wait_bounded(&empty[s], (uint32_t)(((kt / S) & 1) ^ 1));
+                    if (!ok) break;
+                    weights(kt);
+                }
+                pg_tma_2d(smem_u32(smem + (uint32_t)s * stage_bytes), &maps.x[js], (k0 + kt) * DG_K, m0, &full[s]);
+                issued = kt + 1;
+            }
+            // after a failure the copies that were announced must land before the stages are reused
+            for (int kt = max(0, issued - S); kt < issued && !ok; kt++) mbar_wait_bounded(&full[kt % S], (uint32_t)((kt / S) & 1));
+        }
+    } else if (warp == 1) {
+        pdl_wait();   // tensor memory is asked for when no earlier launch can still hold it
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(P.tmem_cols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        __syncwarp();
+        const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(&tmem_slot);
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(P.nt >> 3) << 17) | ((uint32_t)(DG_ROWS >> 4) << 24);
+        if (lane == 0) {
+            for (int kt = 0; kt < KT && ok; kt++) {
+                const int s = kt % S;
+                ok = mbar_wait_bounded(&full[s], (uint32_t)((kt / S) & 1));
+                if (!ok) break;
+                pg_fence_after();
+                const uint32_t x_addr = smem_u32(smem + (uint32_t)s * stage_bytes), w_addr = x_addr + x_bytes;
+#pragma unroll
+                for (int k = 0; k < 4; k++)
+                    ps_mma(tmem, pg_smem_desc(w_addr + (uint32_t)k * 32u), pg_smem_desc(x_addr + (uint32_t)k * 32u), idesc, (kt > 0 || k > 0) ? 1u : 0u);
+                pg_commit(&empty[s]);
+            }
+            if (ok) pg_commit(&done_bar);
+        }
+        __syncwarp();
+    }
+    if (!ok) s_failed = 1;
+    __syncthreads();   // the accumulators' address; a failure of any role
+    pdl_wait();        // every thread that stores comes after the launches before this one
+    const bool fin = __all_sync(0xffffffffu, s_failed == 0 && mbar_wait_bounded(&done_bar, 0u));
+    if (!fin) s_failed = 1;
+    pg_fence_after();
+    const uint32_t tmem = tmem_slot;
+    if (P.ks > 1) ps_cluster_sync();   // every CTA's MMAs have read their stages: the slots may be written
+    const int q = warp & 3;
+    float *ex = reinterpret_cast<float *>(smem + PS_SLOT_BYTES);   // gate / up exchange, two buffers in turn
+    ps_reduce<DP_SUB, 1>(P.ks, kr, (end - m0 + DP_SUB - 1) / DP_SUB, smem, tmem, warp >= 2, q, 0, fin, [&](int cc, int j, const float (&v)[DP_SUB]) {
+        const int tok0 = m0 + cc * DP_SUB;
+        auto put = [&](int t, int row, float a) {
+            if (tok0 + t >= end) return;
+            if (job.out_bf16) dg_store<bf16>(job.y, (size_t)(tok0 + t) * job.ld + row, a);
+            else dg_store<float>(job.y, (size_t)(tok0 + t) * job.ld + row, a);
+        };
+        if (pair) {
+            // gate rows on lane quarters 0 and 1, the same rows of up on 2 and 3: each warp finishes half of the tokens
+            float *buf = ex + (size_t)(j & 1) * (DP_SUB * DG_ROWS);
+#pragma unroll
+            for (int t = 0; t < DP_SUB; t++) buf[t * DG_ROWS + q * 32 + lane] = v[t];
+            asm volatile("bar.sync 1, 128;" ::: "memory");
+            const int row = n0 + (q & 1) * 32 + lane, t_lo = (q >> 1) * (DP_SUB / 2);
+            if (fin && row < rows) {
+#pragma unroll
+                for (int t = t_lo; t < t_lo + DP_SUB / 2; t++) {
+                    const float z = buf[t * DG_ROWS + (q & 1) * 32 + lane], u = buf[t * DG_ROWS + 64 + (q & 1) * 32 + lane];
+                    put(t, row, (job.out_bf16 ? gate_act_fast(job.act, z) : gate_act(job.act, z)) * u);
+                }
+            }
+        } else if (fin && n0 + q * 32 + lane < rows) {
+            const int row = n0 + q * 32 + lane;
+            const float b = job.decay_bias ? job.decay_bias[row] : 0.f;
+#pragma unroll
+            for (int t = 0; t < DP_SUB; t++)
+                put(t, row, !job.decay_bias ? v[t] : job.decay_kind == DECAY_SIGMOID_ROOT ? sigmoid_root_fast(v[t] + b, job.inv_tau) : expf(-expf(v[t] + b)));
+        }
+    });
+    pg_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(P.tmem_cols) : "memory");
         if (lane == 0 && s_failed && err_flag) atomicExch(err_flag, DEV_ERR_GEMM_TIMEOUT);
     }
 }

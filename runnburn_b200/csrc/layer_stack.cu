@@ -653,7 +653,7 @@ int LayerStack::ready(cudaStream_t s) {
         return RNB_B200_OK;
     };
     const void *fns[] = {(const void *)residual_norm_kernel<float, 4>, (const void *)residual_norm_kernel<float, 1>, (const void *)residual_norm_kernel<bf16, 4>,
-                         (const void *)residual_norm_kernel<bf16, 1>, (const void *)dense_gemm_kernel, (const void *)decay_rows_kernel,
+                         (const void *)residual_norm_kernel<bf16, 1>, (const void *)dense_gemm_kernel, (const void *)dense_gemm_split_kernel, (const void *)decay_rows_kernel,
                          (const void *)linear_state_step_kernel<4>, (const void *)linear_state_step_kernel<8>, (const void *)linear_state_step_kernel<16>,
                          (const void *)linear_state_step_kernel<32>, (const void *)linear_state_step_kernel<64>, (const void *)causal_attention_kernel<4>,
                          (const void *)causal_attention_kernel<8>, (const void *)causal_attention_kernel<16>, (const void *)causal_attention_kernel<32>,
@@ -782,7 +782,26 @@ int LayerStack::matmul(cudaStream_t s, int n, const Mm *jobs, int n_jobs, int *e
         memset(&M, 0, sizeof(M));
         J.n = n_jobs;
         J.seq = n;
-        int tiles = 0;
+        int tiles = 0, depth = 1 << 30;
+        for (int i = 0; i < n_jobs; i++) {
+            const int per = jobs[i].w2 ? DG_ROWS / 2 : DG_ROWS;
+            tiles += (jobs[i].w->rows + per - 1) / per;
+            depth = std::min(depth, (jobs[i].w->cols + DG_K - 1) / DG_K);
+        }
+        // K is cut where the tiles leave SMs idle: up to two CTAs per SM, at least two stages of K each.  Prompts in ms, 256-token
+        // tiles / this rule: 8 Punisun layers of width 2048 at 64, 333, 1000 tokens 2.45 / 1.46, 3.28 / 2.69, 4.23 / 3.95;
+        // 6 Dutivik layers 1.41 / 0.77, 1.94 / 1.37, 2.80 / 2.41; of width 4096 at 64 tokens 1.66 / 0.95 and 1.30 / 0.69.
+        // A cut in two pays only where K is long (2048 tokens: Dutivik's 12288 columns 4.40 / 4.31, Punisun's 2048 6.34 / 6.64).
+        // Uncut tiles of up to 128 tokens also go there, for the deeper ring; at 256 tokens the other kernel's order of the
+        // grid is better (2048 tokens: 6.4 against 5.2 ms at width 4096).
+        DenseSplit P;
+        const int token_tiles = (n + DG_TOK - 1) / DG_TOK;
+        P.ks = 1;
+        while (P.ks * 2 <= PS_MAX_KS && tiles * token_tiles * P.ks * 2 <= 296 && P.ks * 4 <= depth) P.ks *= 2;
+        if (P.ks == 2 && depth < 64) P.ks = 1;
+        P.nt = ((n + token_tiles - 1) / token_tiles + 15) & ~15;
+        const bool split = P.ks > 1 || P.nt <= 128;
+        tiles = 0;
         for (int i = 0; i < n_jobs; i++) {
             DenseGemmJob &j = J.j[i];
             j.y = jobs[i].y;
@@ -797,11 +816,19 @@ int LayerStack::matmul(cudaStream_t s, int n, const Mm *jobs, int n_jobs, int *e
             j.pair = jobs[i].w2 != nullptr;
             const int per = j.pair ? DG_ROWS / 2 : DG_ROWS;
             tiles += (j.rows + per - 1) / per;
-            RNB_TRY(encode_token_map(&M.x[i], reinterpret_cast<const uint16_t *>(jobs[i].x), (size_t)n, (size_t)j.cols, jobs[i].ldx, DG_TOK));
+            RNB_TRY(encode_token_map(&M.x[i], reinterpret_cast<const uint16_t *>(jobs[i].x), (size_t)n, (size_t)j.cols, jobs[i].ldx, split ? P.nt : DG_TOK));
             memcpy(&M.w[i], jobs[i].w->map, sizeof(PgTensorMap));
             if (j.pair) memcpy(&M.w2[i], jobs[i].w2->map, sizeof(PgTensorMap));
         }
-        RNB_CU(launch_k(dense_gemm_kernel, dim3((unsigned)((n + DG_TOK - 1) / DG_TOK), (unsigned)tiles), dim3(DG_THREADS), DG_SMEM, s, J, M, err));
+        if (split) {
+            P.stages = std::min<int>(DP_MAX_STAGES, (int)((DG_SMEM - 1024) / ((uint32_t)P.nt * 128u + DG_W_BYTES)));
+            P.tmem_cols = 32;
+            while ((int)P.tmem_cols < P.nt) P.tmem_cols *= 2;
+            RNB_CU(launch_k_cluster(dense_gemm_split_kernel, dim3((unsigned)(tiles * P.ks), (unsigned)token_tiles), dim3(DG_THREADS), DG_SMEM, s, dim3((unsigned)P.ks), J, M, P,
+                                    err));
+            return RNB_B200_OK;
+        }
+        RNB_CU(launch_k(dense_gemm_kernel, dim3((unsigned)token_tiles, (unsigned)tiles), dim3(DG_THREADS), DG_SMEM, s, J, M, err));
         return RNB_B200_OK;
     }
     DenseSimtJobs J;

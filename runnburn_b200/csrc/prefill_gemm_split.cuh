@@ -24,7 +24,7 @@ namespace rnb {
 constexpr int PS_TOK = 256;        // most tokens per CTA
 constexpr int PS_THREADS = 320;
 constexpr int PS_MAX_STAGES = 5;
-constexpr uint32_t PS_SMEM_STAGES = 96 * 1024;   // operand stages; the reduction reuses them
+constexpr uint32_t PS_SMEM_STAGES = 96 * 1024;   // operand stages; the reduction reuses them: 64 KB of slots, 32 KB of exchange
 constexpr size_t PS_SMEM = PS_SMEM_STAGES + 1024;
 constexpr int PS_MAX_KS = 8;
 
@@ -64,72 +64,90 @@ __device__ __forceinline__ uint32_t ps_map(uint32_t addr, int rank) {
 }
 __device__ __forceinline__ void ps_st_remote(uint32_t addr, uint32_t v) { asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
 
-// Sums and stores the tile.  A round gives every CTA of the cluster one chunk of 2 * SUB tokens: the others send it
-// their accumulators of that chunk, it adds them in rank order with its own.  Warp w holds the rows of lane quarter
-// w & 3 and the chunk's tokens (w >> 2) * SUB ..; all threads of the CTA come through here (cluster barriers).
-template <int SUB>
-__device__ __forceinline__ void ps_finish(const PgJob &job, const PsParams &P, uint8_t *smem, uint32_t tmem, int kr, int n0, int m0, bool fin) {
-    constexpr int CT = 2 * SUB;                       // tokens per chunk
+// Adds the accumulators of a cluster's ks CTAs (one: its own).  A round gives every CTA up to ps_per_round chunks of
+// SUB * GROUPS tokens: the others send it theirs of those chunks, it adds them in rank order with its own and calls
+// f(chunk, count, sums).  Two cluster barriers a round, so few rounds: one or two at 256 tokens.  A worker warp holds the rows of lane quarter q and a chunk's tokens group * SUB ..; all
+// threads of the CTA come through here.  `smem` takes PS_SLOT_BYTES for the accumulators that arrive.
+constexpr uint32_t PS_SLOT_BYTES = 64 * 1024;
+__host__ __device__ inline int ps_per_round(int ks, uint32_t slot) { return ks > 1 ? (int)(PS_SLOT_BYTES / slot) / (ks - 1) : 1; }
+template <int SUB, int GROUPS, class F>
+__device__ __forceinline__ void ps_reduce(int ks, int kr, int n_chunks, uint8_t *smem, uint32_t tmem, bool worker, int q, int group, bool fin, F &&f) {
+    constexpr int CT = SUB * GROUPS;                  // tokens per chunk
     constexpr uint32_t SLOT = CT * PG_ROWS * 4;       // one CTA's accumulators of a chunk: [token][row]
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, ks = P.ks;
-    const bool worker = warp < 8, pair = job.w2 != nullptr;
-    const int q = warp & 3, sub = (warp >> 2) & 1, rows = job.rows;
-    const int end = min(P.seq, m0 + P.nt), n_chunks = (end - m0 + CT - 1) / CT;
-    const uint32_t base = smem_u32(smem), mine = (uint32_t)(sub * SUB * PG_ROWS + q * 32 + lane) * 4u;
-    const uint32_t lanes = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(sub * SUB);
-    float *ex = reinterpret_cast<float *>(smem + (size_t)(ks - 1) * SLOT);   // gate / up exchange, two buffers in turn
-    for (int j = 0; j * ks < n_chunks; j++) {
+    static_assert((PS_MAX_KS / 2 - 1) * SLOT <= PS_SLOT_BYTES, "a slot per sender");
+    const int lane = threadIdx.x & 31, M = ps_per_round(ks, SLOT);
+    const uint32_t base = smem_u32(smem), mine = (uint32_t)(group * SUB * PG_ROWS + q * 32 + lane) * 4u;
+    const uint32_t lanes = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(group * SUB);
+    int count = 0;
+    for (int c0 = 0; c0 < n_chunks; c0 += M * ks) {
         if (ks > 1) {
+            if (c0 > 0) ps_cluster_sync();   // the slots are free again
             if (worker)
                 for (int i = 1; i < ks; i++) {
-                    const int to = (kr + i) % ks, cc = j * ks + to;
-                    if (cc >= n_chunks) continue;
-                    uint32_t v[SUB];
-                    if (fin) ps_tmem_ld<SUB>(lanes + (uint32_t)(cc * CT), v);
-                    const uint32_t dst = ps_map(base + (uint32_t)(kr < to ? kr : kr - 1) * SLOT + mine, to);
+                    const int to = (kr + i) % ks;
+                    for (int m = 0; m < M; m++) {
+                        const int cc = c0 + m * ks + to;
+                        if (cc >= n_chunks) break;
+                        uint32_t v[SUB];
+                        if (fin) ps_tmem_ld<SUB>(lanes + (uint32_t)(cc * CT), v);
+                        const uint32_t dst = ps_map(base + (uint32_t)((kr < to ? kr : kr - 1) * M + m) * SLOT + mine, to);
 #pragma unroll
-                    for (int t = 0; t < SUB; t++) ps_st_remote(dst + (uint32_t)(t * PG_ROWS * 4), fin ? v[t] : 0u);
+                        for (int t = 0; t < SUB; t++) ps_st_remote(dst + (uint32_t)(t * PG_ROWS * 4), fin ? v[t] : 0u);
+                    }
                 }
             ps_cluster_sync();
         }
-        const int cc = j * ks + kr;
-        if (worker && cc < n_chunks) {
+        for (int m = 0; m < M; m++) {
+            const int cc = c0 + m * ks + kr;
+            if (!worker || cc >= n_chunks) break;
             uint32_t v[SUB];
             if (fin) ps_tmem_ld<SUB>(lanes + (uint32_t)(cc * CT), v);
             float s[SUB];
 #pragma unroll
             for (int t = 0; t < SUB; t++) {
                 const float own = fin ? __uint_as_float(v[t]) : 0.f;
-                const float *part = reinterpret_cast<const float *>(smem + mine) + t * PG_ROWS;
+                const float *part = reinterpret_cast<const float *>(smem + (size_t)m * SLOT + mine) + t * PG_ROWS;
                 s[t] = kr == 0 ? own : part[0];
-                for (int r = 1; r < ks; r++) s[t] += r == kr ? own : part[(size_t)(r < kr ? r : r - 1) * (SLOT / 4)];
+                for (int r = 1; r < ks; r++) s[t] += r == kr ? own : part[(size_t)(r < kr ? r : r - 1) * M * (SLOT / 4)];
             }
-            const int tok0 = m0 + cc * CT;
-            if (pair) {
-                // gate rows on lane quarters 0 and 1, the same rows of up on 2 and 3: each warp finishes half of its tokens
-                float *buf = ex + (size_t)(j & 1) * (SLOT / 4);
-#pragma unroll
-                for (int t = 0; t < SUB; t++) buf[(sub * SUB + t) * PG_ROWS + q * 32 + lane] = s[t];
-                asm volatile("bar.sync 1, 256;" ::: "memory");
-                const int row = n0 + (q & 1) * 32 + lane, t_lo = sub * SUB + (q >> 1) * (SUB / 2);
-                if (fin && row < rows) {
-#pragma unroll
-                    for (int t = t_lo; t < t_lo + SUB / 2; t++) {
-                        const float g = buf[t * PG_ROWS + (q & 1) * 32 + lane], u = buf[t * PG_ROWS + 64 + (q & 1) * 32 + lane];
-                        // fast exponential and division: their 2^-21 relative error disappears in the bf16 rounding below
-                        const float a = __fdividef(g, 1.0f + __expf(-g)) * u;
-                        if (tok0 + t < end) job.yb[(size_t)(tok0 + t) * rows + row] = (uint16_t)(pg_pack_bf16(a, 0.f) & 0xffffu);
-                    }
-                }
-            } else if (fin && n0 + q * 32 + lane < rows) {
-                float *dst = job.y + (size_t)(tok0 + sub * SUB) * rows + n0 + q * 32 + lane;
-#pragma unroll
-                for (int t = 0; t < SUB; t++)
-                    if (tok0 + sub * SUB + t < end) dst[(size_t)t * rows] = s[t];
-            }
+            f(cc, count++, s);
         }
-        if (ks > 1 && (j + 1) * ks < n_chunks) ps_cluster_sync();   // the slots are free for the next round
     }
+}
+
+// Sums and stores a tile with eight worker warps: warp w holds tokens (w >> 2) * SUB .. of a chunk.
+template <int SUB>
+__device__ __forceinline__ void ps_finish(const PgJob &job, const PsParams &P, uint8_t *smem, uint32_t tmem, int kr, int n0, int m0, bool fin) {
+    constexpr int CT = 2 * SUB;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, q = warp & 3, sub = (warp >> 2) & 1, rows = job.rows;
+    const int end = min(P.seq, m0 + P.nt), n_chunks = (end - m0 + CT - 1) / CT;
+    float *ex = reinterpret_cast<float *>(smem + PS_SLOT_BYTES);   // gate / up exchange, two buffers in turn
+    const bool pair = job.w2 != nullptr;
+    ps_reduce<SUB, 2>(P.ks, kr, n_chunks, smem, tmem, warp < 8, q, sub, fin, [&](int cc, int j, const float (&s)[SUB]) {
+        const int tok0 = m0 + cc * CT;
+        if (pair) {
+            // gate rows on lane quarters 0 and 1, the same rows of up on 2 and 3: each warp finishes half of its tokens
+            float *buf = ex + (size_t)(j & 1) * (CT * PG_ROWS);
+#pragma unroll
+            for (int t = 0; t < SUB; t++) buf[(sub * SUB + t) * PG_ROWS + q * 32 + lane] = s[t];
+            asm volatile("bar.sync 1, 256;" ::: "memory");
+            const int row = n0 + (q & 1) * 32 + lane, t_lo = sub * SUB + (q >> 1) * (SUB / 2);
+            if (fin && row < rows) {
+#pragma unroll
+                for (int t = t_lo; t < t_lo + SUB / 2; t++) {
+                    const float g = buf[t * PG_ROWS + (q & 1) * 32 + lane], u = buf[t * PG_ROWS + 64 + (q & 1) * 32 + lane];
+                    // fast exponential and division: their 2^-21 relative error disappears in the bf16 rounding below
+                    const float a = __fdividef(g, 1.0f + __expf(-g)) * u;
+                    if (tok0 + t < end) job.yb[(size_t)(tok0 + t) * rows + row] = (uint16_t)(pg_pack_bf16(a, 0.f) & 0xffffu);
+                }
+            }
+        } else if (fin && n0 + q * 32 + lane < rows) {
+            float *dst = job.y + (size_t)(tok0 + sub * SUB) * rows + n0 + q * 32 + lane;
+#pragma unroll
+            for (int t = 0; t < SUB; t++)
+                if (tok0 + sub * SUB + t < end) dst[(size_t)t * rows] = s[t];
+        }
+    });
 }
 
 // grid = (row tiles of all jobs x ks, token tiles), cluster (ks, 1, 1); 320 threads; dynamic shared memory PS_SMEM.

@@ -51,3 +51,24 @@ def test_short_prompt_gate_up(ops, t, rows, cols, seq):
     assert ops.dev_error_flag() == 0
     got = act.float().cpu().numpy().astype(np.float64)
     assert np.max(np.abs(got - ref) - 2.0 ** -8 * np.abs(ref)) <= 1e-4 * np.max(np.abs(ref))
+
+
+@pytest.mark.parametrize("n", [9, 16, 17, 128, 129, 256, 257, 300])
+@pytest.mark.parametrize("design", ["dutivik", "punisun"])
+def test_prompt_products_cut_along_k(design, n):
+    """bf16 stacks whose products have 16 to 48 stages of K and few tiles (4 or 8 CTAs along K; the gate and up pair too),
+    at the edges of the token tiles, against the plain reference: every projection rounds its input to bf16, the bound
+    of the stack tests (3e-2 of the rows' scale)."""
+    import stack_util as su
+    from hybrid_ref import Model
+    if design == "dutivik":
+        cfg = su.dutivik([su.gla(heads=4, dim=64, vdim=64, ff=2816)], width=1024)
+    else:
+        cfg = su.config([su.retention(heads=4, dim=64, vdim=64, ff=1920)], width=1024)
+    w = su.weights(cfg, seed=n, rank=16)
+    toks = su.tokens(cfg, n, seed=1)
+    dec = su.decoder(cfg, w, "bfloat16", max_ctx=512)
+    want = Model(cfg, w).forward(toks)
+    got = dec.prefill_logits(toks, 0, list(range(n)))[0]
+    dec.close()
+    assert not (why := su.bad(got, want, "bfloat16")), why
