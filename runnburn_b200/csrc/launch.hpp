@@ -11,6 +11,7 @@
 #include "gemv_q5k.cuh"
 #include "moe.cuh"
 #include "prefill_gemm.cuh"
+#include "prefill_gemm_pair.cuh"
 #include "prefill_gemm_split.cuh"
 #include "q8k.cuh"
 #include "state.hpp"
@@ -202,8 +203,8 @@ inline const KsplitTuning &ksplit_tuning() {
 // on a 16-byte boundary).  RNB_B200_MMA=0 turns it off, _MMA_STAGES / _MMA_CTAS set the ring depth
 // and the resident CTAs per SM the persistent grid is sized for.
 // Descriptor of a weight matrix for the integer-MMA matvec's tiled copies: [rows][row_bytes / 8] 8-byte
-// words, boxes of 16 rows x box_bytes / 8 words, no swizzle, zeros outside the matrix.
-int encode_weight_map(GmTensorMap *out, const uint8_t *w, size_t rows, size_t row_bytes, uint32_t box_bytes);
+// words, boxes of box_rows rows x box_bytes / 8 words, no swizzle, zeros outside the matrix.
+int encode_weight_map(GmTensorMap *out, const uint8_t *w, size_t rows, size_t row_bytes, uint32_t box_bytes, int box_rows = GM_ROWS);
 struct MmaTuning {
     int enabled, stages, ctas_per_sm, chunk16, tmap;
 };
@@ -712,9 +713,9 @@ inline int launch_attention_decode(cudaStream_t s, const float *q, const uint16_
 // elements) and runs the tcgen05 kernel.  y is [seq][rows] f32.
 int prefill_gemm_setup();   // raises the kernels' dynamic shared-memory limit once
 // Descriptor of a bf16 matrix [seq][cols] (row pitch ld elements, 0: cols) for the kernels' tiled copies:
-// boxes of 64 columns x box_rows rows (256 tokens), 128-byte swizzle, zeros past either end.  The encoder is a driver
+// boxes of 64 columns x box_rows rows, 128-byte swizzle, zeros past either end.  The encoder is a driver
 // entry point, looked up once through the runtime.
-inline int encode_token_map(PgTensorMap *out, const uint16_t *xb, size_t seq, size_t cols, size_t ld = 0, int box_rows = PG_BOX_ROWS) {
+inline int encode_token_map(PgTensorMap *out, const uint16_t *xb, size_t seq, size_t cols, size_t ld, int box_rows) {
     static_assert(sizeof(PgTensorMap) == sizeof(CUtensorMap) && alignof(PgTensorMap) >= alignof(CUtensorMap), "descriptor size");
     typedef CUresult (*EncodeTiled)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
                                     const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -735,7 +736,8 @@ inline int encode_token_map(PgTensorMap *out, const uint16_t *xb, size_t seq, si
     if (r != CUDA_SUCCESS) return fail(RNB_B200_CUDA_ERROR, "cuTensorMapEncodeTiled failed with driver code %d", (int)r);
     return RNB_B200_OK;
 }
-// CTAs along K for a short prompt, 0: the 512-token tiles.  Measured on the matrices of the 8B and 1B shapes, 16 to 512
+// CTAs along K for a short prompt, 0: pairs of SMs (prefill_gemm_pair.cuh).  Measured against the kernel of 512-token tiles
+// that the pairs replaced, on the matrices of the 8B and 1B shapes, 16 to 512
 // tokens (us, 512-token tiles / this rule):
 //   matrices of their own: 203 tokens 4096 x 4096 55 / 29, 4096 x 14336 251 / 61, q + k + v 77 / 43, 2048 x 8192 147 / 38;
 //     400 tokens 55 / 37, 255 / 112, 77 / 71, 148 / 41.  With 4 to 7, 8 to 31 and more blocks of 256 columns 2, 4 and 8
@@ -752,19 +754,56 @@ inline int prefill_split_ks(bool pair, int tiles, size_t seq, size_t cols) {
         while (ks * 2 * tiles <= 148 && ks * 2 <= std::min(nb / 2, PS_MAX_KS)) ks *= 2;
         return ks;
     }
-    if (seq >= (size_t)PG_TOK) return 0;
+    if (seq >= (size_t)PT_MAX_TOK) return 0;
     return nb < 4 ? 1 : nb < 8 ? 2 : nb < 32 ? 4 : PS_MAX_KS;
+}
+inline int pg_pairs() { return std::max(1, (state().sm_count > 0 ? state().sm_count : 148) / 2); }
+// Tokens per tile of the paired kernels (two parts, multiples of 32): the width that gives the least rounds x cost(width).
+template <class P, class F>
+inline void pg_pair_tiles(P &p, int row_pairs, int seq, F &&cost) {
+    const int first = (seq + PT_MAX_TOK - 1) / PT_MAX_TOK;
+    long best = -1;
+    int nt = PT_MAX_TOK;
+    for (int n = first; n <= 2 * first; n++) {
+        const int w = std::max(((seq + n - 1) / n + 31) & ~31, 64);
+        const long c = (long)((row_pairs * ((seq + w - 1) / w) + pg_pairs() - 1) / pg_pairs()) * cost(w);
+        if (best < 0 || c < best) best = c, nt = w;
+    }
+    p.n1 = (nt / 2 + 31) & ~31;
+    p.n2 = nt - p.n1;
+    p.token_tiles = (seq + nt - 1) / nt;
+    p.tiles = row_pairs * p.token_tiles;
 }
 // `tiles`: row tiles of all jobs
 inline int launch_prefill_gemm_tiles(cudaStream_t s, const PgJobs &jobs, int tiles, size_t seq, size_t cols, const uint16_t *xb, int *dev_error) {
-    PgTensorMap tmap;
     const int ks = prefill_split_ks(jobs.j[0].w2 != nullptr, tiles, seq, cols);
     if (ks == 0) {
-        RNB_TRY(encode_token_map(&tmap, xb, seq, cols));
-        const dim3 grid((unsigned)tiles, (unsigned)((seq + PG_TOK - 1) / PG_TOK));
-        RNB_CU(launch_k(prefill_gemm_kernel, grid, dim3(PG_THREADS), PG_SMEM, s, jobs, tmap, (int)seq, (int)cols, dev_error));
+        PtParams P;
+        PtMaps maps;
+        memset(&maps, 0, sizeof(maps));
+        P.seq = (int)seq;
+        P.cols = (int)cols;
+        P.row_tiles = tiles;
+        P.direct = 0;
+        // a narrower tile than 450 tokens is no faster: its stages take as long as dequantising them does
+        pg_pair_tiles(P, (tiles + 1) / 2, P.seq, [](int w) { return std::max(w, 450) + 24; });
+        RNB_TRY(encode_token_map(&maps.xa, xb, seq, cols, 0, P.n1 / 2));
+        RNB_TRY(encode_token_map(&maps.xb, xb, seq, cols, 0, P.n2 / 2));
+        for (int i = 0; i < jobs.n; i++) {
+            const PgJob &j = jobs.j[i];
+            const size_t rb = row_bytes_of(j.type, cols);
+            if ((((uintptr_t)j.w | (uintptr_t)j.w2 | rb) & 15u) != 0) {
+                P.direct |= 1 << i;
+                continue;
+            }
+            const uint32_t box = j.type == TYPE_Q4_K ? PT_Q4_PITCH : PT_Q6_PITCH;
+            RNB_TRY(encode_weight_map(reinterpret_cast<GmTensorMap *>(&maps.w[i]), j.w, (size_t)j.rows, rb, box, PG_ROWS / 2));
+            if (j.w2) RNB_TRY(encode_weight_map(reinterpret_cast<GmTensorMap *>(&maps.w2), j.w2, (size_t)j.rows, rb, box, PG_ROWS / 2));
+        }
+        RNB_CU(launch_k_cluster(prefill_gemm_pair_kernel, dim3((unsigned)(2 * std::min(P.tiles, pg_pairs()))), dim3(PT_THREADS), PT_SMEM, s, dim3(2), jobs, maps, P, dev_error));
         return RNB_B200_OK;
     }
+    PgTensorMap tmap;
     PsParams P;
     const int token_tiles = (int)((seq + PS_TOK - 1) / PS_TOK);
     P.seq = (int)seq;

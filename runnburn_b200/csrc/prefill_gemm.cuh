@@ -6,21 +6,14 @@
 // crates/rnb-cpu/src/quantize/dequant.rs:353-381 (Q4_K) and :780-807 (Q6_K) in f32 and rounds
 // once to bf16.
 //
-// One CTA owns a 512-token x 128-row output tile: two fp32 accumulators of 128 rows x 256 tokens =
-// all 512 columns of the SM's tensor memory; the weight tile is the M operand (TMEM lane = weight
-// row), a token half the N operand.  A dequantised weight tile serves 512 tokens - the dequantising
-// warps, not the tensor pipe, bounded a 256 x 256 tile.  K advances 64 elements (one Q4_K group, a
-// quarter of a super-block) per pipeline stage; a stage holds the token tile (512 x 64 bf16 = 64 KB,
-// brought in by two tiled TMA copies; rows past the end of the batch read as zeros) and the weight
-// tile (128 x 64 bf16), both K-major in the 128-byte swizzle the MMA descriptors expect:
+// What the two kernels share (prefill_gemm_pair.cuh: long prompts on pairs of SMs; prefill_gemm_split.cuh: short ones with K
+// cut over a cluster): the weight tile is the M operand (tensor-memory lane = weight row), the tokens the N operand.  K
+// advances 64 elements per stage (one Q4_K group, a quarter of a super-block); the operand tiles are K-major in the 128-byte
+// swizzle the MMA descriptors expect:
 //   byte offset of (row r, 16-byte chunk c) = (r / 8) * 1024 + (r % 8) * 128 + ((c ^ (r % 8)) * 16).
-// Two stages of 80 KB; a stage is refilled as soon as the MMAs that read it have been committed.
-// Warp roles: 0-7 dequantise (thread t owns weight row t / 2 and half t % 2 of the 64-element group:
-// Q4_K low or high nibbles, Q6_K the first or second 32 elements), thread 0 also issues the token
-// copies; warp 8 allocates tensor memory and issues the MMAs (eight per stage: 2 token halves x 4
-// K-steps of 16); afterwards warps 0-7 read the accumulators back (tcgen05.ld, one TMEM lane quarter
-// per warp) and store f32 rows.  Every wait is bounded; a timeout sets the error flag and all roles
-// still meet at the final barrier, where the tensor memory is freed.
+// Tokens come in by tiled TMA copies (rows past the end of the batch read as zeros); a weight row's stage is dequantised by two
+// threads, each half of the 64 elements: Q4_K low or high nibbles, Q6_K the first or second 32.  Every wait is bounded; a
+// timeout sets the error flag and all roles still meet at the final barrier, where the tensor memory is freed.
 #pragma once
 #include <cuda_bf16.h>
 
@@ -30,16 +23,9 @@
 
 namespace rnb {
 
-constexpr int PG_TOK = 512;      // tokens per CTA
 constexpr int PG_ROWS = 128;     // weight rows per CTA
 constexpr int PG_K = 64;         // elements per stage
-constexpr int PG_STAGES = 2;
-constexpr int PG_THREADS = 288;
-constexpr uint32_t PG_A_BYTES = PG_TOK * 128;    // token tile of a stage
 constexpr uint32_t PG_B_BYTES = PG_ROWS * 128;   // weight tile of a stage
-constexpr uint32_t PG_STAGE_BYTES = PG_A_BYTES + PG_B_BYTES;
-constexpr size_t PG_SMEM = (size_t)PG_STAGES * PG_STAGE_BYTES + 1024;   // + slack to align to 1024
-constexpr int PG_BOX_ROWS = 256;                 // tokens per TMA copy
 
 // K-major, 128-byte swizzle, 8-row groups 1024 bytes apart; descriptor version 1 (sm_100)
 __device__ __forceinline__ uint64_t pg_smem_desc(uint32_t saddr) {
@@ -54,6 +40,14 @@ __device__ __forceinline__ void pg_mma(uint32_t tmem_d, uint64_t da, uint64_t db
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(tmem_d), "l"(da), "l"(db), "r"(PG_IDESC), "r"(accumulate)
         : "memory");
+}
+// One lane of a converged warp.  The MMAs are issued behind this and not behind `lane == 0`: their operands live in uniform
+// registers, and where the compiler cannot see that a single thread gets there it moves them there once per lane (a stage of
+// eight MMAs took 1000 cycles to issue).
+__device__ __forceinline__ bool pg_elect() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
 }
 __device__ __forceinline__ void pg_commit(uint64_t *bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -75,13 +69,25 @@ __device__ __forceinline__ void pg_tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) 
         : "r"(taddr));
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
-// q in 0..255 -> exact f32 without an int-to-float conversion: 2^23 + q, minus 2^23
-__device__ __forceinline__ float pg_byte_to_f32(uint32_t word, int byte) {
-    return __uint_as_float(__byte_perm(word, 0x4b000000u, 0x7650 + byte) ) - 8388608.0f;
+// q in 0..255 -> exact f32 without an int-to-float conversion: the bits of 2^23 + q, minus 2^23 (Q6_K: minus 2^23 + 32);
+// two of them at a time as packed f32: ((2^23 + q) - 2^23) * s + m of bytes b and b + 1 of `word`, rounded to a bf16 pair.  The
+// same roundings as one by one, five instructions for two elements instead of seven.
+__device__ __forceinline__ uint64_t pg_pair_f32(float a, float b) { return (uint64_t)__float_as_uint(a) | (uint64_t)__float_as_uint(b) << 32; }
+__device__ __forceinline__ uint32_t pg_dequant_pair_fma(uint32_t word, int b, uint64_t s, uint64_t m) {
+    uint32_t r;
+    asm("{\n\t.reg .b64 t;\n\t.reg .b32 x, y;\n\tmov.b64 t, {%1, %2};\n\tadd.rn.f32x2 t, t, %3;\n\tfma.rn.f32x2 t, t, %4, %5;\n\tmov.b64 {x, y}, t;\n\t"
+        "cvt.rn.bf16x2.f32 %0, y, x;\n\t}"
+        : "=r"(r)
+        : "r"(__byte_perm(word, 0x4b000000u, 0x7650 + b)), "r"(__byte_perm(word, 0x4b000000u, 0x7651 + b)), "l"(0xcb000000cb000000ull), "l"(s), "l"(m));
+    return r;
 }
-// same, minus 32 (Q6_K's offset): 2^23 + q - (2^23 + 32) is exact
-__device__ __forceinline__ float pg_byte_to_f32_m32(uint32_t word, int byte) {
-    return __uint_as_float(__byte_perm(word, 0x4b000000u, 0x7650 + byte)) - 8388640.0f;
+__device__ __forceinline__ uint32_t pg_dequant_pair_mul_m32(uint32_t word, int b, uint64_t s) {   // (q - 32) * s
+    uint32_t r;
+    asm("{\n\t.reg .b64 t;\n\t.reg .b32 x, y;\n\tmov.b64 t, {%1, %2};\n\tadd.rn.f32x2 t, t, %3;\n\tmul.rn.f32x2 t, t, %4;\n\tmov.b64 {x, y}, t;\n\t"
+        "cvt.rn.bf16x2.f32 %0, y, x;\n\t}"
+        : "=r"(r)
+        : "r"(__byte_perm(word, 0x4b000000u, 0x7650 + b)), "r"(__byte_perm(word, 0x4b000000u, 0x7651 + b)), "l"(0xcb000020cb000020ull), "l"(s));
+    return r;
 }
 __device__ __forceinline__ uint32_t pg_pack_bf16(float lo, float hi) {
     const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
@@ -92,14 +98,6 @@ __device__ __forceinline__ uint32_t pg_pack_bf16(float lo, float hi) {
 // The two threads of a row fetch disjoint halves of what both need (the block header once per
 // block, the group's 32 qs bytes every stage) and exchange them by shuffle when the bytes are
 // used: every byte of a weight tile crosses the L2 -> SM path once.
-struct PgRawQ4 {
-    uint2 hdr_half;   // bytes 8h .. 8h+7 of {d, dmin, 12 scale bytes}; valid for group 0 of a block
-    uint4 qm;         // qs bytes 16h .. 16h+15 of the group
-};
-__device__ __forceinline__ void pg_load_q4(PgRawQ4 &r, const uint8_t *blk, int g, int h) {
-    if (g == 0) r.hdr_half = ldg_nc_u2(blk + 8 * h);
-    r.qm = ldg_nc_u4(blk + 16 + 32 * g + 16 * h);
-}
 __device__ __forceinline__ uint4 pg_pair_exchange(const uint4 &mine) {
     return make_uint4(__shfl_xor_sync(0xffffffffu, mine.x, 1), __shfl_xor_sync(0xffffffffu, mine.y, 1), __shfl_xor_sync(0xffffffffu, mine.z, 1),
                       __shfl_xor_sync(0xffffffffu, mine.w, 1));
@@ -200,14 +198,14 @@ __device__ __forceinline__ void pg_tma_2d(uint32_t dst, const void *tmap, int x,
 }
 
 // Up to three matrices that share the token tile go out in one launch (q/k/v, gate/up): the
-// x dimension of the grid runs over the 256-row tiles of all of them.
+// row tiles of all of them are numbered through.
 constexpr int PG_MAX_JOBS = 3;
 struct PgJob {
     const uint8_t *w;
     float *y;     // [seq][rows]
     int rows, type, tile0, pad;
-    // gate + up form (w2 != null): a tile is 64 rows of w (gate) on TMEM lanes 0-63 and the same 64 rows of w2 (up) on
-    // lanes 64-127; the epilogue writes silu(gate) * up as bf16 [seq][rows] to yb - the token matrix of the down matmul
+    // gate + up form (w2 != null): a tile is 64 rows of w (gate) and the same 64 rows of w2 (up); the epilogue writes
+    // silu(gate) * up as bf16 [seq][rows] to yb - the token matrix of the down matmul
     const uint8_t *w2;
     uint16_t *yb;
 };
@@ -228,6 +226,7 @@ __device__ __forceinline__ void pg_dequant_q4(const uint4 &hdr, const uint4 &q0,
     const uint32_t scw = g < 2 ? sc03 : sc47, mnw = g < 2 ? mn03 : mn47;
     const int sh = 16 * (g & 1) + 8 * h;
     const float ds = __fmul_rn(d, (float)((scw >> sh) & 0xffu)), nm = -__fmul_rn(dmin, (float)((mnw >> sh) & 0xffu));
+    const uint64_t ds2 = pg_pair_f32(ds, ds), nm2 = pg_pair_f32(nm, nm);
     const uint32_t qw[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
     const int nsh = 4 * h;
 #pragma unroll
@@ -236,8 +235,8 @@ __device__ __forceinline__ void pg_dequant_q4(const uint4 &hdr, const uint4 &q0,
 #pragma unroll
         for (int w = 0; w < 2; w++) {
             const uint32_t n4 = (qw[2 * c + w] >> nsh) & 0x0f0f0f0fu;
-            o[2 * w] = pg_pack_bf16(__fmaf_rn(ds, pg_byte_to_f32(n4, 0), nm), __fmaf_rn(ds, pg_byte_to_f32(n4, 1), nm));
-            o[2 * w + 1] = pg_pack_bf16(__fmaf_rn(ds, pg_byte_to_f32(n4, 2), nm), __fmaf_rn(ds, pg_byte_to_f32(n4, 3), nm));
+            o[2 * w] = pg_dequant_pair_fma(n4, 0, ds2, nm2);
+            o[2 * w + 1] = pg_dequant_pair_fma(n4, 2, ds2, nm2);
         }
         *reinterpret_cast<uint4 *>(row_base + (((c + 4 * h) ^ rr) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
     }
@@ -253,16 +252,18 @@ struct PgRawQ6 {
 // threads of a warp read rows that lie kilobytes apart, so every load instruction costs 32 cache-line accesses
 // whatever its width: seven 16-byte loads per half block instead of eighteen 4-byte ones is what lifts the Q6_K
 // producer off the load pipe.  An aligned 16-byte load that contains one byte of the tensor cannot leave its page.
-template <int NW, int NV>
+template <int NW, int NV, bool SHARED = false>
 __device__ __forceinline__ void pg_ldg_window(const uint8_t *p, uint32_t *out, uint32_t *raw = nullptr) {
     static_assert(4 * NV >= NW + 4, "window too small");
     const uintptr_t a = reinterpret_cast<uintptr_t>(p);
-    const uint8_t *base = reinterpret_cast<const uint8_t *>(a & ~(uintptr_t)15);
+    const uint8_t *base = p - (a & 15);
     const uint32_t off = (uint32_t)(a & 15), k = off >> 2, sh = (off & 3u) * 8u;
     uint32_t v[4 * NV];
 #pragma unroll
     for (int j = 0; j < NV; j++) {
-        const uint4 t = ldg_nc_u4(base + 16 * j);
+        uint4 t;
+        if constexpr (SHARED) t = *reinterpret_cast<const uint4 *>(base + 16 * j);
+        else t = ldg_nc_u4(base + 16 * j);
         v[4 * j] = t.x, v[4 * j + 1] = t.y, v[4 * j + 2] = t.z, v[4 * j + 3] = t.w;
     }
     if (raw) {
@@ -290,6 +291,25 @@ __device__ __forceinline__ void pg_load_q6(PgRawQ6 &r, const uint8_t *blk, int n
     const uint32_t dlo = (dk & 2u) ? ((dk & 1u) ? raw[7] : raw[6]) : ((dk & 1u) ? raw[5] : raw[4]);
     r.d = f16_bits_to_f32((dlo >> ((dpos & 2u) * 8u)) & 0xffffu);
 }
+// ql, qh: this half's 32 low and high bytes; scw: its two scale bytes
+__device__ __forceinline__ void pg_dequant_q6_half(const uint32_t (&ql)[8], const uint32_t (&qh)[8], uint32_t scw, float d, bool odd, int h, uint8_t *row_base, int rr) {
+    const float ds0 = __fmul_rn(d, (float)(int)(int8_t)(scw & 0xffu)), ds1 = __fmul_rn(d, (float)(int)(int8_t)((scw >> 8) & 0xffu));
+    const uint64_t sp[2] = {pg_pair_f32(ds0, ds0), pg_pair_f32(ds1, ds1)};
+    // the two high bits of this half's elements sit at bit 2h (even group) or 4 + 2h (odd group) of qh
+    const int hs = (odd ? 4 : 0) + 2 * h, ls = odd ? 4 : 0;
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+        uint32_t o[4];
+#pragma unroll
+        for (int w = 0; w < 2; w++) {
+            const int i = 2 * c + w;
+            const uint32_t q = ((ql[i] >> ls) & 0x0f0f0f0fu) | (((qh[i] >> hs) << 4) & 0x30303030u);
+            o[2 * w] = pg_dequant_pair_mul_m32(q, 0, sp[c >> 1]);
+            o[2 * w + 1] = pg_dequant_pair_mul_m32(q, 2, sp[c >> 1]);
+        }
+        *reinterpret_cast<uint4 *>(row_base + (((c + 4 * h) ^ rr) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+}
 __device__ __forceinline__ void pg_dequant_q6(const PgRawQ6 &r, int g, int h, uint8_t *row_base, int rr) {
     const bool odd = g & 1;
     uint32_t qh[8];
@@ -299,216 +319,7 @@ __device__ __forceinline__ void pg_dequant_q6(const PgRawQ6 &r, int g, int h, ui
         qh[i] = h ? other : r.qh[i];
         qh[4 + i] = h ? r.qh[i] : other;
     }
-    const uint32_t scw = (odd ? r.sc[1] : r.sc[0]) >> (16 * h);   // this half's two scale bytes
-    const float ds0 = __fmul_rn(r.d, (float)(int)(int8_t)(scw & 0xffu)), ds1 = __fmul_rn(r.d, (float)(int)(int8_t)((scw >> 8) & 0xffu));
-    // the two high bits of this half's elements sit at bit 2h (even group) or 4 + 2h (odd group) of qh
-    const int hs = (odd ? 4 : 0) + 2 * h;
-#pragma unroll
-    for (int c = 0; c < 4; c++) {
-        uint32_t o[4];
-        const float sa = c < 2 ? ds0 : ds1;
-#pragma unroll
-        for (int w = 0; w < 2; w++) {
-            const int i = 2 * c + w;
-            const uint32_t lo = (odd ? (r.ql[i] >> 4) : r.ql[i]) & 0x0f0f0f0fu;
-            const uint32_t q = lo | (((qh[i] >> hs) << 4) & 0x30303030u);
-            o[2 * w] = pg_pack_bf16(__fmul_rn(sa, pg_byte_to_f32_m32(q, 0)), __fmul_rn(sa, pg_byte_to_f32_m32(q, 1)));
-            o[2 * w + 1] = pg_pack_bf16(__fmul_rn(sa, pg_byte_to_f32_m32(q, 2)), __fmul_rn(sa, pg_byte_to_f32_m32(q, 3)));
-        }
-        *reinterpret_cast<uint4 *>(row_base + (((c + 4 * h) ^ rr) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
-    }
-}
-
-
-// grid = (sum over jobs of ceil(rows / 128), ceil(seq / 512)); 288 threads; dynamic shared memory PG_SMEM.
-RNB_GLOBAL void __launch_bounds__(PG_THREADS, 1)
-prefill_gemm_kernel(const __grid_constant__ PgJobs jobs, const __grid_constant__ PgTensorMap tmap_x, int seq, int cols,
-                         int *__restrict__ err_flag) {
-    extern __shared__ __align__(1024) uint8_t pg_smem_raw[];
-    __shared__ __align__(8) uint64_t full[PG_STAGES], empty[PG_STAGES], done_bar;
-    __shared__ uint32_t tmem_base_slot;
-    __shared__ int s_failed;
-    pdl_launch_dependents();
-    pdl_wait();
-    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(pg_smem_raw) + 1023) & ~(uintptr_t)1023);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    int jsel = 0;
-    for (int i = 1; i < jobs.n; i++)
-        if ((int)blockIdx.x >= jobs.j[i].tile0) jsel = i;
-    const PgJob &job = jobs.j[jsel];
-    const int rows = job.rows, TYPE = job.type;
-    const uint8_t *__restrict__ w = job.w;
-    float *__restrict__ y = job.y;
-    const uint32_t BLK = TYPE == TYPE_Q4_K ? Q4K_BYTES : Q6K_BYTES;
-    const bool pair = job.w2 != nullptr;
-    const int n0 = ((int)blockIdx.x - job.tile0) * (pair ? PG_ROWS / 2 : PG_ROWS), m0 = blockIdx.y * PG_TOK;
-    const int nb = cols >> 8, KT = cols / PG_K;
-    if (tid == 0) {
-        for (int s = 0; s < PG_STAGES; s++) {
-            mbar_init(&full[s], 9);    // one arrival per producer warp + the thread that issues the token copies
-            mbar_init(&empty[s], 1);   // tcgen05.commit
-        }
-        mbar_init(&done_bar, 1);
-        mbar_fence_init();
-        s_failed = 0;
-    }
-    if (warp == 8) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)), "r"(512) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    pg_fence_before();
-    __syncthreads();
-    pg_fence_after();
-    const uint32_t tmem_base = tmem_base_slot;
-    bool ok = true;
-
-    if (warp < 8) {
-        const int row = tid >> 1, h = tid & 1, rr = row & 7;
-        const size_t rb = (size_t)nb * BLK;
-        // rows past the end repeat the last one (never stored)
-        const uint8_t *wr = pair ? (row < PG_ROWS / 2 ? w : job.w2) + (size_t)min(n0 + (row & (PG_ROWS / 2 - 1)), rows - 1) * rb
-                                 : w + (size_t)min(n0 + row, rows - 1) * rb;
-        uint8_t *const brow = smem + PG_A_BYTES + (row >> 3) * 1024 + rr * 128;
-        // token tile of stage kt: thread 0 announces the bytes and issues the two copies
-        auto issue_tokens = [&](int kt) {
-            if (tid != 0) return;
-            const int s = kt % PG_STAGES;
-            const uint32_t dst = smem_u32(smem + (uint32_t)s * PG_STAGE_BYTES);
-            mbar_arrive_expect_tx(&full[s], PG_A_BYTES);
-#pragma unroll
-            for (int i = 0; i < PG_TOK / PG_BOX_ROWS; i++)
-                pg_tma_2d(dst + (uint32_t)i * (PG_BOX_ROWS * 128), &tmap_x, kt * PG_K, m0 + i * PG_BOX_ROWS, &full[s]);
-        };
-        auto stage_tail = [&](int kt) -> bool {
-            pg_proxy_fence();
-            __syncwarp();
-            if (lane == 0) pg_arrive(&full[kt % PG_STAGES]);
-            if (kt + 1 < KT) {
-                // the next stage may be written once the MMAs that read it have been committed
-                if (!mbar_wait_bounded(&empty[(kt + 1) % PG_STAGES], (uint32_t)((((kt + 1) / PG_STAGES) & 1) ^ 1))) return false;
-                issue_tokens(kt + 1);
-            }
-            return true;
-        };
-        ok = mbar_wait_bounded(&empty[0], 1u);
-        if (ok) issue_tokens(0);
-        if (TYPE == TYPE_Q4_K) {
-            PgRawQ4 cur, nxt;
-            uint4 hdr = make_uint4(0u, 0u, 0u, 0u);
-            pg_load_q4(cur, wr, 0, h);
-            for (int kt = 0; kt < KT && ok; kt++) {
-                const int g = kt & 3;
-                if (kt + 1 < KT) pg_load_q4(nxt, wr + (size_t)((kt + 1) >> 2) * BLK, (kt + 1) & 3, h);
-                if (g == 0) {   // a new block: put the header halves together
-                    const uint32_t ox = __shfl_xor_sync(0xffffffffu, cur.hdr_half.x, 1), oy = __shfl_xor_sync(0xffffffffu, cur.hdr_half.y, 1);
-                    hdr = h ? make_uint4(ox, oy, cur.hdr_half.x, cur.hdr_half.y) : make_uint4(cur.hdr_half.x, cur.hdr_half.y, ox, oy);
-                }
-                const uint4 other = pg_pair_exchange(cur.qm);
-                pg_dequant_q4(hdr, h ? other : cur.qm, h ? cur.qm : other, g, h, brow + (uint32_t)(kt % PG_STAGES) * PG_STAGE_BYTES, rr);
-                ok = __all_sync(0xffffffffu, stage_tail(kt));   // warp-uniform: the shuffles above need the whole warp
-                cur = nxt;
-            }
-        } else {
-            PgRawQ6 cur, nxt;
-            pg_load_q6(cur, wr, 0, h);
-            for (int kt = 0; kt < KT && ok; kt++) {
-                // a half block (128 elements) serves two stages: fetch the next half two stages ahead
-                if (!(kt & 1) && kt + 2 < KT) pg_load_q6(nxt, wr + (size_t)((kt + 2) >> 2) * BLK, ((kt + 2) >> 1) & 1, h);
-                pg_dequant_q6(cur, kt & 3, h, brow + (uint32_t)(kt % PG_STAGES) * PG_STAGE_BYTES, rr);
-                ok = __all_sync(0xffffffffu, stage_tail(kt));   // warp-uniform: the shuffles in the dequantisation need the whole warp
-                if (kt & 1) cur = nxt;
-            }
-        }
-    } else {
-        // ---- MMA issuer: per stage 2 token halves x 4 K-steps of 16; the weight tile is the M operand (128 rows =
-        // 128 TMEM lanes), a token half the N operand (256 columns): fewer shared-memory reads per flop than four
-        // 128 x 128 products ----
-        for (int kt = 0; kt < KT && ok; kt++) {
-            const int s = kt % PG_STAGES;
-            ok = mbar_wait_bounded(&full[s], (uint32_t)((kt / PG_STAGES) & 1));
-            if (!ok) break;
-            pg_fence_after();
-            if (lane == 0) {
-                const uint32_t x_addr = smem_u32(smem + (uint32_t)s * PG_STAGE_BYTES), w_addr = x_addr + PG_A_BYTES;
-#pragma unroll
-                for (int nh = 0; nh < 2; nh++)
-#pragma unroll
-                    for (int k = 0; k < 4; k++)
-                        pg_mma(tmem_base + (uint32_t)nh * 256u, pg_smem_desc(w_addr + (uint32_t)k * 32u),
-                               pg_smem_desc(x_addr + (uint32_t)nh * 256u * 128u + (uint32_t)k * 32u), (kt > 0 || k > 0) ? 1u : 0u);
-                pg_commit(&empty[s]);
-            }
-            __syncwarp();
-        }
-        if (ok && lane == 0) pg_commit(&done_bar);
-        __syncwarp();
-    }
-    if (!ok) atomicExch(&s_failed, 1);
-
-    // ---- epilogue: warps 0-7; TMEM lane = weight row (lane quarter = warp % 4), column = token (half = warp / 4).
-    // A warp's 32 lanes hold 32 consecutive rows of one token: each store instruction writes 128 contiguous bytes ----
-    if (warp < 8) {
-        bool fin = ok && mbar_wait_bounded(&done_bar, 0u);
-        // token copies that were announced but never consumed must land before the CTA exits
-        if (!fin) {
-            atomicExch(&s_failed, 1);
-            for (int s = 0; s < PG_STAGES; s++) mbar_wait_bounded(&full[s], 0u);
-        }
-        pg_fence_after();
-        if (pair) {
-            // gate rows sit on lanes 0-63 (lane quarters 0, 1), the same rows of up on lanes 64-127 (quarters 2, 3): the
-            // eight warps put their 32 rows x 32 tokens into shared memory (the operand stages are free by now), then
-            // each computes silu(gate) * up for 16 of the 32 tokens of its row.  Every warp takes part in every
-            // barrier, whatever its own wait returned.
-            float *ex = reinterpret_cast<float *>(smem);
-            const int q = warp & 3, nh = warp >> 2, qp = q & 1;
-            const int row = n0 + qp * 32 + lane, t_lo = (q >> 1) * 16;
-#pragma unroll 1
-            for (int cc = 0; cc < 256 / 32; cc++) {
-                // two exchange buffers in turn: the barrier of the next pass also covers the reads of this one
-                float *buf = ex + (size_t)(cc & 1) * (8 * 32 * 33);
-                float *mine = buf + (size_t)warp * (32 * 33);
-                const float *gsrc = buf + (size_t)(nh * 4 + qp) * (32 * 33), *usrc = buf + (size_t)(nh * 4 + qp + 2) * (32 * 33);
-                uint32_t v[32];
-                if (fin) pg_tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(nh * 256 + cc * 32), v);
-#pragma unroll
-                for (int i = 0; i < 32; i++) mine[lane * 33 + i] = fin ? __uint_as_float(v[i]) : 0.f;
-                asm volatile("bar.sync 1, 256;" ::: "memory");
-                const int tok0 = m0 + nh * 256 + cc * 32 + t_lo;
-                if (fin && row < rows) {
-                    uint16_t *dst = job.yb + (size_t)tok0 * rows + row;
-#pragma unroll
-                    for (int i = 0; i < 16; i++) {
-                        const float g = gsrc[lane * 33 + t_lo + i], u = usrc[lane * 33 + t_lo + i];
-                        // fast exponential and division: their 2^-21 relative error disappears in the bf16 rounding below
-                        const float a = __fdividef(g, 1.0f + __expf(-g)) * u;
-                        if (tok0 + i < seq) dst[(size_t)i * rows] = (uint16_t)(pg_pack_bf16(a, 0.f) & 0xffffu);
-                    }
-                }
-            }
-        } else if (fin) {
-            const int q = warp & 3, nh = warp >> 2;
-            const int row = n0 + q * 32 + lane;
-#pragma unroll 1
-            for (int cc = 0; cc < 256 / 32; cc++) {
-                uint32_t v[32];
-                pg_tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(nh * 256 + cc * 32), v);
-                const int tok0 = m0 + nh * 256 + cc * 32;
-                if (row < rows) {
-                    float *dst = y + (size_t)tok0 * rows + row;
-#pragma unroll
-                    for (int i = 0; i < 32; i++)
-                        if (tok0 + i < seq) dst[(size_t)i * rows] = __uint_as_float(v[i]);
-                }
-            }
-        }
-    }
-    pg_fence_before();
-    __syncthreads();
-    if (warp == 8) {
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
-        if (lane == 0 && s_failed && err_flag) atomicExch(err_flag, DEV_ERR_GEMM_TIMEOUT);
-    }
+    pg_dequant_q6_half(r.ql, qh, (odd ? r.sc[1] : r.sc[0]) >> (16 * h), r.d, odd, h, row_base, rr);
 }
 
 }  // namespace rnb

@@ -1,9 +1,9 @@
-// Prefill matmul for short prompts: the same product as prefill_gemm_kernel (dequantised bf16 weights x bf16 tokens,
+// Prefill matmul for short prompts: the same product as prefill_gemm_pair_kernel (dequantised bf16 weights x bf16 tokens,
 // f32 accumulators in tensor memory), cut so that a few hundred tokens still occupy the chip.
 //
 // A CTA owns 128 weight rows x up to 256 tokens and a part of K; the `ks` CTAs of a thread-block cluster share a tile
 // and add their accumulators over distributed shared memory in rank order (the same bits on every run, whichever CTA
-// adds).  A 512-token tile per CTA leaves 32 CTAs for the 4096 rows of an output projection on 148 SMs, each with a
+// adds).  A tile of all tokens per CTA leaves 32 CTAs for the 4096 rows of an output projection on 148 SMs, each with a
 // chain of 64 to 224 stages; with K cut in 8 the chain is 8 to 28 stages on 256 CTAs.
 //
 // Two CTAs per SM.  A stage is 64 elements of K: nt tokens x 128 bytes by one tiled TMA copy, and 128 weight rows that
