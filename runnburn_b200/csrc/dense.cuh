@@ -422,20 +422,21 @@ dense_gemm_split_kernel(const __grid_constant__ DenseGemmJobs jobs, const __grid
         __syncwarp();
         const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(&tmem_slot);
         const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(P.nt >> 3) << 17) | ((uint32_t)(DG_ROWS >> 4) << 24);
-        if (lane == 0) {
-            for (int kt = 0; kt < KT && ok; kt++) {
-                const int s = kt % S;
-                ok = mbar_wait_bounded(&full[s], (uint32_t)((kt / S) & 1));
-                if (!ok) break;
-                pg_fence_after();
-                const uint32_t x_addr = smem_u32(smem + (uint32_t)s * stage_bytes), w_addr = x_addr + x_bytes;
+        for (int kt = 0; kt < KT && ok; kt++) {
+            const int s = kt % S;
+            ok = __all_sync(0xffffffffu, mbar_wait_bounded(&full[s], (uint32_t)((kt / S) & 1)));
+            if (!ok) break;
+            pg_fence_after();
+            if (pg_elect()) {
+                const uint32_t x_addr = smem_u32(smem + (uint32_t)s * stage_bytes);
+                const uint64_t dx = pg_smem_desc(x_addr), dw = pg_smem_desc(x_addr + x_bytes);
 #pragma unroll
-                for (int k = 0; k < 4; k++)
-                    ps_mma(tmem, pg_smem_desc(w_addr + (uint32_t)k * 32u), pg_smem_desc(x_addr + (uint32_t)k * 32u), idesc, (kt > 0 || k > 0) ? 1u : 0u);
+                for (int k = 0; k < 4; k++) ps_mma(tmem, dw + 2u * k, dx + 2u * k, idesc, (kt > 0 || k > 0) ? 1u : 0u);   // 32 bytes on
                 pg_commit(&empty[s]);
             }
-            if (ok) pg_commit(&done_bar);
+            __syncwarp();
         }
+        if (ok && pg_elect()) pg_commit(&done_bar);
         __syncwarp();
     }
     if (!ok) s_failed = 1;

@@ -254,17 +254,17 @@ prefill_gemm_split_kernel(const __grid_constant__ PgJobs jobs, const __grid_cons
             ok = __all_sync(0xffffffffu, mbar_wait_bounded(&full[s], phase));
             if (!ok) break;
             pg_fence_after();
-            if (lane == 0) {
-                const uint32_t x_addr = smem_u32(smem + (uint32_t)s * stage_bytes), w_addr = x_addr + x_bytes;
+            if (pg_elect()) {
+                const uint32_t x_addr = smem_u32(smem + (uint32_t)s * stage_bytes);
+                const uint64_t dx = pg_smem_desc(x_addr), dw = pg_smem_desc(x_addr + x_bytes);
 #pragma unroll
-                for (int k = 0; k < 4; k++)
-                    ps_mma(tmem, pg_smem_desc(w_addr + (uint32_t)k * 32u), pg_smem_desc(x_addr + (uint32_t)k * 32u), idesc, (kt > 0 || k > 0) ? 1u : 0u);
+                for (int k = 0; k < 4; k++) ps_mma(tmem, dw + 2u * k, dx + 2u * k, idesc, (kt > 0 || k > 0) ? 1u : 0u);   // 32 bytes on
                 pg_commit(&empty[s]);
             }
             __syncwarp();
             if (++s == S) s = 0, phase ^= 1u;
         }
-        if (ok && lane == 0) pg_commit(&done_bar);
+        if (ok && pg_elect()) pg_commit(&done_bar);
         __syncwarp();
     } else if (lane == 0) {
         pdl_wait();   // the tokens are the previous launch's result
