@@ -2,7 +2,7 @@
 //
 //   dense_gemv_kernel       1..8 tokens, f32 activations: one warp per two rows, weights streamed by
 //                           16-byte loads (the first ones issued before the dependency wait)
-//   dense_gemm_kernel       many tokens, bf16 activations, tcgen05: 128 rows x 256 tokens per CTA
+//   dense_gemm_pair_kernel  many tokens, bf16 activations, tcgen05: 256 rows x up to 512 tokens per pair of SMs
 //   dense_gemm_split_kernel the same for prompts whose tiles do not fill the chip: K cut over a cluster
 //   dense_gemm_simt_kernel  many tokens in true f32 (and bf16 activations whose rows are not
 //                           16-byte aligned, which the tiled copies cannot describe)
@@ -14,6 +14,7 @@
 
 #include "common.cuh"
 #include "prefill_gemm.cuh"
+#include "prefill_gemm_pair.cuh"
 #include "prefill_gemm_split.cuh"
 
 namespace rnb {
@@ -172,18 +173,11 @@ dense_gemv_kernel(const __grid_constant__ DenseVecJobs jobs) {
 }
 
 // ---- many tokens, tcgen05 -----------------------------------------------------------------------
-// One CTA: 128 weight rows (M operand, TMEM lane = row) x 256 tokens (N operand), f32 accumulators in
-// 256 tensor-memory columns.  K advances 64 per stage; a stage is one copy of 256 tokens and two of 64
-// weight rows (a gate + up pair takes its second half from the other matrix), both in the 128-byte
-// swizzle the descriptors expect, zeros past either end.  Two stages of 48 KB let two CTAs share an SM:
-// one's epilogue overlaps the other's matmul.  Warp 0 issues the copies, warp 1 the MMAs, warps 2-5
-// read the accumulators back.  Every wait is bounded; after a timeout the error flag is set, the
-// copies in flight are waited for and the tensor memory is freed.
-// grid = (token tiles, row tiles of all jobs): CTAs that run together share weight rows, so a weight matrix
-// larger than L2 still crosses DRAM once.
-constexpr int DG_TOK = 256, DG_ROWS = 128, DG_K = 64, DG_STAGES = 2, DG_THREADS = 192;
-constexpr uint32_t DG_X_BYTES = DG_TOK * 128, DG_W_BYTES = DG_ROWS * 128, DG_STAGE_BYTES = DG_X_BYTES + DG_W_BYTES;
-constexpr size_t DG_SMEM = (size_t)DG_STAGES * DG_STAGE_BYTES + 1024;
+// Weights are the M operand (tensor-memory lane = row), tokens the N operand, f32 accumulators.  K advances 64 per stage, in
+// the 128-byte swizzle the descriptors expect, zeros past either end.  Every wait is bounded; after a timeout the error flag
+// is set, the copies in flight are waited for and the tensor memory is freed.
+constexpr int DG_ROWS = 128, DG_K = 64;
+constexpr uint32_t DG_W_BYTES = DG_ROWS * 128;
 
 struct DenseGemmJob {
     void *y;             // [seq][ld]
@@ -202,122 +196,169 @@ struct DenseMaps {   // per job: tokens, weights, second weights
 template <class OT>
 __device__ __forceinline__ void dg_store(void *y, size_t idx, float v) { reinterpret_cast<OT *>(y)[idx] = from_f32<OT>(v); }
 
-RNB_GLOBAL void __launch_bounds__(DG_THREADS)
-dense_gemm_kernel(const __grid_constant__ DenseGemmJobs jobs, const __grid_constant__ DenseMaps maps, int *__restrict__ err_flag) {
+// A pair of CTAs (a cluster of two) multiplies 256 rows x up to 512 tokens: each CTA takes 128 rows (64 of gate and 64 of up
+// in the pair form) and half of the tokens, the MMAs read the token halves of both SMs, and a CTA's rows x tokens fill its
+// tensor memory (parts of n1 and n2 tokens).  A stage of K moves 48 KB into an SM per 1024 cycles of the tensor pipe; a
+// CTA by itself with 256 tokens moved 48 KB per 512 cycles, more than an SM gets from L2.  Four stages.
+// Persistent: a pair walks its tiles, token tiles fastest, so that a weight matrix larger than L2 crosses DRAM once.  Warp 0
+// issues the copies (the first stages' weights before the dependency wait), warp 1 of the even CTA the MMAs, warps 2-9 read
+// the accumulators back, four per part; a part of the next tile starts when its columns are free.
+constexpr int DQ_STAGES = 4, DQ_THREADS = 320;
+constexpr uint32_t DQ_STAGE_BYTES = PT_MAX_TOK / 2 * 128 + DG_W_BYTES;
+constexpr uint32_t DQ_EXCHANGE = 2 * 2 * 4 * 8 * 32 * 4;   // parts x buffers in turn x warps x tokens x rows
+constexpr size_t DQ_SMEM = (size_t)DQ_STAGES * DQ_STAGE_BYTES + DQ_EXCHANGE + 1024;
+struct DenseMapsPair {   // per job: tokens of part 1 and 2 (boxes of n1 / 2 and n2 / 2), weights, second weights
+    PgTensorMap x1[DENSE_MAX_JOBS], x2[DENSE_MAX_JOBS], w[DENSE_MAX_JOBS], w2[DENSE_MAX_JOBS];
+};
+struct DensePair {
+    int n1, n2, token_tiles, tiles;   // n1, n2: multiples of 32, at most 256; tiles: pairs of row tiles of all jobs x token tiles
+};
+RNB_GLOBAL void __launch_bounds__(DQ_THREADS, 1)
+dense_gemm_pair_kernel(const __grid_constant__ DenseGemmJobs jobs, const __grid_constant__ DenseMapsPair maps, const DensePair P, int *__restrict__ err_flag) {
     extern __shared__ __align__(1024) uint8_t dg_smem_raw[];
-    __shared__ __align__(8) uint64_t full[DG_STAGES], empty[DG_STAGES], done_bar;
+    __shared__ __align__(8) uint64_t full[DQ_STAGES], empty[DQ_STAGES], acc_full, acc_free[2];
     __shared__ uint32_t tmem_slot;
     __shared__ int s_failed;
     pdl_launch_dependents();
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(dg_smem_raw) + 1023) & ~(uintptr_t)1023);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    int js = 0;
-    for (int i = 1; i < jobs.n; i++)
-        if ((int)blockIdx.y >= jobs.j[i].tile0) js = i;
-    const DenseGemmJob &job = jobs.j[js];
-    const bool pair = job.pair != 0;
-    const int rows = job.rows, seq = jobs.seq;
-    const int n0 = ((int)blockIdx.y - job.tile0) * (pair ? DG_ROWS / 2 : DG_ROWS), m0 = blockIdx.x * DG_TOK;
-    const int KT = (job.cols + DG_K - 1) / DG_K;
+    const int rank = (int)blockIdx.x & 1, pair0 = (int)blockIdx.x >> 1, n_pairs = (int)gridDim.x >> 1, nt = P.n1 + P.n2;
+    const uint32_t tok_bytes = (uint32_t)(nt / 2) * 128u, stage_bytes = tok_bytes + DG_W_BYTES;
     if (tid == 0) {
-        for (int s = 0; s < DG_STAGES; s++) {
+        for (int s = 0; s < DQ_STAGES; s++) {
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], 1);
         }
-        mbar_init(&done_bar, 1);
+        mbar_init(&acc_full, 1);
+        for (int i = 0; i < 2; i++) mbar_init(&acc_free[i], 8);
         mbar_fence_init();
         s_failed = 0;
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(256) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        // no launch that holds tensor memory can share an SM with this much shared memory
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(512) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
     pg_fence_before();
     __syncthreads();
+    ps_cluster_sync();   // barriers and tensor memory of both CTAs stand
     pg_fence_after();
     const uint32_t tmem = tmem_slot;
-    pdl_wait();
+    auto job_of = [&](int tile) {
+        int js = 0;
+        for (int i = 1; i < jobs.n; i++)
+            if (tile / P.token_tiles >= jobs.j[i].tile0) js = i;
+        return js;
+    };
+    // first row of this CTA's part of a tile: rows past the end read as zeros and are never stored
+    auto first_row = [&](int tile, const DenseGemmJob &job) { return (2 * (tile / P.token_tiles - job.tile0) + rank) * (job.pair ? DG_ROWS / 2 : DG_ROWS); };
+    bool ok = true;
 
     if (warp == 0) {
         if (lane == 0) {
-            bool ok = true;
-            int issued = 0;
-            for (int kt = 0; kt < KT && ok; kt++) {
-                const int s = kt % DG_STAGES;
-                ok = mbar_wait_bounded(&empty[s], (uint32_t)(((kt / DG_STAGES) & 1) ^ 1));
-                if (!ok) break;
-                const uint32_t dst = smem_u32(smem + (uint32_t)s * DG_STAGE_BYTES);
-                mbar_arrive_expect_tx(&full[s], DG_STAGE_BYTES);
-                pg_tma_2d(dst, &maps.x[js], kt * DG_K, m0, &full[s]);
-                pg_tma_2d(dst + DG_X_BYTES, &maps.w[js], kt * DG_K, n0, &full[s]);
-                pg_tma_2d(dst + DG_X_BYTES + DG_W_BYTES / 2, pair ? &maps.w2[js] : &maps.w[js], kt * DG_K, pair ? n0 : n0 + DG_ROWS / 2, &full[s]);
-                issued = kt + 1;
+            uint32_t it = 0;
+            auto weights = [&](uint32_t at, int js, int kt, int n0) {
+                const uint32_t s = at % DQ_STAGES, dst = smem_u32(smem + s * stage_bytes) + tok_bytes, bar = ps_map(smem_u32(&full[s]), 0);
+                const bool pair = jobs.j[js].pair != 0;
+                if (rank == 0) mbar_arrive_expect_tx(&full[s], 2 * stage_bytes);   // both CTAs' copies
+                pt_tma_2d(dst, &maps.w[js], kt * DG_K, n0, bar);
+                pt_tma_2d(dst + DG_W_BYTES / 2, pair ? &maps.w2[js] : &maps.w[js], kt * DG_K, pair ? n0 : n0 + DG_ROWS / 2, bar);
+            };
+            int head = 0;
+            for (int tile = pair0; tile < P.tiles && ok; tile += n_pairs) {
+                const int js = job_of(tile), n0 = first_row(tile, jobs.j[js]), m0 = (tile % P.token_tiles) * nt, KT = (jobs.j[js].cols + DG_K - 1) / DG_K;
+                if (tile == pair0) {
+                    head = min(KT, DQ_STAGES);
+                    for (int kt = 0; kt < head; kt++) weights((uint32_t)kt, js, kt, n0);
+                    pdl_wait();   // the tokens are the previous launch's result
+                }
+                for (int kt = 0; kt < KT; kt++, it++) {
+                    const uint32_t s = it % DQ_STAGES, dst = smem_u32(smem + s * stage_bytes), bar = ps_map(smem_u32(&full[s]), 0);
+                    if (it >= (uint32_t)head) {
+                        ok = mbar_wait_bounded(&empty[s], ((it / DQ_STAGES) & 1u) ^ 1u);
+                        if (!ok) break;
+                        weights(it, js, kt, n0);
+                    }
+                    pt_tma_2d(dst, &maps.x1[js], kt * DG_K, m0 + rank * (P.n1 / 2), bar);
+                    pt_tma_2d(dst + (uint32_t)(P.n1 / 2) * 128u, &maps.x2[js], kt * DG_K, m0 + P.n1 + rank * (P.n2 / 2), bar);
+                }
             }
-            if (!ok) {
-                // copies that were announced must land before the CTA may leave
-                atomicExch(&s_failed, 1);
-                for (int kt = max(0, issued - DG_STAGES); kt < issued; kt++) mbar_wait_bounded(&full[kt % DG_STAGES], (uint32_t)((kt / DG_STAGES) & 1));
-            }
+            // after a failure the copies that were announced must land before the CTAs may leave
+            if (!ok && rank == 0)
+                for (uint32_t i = it > DQ_STAGES ? it - DQ_STAGES : 0; i < it; i++) mbar_wait_bounded(&full[i % DQ_STAGES], (i / DQ_STAGES) & 1u);
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            bool ok = true;
-            for (int kt = 0; kt < KT && ok; kt++) {
-                const int s = kt % DG_STAGES;
-                ok = mbar_wait_bounded(&full[s], (uint32_t)((kt / DG_STAGES) & 1));
-                if (!ok) break;
-                pg_fence_after();
-                const uint32_t x_addr = smem_u32(smem + (uint32_t)s * DG_STAGE_BYTES), w_addr = x_addr + DG_X_BYTES;
+        if (rank == 0) {
+            const uint32_t id1 = pt_idesc(P.n1), id2 = pt_idesc(P.n2);
+            uint32_t s = 0, phase = 0;
+            int count = 0;
+            for (int tile = pair0; tile < P.tiles && ok; tile += n_pairs, count++) {
+                const int KT = (jobs.j[job_of(tile)].cols + DG_K - 1) / DG_K;
+                for (int kt = 0; kt < KT && ok; kt++) {
+                    ok = __all_sync(0xffffffffu, mbar_wait_bounded(&full[s], phase));
+                    const uint32_t x1 = smem_u32(smem + s * stage_bytes);
+                    const uint64_t dx1 = pg_smem_desc(x1), dx2 = pg_smem_desc(x1 + (uint32_t)(P.n1 / 2) * 128u), dw = pg_smem_desc(x1 + tok_bytes);
+                    for (int part = 0; part < 2 && ok; part++) {
+                        if (kt == 0 && count > 0) ok = __all_sync(0xffffffffu, pt_wait(&acc_free[part], (uint32_t)((count - 1) & 1)));
+                        if (!ok) break;
+                        pg_fence_after();
+                        if (pg_elect()) {
+                            const uint64_t dx = part ? dx2 : dx1;
 #pragma unroll
-                for (int k = 0; k < 4; k++)
-                    pg_mma(tmem, pg_smem_desc(w_addr + (uint32_t)k * 32u), pg_smem_desc(x_addr + (uint32_t)k * 32u), (kt > 0 || k > 0) ? 1u : 0u);
-                pg_commit(&empty[s]);
+                            for (int k = 0; k < 4; k++) pt_mma(tmem + (uint32_t)part * 256u, dw + 2u * k, dx + 2u * k, part ? id2 : id1, (kt | k) != 0);   // 32 bytes on
+                            if (part) pt_commit(&empty[s]);
+                        }
+                        __syncwarp();
+                    }
+                    if (++s == DQ_STAGES) s = 0, phase ^= 1u;
+                }
+                if (ok && pg_elect()) pt_commit(&acc_full);
+                __syncwarp();
             }
-            if (ok) pg_commit(&done_bar);
-            else atomicExch(&s_failed, 1);
         }
     } else {
-        const int q = warp & 3;   // tensor-memory lane quarter of this warp
-        const bool fin = mbar_wait_bounded(&done_bar, 0u);
-        if (!fin) atomicExch(&s_failed, 1);
-        pg_fence_after();
-        const int n_cc = min(DG_TOK, seq - m0 + 31) / 32;   // 32-token column groups that hold tokens
-        if (pair) {
-            // gate rows on lanes 0-63, the same rows of up on lanes 64-127: the four warps exchange them through
-            // shared memory (the stages are free: every MMA has been committed) and each finishes 16 of the 32 tokens
-            float *ex = reinterpret_cast<float *>(smem);
-            const int qp = q & 1, t_lo = (q >> 1) * 16;
-            const int row = n0 + qp * 32 + lane;
-            for (int cc = 0; cc < n_cc; cc++) {
-                float *buf = ex + (size_t)(cc & 1) * (4 * 32 * 33);
-                float *mine = buf + (size_t)q * (32 * 33);
-                const float *gs = buf + (size_t)qp * (32 * 33), *us = buf + (size_t)(qp + 2) * (32 * 33);
-                uint32_t v[32];
-                if (fin) pg_tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(cc * 32), v);
+        const int q = warp & 3, part = (warp - 2) >> 2, cols = part ? P.n2 : P.n1;   // tensor-memory lane quarter and columns of this warp
+        float *const ex = reinterpret_cast<float *>(smem + (size_t)DQ_STAGES * DQ_STAGE_BYTES + (size_t)part * (DQ_EXCHANGE / 2));
+        const uint32_t at = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(part * 256);
+        pdl_wait();   // stores come after the launches before this one
+        int count = 0, turn = 0;
+        for (int tile = pair0; tile < P.tiles && ok; tile += n_pairs, count++) {
+            const DenseGemmJob &job = jobs.j[job_of(tile)];
+            const int n0 = first_row(tile, job), m0 = (tile % P.token_tiles) * nt + part * P.n1, rows = job.rows;
+            ok = __all_sync(0xffffffffu, mbar_wait_bounded(&acc_full, (uint32_t)(count & 1)));
+            pg_fence_after();
+            if (job.pair)   // every warp of the part takes part in the exchange, whatever its own wait returned
+                for (int c = 0; c < cols && m0 + c < jobs.seq; c += 16, turn ^= 1) {
+                    // gate rows on lanes 0-63, the same rows of up on lanes 64-127: a warp hands eight of 16 tokens to its partner
+                    uint32_t v[16];
+                    if (ok) ps_tmem_ld<16>(at + (uint32_t)c, v);
+                    const bool up = q >= 2;
+                    float *buf = ex + turn * (4 * 8 * 32);
 #pragma unroll
-                for (int i = 0; i < 32; i++) mine[lane * 33 + i] = fin ? __uint_as_float(v[i]) : 0.f;
-                asm volatile("bar.sync 1, 128;" ::: "memory");
-                if (fin && row < rows) {
+                    for (int i = 0; i < 8; i++) buf[((q ^ 2) * 8 + i) * 32 + lane] = ok ? __uint_as_float(up ? v[i] : v[8 + i]) : 0.f;
+                    asm volatile("bar.sync %0, 128;" ::"r"(1 + part) : "memory");
+                    const int row = n0 + (q & 1) * 32 + lane;
+                    if (ok && row < rows) {
 #pragma unroll
-                    for (int i = 0; i < 16; i++) {
-                        const int tok = m0 + cc * 32 + t_lo + i;
-                        const float z = gs[lane * 33 + t_lo + i];
-                        const float a = (job.out_bf16 ? gate_act_fast(job.act, z) : gate_act(job.act, z)) * us[lane * 33 + t_lo + i];
-                        if (tok < seq) {
+                        for (int i = 0; i < 8; i++) {
+                            const int tok = m0 + c + i + (up ? 8 : 0);
+                            const float other = buf[(q * 8 + i) * 32 + lane], own = __uint_as_float(up ? v[8 + i] : v[i]);
+                            const float z = up ? other : own, u = up ? own : other;
+                            if (tok >= jobs.seq) continue;
+                            const float a = (job.out_bf16 ? gate_act_fast(job.act, z) : gate_act(job.act, z)) * u;
                             if (job.out_bf16) dg_store<bf16>(job.y, (size_t)tok * job.ld + row, a);
                             else dg_store<float>(job.y, (size_t)tok * job.ld + row, a);
                         }
                     }
                 }
-            }
-        } else if (fin) {
-            const int row = n0 + q * 32 + lane;
-            for (int cc = 0; cc < n_cc; cc++) {
-                uint32_t v[32];
-                pg_tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(cc * 32), v);
-                if (row < rows) {
+            else if (ok) {
+                const int row = n0 + q * 32 + lane;
+                const float b = job.decay_bias && row < rows ? job.decay_bias[row] : 0.f;
+                for (int c = 0; c < cols && m0 + c < jobs.seq; c += 32) {
+                    uint32_t v[32];
+                    pg_tmem_ld32(at + (uint32_t)c, v);
+                    if (row >= rows) continue;
                     if (job.decay_bias) {
-                        const float b = job.decay_bias[row];
                         if (job.decay_kind == DECAY_SIGMOID_ROOT) {
 #pragma unroll
                             for (int i = 0; i < 32; i++) v[i] = __float_as_uint(sigmoid_root_fast(__uint_as_float(v[i]) + b, job.inv_tau));
@@ -328,20 +369,26 @@ dense_gemm_kernel(const __grid_constant__ DenseGemmJobs jobs, const __grid_const
                     }
 #pragma unroll
                     for (int i = 0; i < 32; i++) {
-                        const int tok = m0 + cc * 32 + i;
-                        if (tok < seq) {
+                        const int tok = m0 + c + i;
+                        if (tok < jobs.seq) {
                             if (job.out_bf16) dg_store<bf16>(job.y, (size_t)tok * job.ld + row, __uint_as_float(v[i]));
                             else dg_store<float>(job.y, (size_t)tok * job.ld + row, __uint_as_float(v[i]));
                         }
                     }
                 }
             }
+            pg_fence_before();
+            __syncwarp();
+            if (lane == 0) pt_arrive(ps_map(smem_u32(&acc_free[part]), 0));
         }
     }
+    if (!ok) s_failed = 1;
+    __syncwarp();
     pg_fence_before();
     __syncthreads();
+    ps_cluster_sync();   // the other CTA's memory and barriers are no longer used
     if (warp == 1) {
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
         if (lane == 0 && s_failed && err_flag) atomicExch(err_flag, DEV_ERR_GEMM_TIMEOUT);
     }
 }
@@ -354,12 +401,13 @@ dense_gemm_kernel(const __grid_constant__ DenseGemmJobs jobs, const __grid_const
 // rows gave the 256-token tiles 16 CTAs at 150 tokens; a prompt of 64 tokens through 8 Punisun layers of width 2048 takes
 // 1.46 ms (2.45 with those tiles), one of 150 through 6 Dutivik layers 1.06 ms (1.58).
 // Warp 0 issues the copies, warp 1 the MMAs, warps 2-5 reduce and store.  grid = (row tiles of all jobs x ks, token tiles).
-constexpr int DP_SUB = 16, DP_MAX_STAGES = 5;
+constexpr int DP_SUB = 16, DP_MAX_STAGES = 5, DP_THREADS = 192, DP_TOK = 256;   // DP_TOK: most tokens per CTA
+constexpr size_t DP_SMEM = PS_SMEM;   // two CTAs per SM
 struct DenseSplit {
     int nt, stages, ks;
     uint32_t tmem_cols;
 };
-RNB_GLOBAL void __launch_bounds__(DG_THREADS)
+RNB_GLOBAL void __launch_bounds__(DP_THREADS)
 dense_gemm_split_kernel(const __grid_constant__ DenseGemmJobs jobs, const __grid_constant__ DenseMaps maps, const DenseSplit P, int *__restrict__ err_flag) {
     extern __shared__ __align__(1024) uint8_t dg_smem_raw[];
     __shared__ __align__(8) uint64_t full[DP_MAX_STAGES], empty[DP_MAX_STAGES], done_bar;

@@ -653,7 +653,7 @@ int LayerStack::ready(cudaStream_t s) {
         return RNB_B200_OK;
     };
     const void *fns[] = {(const void *)residual_norm_kernel<float, 4>, (const void *)residual_norm_kernel<float, 1>, (const void *)residual_norm_kernel<bf16, 4>,
-                         (const void *)residual_norm_kernel<bf16, 1>, (const void *)dense_gemm_kernel, (const void *)dense_gemm_split_kernel, (const void *)decay_rows_kernel,
+                         (const void *)residual_norm_kernel<bf16, 1>, (const void *)dense_gemm_pair_kernel, (const void *)dense_gemm_split_kernel, (const void *)decay_rows_kernel,
                          (const void *)linear_state_step_kernel<4>, (const void *)linear_state_step_kernel<8>, (const void *)linear_state_step_kernel<16>,
                          (const void *)linear_state_step_kernel<32>, (const void *)linear_state_step_kernel<64>, (const void *)causal_attention_kernel<4>,
                          (const void *)causal_attention_kernel<8>, (const void *)causal_attention_kernel<16>, (const void *)causal_attention_kernel<32>,
@@ -795,12 +795,23 @@ int LayerStack::matmul(cudaStream_t s, int n, const Mm *jobs, int n_jobs, int *e
         // Uncut tiles of up to 128 tokens also go there, for the deeper ring; at 256 tokens the other kernel's order of the
         // grid is better (2048 tokens: 6.4 against 5.2 ms at width 4096).
         DenseSplit P;
-        const int token_tiles = (n + DG_TOK - 1) / DG_TOK;
+        const int token_tiles = (n + DP_TOK - 1) / DP_TOK;
         P.ks = 1;
         while (P.ks * 2 <= PS_MAX_KS && tiles * token_tiles * P.ks * 2 <= 296 && P.ks * 4 <= depth) P.ks *= 2;
         if (P.ks == 2 && depth < 64) P.ks = 1;
         P.nt = ((n + token_tiles - 1) / token_tiles + 15) & ~15;
         const bool split = P.ks > 1 || P.nt <= 128;
+        DenseMapsPair MP;
+        DensePair Q;
+        memset(&MP, 0, sizeof(MP));
+        memset(&Q, 0, sizeof(Q));
+        int row_pairs = 0;
+        for (int i = 0; i < n_jobs; i++) {
+            const int per = jobs[i].w2 ? DG_ROWS : 2 * DG_ROWS;
+            row_pairs += (jobs[i].w->rows + per - 1) / per;
+        }
+        // a stage is bound by the tensor pipe (two cycles a token) or by its copies (16 KB of weights cost as much as 256 tokens)
+        if (!split) pg_pair_tiles(Q, row_pairs, n, [](int w) { return std::max(2 * w, w + 256) + 48; });
         tiles = 0;
         for (int i = 0; i < n_jobs; i++) {
             DenseGemmJob &j = J.j[i];
@@ -814,21 +825,27 @@ int LayerStack::matmul(cudaStream_t s, int n, const Mm *jobs, int n_jobs, int *e
             j.tile0 = tiles;
             j.out_bf16 = !jobs[i].f32_out;
             j.pair = jobs[i].w2 != nullptr;
-            const int per = j.pair ? DG_ROWS / 2 : DG_ROWS;
+            const int per = (j.pair ? DG_ROWS / 2 : DG_ROWS) * (split ? 1 : 2);
             tiles += (j.rows + per - 1) / per;
-            RNB_TRY(encode_token_map(&M.x[i], reinterpret_cast<const uint16_t *>(jobs[i].x), (size_t)n, (size_t)j.cols, jobs[i].ldx, split ? P.nt : DG_TOK));
-            memcpy(&M.w[i], jobs[i].w->map, sizeof(PgTensorMap));
-            if (j.pair) memcpy(&M.w2[i], jobs[i].w2->map, sizeof(PgTensorMap));
+            const uint16_t *x = reinterpret_cast<const uint16_t *>(jobs[i].x);
+            if (split)
+                RNB_TRY(encode_token_map(&M.x[i], x, (size_t)n, (size_t)j.cols, jobs[i].ldx, P.nt));
+            else {
+                RNB_TRY(encode_token_map(&MP.x1[i], x, (size_t)n, (size_t)j.cols, jobs[i].ldx, Q.n1 / 2));
+                RNB_TRY(encode_token_map(&MP.x2[i], x, (size_t)n, (size_t)j.cols, jobs[i].ldx, Q.n2 / 2));
+            }
+            memcpy(split ? &M.w[i] : &MP.w[i], jobs[i].w->map, sizeof(PgTensorMap));
+            if (j.pair) memcpy(split ? &M.w2[i] : &MP.w2[i], jobs[i].w2->map, sizeof(PgTensorMap));
         }
         if (split) {
-            P.stages = std::min<int>(DP_MAX_STAGES, (int)((DG_SMEM - 1024) / ((uint32_t)P.nt * 128u + DG_W_BYTES)));
+            P.stages = std::min<int>(DP_MAX_STAGES, (int)((DP_SMEM - 1024) / ((uint32_t)P.nt * 128u + DG_W_BYTES)));
             P.tmem_cols = 32;
             while ((int)P.tmem_cols < P.nt) P.tmem_cols *= 2;
-            RNB_CU(launch_k_cluster(dense_gemm_split_kernel, dim3((unsigned)(tiles * P.ks), (unsigned)token_tiles), dim3(DG_THREADS), DG_SMEM, s, dim3((unsigned)P.ks), J, M, P,
+            RNB_CU(launch_k_cluster(dense_gemm_split_kernel, dim3((unsigned)(tiles * P.ks), (unsigned)token_tiles), dim3(DP_THREADS), DP_SMEM, s, dim3((unsigned)P.ks), J, M, P,
                                     err));
             return RNB_B200_OK;
         }
-        RNB_CU(launch_k(dense_gemm_kernel, dim3((unsigned)token_tiles, (unsigned)tiles), dim3(DG_THREADS), DG_SMEM, s, J, M, err));
+        RNB_CU(launch_k_cluster(dense_gemm_pair_kernel, dim3((unsigned)(2 * std::min(Q.tiles, pg_pairs()))), dim3(DQ_THREADS), DQ_SMEM, s, dim3(2), J, MP, Q, err));
         return RNB_B200_OK;
     }
     DenseSimtJobs J;

@@ -31,16 +31,6 @@ constexpr uint32_t PG_B_BYTES = PG_ROWS * 128;   // weight tile of a stage
 __device__ __forceinline__ uint64_t pg_smem_desc(uint32_t saddr) {
     return (uint64_t)((saddr & 0x3ffffu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
-// D = f32, A = B = bf16, both K-major, N = 256 (a token half), M = 128 (the weight rows)
-constexpr uint32_t PG_IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(256 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-
-__device__ __forceinline__ void pg_mma(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(da), "l"(db), "r"(PG_IDESC), "r"(accumulate)
-        : "memory");
-}
 // One lane of a converged warp.  The MMAs are issued behind this and not behind `lane == 0`: their operands live in uniform
 // registers, and where the compiler cannot see that a single thread gets there it moves them there once per lane (a stage of
 // eight MMAs took 1000 cycles to issue).
