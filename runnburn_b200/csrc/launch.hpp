@@ -712,7 +712,7 @@ inline int launch_attention_decode(cudaStream_t s, const float *q, const uint16_
 // Tensor-core prefill matmul: converts the f32 token rows to bf16 (scratch `xb`, seq*cols
 // elements) and runs the tcgen05 kernel.  y is [seq][rows] f32.
 int prefill_gemm_setup();   // raises the kernels' dynamic shared-memory limit once
-// Descriptor of a bf16 matrix [seq][cols] (row pitch ld elements, 0: cols) for the kernels' tiled copies:
+// Descriptor of a bf16 (or f16) matrix [seq][cols] (row pitch ld elements, 0: cols) for the kernels' tiled copies:
 // boxes of 64 columns x box_rows rows, 128-byte swizzle, zeros past either end.  The encoder is a driver
 // entry point, looked up once through the runtime.
 inline int encode_token_map(PgTensorMap *out, const uint16_t *xb, size_t seq, size_t cols, size_t ld, int box_rows) {

@@ -2,6 +2,7 @@
 // f32 tensors: crates/rnb-backend/cuda/src/runtime/api/attention_api.rs:661-700).
 #pragma once
 #include "attention.cuh"
+#include "launch.hpp"
 #include "prefill_attention_tiled.cuh"
 #include "state.hpp"
 
@@ -62,17 +63,18 @@ inline int launch_prefill_attention_f16kv(cudaStream_t s, const float *q, const 
     cfg.stream = s;
     const bool aligned = (((uintptr_t)k | (uintptr_t)v) & 15) == 0;
     if (!simt && tiled && aligned && group >= 1 && group <= PAT_ROWS && (group & (group - 1)) == 0 && num_heads == group * num_kv_heads &&
-        ((uintptr_t)q & 7) == 0 && ((uintptr_t)out & 7) == 0 && kv_len >= seq_len) {
+        ((uintptr_t)q & 15) == 0 && ((uintptr_t)out & 15) == 0 && kv_len >= seq_len && seq_len > 0) {
         static bool attr_set = false;
         if (!attr_set) {
             RNB_CU(cudaFuncSetAttribute(prefill_attention_tiled_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PAT_SMEM));
             attr_set = true;
         }
         const int qpc = PAT_ROWS / group;
-        cfg.blockDim = dim3(PAT_THREADS);
-        cfg.gridDim = dim3((seq_len + qpc - 1) / qpc, num_kv_heads);
-        cfg.dynamicSmemBytes = PAT_SMEM;
-        RNB_CU(cudaLaunchKernelEx(&cfg, prefill_attention_tiled_kernel, q, k, v, seq_len, kv_len, num_heads, num_kv_heads, scale, out));
+        PatMaps maps;
+        RNB_TRY(encode_token_map(&maps.k, k, (size_t)kv_len, (size_t)num_kv_heads * HD, 0, PAT_KEYS));
+        RNB_TRY(encode_token_map(&maps.v, v, (size_t)kv_len, (size_t)num_kv_heads * HD, 0, PAT_KEYS));
+        RNB_CU(launch_k(prefill_attention_tiled_kernel, dim3((seq_len + qpc - 1) / qpc, num_kv_heads), dim3(PAT_THREADS), PAT_SMEM, s, q, maps, seq_len, kv_len,
+                        num_heads, num_kv_heads, scale, out, dev_error));
         return RNB_B200_OK;
     }
     cfg.blockDim = dim3(FD_THREADS);

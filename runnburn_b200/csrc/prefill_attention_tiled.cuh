@@ -1,195 +1,290 @@
-// Causal prefill attention, query-tiled: one CTA owns 128 (query, head) rows of one KV head -
-// 128 / group consecutive query positions x the group's heads - and walks the visible keys in
-// tiles of 64, so a K/V tile fetched once serves all 128 rows (the split-KV decode kernel reused
-// for prefill served 8).  Arithmetic as in the decode kernel: scores and P*V on mma.sync
-// m16n8k16 (f16 operands, fp32 accumulators), q and the probabilities enter as f16 "hi" + f16
-// remainder "lo" so that the products keep fp32-level accuracy against the f16 cache;
-// softmax(q.K^T * scale).V per head with the online maximum, as rnb-cpu's
-// attention_with_scale_window_and_softcap (crates/rnb-cpu/src/kernels/attention/batch_f32.rs:76+);
-// query i sees keys 0 .. kv_len - seq_len + i.
+// Causal prefill attention on the 5th-generation tensor cores: one CTA owns 128 (query, head) rows of one KV head -
+// 128 / group consecutive query positions x the group's heads - and walks the visible keys in tiles of 64.  Arithmetic:
+// f16 operands, fp32 accumulators; q and the probabilities enter as f16 "hi" + f16 remainder "lo" so that the products
+// keep fp32-level accuracy against the f16 cache; softmax(q.K^T * scale).V per head with the online maximum, as
+// rnb-cpu's attention_with_scale_window_and_softcap (crates/rnb-cpu/src/kernels/attention/batch_f32.rs:76+); query i sees
+// keys 0 .. kv_len - seq_len + i.
 //
-// 8 warps, warp w owns rows 16w .. 16w+15; row r = (query r / group, head r % group).  K and V
-// tiles (64 keys x 128 dims f16, 272-byte padded rows) are double-buffered with cp.async;
-// keys past the end of the cache are zero-filled and always masked.
+// Row r = (query r / group, head r % group) is tensor-memory lane r and belongs to one thread of warps 0-3: a row's maximum
+// and sum need no shuffles.  Warp 4 issues the products: scores (128 rows x 64 keys, queries and keys from shared memory), then
+// probabilities from tensor memory x values.  The scores of tile t + 1 are under way while the softmax of tile t runs.  Warp 5
+// copies K and V tiles into a ring of three 16 KB slots in the order of their use (K0 K1 V0 K2 V1 ...).  The output stays in
+// tensor memory; it is scaled only when a row's maximum has grown by more than a factor 2^8 over the one in use, so that
+// probabilities are at most 2^8.  Two CTAs per SM (112 KB, 256 tensor-memory columns each: 64 scores, 128 outputs, 32 + 32
+// probabilities).  Long rows are scheduled first.  Every wait is bounded.
+//
+// What bounds it: the softmax warps (tensor pipe 25 % busy).  2048 tokens of 32 / 8 heads: 134 us cold (262 with mma.sync
+// and eight warps that shared a CTA); 203 tokens behind 1000 positions through 32 layers 10.2 -> 9.4 ms.
 #pragma once
 #include "attention.cuh"
+#include "prefill_gemm_split.cuh"
 
 namespace rnb {
 
 constexpr int PAT_ROWS = 128;                      // (query, head) rows per CTA
 constexpr int PAT_KEYS = 64;                       // keys per tile
-constexpr int PAT_THREADS = 256;
-constexpr int PAT_PITCH = 2 * HD + 16;             // bytes per padded K/V row
-constexpr int PAT_TILE_BYTES = PAT_KEYS * PAT_PITCH;
-constexpr size_t PAT_SMEM = 4 * (size_t)PAT_TILE_BYTES;   // 2 stages x (K, V)
+constexpr int PAT_THREADS = 192;
+constexpr int PAT_SLOTS = 3;
+constexpr uint32_t PAT_PANEL = PAT_ROWS * 128;     // 64 dims of the queries, 128-byte swizzle
+constexpr uint32_t PAT_Q_BYTES = 4 * PAT_PANEL;    // hi, lo x two panels
+constexpr uint32_t PAT_TILE_BYTES = PAT_KEYS * 2 * HD;
+constexpr size_t PAT_SMEM = PAT_Q_BYTES + PAT_SLOTS * PAT_TILE_BYTES + 128;   // + barriers; two CTAs per SM leave no room to align
+constexpr float PAT_GROWTH = 8.0f;                 // log2
 
-// grid = (ceil(seq_len / (128 / group)), num_kv_heads); group = num_heads / num_kv_heads in {1, 2, 4, 8, 16}.
-RNB_GLOBAL void __launch_bounds__(PAT_THREADS, 1)
-prefill_attention_tiled_kernel(const float *__restrict__ q, const uint16_t *__restrict__ k, const uint16_t *__restrict__ v, int seq_len, int kv_len,
-                               int num_heads, int num_kv_heads, float scale, float *__restrict__ out) {
-    extern __shared__ __align__(128) uint8_t pat_smem[];
+struct PatMaps {
+    PgTensorMap k, v;   // [kv_len][kv heads * 128] f16, boxes of 64 columns x 64 rows
+};
+
+// V as the second operand: dims contiguous ("MN-major"), 128-byte swizzle: 8 keys x 64 dims are 1024 bytes, the next 8 keys follow,
+// the other 64 dims are a panel of 64 keys further
+__device__ __forceinline__ uint64_t pat_v_desc(uint32_t saddr) {
+    return (uint64_t)((saddr & 0x3ffffu) >> 4) | ((uint64_t)((PAT_KEYS * 128) >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+}
+// D = f32, A = B = f16, M = 128
+constexpr uint32_t PAT_IDESC_S = (1u << 4) | ((uint32_t)(PAT_KEYS >> 3) << 17) | ((uint32_t)(PAT_ROWS >> 4) << 24);
+constexpr uint32_t PAT_IDESC_O = (1u << 4) | (1u << 16) | ((uint32_t)(HD >> 3) << 17) | ((uint32_t)(PAT_ROWS >> 4) << 24);   // second operand MN-major
+// D += A (tensor memory) x B
+__device__ __forceinline__ void pat_mma_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void pat_tmem_st32(uint32_t taddr, const uint32_t (&v)[32]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,"
+        "%26,%27,%28,%29,%30,%31,%32};"
+        ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]),
+        "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]),
+        "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
+        : "memory");
+}
+__device__ __forceinline__ void pat_tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// grid = (ceil(seq_len / (128 / group)), num_kv_heads); group = num_heads / num_kv_heads a power of two up to 128.
+RNB_GLOBAL void __launch_bounds__(PAT_THREADS, 2)
+prefill_attention_tiled_kernel(const float *__restrict__ q, const __grid_constant__ PatMaps maps, int seq_len, int kv_len, int num_heads, int num_kv_heads,
+                               float scale, float *__restrict__ out, int *__restrict__ err_flag) {
+    extern __shared__ __align__(1024) uint8_t pat_smem[];
     pdl_launch_dependents();
-    pdl_wait();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    uint64_t *const bars = reinterpret_cast<uint64_t *>(pat_smem + PAT_Q_BYTES + PAT_SLOTS * PAT_TILE_BYTES);
+    uint64_t *const full = bars, *const empty = bars + PAT_SLOTS, *const q_full = bars + 6, *const s_full = bars + 7, *const s_free = bars + 8, *const p_full = bars + 9,
+                    *const pv_done = bars + 10;
+    volatile uint32_t *const tmem_slot = reinterpret_cast<volatile uint32_t *>(bars + 11);
+    volatile int *const s_failed = reinterpret_cast<volatile int *>(bars + 12);
+    const uint32_t smem = smem_u32(pat_smem);
     const int group = num_heads / num_kv_heads, qpc = PAT_ROWS / group;
-    const int qb = (int)gridDim.x - 1 - (int)blockIdx.x;   // long rows first
-    const int kv_h = blockIdx.y;
-    const int i0 = qb * qpc;
-    const int shift = kv_len - seq_len;                    // query i sits at position shift + i
-    const int last_q = min(i0 + qpc, seq_len) - 1;
-    const int n_keys = min(kv_len, shift + last_q + 1);    // keys visible to the CTA's last query
+    const int kv_h = blockIdx.y, i0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * qpc;   // long rows first
+    const int shift = kv_len - seq_len;                                              // query i sits at position shift + i
+    const int n_keys = min(kv_len, shift + min(i0 + qpc, seq_len));                  // keys visible to the CTA's last query
     const int n_tiles = (n_keys + PAT_KEYS - 1) / PAT_KEYS;
-    const uint32_t smem_base = smem_u32(pat_smem);
-
-    // ---- K/V tile t -> stage t & 1: 2 x 64 rows x 16 chunks of 16 bytes, 8 per thread ----
-    auto load_tile = [&](int t) {
-        const uint32_t st = smem_base + (uint32_t)(t & 1) * 2u * PAT_TILE_BYTES;
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const int idx = i * PAT_THREADS + tid;          // 0..2047
-            const int which = idx >> 10, row = (idx >> 4) & 63, c = idx & 15;
-            const int key = t * PAT_KEYS + row;
-            const uint16_t *base = which ? v : k;
-            const uint16_t *src = base + ((size_t)min(key, kv_len - 1) * num_kv_heads + kv_h) * HD + c * 8;
-            const uint32_t nbytes = key < kv_len ? 16u : 0u;
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(st + (uint32_t)which * PAT_TILE_BYTES + (uint32_t)row * PAT_PITCH + (uint32_t)c * 16u),
-                         "l"(src), "r"(nbytes)
-                         : "memory");
+    if (tid == 0) {
+        for (int s = 0; s < PAT_SLOTS; s++) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    if (n_tiles > 0) load_tile(0);
-
-    // ---- this thread's two rows: g = lane / 4 -> rows 16w + g and 16w + g + 8 ----
-    const int g = lane >> 2, tq = lane & 3;
-    int qi[2], hd[2], pos[2];
-    bool live[2];
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-        const int r = warp * 16 + g + 8 * h;
-        qi[h] = i0 + r / group;
-        hd[h] = kv_h * group + r % group;
-        live[h] = qi[h] < seq_len;
-        pos[h] = live[h] ? shift + qi[h] : kv_len - 1;   // dead rows see everything (finite numbers) and are never stored
+        mbar_init(q_full, 4);
+        mbar_init(s_full, 1);
+        mbar_init(s_free, 4);
+        mbar_init(p_full, 4);
+        mbar_init(pv_done, 1);
+        mbar_fence_init();
+        *s_failed = (smem & 1023u) != 0;
     }
-    // q A-fragments (hi, lo): k-step ks covers dims 16ks..16ks+15; regs: (row g, dims 2tq..), (row g+8, same), (row g, +8), (row g+8, +8)
-    uint32_t qh[8][4], ql[8][4];
-#pragma unroll
-    for (int ks = 0; ks < 8; ks++)
-#pragma unroll
-        for (int h = 0; h < 2; h++)
-#pragma unroll
-            for (int half = 0; half < 2; half++) {
-                float2 x = make_float2(0.f, 0.f);
-                if (live[h]) x = *reinterpret_cast<const float2 *>(q + ((size_t)qi[h] * num_heads + hd[h]) * HD + ks * 16 + half * 8 + 2 * tq);
-                split_f16x2(x.x, x.y, qh[ks][h + 2 * half], ql[ks][h + 2 * half]);
-            }
-    float o[16][4];
-#pragma unroll
-    for (int j = 0; j < 16; j++) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
-    float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
-    const float sl2 = scale * 1.4426950408889634f;   // scores are kept in log2 units: exp(x) = exp2(x * log2 e)
-    const int mi = lane >> 3, mr = lane & 7;         // ldmatrix: this lane addresses row mr of matrix mi
-
-    for (int t = 0; t < n_tiles; t++) {
-        if (t + 1 < n_tiles) {
-            load_tile(t + 1);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-        }
-        __syncthreads();
-        const uint32_t k_st = smem_base + (uint32_t)(t & 1) * 2u * PAT_TILE_BYTES, v_st = k_st + PAT_TILE_BYTES;
-        // ---- S = q . K^T for 16 rows x 64 keys ----
-        float s[8][4];
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
-            // B fragments of key tile j: matrices (dims 16ks2*2 + 8 mi) for two k-steps per ldmatrix
-            const uint32_t row_addr = k_st + (uint32_t)(j * 8 + mr) * PAT_PITCH + (uint32_t)mi * 16u;
-#pragma unroll
-            for (int kp = 0; kp < 4; kp++) {
-                uint32_t b[4];
-                ldmatrix_x4(b, row_addr + (uint32_t)kp * 64u);
-                mma_f16_16816(s[j], qh[2 * kp], b[0], b[1]);
-                mma_f16_16816(s[j], ql[2 * kp], b[0], b[1]);
-                mma_f16_16816(s[j], qh[2 * kp + 1], b[2], b[3]);
-                mma_f16_16816(s[j], ql[2 * kp + 1], b[2], b[3]);
-            }
-        }
-        // ---- scale, causal mask, online softmax (rows g and g + 8; a row's 64 scores live in a quad) ----
-        const int key0 = t * PAT_KEYS + 2 * tq;
-        const bool need_mask = t * PAT_KEYS + PAT_KEYS - 1 > min(pos[0], pos[1]);
-        float mx[2] = {-INFINITY, -INFINITY};
-#pragma unroll
-        for (int j = 0; j < 8; j++)
-#pragma unroll
-            for (int e = 0; e < 4; e++) {
-                const int h = e >> 1, key = key0 + j * 8 + (e & 1);
-                float x = s[j][e] * sl2;
-                if (need_mask && key > pos[h]) x = -INFINITY;
-                s[j][e] = x;
-                mx[h] = fmaxf(mx[h], x);
-            }
-        float corr[2], m_use[2];
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-            mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 1));
-            mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 2));
-            const float m_new = fmaxf(m_run[h], mx[h]);
-            m_use[h] = m_new == -INFINITY ? 0.f : m_new;   // a fully masked row so far: keep everything at zero
-            corr[h] = exp2f(m_run[h] - m_use[h]);           // exp2(-inf) = 0 on the first tile
-            m_run[h] = m_new;
-        }
-        float rs[2] = {0.f, 0.f};
-        uint32_t ph[4][4], pl[4][4];   // P as A fragments of the 4 key k-steps (16 keys each)
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const float p0 = exp2f(s[j][0] - m_use[0]), p1 = exp2f(s[j][1] - m_use[0]);
-            const float p2 = exp2f(s[j][2] - m_use[1]), p3 = exp2f(s[j][3] - m_use[1]);
-            rs[0] += p0 + p1;
-            rs[1] += p2 + p3;
-            // key tile j = half (j & 1) of k-step j / 2: regs (row g), (row g + 8) then the + 8 keys pair
-            split_f16x2(p0, p1, ph[j >> 1][2 * (j & 1)], pl[j >> 1][2 * (j & 1)]);
-            split_f16x2(p2, p3, ph[j >> 1][2 * (j & 1) + 1], pl[j >> 1][2 * (j & 1) + 1]);
-        }
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-            rs[h] += __shfl_xor_sync(0xffffffffu, rs[h], 1);
-            rs[h] += __shfl_xor_sync(0xffffffffu, rs[h], 2);
-            l_run[h] = l_run[h] * corr[h] + rs[h];
-        }
-#pragma unroll
-        for (int j = 0; j < 16; j++) {
-            o[j][0] *= corr[0];
-            o[j][1] *= corr[0];
-            o[j][2] *= corr[1];
-            o[j][3] *= corr[1];
-        }
-        // ---- O += P . V: k-step kk = keys 16kk..16kk+15, dim tiles jp*2, jp*2+1 per transposed ldmatrix ----
-#pragma unroll
-        for (int kk = 0; kk < 4; kk++) {
-            const uint32_t row_addr = v_st + (uint32_t)(kk * 16 + (mi & 1) * 8 + mr) * PAT_PITCH + (uint32_t)(mi >> 1) * 16u;
-#pragma unroll
-            for (int jp = 0; jp < 8; jp++) {
-                uint32_t b[4];
-                ldmatrix_x4_trans(b, row_addr + (uint32_t)jp * 32u);
-                mma_f16_16816(o[2 * jp], ph[kk], b[0], b[1]);
-                mma_f16_16816(o[2 * jp], pl[kk], b[0], b[1]);
-                mma_f16_16816(o[2 * jp + 1], ph[kk], b[2], b[3]);
-                mma_f16_16816(o[2 * jp + 1], pl[kk], b[2], b[3]);
-            }
-        }
-        __syncthreads();   // every warp is done with this stage before the copy of tile t + 2 lands in it
+    pdl_wait();   // the queries and the cache are the previous launch's result; tensor memory is asked for when no earlier launch can still hold it
+    if (warp == 4) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(const_cast<uint32_t *>(tmem_slot))), "r"(256) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    // ---- normalise and store: row h of this thread, dims 8j + 2tq, + 1 ----
+    pg_fence_before();
+    __syncthreads();
+    pg_fence_after();
+    const uint32_t tmem = *tmem_slot, t_s = tmem, t_o = tmem + 64, t_ph = tmem + 192, t_pl = tmem + 224;
+    bool ok = *s_failed == 0;
+
+    if (warp < 4) {
+        // ---- queries as f16 hi + lo: a warp takes its 32 rows one by one, four dims per lane ----
+        for (int i = 0; i < 32 && ok; i++) {
+            const int r = warp * 32 + i, qi = i0 + r / group;
+            float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (qi < seq_len) x = *reinterpret_cast<const float4 *>(q + ((size_t)qi * num_heads + kv_h * group + r % group) * HD + lane * 4);
+            uint2 hi, lo;
+            split_f16x2(x.x, x.y, hi.x, lo.x);
+            split_f16x2(x.z, x.w, hi.y, lo.y);
+            const uint32_t at = (uint32_t)(lane >> 4) * PAT_PANEL + (uint32_t)(r >> 3) * 1024u + (uint32_t)(r & 7) * 128u + (((uint32_t)((lane & 15) >> 1) ^ (uint32_t)(r & 7)) << 4) +
+                                (uint32_t)(lane & 1) * 8u;
+            *reinterpret_cast<uint2 *>(pat_smem + at) = hi;
+            *reinterpret_cast<uint2 *>(pat_smem + 2 * PAT_PANEL + at) = lo;
+        }
+        pg_proxy_fence();
+        __syncwarp();
+        if (lane == 0) pg_arrive(q_full);
+        // ---- softmax: this thread's row ----
+        const int r = warp * 32 + lane, qi = i0 + r / group;
+        const bool live = qi < seq_len;
+        const int pos = live ? shift + qi : kv_len - 1;   // dead rows see everything (finite numbers) and are never stored
+        const uint32_t lanes = (uint32_t)(warp * 32) << 16;
+        const float sl2 = scale * 1.4426950408889634f;    // scores are kept in log2 units: exp(x) = exp2(x * log2 e)
+        float m_ref = -INFINITY, l_run = 0.f;
+        for (int t = 0; t < n_tiles && ok; t++) {
+            ok = __all_sync(0xffffffffu, mbar_wait_bounded(s_full, (uint32_t)(t & 1)));
+            if (!ok) break;
+            pg_fence_after();
+            float s[PAT_KEYS];
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
-        if (!live[h]) continue;
-        const float inv = l_run[h] > 0.f ? 1.0f / l_run[h] : 0.f;
-        float *dst = out + ((size_t)qi[h] * num_heads + hd[h]) * HD + 2 * tq;
+            for (int c = 0; c < 2; c++) {
+                uint32_t v[32];
+                pg_tmem_ld32(t_s + lanes + (uint32_t)c * 32u, v);
 #pragma unroll
-        for (int j = 0; j < 16; j++) *reinterpret_cast<float2 *>(dst + 8 * j) = make_float2(o[j][2 * h] * inv, o[j][2 * h + 1] * inv);
+                for (int i = 0; i < 32; i++) s[c * 32 + i] = __uint_as_float(v[i]) * sl2;
+            }
+            pg_fence_before();
+            __syncwarp();
+            if (lane == 0) pg_arrive(s_free);
+            const int seen = pos - t * PAT_KEYS;   // the tile's keys 0 .. seen are visible
+            if (seen < PAT_KEYS - 1) {
+#pragma unroll
+                for (int i = 0; i < PAT_KEYS; i++)
+                    if (i > seen) s[i] = -INFINITY;
+            }
+            float mx = s[0];
+#pragma unroll
+            for (int i = 1; i < PAT_KEYS; i++) mx = fmaxf(mx, s[i]);
+            // the maximum in use; the output is scaled when it falls behind by more than PAT_GROWTH
+            float corr = 1.0f;
+            if (mx > m_ref + PAT_GROWTH || m_ref == -INFINITY) {
+                const float m_new = fmaxf(mx, m_ref);
+                corr = exp2f(m_ref - (m_new == -INFINITY ? 0.f : m_new));   // exp2(-inf) = 0 on the first tile
+                m_ref = m_new;
+            }
+            const float m_use = m_ref == -INFINITY ? 0.f : m_ref;   // a fully masked row so far: keep everything at zero
+            float sum[4] = {0.f, 0.f, 0.f, 0.f};
+            uint32_t ph[32], pl[32];
+#pragma unroll
+            for (int i = 0; i < 32; i++) {
+                const float p0 = exp2f(s[2 * i] - m_use), p1 = exp2f(s[2 * i + 1] - m_use);
+                sum[i & 3] += p0 + p1;
+                split_f16x2(p0, p1, ph[i], pl[i]);
+            }
+            l_run = l_run * corr + ((sum[0] + sum[1]) + (sum[2] + sum[3]));
+            if (t > 0) {
+                ok = __all_sync(0xffffffffu, mbar_wait_bounded(pv_done, (uint32_t)((t - 1) & 1)));   // the probabilities' columns are free, the output stands
+                if (!ok) break;
+                pg_fence_after();
+                if (__any_sync(0xffffffffu, corr != 1.0f)) {
+#pragma unroll 1
+                    for (int c = 0; c < 4; c++) {
+                        uint32_t v[32];
+                        pg_tmem_ld32(t_o + lanes + (uint32_t)c * 32u, v);
+#pragma unroll
+                        for (int i = 0; i < 32; i++) v[i] = __float_as_uint(__uint_as_float(v[i]) * corr);
+                        pat_tmem_st32(t_o + lanes + (uint32_t)c * 32u, v);
+                    }
+                }
+            }
+            __syncwarp();
+            pat_tmem_st32(t_ph + lanes, ph);
+            pat_tmem_st32(t_pl + lanes, pl);
+            pat_tmem_st_wait();
+            pg_fence_before();
+            __syncwarp();
+            if (lane == 0) pg_arrive(p_full);
+        }
+        if (ok && n_tiles > 0) ok = __all_sync(0xffffffffu, mbar_wait_bounded(pv_done, (uint32_t)((n_tiles - 1) & 1)));
+        if (ok) {
+            pg_fence_after();
+            const float inv = l_run > 0.f ? 1.0f / l_run : 0.f;
+            float *dst = out + ((size_t)min(qi, seq_len - 1) * num_heads + kv_h * group + r % group) * HD;
+#pragma unroll 1
+            for (int c = 0; c < 4; c++) {
+                uint32_t v[32];
+                pg_tmem_ld32(t_o + lanes + (uint32_t)c * 32u, v);
+                if (live) {
+#pragma unroll
+                    for (int i = 0; i < 32; i += 4)
+                        *reinterpret_cast<float4 *>(dst + c * 32 + i) =
+                            make_float4(__uint_as_float(v[i]) * inv, __uint_as_float(v[i + 1]) * inv, __uint_as_float(v[i + 2]) * inv, __uint_as_float(v[i + 3]) * inv);
+                }
+            }
+        }
+    } else if (warp == 4) {
+        // ---- products; item i of the ring lies in slot i % 3 ----
+        const uint32_t ring = smem + PAT_Q_BYTES;
+        uint32_t it = 0;
+        auto arrived = [&]() { return __all_sync(0xffffffffu, mbar_wait_bounded(&full[it % PAT_SLOTS], (it / PAT_SLOTS) & 1u)); };
+        auto scores = [&]() {   // of the K tile that is next in the ring
+            ok = ok && arrived();
+            if (!ok) return;
+            pg_fence_after();
+            if (pg_elect()) {
+                const uint32_t kt = ring + (it % PAT_SLOTS) * PAT_TILE_BYTES;
+#pragma unroll
+                for (int part = 0; part < 2; part++)   // hi, lo
+#pragma unroll
+                    for (int p = 0; p < 2; p++) {
+                        const uint64_t dq = pg_smem_desc(smem + (uint32_t)(2 * part + p) * PAT_PANEL), dk = pg_smem_desc(kt + (uint32_t)p * (PAT_KEYS * 128));
+#pragma unroll
+                        for (int k = 0; k < 4; k++) ps_mma(t_s, dq + 2u * k, dk + 2u * k, PAT_IDESC_S, (part | p | k) != 0);   // 16 dims, 32 bytes on
+                    }
+                pg_commit(&empty[it % PAT_SLOTS]);
+                pg_commit(s_full);
+            }
+            __syncwarp();
+            it++;
+        };
+        if (n_tiles > 0) {
+            ok = ok && __all_sync(0xffffffffu, mbar_wait_bounded(q_full, 0u));
+            scores();
+        }
+        for (int t = 0; t < n_tiles && ok; t++) {
+            if (t + 1 < n_tiles) {
+                ok = __all_sync(0xffffffffu, mbar_wait_bounded(s_free, (uint32_t)(t & 1)));
+                scores();
+            }
+            ok = ok && arrived() && __all_sync(0xffffffffu, mbar_wait_bounded(p_full, (uint32_t)(t & 1)));
+            if (!ok) break;
+            pg_fence_after();
+            if (pg_elect()) {
+                const uint64_t dv = pat_v_desc(ring + (it % PAT_SLOTS) * PAT_TILE_BYTES);
+#pragma unroll
+                for (int k = 0; k < 4; k++) {   // 16 keys: 2048 bytes of V, eight columns of probabilities on
+                    pat_mma_ta(t_o, t_ph + 8u * k, dv + (uint64_t)(k * (2048 >> 4)), PAT_IDESC_O, (t | k) != 0);
+                    pat_mma_ta(t_o, t_pl + 8u * k, dv + (uint64_t)(k * (2048 >> 4)), PAT_IDESC_O, 1u);
+                }
+                pg_commit(&empty[it % PAT_SLOTS]);
+                pg_commit(pv_done);
+            }
+            __syncwarp();
+            it++;
+        }
+    } else if (lane == 0) {
+        uint32_t it = 0;
+        auto copy = [&](const PgTensorMap *map, int t) {
+            const uint32_t s = it % PAT_SLOTS, dst = smem + PAT_Q_BYTES + s * PAT_TILE_BYTES;
+            ok = ok && mbar_wait_bounded(&empty[s], ((it / PAT_SLOTS) & 1u) ^ 1u);
+            if (!ok) return;
+            mbar_arrive_expect_tx(&full[s], PAT_TILE_BYTES);
+            pg_tma_2d(dst, map, kv_h * HD, t * PAT_KEYS, &full[s]);
+            pg_tma_2d(dst + PAT_KEYS * 128, map, kv_h * HD + 64, t * PAT_KEYS, &full[s]);
+            it++;
+        };
+        if (n_tiles > 0) copy(&maps.k, 0);
+        for (int t = 0; t < n_tiles && ok; t++) {
+            if (t + 1 < n_tiles) copy(&maps.k, t + 1);
+            copy(&maps.v, t);
+        }
+        // after a failure the copies that were announced must land before the CTA may leave
+        for (uint32_t i = it > PAT_SLOTS ? it - PAT_SLOTS : 0; i < it && !ok; i++) mbar_wait_bounded(&full[i % PAT_SLOTS], (i / PAT_SLOTS) & 1u);
+    }
+    if (!ok) *s_failed = 1;
+    __syncwarp();
+    pg_fence_before();
+    __syncthreads();
+    if (warp == 4) {
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256) : "memory");
+        if (lane == 0 && *s_failed && err_flag) atomicExch(err_flag, DEV_ERR_GEMM_TIMEOUT);
     }
 }
 

@@ -1,0 +1,45 @@
+"""Prefill attention on tensor memory: sizes at the edges of its tiles (128 rows of query x head, 64 keys), every group of
+heads, and rows whose maximum grows from tile to tile (the output in tensor memory is scaled) or falls, against f64.
+
+Bound: queries and probabilities enter as two f16 terms (2^-21 of each product at worst) and sums are f32: a row's error
+is below 2^-18 of the largest value of V for scores of a few units; a score of size s carries 2^-22 s into the exponent.
+1e-4 of the largest output covers scores up to 200."""
+import numpy as np
+import pytest
+
+from test_gpu_prefill_gemm import ops  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+def reference(q, k, v, scale):
+    seq, heads, _ = q.shape
+    kv_len, kvh, _ = k.shape
+    out = np.empty(q.shape)
+    seen = np.arange(kv_len)[None] <= np.arange(seq)[:, None] + kv_len - seq
+    for h in range(heads):
+        s = np.where(seen, q[:, h].astype(np.float64) @ k[:, h * kvh // heads].astype(np.float64).T * scale, -np.inf)
+        p = np.exp(s - s.max(1, keepdims=True))
+        out[:, h] = (p / p.sum(1, keepdims=True)) @ v[:, h * kvh // heads].astype(np.float64)
+    return out
+
+
+@pytest.mark.parametrize("shape", ["flat", "growing", "falling"])
+@pytest.mark.parametrize("heads,kvh,seq,kv_len", [
+    (8, 8, 1, 1), (2, 2, 128, 128), (4, 2, 64, 65), (8, 2, 33, 129), (16, 2, 17, 300), (16, 1, 8, 64), (32, 1, 5, 191), (64, 1, 3, 192), (128, 1, 2, 257),
+    (32, 8, 513, 1200), (4, 1, 640, 640),
+])
+def test_prefill_attention(ops, heads, kvh, seq, kv_len, shape):
+    rng = np.random.default_rng(heads + 31 * seq + kv_len)
+    q = rng.standard_normal((seq, heads, 128)).astype(np.float32)
+    k = rng.standard_normal((kv_len, kvh, 128))
+    if shape != "flat":
+        # the keys share a direction with the queries, more of it towards one end: scores move by up to 60
+        q += 1.0
+        k += np.linspace(0.0, 5.0, kv_len)[:, None, None] * (1.0 if shape == "growing" else -1.0)
+    k, v = k.astype(np.float16), rng.standard_normal((kv_len, kvh, 128)).astype(np.float16)
+    scale = 1.0 / np.sqrt(128.0)
+    got = ops.attention_prefill_flash_hd128_f16kv(q.reshape(-1), k.view(np.uint16).reshape(-1), v.view(np.uint16).reshape(-1), seq, kv_len, heads, kvh, scale)
+    want = reference(q, k, v, scale)
+    assert ops.dev_error_flag() == 0
+    assert np.max(np.abs(np.asarray(got).reshape(want.shape) - want)) <= 1e-4 * np.max(np.abs(want))
