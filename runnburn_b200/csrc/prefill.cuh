@@ -44,11 +44,12 @@ inline int launch_prefill_attention_f32kv(cudaStream_t s, const float *q, const 
                               num_heads, num_kv_heads, scale, out));
     return RNB_B200_OK;
 }
-// f16 caches on 16-byte boundaries take the tensor-core kernel, anything else the CUDA-core one.
+// f16 caches on 16-byte boundaries take the tensor-core kernel, anything else the CUDA-core one.  `out_bf16`: where the
+// result may go as bf16 instead; *wrote_bf16 says whether it did.
 inline int launch_prefill_attention_f16kv(cudaStream_t s, const float *q, const uint16_t *k,
                                           const uint16_t *v, int seq_len, int kv_len,
                                           int num_heads, int num_kv_heads, float scale,
-                                          float *out, int *dev_error = nullptr) {
+                                          float *out, int *dev_error = nullptr, uint16_t *out_bf16 = nullptr, bool *wrote_bf16 = nullptr) {
     const int group = num_heads / num_kv_heads;
     static const bool simt = [] {
         const char *e = getenv("RNB_B200_FD_SIMT");
@@ -63,7 +64,7 @@ inline int launch_prefill_attention_f16kv(cudaStream_t s, const float *q, const 
     cfg.stream = s;
     const bool aligned = (((uintptr_t)k | (uintptr_t)v) & 15) == 0;
     if (!simt && tiled && aligned && group >= 1 && group <= PAT_ROWS && (group & (group - 1)) == 0 && num_heads == group * num_kv_heads &&
-        ((uintptr_t)q & 15) == 0 && ((uintptr_t)out & 15) == 0 && kv_len >= seq_len && seq_len > 0) {
+        ((uintptr_t)q & 15) == 0 && ((uintptr_t)out & 15) == 0 && kv_len >= seq_len && seq_len > 0 && scale > 0.f && ((uintptr_t)out_bf16 & 15) == 0) {
         static bool attr_set = false;
         if (!attr_set) {
             RNB_CU(cudaFuncSetAttribute(prefill_attention_tiled_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PAT_SMEM));
@@ -74,7 +75,8 @@ inline int launch_prefill_attention_f16kv(cudaStream_t s, const float *q, const 
         RNB_TRY(encode_token_map(&maps.k, k, (size_t)kv_len, (size_t)num_kv_heads * HD, 0, PAT_KEYS));
         RNB_TRY(encode_token_map(&maps.v, v, (size_t)kv_len, (size_t)num_kv_heads * HD, 0, PAT_KEYS));
         RNB_CU(launch_k(prefill_attention_tiled_kernel, dim3((seq_len + qpc - 1) / qpc, num_kv_heads), dim3(PAT_THREADS), PAT_SMEM, s, q, maps, seq_len, kv_len,
-                        num_heads, num_kv_heads, scale, out, dev_error));
+                        num_heads, num_kv_heads, scale, out, out_bf16, dev_error));
+        if (wrote_bf16) *wrote_bf16 = out_bf16 != nullptr;
         return RNB_B200_OK;
     }
     cfg.blockDim = dim3(FD_THREADS);

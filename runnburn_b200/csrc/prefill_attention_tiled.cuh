@@ -60,12 +60,33 @@ __device__ __forceinline__ void pat_tmem_st32(uint32_t taddr, const uint32_t (&v
         "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
         : "memory");
 }
+__device__ __forceinline__ void pat_tmem_ld64(uint32_t taddr, uint32_t (&v)[64]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x64.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,"
+        "%26,%27,%28,%29,%30,%31,%32,%33,%34,%35,%36,%37,%38,%39,%40,%41,%42,%43,%44,%45,%46,%47,%48,%49,%50,%51,%52,%53,%54,%55,%56,%57,%58,%59,%60,"
+        "%61,%62,%63}, [%64];\n\ttcgen05.wait::ld.sync.aligned;"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]),
+          "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]),
+          "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31]), "=r"(v[32]), "=r"(v[33]),
+          "=r"(v[34]), "=r"(v[35]), "=r"(v[36]), "=r"(v[37]), "=r"(v[38]), "=r"(v[39]), "=r"(v[40]), "=r"(v[41]), "=r"(v[42]), "=r"(v[43]), "=r"(v[44]),
+          "=r"(v[45]), "=r"(v[46]), "=r"(v[47]), "=r"(v[48]), "=r"(v[49]), "=r"(v[50]), "=r"(v[51]), "=r"(v[52]), "=r"(v[53]), "=r"(v[54]), "=r"(v[55]),
+          "=r"(v[56]), "=r"(v[57]), "=r"(v[58]), "=r"(v[59]), "=r"(v[60]), "=r"(v[61]), "=r"(v[62]), "=r"(v[63])
+        : "r"(taddr)
+        : "memory");
+}
+// 2^x; what is below 2^-126 of the largest probability is zero
+__device__ __forceinline__ float pat_exp2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
 __device__ __forceinline__ void pat_tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// grid = (ceil(seq_len / (128 / group)), num_kv_heads); group = num_heads / num_kv_heads a power of two up to 128.
+// grid = (ceil(seq_len / (128 / group)), num_kv_heads); group = num_heads / num_kv_heads a power of two up to 128; scale > 0.
+// out_bf16 (may be null): the result rounded to bf16 there instead of f32 in `out`.
 RNB_GLOBAL void __launch_bounds__(PAT_THREADS, 2)
 prefill_attention_tiled_kernel(const float *__restrict__ q, const __grid_constant__ PatMaps maps, int seq_len, int kv_len, int num_heads, int num_kv_heads,
-                               float scale, float *__restrict__ out, int *__restrict__ err_flag) {
+                               float scale, float *__restrict__ out, uint16_t *__restrict__ out_bf16, int *__restrict__ err_flag) {
     extern __shared__ __align__(1024) uint8_t pat_smem[];
     pdl_launch_dependents();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -132,14 +153,8 @@ prefill_attention_tiled_kernel(const float *__restrict__ q, const __grid_constan
             ok = __all_sync(0xffffffffu, mbar_wait_bounded(s_full, (uint32_t)(t & 1)));
             if (!ok) break;
             pg_fence_after();
-            float s[PAT_KEYS];
-#pragma unroll
-            for (int c = 0; c < 2; c++) {
-                uint32_t v[32];
-                pg_tmem_ld32(t_s + lanes + (uint32_t)c * 32u, v);
-#pragma unroll
-                for (int i = 0; i < 32; i++) s[c * 32 + i] = __uint_as_float(v[i]) * sl2;
-            }
+            uint32_t s[PAT_KEYS];
+            pat_tmem_ld64(t_s + lanes, s);
             pg_fence_before();
             __syncwarp();
             if (lane == 0) pg_arrive(s_free);
@@ -147,11 +162,14 @@ prefill_attention_tiled_kernel(const float *__restrict__ q, const __grid_constan
             if (seen < PAT_KEYS - 1) {
 #pragma unroll
                 for (int i = 0; i < PAT_KEYS; i++)
-                    if (i > seen) s[i] = -INFINITY;
+                    if (i > seen) s[i] = 0xff800000u;   // -inf
             }
-            float mx = s[0];
+            float mxs[4];
 #pragma unroll
-            for (int i = 1; i < PAT_KEYS; i++) mx = fmaxf(mx, s[i]);
+            for (int j = 0; j < 4; j++) mxs[j] = __uint_as_float(s[j]);
+#pragma unroll
+            for (int i = 4; i < PAT_KEYS; i++) mxs[i & 3] = fmaxf(mxs[i & 3], __uint_as_float(s[i]));
+            const float mx = fmaxf(fmaxf(mxs[0], mxs[1]), fmaxf(mxs[2], mxs[3])) * sl2;   // sl2 > 0
             // the maximum in use; the output is scaled when it falls behind by more than PAT_GROWTH
             float corr = 1.0f;
             if (mx > m_ref + PAT_GROWTH || m_ref == -INFINITY) {
@@ -164,7 +182,7 @@ prefill_attention_tiled_kernel(const float *__restrict__ q, const __grid_constan
             uint32_t ph[32], pl[32];
 #pragma unroll
             for (int i = 0; i < 32; i++) {
-                const float p0 = exp2f(s[2 * i] - m_use), p1 = exp2f(s[2 * i + 1] - m_use);
+                const float p0 = pat_exp2(fmaf(__uint_as_float(s[2 * i]), sl2, -m_use)), p1 = pat_exp2(fmaf(__uint_as_float(s[2 * i + 1]), sl2, -m_use));
                 sum[i & 3] += p0 + p1;
                 split_f16x2(p0, p1, ph[i], pl[i]);
             }
@@ -196,16 +214,21 @@ prefill_attention_tiled_kernel(const float *__restrict__ q, const __grid_constan
         if (ok) {
             pg_fence_after();
             const float inv = l_run > 0.f ? 1.0f / l_run : 0.f;
-            float *dst = out + ((size_t)min(qi, seq_len - 1) * num_heads + kv_h * group + r % group) * HD;
+            const size_t at = ((size_t)min(qi, seq_len - 1) * num_heads + kv_h * group + r % group) * HD;
 #pragma unroll 1
             for (int c = 0; c < 4; c++) {
                 uint32_t v[32];
                 pg_tmem_ld32(t_o + lanes + (uint32_t)c * 32u, v);
-                if (live) {
+                if (!live) continue;
+                auto o = [&](int i) { return __uint_as_float(v[i]) * inv; };
+                if (out_bf16) {
 #pragma unroll
-                    for (int i = 0; i < 32; i += 4)
-                        *reinterpret_cast<float4 *>(dst + c * 32 + i) =
-                            make_float4(__uint_as_float(v[i]) * inv, __uint_as_float(v[i + 1]) * inv, __uint_as_float(v[i + 2]) * inv, __uint_as_float(v[i + 3]) * inv);
+                    for (int i = 0; i < 32; i += 8)
+                        *reinterpret_cast<uint4 *>(out_bf16 + at + c * 32 + i) =
+                            make_uint4(pg_pack_bf16(o(i), o(i + 1)), pg_pack_bf16(o(i + 2), o(i + 3)), pg_pack_bf16(o(i + 4), o(i + 5)), pg_pack_bf16(o(i + 6), o(i + 7)));
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 32; i += 4) *reinterpret_cast<float4 *>(out + at + c * 32 + i) = make_float4(o(i), o(i + 1), o(i + 2), o(i + 3));
                 }
             }
         }
@@ -221,12 +244,12 @@ prefill_attention_tiled_kernel(const float *__restrict__ q, const __grid_constan
             if (pg_elect()) {
                 const uint32_t kt = ring + (it % PAT_SLOTS) * PAT_TILE_BYTES;
 #pragma unroll
-                for (int part = 0; part < 2; part++)   // hi, lo
+                for (int part = 1; part >= 0; part--)   // lo before hi: the accumulator truncates what it adds, and adds less often to full sums
 #pragma unroll
                     for (int p = 0; p < 2; p++) {
                         const uint64_t dq = pg_smem_desc(smem + (uint32_t)(2 * part + p) * PAT_PANEL), dk = pg_smem_desc(kt + (uint32_t)p * (PAT_KEYS * 128));
 #pragma unroll
-                        for (int k = 0; k < 4; k++) ps_mma(t_s, dq + 2u * k, dk + 2u * k, PAT_IDESC_S, (part | p | k) != 0);   // 16 dims, 32 bytes on
+                        for (int k = 0; k < 4; k++) ps_mma(t_s, dq + 2u * k, dk + 2u * k, PAT_IDESC_S, (1 - part) | p | k);   // 16 dims, 32 bytes on
                     }
                 pg_commit(&empty[it % PAT_SLOTS]);
                 pg_commit(s_full);

@@ -108,50 +108,53 @@ f32_to_bf16_kernel(const float *__restrict__ x, uint16_t *__restrict__ y, size_t
 
 // Residual add + RMSNorm of a batch of token rows, written straight as the bf16 token matrix of
 // the next matmul: x += t (when t is given; x is updated in place), then (x / rms) * w with the
-// f64 mean square of rnb-cpu's rms_norm_into (crates/rnb-cpu/src/kernels/norm.rs:177-196) in the
-// reduction order of rmsnorm_q8k_kernel, rounded once to bf16.  One CTA per token; hidden % 8 == 0.
+// f64 mean square of rnb-cpu's rms_norm_into (crates/rnb-cpu/src/kernels/norm.rs:177-196), rounded once to bf16.  One CTA per
+// token; hidden % 256 == 0.  A row of up to 16 elements per thread stays in registers between the sum and the output.
 template <int THREADS>
 RNB_GLOBAL void __launch_bounds__(THREADS)
 add_rmsnorm_bf16_kernel(float *__restrict__ x, const float *__restrict__ t, const float *__restrict__ w, float eps, int hidden,
                         uint16_t *__restrict__ out) {
+    constexpr int KEEP = 4;
     pdl_launch_dependents();
     pdl_wait();
     __shared__ double red[THREADS / 32];
-    __shared__ float s_rms;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    float *xs = x + (size_t)blockIdx.x * hidden;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n4 = hidden / 4;
+    float4 *xs = reinterpret_cast<float4 *>(x + (size_t)blockIdx.x * hidden);
+    const float4 *ts = t ? reinterpret_cast<const float4 *>(t + (size_t)blockIdx.x * hidden) : nullptr;
     double ss = 0.0;
-    if (t) {
-        const float *ts = t + (size_t)blockIdx.x * hidden;
-        for (int i = tid; i < hidden; i += THREADS) {
-            const float v = __fadd_rn(xs[i], ts[i]);
+    float4 keep[KEEP];
+    auto take = [&](int i) {
+        float4 v = xs[i];
+        if (ts) {
+            const float4 a = ts[i];
+            v = make_float4(__fadd_rn(v.x, a.x), __fadd_rn(v.y, a.y), __fadd_rn(v.z, a.z), __fadd_rn(v.w, a.w));
             xs[i] = v;
-            ss += (double)v * (double)v;
         }
-    } else {
-        for (int i = tid; i < hidden; i += THREADS) {
-            const double v = (double)xs[i];
-            ss += v * v;
-        }
-    }
+        ss += ((double)v.x * v.x + (double)v.y * v.y) + ((double)v.z * v.z + (double)v.w * v.w);
+        return v;
+    };
+#pragma unroll
+    for (int k = 0; k < KEEP; k++)
+        if (tid + k * THREADS < n4) keep[k] = take(tid + k * THREADS);
+    for (int i = tid + KEEP * THREADS; i < n4; i += THREADS) take(i);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
     if (lane == 0) red[warp] = ss;
-    __syncthreads();   // also orders this CTA's writes of xs before the reads below
-    if (tid == 0) {
-        double a = 0.0;
-        for (int i = 0; i < THREADS / 32; i++) a += red[i];
-        s_rms = (float)sqrt(a / (double)hidden + (double)eps);
-    }
     __syncthreads();
-    const float rms = s_rms;
-    uint16_t *os = out + (size_t)blockIdx.x * hidden;
-    for (int i = tid * 8; i < hidden; i += THREADS * 8) {
-        float v[8];
+    double a = 0.0;
+    for (int i = 0; i < THREADS / 32; i++) a += red[i];
+    const float rms = (float)sqrt(a / (double)hidden + (double)eps);
+    uint2 *os = reinterpret_cast<uint2 *>(out + (size_t)blockIdx.x * hidden);
+    const float4 *ws = reinterpret_cast<const float4 *>(w);
+    auto put = [&](int i, const float4 &v) {
+        const float4 g = ws[i];
+        os[i] = make_uint2(pg_pack_bf16(__fmul_rn(__fdiv_rn(v.x, rms), g.x), __fmul_rn(__fdiv_rn(v.y, rms), g.y)),
+                           pg_pack_bf16(__fmul_rn(__fdiv_rn(v.z, rms), g.z), __fmul_rn(__fdiv_rn(v.w, rms), g.w)));
+    };
 #pragma unroll
-        for (int j = 0; j < 8; j++) v[j] = __fmul_rn(__fdiv_rn(xs[i + j], rms), w[i + j]);
-        *reinterpret_cast<uint4 *>(os + i) = make_uint4(pg_pack_bf16(v[0], v[1]), pg_pack_bf16(v[2], v[3]), pg_pack_bf16(v[4], v[5]), pg_pack_bf16(v[6], v[7]));
-    }
+    for (int k = 0; k < KEEP; k++)
+        if (tid + k * THREADS < n4) put(tid + k * THREADS, keep[k]);
+    for (int i = tid + KEEP * THREADS; i < n4; i += THREADS) put(i, xs[i]);   // this thread's own stores
 }
 
 // silu(gate) * up (g / (1 + exp(-g)), crates/rnb-cpu/src/kernels/activation.rs:74-89, libm's expf as in
