@@ -13,7 +13,7 @@
 // probabilities are at most 2^8.  Two CTAs per SM (112 KB, 256 tensor-memory columns each: 64 scores, 128 outputs, 32 + 32
 // probabilities).  Long rows are scheduled first.  Every wait is bounded.
 //
-// What bounds it: the softmax warps (tensor pipe 25 % busy).  2048 tokens of 32 / 8 heads: 134 us cold (262 with mma.sync
+// What bounds it: the softmax warps (tensor pipe 31 % busy).  2048 tokens of 32 / 8 heads: 108 us cold (262 with mma.sync
 // and eight warps that shared a CTA); 203 tokens behind 1000 positions through 32 layers 10.2 -> 9.4 ms.
 #pragma once
 #include "attention.cuh"
@@ -80,9 +80,21 @@ __device__ __forceinline__ float pat_exp2(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+// packed f32: {x, y} * m + a, and sums; each half rounds as the single operation does
+__device__ __forceinline__ float2 pat_fma2(float x, float y, uint64_t m, uint64_t a) {
+    float2 r;
+    asm("{\n\t.reg .b64 t;\n\tmov.b64 t, {%2, %3};\n\tfma.rn.f32x2 t, t, %4, %5;\n\tmov.b64 {%0, %1}, t;\n\t}" : "=f"(r.x), "=f"(r.y) : "f"(x), "f"(y), "l"(m), "l"(a));
+    return r;
+}
+__device__ __forceinline__ void pat_add2(uint64_t &sum, float x, float y) {
+    asm("{\n\t.reg .b64 t;\n\tmov.b64 t, {%1, %2};\n\tadd.rn.f32x2 %0, %0, t;\n\t}" : "+l"(sum) : "f"(x), "f"(y));
+}
+__device__ __forceinline__ float pat_total(uint64_t a, uint64_t b) {
+    return (__uint_as_float((uint32_t)a) + __uint_as_float((uint32_t)(a >> 32))) + (__uint_as_float((uint32_t)b) + __uint_as_float((uint32_t)(b >> 32)));
+}
 __device__ __forceinline__ void pat_tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// grid = (ceil(seq_len / (128 / group)), num_kv_heads); group = num_heads / num_kv_heads a power of two up to 128; scale > 0.
+// grid = (num_kv_heads, ceil(seq_len / (128 / group))): the long rows of every head come first; group = num_heads / num_kv_heads a power of two up to 128; scale > 0.
 // out_bf16 (may be null): the result rounded to bf16 there instead of f32 in `out`.
 RNB_GLOBAL void __launch_bounds__(PAT_THREADS, 2)
 prefill_attention_tiled_kernel(const float *__restrict__ q, const __grid_constant__ PatMaps maps, int seq_len, int kv_len, int num_heads, int num_kv_heads,
@@ -97,7 +109,7 @@ prefill_attention_tiled_kernel(const float *__restrict__ q, const __grid_constan
     volatile int *const s_failed = reinterpret_cast<volatile int *>(bars + 12);
     const uint32_t smem = smem_u32(pat_smem);
     const int group = num_heads / num_kv_heads, qpc = PAT_ROWS / group;
-    const int kv_h = blockIdx.y, i0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * qpc;   // long rows first
+    const int kv_h = blockIdx.x, i0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * qpc;   // long rows first
     const int shift = kv_len - seq_len;                                              // query i sits at position shift + i
     const int n_keys = min(kv_len, shift + min(i0 + qpc, seq_len));                  // keys visible to the CTA's last query
     const int n_tiles = (n_keys + PAT_KEYS - 1) / PAT_KEYS;
@@ -178,15 +190,17 @@ prefill_attention_tiled_kernel(const float *__restrict__ q, const __grid_constan
                 m_ref = m_new;
             }
             const float m_use = m_ref == -INFINITY ? 0.f : m_ref;   // a fully masked row so far: keep everything at zero
-            float sum[4] = {0.f, 0.f, 0.f, 0.f};
+            const uint64_t sl22 = pg_pair_f32(sl2, sl2), nm2 = pg_pair_f32(-m_use, -m_use);
+            uint64_t sum[2] = {0, 0};
             uint32_t ph[32], pl[32];
 #pragma unroll
             for (int i = 0; i < 32; i++) {
-                const float p0 = pat_exp2(fmaf(__uint_as_float(s[2 * i]), sl2, -m_use)), p1 = pat_exp2(fmaf(__uint_as_float(s[2 * i + 1]), sl2, -m_use));
-                sum[i & 3] += p0 + p1;
+                const float2 x = pat_fma2(__uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1]), sl22, nm2);
+                const float p0 = pat_exp2(x.x), p1 = pat_exp2(x.y);
+                pat_add2(sum[i & 1], p0, p1);
                 split_f16x2(p0, p1, ph[i], pl[i]);
             }
-            l_run = l_run * corr + ((sum[0] + sum[1]) + (sum[2] + sum[3]));
+            l_run = fmaf(l_run, corr, pat_total(sum[0], sum[1]));
             if (t > 0) {
                 ok = __all_sync(0xffffffffu, mbar_wait_bounded(pv_done, (uint32_t)((t - 1) & 1)));   // the probabilities' columns are free, the output stands
                 if (!ok) break;
