@@ -8,6 +8,7 @@
 
 #include "delta_rule.cuh"
 #include "dense.cuh"
+#include "causal_attention_tc.cuh"
 #include "latent_attention.cuh"
 #include "launch.hpp"
 #include "layer_glue.cuh"
@@ -655,7 +656,7 @@ int LayerStack::ready(cudaStream_t s) {
     const void *fns[] = {(const void *)residual_norm_kernel<float, 4>, (const void *)residual_norm_kernel<float, 1>, (const void *)residual_norm_kernel<bf16, 4>,
                          (const void *)residual_norm_kernel<bf16, 1>, (const void *)dense_gemm_pair_kernel, (const void *)dense_gemm_split_kernel, (const void *)decay_rows_kernel,
                          (const void *)linear_state_step_kernel<4>, (const void *)linear_state_step_kernel<8>, (const void *)linear_state_step_kernel<16>,
-                         (const void *)linear_state_step_kernel<32>, (const void *)linear_state_step_kernel<64>, (const void *)causal_attention_kernel<4>,
+                         (const void *)linear_state_step_kernel<32>, (const void *)linear_state_step_kernel<64>, (const void *)causal_attention_tc_kernel<2>, (const void *)causal_attention_tc_kernel<3>, (const void *)causal_attention_kernel<4>,
                          (const void *)causal_attention_kernel<8>, (const void *)causal_attention_kernel<16>, (const void *)causal_attention_kernel<32>,
                          (const void *)attention_step_kernel<float, float>, (const void *)attention_step_kernel<float, bf16>, (const void *)attention_step_kernel<bf16, bf16>,
                          (const void *)delta_prepare_kernel<0>, (const void *)delta_prepare_kernel<2>,
@@ -964,7 +965,7 @@ static int launch_linear(cudaStream_t s, const LinearChunkArgs &a, bool narrow, 
     return launch_linear_tiles<16, MODE>(s, a);
 }
 
-static int launch_causal_attention(cudaStream_t s, const CausalAttentionArgs &a);
+static int launch_causal_attention(cudaStream_t s, const CausalAttentionArgs &a, int pos_host, int *err);
 
 // Norm and gate of a mixer's heads in b.o; the result is its part of the output matrix's input.
 int LayerStack::head_norm_gate(cudaStream_t s, int n, StackScratch &b, const StackLayer &L, const StackMixer &M, const void *g, int ldg) {
@@ -1083,7 +1084,7 @@ WindowAttentionArgs LayerStack::attention_args(int n, StackScratch &b, StackLaye
     return a;
 }
 
-int LayerStack::mixer_attention(cudaStream_t s, int n, StackScratch &b, StackLayer &L, int i, MixerState &R, const int *pos_dev) {
+int LayerStack::mixer_attention(cudaStream_t s, int n, StackScratch &b, StackLayer &L, int i, MixerState &R, const int *pos_dev, int pos_host, int *err) {
     const rnb_b200_mixer_cfg &m = L.mixers[i].c;
     const bool nb = narrow(n);
     const WindowAttentionArgs a = attention_args(n, b, L, i, R, pos_dev);
@@ -1114,7 +1115,7 @@ int LayerStack::mixer_attention(cudaStream_t s, int n, StackScratch &b, StackLay
     c.tokens = n, c.heads = m.heads, c.group = m.heads / m.kv_heads, c.dim = m.dim, c.vdim = m.vdim;
     c.ring = a.ring, c.window = m.window, c.lda = a.lda, c.ldg = a.ldg;
     c.vec = m.dim % 8 == 0 && m.vdim % 8 == 0;
-    return launch_causal_attention(s, c);
+    return launch_causal_attention(s, c, pos_host, err);
 }
 
 DeltaArgs LayerStack::delta_args(int n, StackScratch &b, StackLayer &L, int i, MixerState &R, const int *pos_dev) const {
@@ -1173,7 +1174,25 @@ int LayerStack::mixer_delta(cudaStream_t s, int n, StackScratch &b, StackLayer &
     return head_norm_gate(s, n, b, L, M, (const char *)b.p[i] + (size_t)a.g_at * (nb ? 2 : 4), M.in_rows);
 }
 
-static int launch_causal_attention(cudaStream_t s, const CausalAttentionArgs &a) {
+// The tensor-memory form takes keys of two or three panels of 64, values of 128, rows on 16-byte boundaries and a ring that has not
+// wrapped (positions are rows); a scale of zero or less (its maxima are of unscaled scores) and everything else stay on mma.sync.
+static int launch_causal_attention(cudaStream_t s, const CausalAttentionArgs &a, int pos_host, int *err) {
+    const int dk = a.dim + a.dim2, kv_len = pos_host + a.tokens, kv_heads = a.heads / a.group;
+    const size_t pitches = a.ldq | a.ldk | a.ldk2 | a.ldv | (size_t)a.lda;
+    if (a.dim % 64 == 0 && a.dim2 % 64 == 0 && (dk == 128 || dk == 192) && a.vdim == 128 && a.scale > 0.f && kv_len <= a.ring && pitches % 8 == 0 &&
+        ((((uintptr_t)a.q | (uintptr_t)a.k | (uintptr_t)a.k2 | (uintptr_t)a.v | (uintptr_t)a.act) & 15u) == 0)) {
+        CausalAttentionMaps m;
+        memset(&m, 0, sizeof(m));
+        auto bits = [](const bf16 *x) { return reinterpret_cast<const uint16_t *>(x); };
+        RNB_TRY(encode_token_map(&m.q, bits(a.q), (size_t)a.tokens, (size_t)a.heads * dk, a.ldq, CA_ROWS));
+        RNB_TRY(encode_token_map(&m.k, bits(a.k), (size_t)kv_len, (size_t)kv_heads * a.dim, a.ldk, CA_KEYS));
+        if (a.dim2) RNB_TRY(encode_token_map(&m.k2, bits(a.k2), (size_t)kv_len, (size_t)a.dim2, a.ldk2, CA_KEYS));
+        RNB_TRY(encode_token_map(&m.v, bits(a.v), (size_t)kv_len, (size_t)kv_heads * a.vdim, a.ldv, CA_KEYS));
+        const dim3 grid((unsigned)a.heads, (unsigned)((a.tokens + CA_ROWS - 1) / CA_ROWS));
+        if (dk == 128) RNB_CU(launch_k(causal_attention_tc_kernel<2>, grid, dim3(PAT_THREADS), ct_smem(2), s, a, m, pos_host, err));
+        else RNB_CU(launch_k(causal_attention_tc_kernel<3>, grid, dim3(PAT_THREADS), ct_smem(3), s, a, m, pos_host, err));
+        return RNB_B200_OK;
+    }
     const dim3 grid((unsigned)((a.tokens + CA_ROWS - 1) / CA_ROWS), (unsigned)a.heads), block(CA_THREADS);
     const size_t smem = causal_attention_smem(a.dim + a.dim2, a.vdim);
     switch (causal_attention_vcols(a.vdim)) {
@@ -1283,13 +1302,13 @@ int LayerStack::mixer_latent(cudaStream_t s, int n, StackScratch &b, StackLayer 
     a.ldq = (size_t)m.heads * (m.dim + m.rot_dim), a.ldk = (size_t)m.heads * m.dim, a.ldk2 = (size_t)d.ld, a.ldv = (size_t)m.heads * m.vdim;
     a.tokens = n, a.heads = m.heads, a.group = 1, a.dim = m.dim, a.dim2 = m.rot_dim, a.vdim = m.vdim, a.ring = cfg.max_ctx, a.lda = L.out_cols;
     a.vec = m.dim % 8 == 0 && m.rot_dim % 8 == 0 && m.vdim % 8 == 0 && m.kv_rank % 8 == 0;
-    return launch_causal_attention(s, a);
+    return launch_causal_attention(s, a, pos_host, err);
 }
 
 int LayerStack::run_mixer(cudaStream_t s, int n, StackScratch &b, StackLayer &L, int i, MixerState &R, const int *pos_dev, int pos_host, int *err) {
     switch (L.mixers[i].c.mixer) {
     case RNB_B200_MIXER_LATENT_ATTENTION: return mixer_latent(s, n, b, L, i, R, pos_dev, pos_host, err);
-    case RNB_B200_MIXER_ATTENTION: return mixer_attention(s, n, b, L, i, R, pos_dev);
+    case RNB_B200_MIXER_ATTENTION: return mixer_attention(s, n, b, L, i, R, pos_dev, pos_host, err);
     case RNB_B200_MIXER_DELTA: return mixer_delta(s, n, b, L, i, R, pos_dev, err);
     default: return mixer_linear(s, n, b, L, i, R, pos_dev, err);
     }

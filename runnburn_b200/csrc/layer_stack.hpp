@@ -131,7 +131,7 @@ private:
     int run_mixer(cudaStream_t s, int n, StackScratch &b, StackLayer &L, int i, MixerState &R, const int *pos_dev, int pos_host, int *err);
     int mixer_linear(cudaStream_t s, int n, StackScratch &b, StackLayer &L, int i, MixerState &R, const int *pos_dev, int *err);
     int mixer_latent(cudaStream_t s, int n, StackScratch &b, StackLayer &L, int i, MixerState &R, const int *pos_dev, int pos_host, int *err);
-    int mixer_attention(cudaStream_t s, int n, StackScratch &b, StackLayer &L, int i, MixerState &R, const int *pos_dev);
+    int mixer_attention(cudaStream_t s, int n, StackScratch &b, StackLayer &L, int i, MixerState &R, const int *pos_dev, int pos_host, int *err);
     WindowAttentionArgs attention_args(int n, StackScratch &b, StackLayer &L, int i, MixerState &R, const int *pos_dev) const;
     DeltaArgs delta_args(int n, StackScratch &b, StackLayer &L, int i, MixerState &R, const int *pos_dev) const;
     int mixers_attention_delta(cudaStream_t s, int n, StackScratch &b, StackLayer &L, LayerRun &R, const int *pos_dev);

@@ -43,3 +43,23 @@ def test_prefill_attention(ops, heads, kvh, seq, kv_len, shape):
     want = reference(q, k, v, scale)
     assert ops.dev_error_flag() == 0
     assert np.max(np.abs(np.asarray(got).reshape(want.shape) - want)) <= 1e-4 * np.max(np.abs(want))
+
+
+@pytest.mark.parametrize("cuts", [[9], [63, 64, 65], [128, 129], [300]])
+@pytest.mark.parametrize("kind", ["window", "wide window", "one group", "latent", "latent 64 + 64"])
+def test_prompt_attention_of_mixed_stacks(kind, cuts):
+    """Keys of 128 and 192 elements and values of 128 in bf16 stacks: portions that start anywhere, windows that reach part of
+    a tile, heads that share keys; the bound of the stack tests."""
+    import stack_util as su
+    from hybrid_ref import Model
+    if "latent" in kind:
+        size = dict(dim=64, rot_dim=64) if "+" in kind else dict(dim=128, rot_dim=64)
+        cfg = su.config([su.latent(heads=2, vdim=128, kv_rank=128, **size)], width=256)
+    else:
+        left = su.window(heads=4, kv_heads=4 if kind == "one group" else 2, dim=128, vdim=128, size=1000 if kind == "wide window" else 70, scale=128 ** -0.5)
+        cfg = su.dutivik([su.parallel(left, su.delta(heads=2, kv_heads=1, dim=32, vdim=32))], width=256)
+    w, toks = su.weights(cfg, seed=len(kind), rank=16), su.tokens(cfg, 333 if cuts != [9] else 45, seed=1)
+    dec = su.decoder(cfg, w, "bfloat16", max_ctx=512)
+    got = su.feed(dec, toks, cuts)
+    dec.close()
+    assert not (why := su.bad(got, Model(cfg, w).forward(toks), "bfloat16")), why
