@@ -1,0 +1,25 @@
+// Control flow around waits that may give up, apart from the kernels that use it so that it also compiles for the host.
+#pragma once
+
+#ifdef __CUDACC__
+#define RNB_WALK __device__ __forceinline__
+#else
+#define RNB_WALK inline
+#endif
+
+namespace rnb {
+
+// The tiles first, first + step, ... below `tiles`, taken in turn by warps that meet at barriers inside `body`.  `wait(i)` waits
+// for the i-th of them with a limit and may give up in one warp while it succeeds in another; `agree` makes the outcome
+// common (true if all warps pass true), so that nobody goes on to a barrier that another warp has left.  False: some warp gave up.
+template <class Wait, class Agree, class Body>
+RNB_WALK bool walk_tiles(int first, int step, int tiles, Wait &&wait, Agree &&agree, Body &&body) {
+    int count = 0;
+    for (int tile = first; tile < tiles; tile += step, count++) {
+        if (!agree(wait(count))) return false;
+        body(tile);
+    }
+    return true;
+}
+
+}  // namespace rnb

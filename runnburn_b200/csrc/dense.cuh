@@ -12,6 +12,7 @@
 #pragma once
 #include <cuda_bf16.h>
 
+#include "bounded_walk.hpp"
 #include "common.cuh"
 #include "prefill_gemm.cuh"
 #include "prefill_gemm_pair.cuh"
@@ -193,6 +194,15 @@ struct DenseMaps {   // per job: tokens, weights, second weights
     PgTensorMap x[DENSE_MAX_JOBS], w[DENSE_MAX_JOBS], w2[DENSE_MAX_JOBS];
 };
 
+// true if all 128 threads of the named barrier bring true
+__device__ __forceinline__ bool dq_agree(int barrier, bool v) {
+    uint32_t all;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\tbarrier.cta.red.and.pred q, %2, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                 : "=r"(all)
+                 : "r"((uint32_t)v), "r"(barrier)
+                 : "memory");
+    return all != 0;
+}
 template <class OT>
 __device__ __forceinline__ void dg_store(void *y, size_t idx, float v) { reinterpret_cast<OT *>(y)[idx] = from_f32<OT>(v); }
 
@@ -321,24 +331,24 @@ dense_gemm_pair_kernel(const __grid_constant__ DenseGemmJobs jobs, const __grid_
         float *const ex = reinterpret_cast<float *>(smem + (size_t)DQ_STAGES * DQ_STAGE_BYTES + (size_t)part * (DQ_EXCHANGE / 2));
         const uint32_t at = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(part * 256);
         pdl_wait();   // stores come after the launches before this one
-        int count = 0, turn = 0;
-        for (int tile = pair0; tile < P.tiles && ok; tile += n_pairs, count++) {
+        int turn = 0;
+        auto landed = [&](int count) { return __all_sync(0xffffffffu, mbar_wait_bounded(&acc_full, (uint32_t)(count & 1))) != 0; };
+        ok = walk_tiles(pair0, n_pairs, P.tiles, landed, [&](bool v) { return dq_agree(1 + part, v); }, [&](int tile) {
             const DenseGemmJob &job = jobs.j[job_of(tile)];
             const int n0 = first_row(tile, job), m0 = (tile % P.token_tiles) * nt + part * P.n1, rows = job.rows;
-            ok = __all_sync(0xffffffffu, mbar_wait_bounded(&acc_full, (uint32_t)(count & 1)));
             pg_fence_after();
-            if (job.pair)   // every warp of the part takes part in the exchange, whatever its own wait returned
+            if (job.pair)
                 for (int c = 0; c < cols && m0 + c < jobs.seq; c += 16, turn ^= 1) {
                     // gate rows on lanes 0-63, the same rows of up on lanes 64-127: a warp hands eight of 16 tokens to its partner
                     uint32_t v[16];
-                    if (ok) ps_tmem_ld<16>(at + (uint32_t)c, v);
+                    ps_tmem_ld<16>(at + (uint32_t)c, v);
                     const bool up = q >= 2;
                     float *buf = ex + turn * (4 * 8 * 32);
 #pragma unroll
-                    for (int i = 0; i < 8; i++) buf[((q ^ 2) * 8 + i) * 32 + lane] = ok ? __uint_as_float(up ? v[i] : v[8 + i]) : 0.f;
+                    for (int i = 0; i < 8; i++) buf[((q ^ 2) * 8 + i) * 32 + lane] = __uint_as_float(up ? v[i] : v[8 + i]);
                     asm volatile("bar.sync %0, 128;" ::"r"(1 + part) : "memory");
                     const int row = n0 + (q & 1) * 32 + lane;
-                    if (ok && row < rows) {
+                    if (row < rows) {
 #pragma unroll
                         for (int i = 0; i < 8; i++) {
                             const int tok = m0 + c + i + (up ? 8 : 0);
@@ -351,7 +361,7 @@ dense_gemm_pair_kernel(const __grid_constant__ DenseGemmJobs jobs, const __grid_
                         }
                     }
                 }
-            else if (ok) {
+            else {
                 const int row = n0 + q * 32 + lane;
                 const float b = job.decay_bias && row < rows ? job.decay_bias[row] : 0.f;
                 for (int c = 0; c < cols && m0 + c < jobs.seq; c += 32) {
@@ -380,7 +390,7 @@ dense_gemm_pair_kernel(const __grid_constant__ DenseGemmJobs jobs, const __grid_
             pg_fence_before();
             __syncwarp();
             if (lane == 0) pt_arrive(ps_map(smem_u32(&acc_free[part]), 0));
-        }
+        });
     }
     if (!ok) s_failed = 1;
     __syncwarp();
