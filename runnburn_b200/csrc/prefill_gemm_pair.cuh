@@ -13,8 +13,10 @@
 // Persistent: a pair walks its tiles (token tiles fastest, so that a weight row crosses DRAM once).  Warps 0-15
 // dequantise, two groups of eight that take two of a block's four stages each; behind the first stage of the next tile
 // they write the finished tile from tensor memory and hand the columns back.  Warp 16 of the even CTA issues the MMAs,
-// warp 17 of each CTA its token copies, which count on the even CTA's barrier, warp 18 those of the weights.  A commit reaches both CTAs.  Every
-// wait is bounded; after a timeout all threads still meet at the cluster barrier.
+// warp 17 of each CTA its token copies, warp 18 those of the weights.  A stage fills on each CTA's own barrier; warp 16 of
+// the odd CTA waits for its own and passes one arrival on to the even CTA's, so that the release and the acquire across the
+// cluster stand between what the odd CTA wrote and the MMA that reads it and cost no dequantising warp anything.
+// A commit reaches both CTAs.  Every wait is bounded; after a timeout all threads still meet at the cluster barrier.
 //
 // What bounds it: the dequantising warps and the tensor pipe, about even at 450 tokens a tile.  Measured with 2048 / 512
 // tokens, us (512-token tiles of a CTA by itself before): gate + up 28672 x 4096 370 / 108 (464 / 132), down 4096 x 14336
@@ -44,12 +46,9 @@ struct PtMaps {   // tokens of the two parts (boxes of n1 / 2 and n2 / 2), block
     PgTensorMap xa, xb, w[PG_MAX_JOBS], w2;
 };
 
-// An arrival at the other CTA's barrier that hands over operand tiles only: pg_proxy_fence has put the writer's stores where
-// the tensor pipe of its own SM reads them, and no thread of the other CTA reads them.  The release across the cluster, which
-// the hand-over of tensor memory below keeps, costs 1200 cycles.
-__device__ __forceinline__ void pt_arrive_tile(uint32_t cluster_addr) { asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory"); }
+// An arrival at the other CTA's barrier, and a wait for one: they order what either CTA did before it.
 __device__ __forceinline__ void pt_arrive(uint32_t cluster_addr) { asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory"); }
-__device__ __forceinline__ bool pt_wait(uint64_t *bar, uint32_t parity) {   // orders what the other CTA did before it arrived
+__device__ __forceinline__ bool pt_wait(uint64_t *bar, uint32_t parity) {
     for (uint32_t i = 0; i < (1u << 22); i++) {
         uint32_t done;
         asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
@@ -96,8 +95,8 @@ prefill_gemm_pair_kernel(const __grid_constant__ PgJobs jobs, const __grid_const
     const uint32_t tok_bytes = (uint32_t)(nt / 2) * 128u, stage_bytes = tok_bytes + PG_B_BYTES;
     if (tid == 0) {
         for (int s = 0; s < PT_STAGES; s++) {
-            mbar_init(&full[s], 2 * (PT_WORKERS / 2) + 1);   // the warps of a group in both CTAs + the thread that announces the token copies
-            mbar_init(&empty[s], 1);                         // tcgen05.commit
+            mbar_init(&full[s], PT_WORKERS / 2 + 1 + (rank == 0));   // the warps of a group + the thread that announces the token copies + the odd CTA
+            mbar_init(&empty[s], 1);                                 // tcgen05.commit
         }
         mbar_init(&raw_full, 1);
         mbar_init(&raw_empty, PT_WORKERS);
@@ -130,12 +129,12 @@ prefill_gemm_pair_kernel(const __grid_constant__ PgJobs jobs, const __grid_const
         const int grp = warp >> 3, row = (tid & 255) >> 1, h = tid & 1, rr = row & 7;
         uint8_t *const brow = smem + tok_bytes + (row >> 3) * 1024 + rr * 128;
         uint32_t uses = 0, raws = 0;   // blocks that have gone through the ring of stages, of raw blocks
-        // a stage: wait for its slot (warp-uniform: shuffles follow), then tell the even CTA
+        // a stage: wait for its slot (warp-uniform: shuffles follow), then hand it over
         auto begin = [&](int i) { return __all_sync(0xffffffffu, mbar_wait_bounded(&empty[2 * grp + i], (uses & 1u) ^ 1u)); };
         auto end = [&](int i) {
             pg_proxy_fence();
             __syncwarp();
-            if (lane == 0) pt_arrive_tile(ps_map(smem_u32(&full[2 * grp + i]), 0));
+            if (lane == 0) pg_arrive(&full[2 * grp + i]);
         };
         uint8_t *const dst[2] = {brow + (uint32_t)(2 * grp) * stage_bytes, brow + (uint32_t)(2 * grp + 1) * stage_bytes};
         // tile `tile`, the pair's `count`-th: tensor memory lane = weight row, a warp takes every fourth group of 32 tokens
@@ -256,7 +255,7 @@ prefill_gemm_pair_kernel(const __grid_constant__ PgJobs jobs, const __grid_const
             for (int tile = pair0; tile < P.tiles && ok; tile += n_pairs, count++) {
                 if (count > 0) ok = __all_sync(0xffffffffu, pt_wait(&acc_free, (uint32_t)((count - 1) & 1)));
                 for (int kt = 0; kt < 4 * nb && ok; kt++) {
-                    ok = __all_sync(0xffffffffu, mbar_wait_bounded(&full[s], phase));
+                    ok = __all_sync(0xffffffffu, pt_wait(&full[s], phase));
                     if (!ok) break;
                     pg_fence_after();
                     if (pg_elect()) {
@@ -274,6 +273,14 @@ prefill_gemm_pair_kernel(const __grid_constant__ PgJobs jobs, const __grid_const
                 if (ok && pg_elect()) pt_commit(&acc_full);
                 __syncwarp();
             }
+        } else if (lane == 0) {
+            uint32_t st = 0;
+            for (int tile = pair0; tile < P.tiles && ok; tile += n_pairs)
+                for (int kt = 0; kt < 4 * nb && ok; kt++, st++) {
+                    const uint32_t s = st % PT_STAGES;
+                    ok = mbar_wait_bounded(&full[s], (st / PT_STAGES) & 1u);
+                    if (ok) pt_arrive(ps_map(smem_u32(&full[s]), 0));
+                }
         }
     } else if (warp == PT_WORKERS + 1) {
         if (lane == 0) {
@@ -285,15 +292,15 @@ prefill_gemm_pair_kernel(const __grid_constant__ PgJobs jobs, const __grid_const
                     const uint32_t s = st % PT_STAGES;
                     ok = mbar_wait_bounded(&empty[s], ((st / PT_STAGES) & 1u) ^ 1u);
                     if (!ok) break;
-                    const uint32_t to = smem_u32(smem + s * stage_bytes), bar = ps_map(smem_u32(&full[s]), 0);
-                    if (rank == 0) mbar_arrive_expect_tx(&full[s], 2 * tok_bytes);   // both CTAs' copies
-                    pt_tma_2d(to, &maps.xa, kt * PG_K, m0 + rank * (P.n1 / 2), bar);
-                    pt_tma_2d(to + (uint32_t)(P.n1 / 2) * 128u, &maps.xb, kt * PG_K, m0 + P.n1 + rank * (P.n2 / 2), bar);
+                    const uint32_t to = smem_u32(smem + s * stage_bytes);
+                    mbar_arrive_expect_tx(&full[s], tok_bytes);
+                    pg_tma_2d(to, &maps.xa, kt * PG_K, m0 + rank * (P.n1 / 2), &full[s]);
+                    pg_tma_2d(to + (uint32_t)(P.n1 / 2) * 128u, &maps.xb, kt * PG_K, m0 + P.n1 + rank * (P.n2 / 2), &full[s]);
                     st++;
                 }
             }
             // after a failure the copies that were announced must land before the CTAs may leave
-            if (!ok && rank == 0)
+            if (!ok)
                 for (uint32_t i = st > PT_STAGES ? st - PT_STAGES : 0; i < st; i++) mbar_wait_bounded(&full[i % PT_STAGES], (i / PT_STAGES) & 1u);
         }
     } else if (lane == 0) {

@@ -84,3 +84,30 @@ def test_long_prompt_gate_up(ops, t, rows, cols, seq):
     assert ops.dev_error_flag() == 0
     got = act.float().cpu().numpy().astype(np.float64)
     assert np.max(np.abs(got - ref) - 2.0 ** -8 * np.abs(ref)) <= 1e-4 * np.max(np.abs(ref))
+
+
+@pytest.mark.parametrize("t,rows,cols,seq", [(Q4_K, 512, 14336, 512), (Q6_K, 512, 14336, 1000), (Q4_K, 20000, 1024, 600)])
+def test_long_prompt_matmul_repeats_its_bits(ops, t, rows, cols, seq):
+    """Weight tiles of one CTA are read by MMAs that the other issues: 200 launches that give the same bits as the first,
+    many stages deep and over several tiles per pair, the weights being the same and the tokens different from launch to
+    launch, so that a stale tile would show."""
+    import torch
+
+    import runnburn_b200 as r
+    rng = np.random.default_rng(cols + seq)
+    w = torch.from_numpy(random_blocks(rng, t, rows, cols)).cuda()
+    xs = [torch.randn(seq, cols, device="cuda", generator=torch.Generator("cuda").manual_seed(i)) for i in range(2)]
+    xb = torch.empty(seq * cols, dtype=torch.int16, device="cuda")
+    ys = [torch.empty(seq, rows, device="cuda") for _ in range(2)]
+    want = []
+    for i in range(200):
+        x, y = xs[i & 1], ys[i & 1]
+        assert r.load().rnb_b200_dev_prefill_gemm_multi(
+            1, (ctypes.c_int * 1)(t), (ctypes.c_void_p * 1)(w.data_ptr()), (ctypes.c_size_t * 1)(rows), (ctypes.c_void_p * 1)(y.data_ptr()), cols, x.data_ptr(), seq,
+            xb.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+        if i < 2:
+            want.append(y.clone())
+        else:
+            assert torch.equal(y, want[i & 1]), i
+    torch.cuda.synchronize()
+    assert ops.dev_error_flag() == 0
