@@ -22,4 +22,12 @@ RNB_WALK bool walk_tiles(int first, int step, int tiles, Wait &&wait, Agree &&ag
     return true;
 }
 
+// What a thread that fills a ring of `ring` slots does before it leaves, whatever came of its own waits: it waits for the last
+// fill of every slot (wait(slot, parity)), so that no copy is still under way when the memory is used for something else or given
+// back.  Another role may have given up although this one has not.
+template <class Wait>
+RNB_WALK void drain_ring(unsigned issued, unsigned ring, Wait &&wait) {
+    for (unsigned i = issued > ring ? issued - ring : 0; i < issued; i++) wait(i % ring, (i / ring) & 1u);
+}
+
 }  // namespace rnb

@@ -218,11 +218,9 @@ causal_attention_tc_kernel(const __grid_constant__ CausalAttentionArgs a, const 
             for (int p = 0; p < 2; p++) pg_tma_2d(v_at + (uint32_t)(t % NV) * CT_V_BYTES + (uint32_t)p * CT_PANEL_K, &maps.v, hk * 128 + 64 * p, (t_first + t) * CA_KEYS, bar);
             nv++;
         }
-        if (!ok) {   // the copies that were announced must land before the CTA may leave
-            mbar_wait_bounded(q_full, 0u);
-            for (int i = max(0, nk - 2); i < nk; i++) mbar_wait_bounded(&kfull[i & 1], (uint32_t)((i >> 1) & 1));
-            for (int i = max(0, nv - NV); i < nv; i++) mbar_wait_bounded(&vfull[i % NV], (uint32_t)((i / NV) & 1));
-        }
+        pg_drain(q_full, 1, 1);
+        pg_drain(kfull, (uint32_t)nk, 2);
+        pg_drain(vfull, (uint32_t)nv, NV);
     }
     if (!ok) *s_failed = 1;
     __syncwarp();

@@ -229,6 +229,7 @@ dense_gemm_pair_kernel(const __grid_constant__ DenseGemmJobs jobs, const __grid_
     __shared__ __align__(8) uint64_t full[DQ_STAGES], empty[DQ_STAGES], acc_full, acc_free[2];
     __shared__ uint32_t tmem_slot;
     __shared__ int s_failed;
+    __shared__ uint32_t s_issued[2];   // of the even CTA: stages that either CTA has asked for
     pdl_launch_dependents();
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(dg_smem_raw) + 1023) & ~(uintptr_t)1023);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -293,9 +294,7 @@ dense_gemm_pair_kernel(const __grid_constant__ DenseGemmJobs jobs, const __grid_
                     pt_tma_2d(dst + (uint32_t)(P.n1 / 2) * 128u, &maps.x2[js], kt * DG_K, m0 + P.n1 + rank * (P.n2 / 2), bar);
                 }
             }
-            // after a failure the copies that were announced must land before the CTAs may leave
-            if (!ok && rank == 0)
-                for (uint32_t i = it > DQ_STAGES ? it - DQ_STAGES : 0; i < it; i++) mbar_wait_bounded(&full[i % DQ_STAGES], (i / DQ_STAGES) & 1u);
+            ps_st_remote(ps_map(smem_u32(&s_issued[rank]), 0), it);
         }
     } else if (warp == 1) {
         if (rank == 0) {
@@ -397,6 +396,17 @@ dense_gemm_pair_kernel(const __grid_constant__ DenseGemmJobs jobs, const __grid_
     pg_fence_before();
     __syncthreads();
     ps_cluster_sync();   // the other CTA's memory and barriers are no longer used
+    if (s_failed) {
+        // A CTA that has read its last accumulators knows that all copies have landed.  One that gave up does not: both CTAs' copies count
+        // on the even CTA's barriers, and what the odd one asked for beyond the even one's last stage is announced here.  The
+        // odd CTA stays for it if it has given up too.
+        if (rank == 0 && tid == 0) {
+            for (uint32_t i = s_issued[0]; i < s_issued[1]; i++) mbar_arrive_expect_tx(&full[i % DQ_STAGES], stage_bytes);
+            pg_drain(full, max(s_issued[0], s_issued[1]), DQ_STAGES);
+        }
+        __syncthreads();
+        ps_cluster_sync();
+    }
     if (warp == 1) {
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
         if (lane == 0 && s_failed && err_flag) atomicExch(err_flag, DEV_ERR_GEMM_TIMEOUT);
@@ -470,8 +480,7 @@ dense_gemm_split_kernel(const __grid_constant__ DenseGemmJobs jobs, const __grid
                 pg_tma_2d(smem_u32(smem + (uint32_t)s * stage_bytes), &maps.x[js], (k0 + kt) * DG_K, m0, &full[s]);
                 issued = kt + 1;
             }
-            // after a failure the copies that were announced must land before the stages are reused
-            for (int kt = max(0, issued - S); kt < issued && !ok; kt++) mbar_wait_bounded(&full[kt % S], (uint32_t)((kt / S) & 1));
+            pg_drain(full, (uint32_t)issued, (uint32_t)S);   // the stages are reused
         }
     } else if (warp == 1) {
         pdl_wait();   // tensor memory is asked for when no earlier launch can still hold it

@@ -312,8 +312,7 @@ prefill_attention_tiled_kernel(const float *__restrict__ q, const __grid_constan
             if (t + 1 < n_tiles) copy(&maps.k, t + 1);
             copy(&maps.v, t);
         }
-        // after a failure the copies that were announced must land before the CTA may leave
-        for (uint32_t i = it > PAT_SLOTS ? it - PAT_SLOTS : 0; i < it && !ok; i++) mbar_wait_bounded(&full[i % PAT_SLOTS], (i / PAT_SLOTS) & 1u);
+        pg_drain(full, it, PAT_SLOTS);
     }
     if (!ok) *s_failed = 1;
     __syncwarp();

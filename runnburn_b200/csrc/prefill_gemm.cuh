@@ -19,6 +19,7 @@
 
 #include <type_traits>
 
+#include "bounded_walk.hpp"
 #include "common.cuh"
 
 namespace rnb {
@@ -47,6 +48,14 @@ __device__ __forceinline__ void pg_fence_after() { asm volatile("tcgen05.fence::
 __device__ __forceinline__ void pg_proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void pg_arrive(uint64_t *bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+// The copies that a producer announced on a ring of barriers have landed (bounded, as every wait).
+__device__ __forceinline__ void pg_drain(uint64_t *full, uint32_t issued, uint32_t ring) {
+    drain_ring(issued, ring, [&](uint32_t slot, uint32_t parity) {
+        for (uint32_t k = 0; k < (1u << 18) && !mbar_try_wait(&full[slot], parity); k++) {
+            if (k > 64) __nanosleep(64);
+        }
+    });
 }
 __device__ __forceinline__ void pg_tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
     asm volatile(

@@ -299,9 +299,7 @@ prefill_gemm_pair_kernel(const __grid_constant__ PgJobs jobs, const __grid_const
                     st++;
                 }
             }
-            // after a failure the copies that were announced must land before the CTAs may leave
-            if (!ok)
-                for (uint32_t i = st > PT_STAGES ? st - PT_STAGES : 0; i < st; i++) mbar_wait_bounded(&full[i % PT_STAGES], (i / PT_STAGES) & 1u);
+            pg_drain(full, st, PT_STAGES);
         }
     } else if (lane == 0) {
         // blocks of K as they are in memory: 64 rows a copy
@@ -323,7 +321,7 @@ prefill_gemm_pair_kernel(const __grid_constant__ PgJobs jobs, const __grid_const
                 pg_tma_2d(to + PG_ROWS / 2 * pitch, job.w2 ? &maps.w2 : &maps.w[js], x, job.w2 ? y : y + PG_ROWS / 2, &raw_full);
             }
         }
-        if (!ok && raws > 0) mbar_wait_bounded(&raw_full, (raws - 1) & 1u);
+        pg_drain(&raw_full, raws, 1);
     }
     if (!ok) s_failed = 1;
     __syncwarp();

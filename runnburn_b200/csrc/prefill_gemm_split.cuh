@@ -278,8 +278,7 @@ prefill_gemm_split_kernel(const __grid_constant__ PgJobs jobs, const __grid_cons
             issued = kt + 1;
             if (++s == S) s = 0, phase ^= 1u;
         }
-        // after a failure the copies that were announced must land before the stages are reused
-        for (int kt = max(0, issued - S); kt < issued && !ok; kt++) mbar_wait_bounded(&full[kt % S], (uint32_t)((kt / S) & 1));
+        pg_drain(full, (uint32_t)issued, (uint32_t)S);   // the stages are reused
     }
     if (!ok) s_failed = 1;
     __syncthreads();   // the accumulators' address; a failure of any role

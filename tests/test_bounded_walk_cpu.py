@@ -1,4 +1,5 @@
 """Control flow around waits that may give up (csrc/bounded_walk.hpp), compiled for the host: threads stand for warps."""
+import re
 import subprocess
 from pathlib import Path
 
@@ -70,6 +71,43 @@ def run(tmp_path, program):
     subprocess.run(["g++", "-std=c++17", "-O1", "-pthread", "-I", str(ROOT / "runnburn_b200" / "csrc"), "-o", str(exe), str(src)], check=True)
     r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, (r.returncode, r.stdout)
+
+
+DRAIN = r"""
+#include "bounded_walk.hpp"
+#include <vector>
+
+int main() {
+    for (unsigned ring = 1; ring <= 5; ring++)
+        for (unsigned issued = 0; issued <= 4 * ring + 1; issued++) {
+            std::vector<int> last(ring, -1), seen(ring, -1);
+            for (unsigned i = 0; i < issued; i++) last[i % ring] = (i / ring) & 1;
+            rnb::drain_ring(issued, ring, [&](unsigned slot, unsigned parity) { seen.at(slot) = (int)parity; });
+            if (seen != last) return 1;
+        }
+    return 0;
+}
+"""
+
+
+def test_drain_waits_for_the_last_fill_of_every_slot(tmp_path):
+    run(tmp_path, DRAIN)
+
+
+@pytest.mark.parametrize("file,kernel", [
+    ("dense.cuh", "dense_gemm_pair_kernel"), ("dense.cuh", "dense_gemm_split_kernel"), ("prefill_gemm_split.cuh", "prefill_gemm_split_kernel"),
+    ("prefill_gemm_pair.cuh", "prefill_gemm_pair_kernel"), ("prefill_attention_tiled.cuh", "prefill_attention_tiled_kernel"),
+    ("causal_attention_tc.cuh", "causal_attention_tc_kernel"),
+])
+def test_producers_drain_whatever_their_own_waits_returned(file, kernel):
+    """Every ring that a kernel announces copies on is drained, and not behind the producer's own outcome (`ok`)."""
+    text = (ROOT / "runnburn_b200" / "csrc" / file).read_text()
+    body = text[text.index(kernel + "("):]
+    body = body[:body.index("\n}\n")]
+    drains = re.findall(r"\n(.*)pg_drain\(&?(\w+),", body)
+    rings = {"raw_full", "full"} if kernel == "prefill_gemm_pair_kernel" else {"q_full", "kfull", "vfull"} if "causal" in kernel else {"full"}
+    assert {d[1] for d in drains} == rings
+    assert not any("ok" in d[0] for d in drains)
 
 
 def test_warps_that_share_barriers_leave_the_tiles_together(tmp_path):
