@@ -304,7 +304,7 @@ dense_gemm_pair_kernel(const __grid_constant__ DenseGemmJobs jobs, const __grid_
             for (int tile = pair0; tile < P.tiles && ok; tile += n_pairs, count++) {
                 const int KT = (jobs.j[job_of(tile)].cols + DG_K - 1) / DG_K;
                 for (int kt = 0; kt < KT && ok; kt++) {
-                    ok = __all_sync(0xffffffffu, mbar_wait_bounded(&full[s], phase));
+                    ok = __all_sync(0xffffffffu, pt_wait_shared(&full[s], phase));
                     const uint32_t x1 = smem_u32(smem + s * stage_bytes);
                     const uint64_t dx1 = pg_smem_desc(x1), dx2 = pg_smem_desc(x1 + (uint32_t)(P.n1 / 2) * 128u), dw = pg_smem_desc(x1 + tok_bytes);
                     for (int part = 0; part < 2 && ok; part++) {

@@ -14,14 +14,14 @@
 // dequantise, two groups of eight that take two of a block's four stages each; behind the first stage of the next tile
 // they write the finished tile from tensor memory and hand the columns back.  Warp 16 of the even CTA issues the MMAs,
 // warp 17 of each CTA its token copies, warp 18 those of the weights.  A stage fills on each CTA's own barrier; warp 16 of
-// the odd CTA waits for its own and passes one arrival on to the even CTA's, so that the release and the acquire across the
-// cluster stand between what the odd CTA wrote and the MMA that reads it and cost no dequantising warp anything.
+// the odd CTA waits for its own and passes one arrival on to the even CTA's: a release and an acquire across the cluster
+// stand between what the odd CTA wrote and the MMA that reads it, and the dequantising warps do not wait for them.
 // A commit reaches both CTAs.  Every wait is bounded; after a timeout all threads still meet at the cluster barrier.
 //
 // What bounds it: the dequantising warps and the tensor pipe, about even at 450 tokens a tile.  Measured with 2048 / 512
-// tokens, us (512-token tiles of a CTA by itself before): gate + up 28672 x 4096 370 / 108 (464 / 132), down 4096 x 14336
-// Q6_K 197 / 156 (272 / 258), q + k + v 98 / 53 (139 / 79), o 59 / 44 (65 / 58): 1300 TFLOP/s for gate + up, 0.80 of the
-// measured 1632.
+// tokens, us, cold, with the conversion of the tokens to bf16 (512-token tiles of a CTA by itself before): gate + up
+// 28672 x 4096 388 / 116 (484 / 148), down 4096 x 14336 Q6_K 193 / 150 (290 / 265), q + k + v 105 / 54 (146 / 87),
+// o 68 / 48 (73 / 64): 1240 TFLOP/s for gate + up, 0.73 of the measured 1701.
 #pragma once
 #include "prefill_gemm.cuh"
 #include "prefill_gemm_split.cuh"
@@ -48,18 +48,35 @@ struct PtMaps {   // tokens of the two parts (boxes of n1 / 2 and n2 / 2), block
 
 // An arrival at the other CTA's barrier, and a wait for one: they order what either CTA did before it.
 __device__ __forceinline__ void pt_arrive(uint32_t cluster_addr) { asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory"); }
-__device__ __forceinline__ bool pt_wait(uint64_t *bar, uint32_t parity) {
+// The same for what lies in shared memory alone, the stages of operands.  As a thread's release of all its memory a stage took
+// 1900 cycles (2048 tokens: gate + up 474 us, down 247; with the restricted fences 388 and 193).
+__device__ __forceinline__ void pt_arrive_shared(uint32_t cluster_addr) {
+    asm volatile("fence.release.sync_restrict::shared::cta.cluster;\n\tmbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+template <bool SHARED>
+__device__ __forceinline__ bool pt_wait_in(uint64_t *bar, uint32_t parity) {
     for (uint32_t i = 0; i < (1u << 22); i++) {
         uint32_t done;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                     : "=r"(done)
-                     : "r"(smem_u32(bar)), "r"(parity)
-                     : "memory");
-        if (done) return true;
+        if constexpr (SHARED)
+            asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.relaxed.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                         : "=r"(done)
+                         : "r"(smem_u32(bar)), "r"(parity)
+                         : "memory");
+        else
+            asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                         : "=r"(done)
+                         : "r"(smem_u32(bar)), "r"(parity)
+                         : "memory");
+        if (done) {
+            if constexpr (SHARED) asm volatile("fence.acquire.sync_restrict::shared::cluster.cluster;" ::: "memory");
+            return true;
+        }
         if (i > 64) __nanosleep(i > 4096 ? 256 : 32);
     }
     return false;
 }
+__device__ __forceinline__ bool pt_wait(uint64_t *bar, uint32_t parity) { return pt_wait_in<false>(bar, parity); }
+__device__ __forceinline__ bool pt_wait_shared(uint64_t *bar, uint32_t parity) { return pt_wait_in<true>(bar, parity); }
 __device__ __forceinline__ void pt_mma(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
@@ -255,7 +272,7 @@ prefill_gemm_pair_kernel(const __grid_constant__ PgJobs jobs, const __grid_const
             for (int tile = pair0; tile < P.tiles && ok; tile += n_pairs, count++) {
                 if (count > 0) ok = __all_sync(0xffffffffu, pt_wait(&acc_free, (uint32_t)((count - 1) & 1)));
                 for (int kt = 0; kt < 4 * nb && ok; kt++) {
-                    ok = __all_sync(0xffffffffu, pt_wait(&full[s], phase));
+                    ok = __all_sync(0xffffffffu, pt_wait_shared(&full[s], phase));
                     if (!ok) break;
                     pg_fence_after();
                     if (pg_elect()) {
@@ -279,7 +296,7 @@ prefill_gemm_pair_kernel(const __grid_constant__ PgJobs jobs, const __grid_const
                 for (int kt = 0; kt < 4 * nb && ok; kt++, st++) {
                     const uint32_t s = st % PT_STAGES;
                     ok = mbar_wait_bounded(&full[s], (st / PT_STAGES) & 1u);
-                    if (ok) pt_arrive(ps_map(smem_u32(&full[s]), 0));
+                    if (ok) pt_arrive_shared(ps_map(smem_u32(&full[s]), 0));
                 }
         }
     } else if (warp == PT_WORKERS + 1) {
