@@ -736,29 +736,36 @@ inline int encode_token_map(PgTensorMap *out, const uint16_t *xb, size_t seq, si
     if (r != CUDA_SUCCESS) return fail(RNB_B200_CUDA_ERROR, "cuTensorMapEncodeTiled failed with driver code %d", (int)r);
     return RNB_B200_OK;
 }
-// CTAs along K for a short prompt, 0: pairs of SMs (prefill_gemm_pair.cuh).  Measured against the kernel of 512-token tiles
-// that the pairs replaced, on the matrices of the 8B and 1B shapes, 16 to 512
-// tokens (us, 512-token tiles / this rule):
-//   matrices of their own: 203 tokens 4096 x 4096 55 / 29, 4096 x 14336 251 / 61, q + k + v 77 / 43, 2048 x 8192 147 / 38;
-//     400 tokens 55 / 37, 255 / 112, 77 / 71, 148 / 41.  With 4 to 7, 8 to 31 and more blocks of 256 columns 2, 4 and 8
-//     CTAs were the fastest or within 5 % of it; the count depends on K and the tokens alone, so that a matrix gives the
-//     same bits in every launch that it can be part of.
-//   gate + up: 45 tokens 116 / 67 (14336 x 4096) and 35 / 26 (8192 x 2048), 203 tokens 124 / 93 and 39 / 40, 320 tokens
-//     128 / 159 and 41 / 51 - two token tiles dequantise twice, so longer prompts keep the 512-token tile.  Its row tiles
-//     fill the chip without a cut from 128 on (cut in 2: 119 and 46 at 203 tokens).
-inline int prefill_split_ks(bool pair, int tiles, size_t seq, size_t cols) {
-    const int nb = (int)(cols / 256);
-    if (pair) {
-        if (seq > PS_TOK) return 0;
-        int ks = 1;
-        while (ks * 2 * tiles <= 148 && ks * 2 <= std::min(nb / 2, PS_MAX_KS)) ks *= 2;
-        return ks;
-    }
+// CTAs along K of a launch, 0: pairs of SMs.  Four CTAs, or eight from 32 blocks of 256 columns on, while the tiles of all
+// matrices, the token tiles and the cut fill the chip at most once (two CTAs per SM); else nothing is cut, and the pairs are the
+// faster kernel, but for a few tokens of very short rows and for up to 128 tokens of more Q4_K tiles than SMs.  Rows of less
+// than 16 blocks are cut up to 128 tokens: above, their chain is short enough for the pairs.  Measured (us, cold, cut / pairs, in
+// brackets the 512-token tiles of one CTA before either kernel; rows x K):
+//   tokens               45                128               203              257              384               511
+//   4096 x 4096          28 / 42 [60]      30 / 42 [60]      38 / 44 [61]     40 / 46 [61]     44 / 49 [63]      48 / 47 [64]
+//   q + k + v, 6144      36 / 47 [81]      38 / 49 [82]      48 / 51 [83]     68 / 52 [83]     79 / 54 [84]      77 / 54 [85]
+//   10240 x 4096         44 / 42 [61]      53 / 44 [60]      71 / 46 [61]     90 / 48 [62]     102 / 50 [63]     108 / 58 [64]
+//   14336 x 4096         53 / 42 [60]      60 / 44 [60]      79 / 47 [62]     114 / 48 [62]    132 / 52 [63]     142 / 59 [65]
+//   4096 x 14336 Q6_K    52 / 136 [256]    56 / 139 [257]    67 / 143 [259]   95 / 144 [260]   106 / 147 [263]   111 / 147 [265]
+//   2048 x 8192 Q6_K     34 / 82 [152]     36 / 84 [153]     43 / 87 [154]    42 / 87 [155]    47 / 90 [157]     50 / 89 [159]
+//   2048 x 2048          24 / 27 [36]      24 / 28 [38]      32 / 30 [38]     30 / 30 [38]     32 / 33 [38]      32 / 31 [39]
+//   8192 x 2048          26 / 28 [36]      28 / 29 [37]      36 / 30 [38]     53 / 32 [38]     62 / 34 [38]      65 / 33 [40]
+//   1024 x 1024          22 / 19 [24]      22 / 20 [25]      28 / 22 [26]     28 / 22 [26]     28 / 24 [26]      30 / 22 [26]
+//   gate + up 2 x 14336  71 / 82 [120]     81 / 85 [124]     95 / 89 [128]    151 / 93 [130]   162 / 98 [133]    177 / 110 [136]   (one CTA along K)
+// What is not cut gives the same bits in every launch and on either kernel; a matrix that is cut by itself may not be in a
+// launch with others.
+inline int pg_sms() { return state().sm_count > 0 ? state().sm_count : 148; }
+inline int prefill_split_ks(bool q4, int tiles, size_t seq, size_t cols) {
     if (seq >= (size_t)PT_MAX_TOK) return 0;
-    return nb < 4 ? 1 : nb < 8 ? 2 : nb < 32 ? 4 : PS_MAX_KS;
+    const int nb = (int)(cols / 256), token_tiles = (int)((seq + PS_TOK - 1) / PS_TOK);
+    int ks = nb < 4 || (nb < 16 && seq > 128) ? 1 : nb < 32 ? 4 : PS_MAX_KS;
+    while (ks >= 4 && tiles * token_tiles * ks > 2 * pg_sms()) ks /= 2;
+    if (ks >= 4) return ks;
+    return (nb < 4 && seq <= 64) || (q4 && tiles >= pg_sms() && seq <= 128) ? 1 : 0;
 }
-inline int pg_pairs() { return std::max(1, (state().sm_count > 0 ? state().sm_count : 148) / 2); }
-// Tokens per tile of the paired kernels (two parts, multiples of 32): the width that gives the least rounds x cost(width).
+inline int pg_pairs() { return std::max(1, pg_sms() / 2); }
+// Tokens per tile of the paired kernels (two parts, multiples of 32): the width that gives the least rounds x cost(width), of
+// those the narrowest: more pairs share the last accumulators (448 tokens, 4096 x 4096, in two tiles instead of one: 51 -> 46 us).
 template <class P, class F>
 inline void pg_pair_tiles(P &p, int row_pairs, int seq, F &&cost) {
     const int first = (seq + PT_MAX_TOK - 1) / PT_MAX_TOK;
@@ -767,7 +774,7 @@ inline void pg_pair_tiles(P &p, int row_pairs, int seq, F &&cost) {
     for (int n = first; n <= 2 * first; n++) {
         const int w = std::max(((seq + n - 1) / n + 31) & ~31, 64);
         const long c = (long)((row_pairs * ((seq + w - 1) / w) + pg_pairs() - 1) / pg_pairs()) * cost(w);
-        if (best < 0 || c < best) best = c, nt = w;
+        if (best < 0 || c <= best) best = c, nt = w;
     }
     p.n1 = (nt / 2 + 31) & ~31;
     p.n2 = nt - p.n1;
@@ -776,7 +783,9 @@ inline void pg_pair_tiles(P &p, int row_pairs, int seq, F &&cost) {
 }
 // `tiles`: row tiles of all jobs
 inline int launch_prefill_gemm_tiles(cudaStream_t s, const PgJobs &jobs, int tiles, size_t seq, size_t cols, const uint16_t *xb, int *dev_error) {
-    const int ks = prefill_split_ks(jobs.j[0].w2 != nullptr, tiles, seq, cols);
+    bool q4 = true;
+    for (int i = 0; i < jobs.n; i++) q4 = q4 && jobs.j[i].type == TYPE_Q4_K;
+    const int ks = prefill_split_ks(q4, tiles, seq, cols);
     if (ks == 0) {
         PtParams P;
         PtMaps maps;

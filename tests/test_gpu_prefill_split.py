@@ -16,6 +16,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("t,rows,cols,seq", [
     (Q4_K, 128, 256, 1), (Q4_K, 129, 768, 16), (Q6_K, 127, 512, 17), (Q4_K, 200, 1024, 255), (Q6_K, 130, 1280, 256), (Q4_K, 256, 2304, 257),
     (Q6_K, 100, 2048, 290), (Q4_K, 260, 4096, 33), (Q6_K, 256, 8448, 48), (Q4_K, 128, 14336, 300), (Q6_K, 384, 14336, 511), (Q4_K, 64, 8192, 511),
+    (Q4_K, 9700, 1024, 1), (Q6_K, 9700, 1024, 17), (Q4_K, 200, 1024, 128), (Q4_K, 19000, 256, 64), (Q4_K, 19000, 512, 128), (Q6_K, 100, 2048, 129),
 ])
 def test_short_prompt_matmul(ops, t, rows, cols, seq):
     rng = np.random.default_rng(rows + 7 * cols + seq)
@@ -72,3 +73,33 @@ def test_prompt_products_cut_along_k(design, n):
     got = dec.prefill_logits(toks, 0, list(range(n)))[0]
     dec.close()
     assert not (why := su.bad(got, want, "bfloat16")), why
+
+
+@pytest.mark.parametrize("specs,cols,seq", [
+    ([(Q4_K, 9600)], 1024, 128), ([(Q4_K, 19000)], 1024, 128), ([(Q4_K, 19000)], 1024, 129), ([(Q6_K, 19000)], 1024, 65), ([(Q4_K, 4700), (Q6_K, 4700)], 2048, 300),
+    ([(Q4_K, 2500)] * 3, 2048, 511), ([(Q6_K, 300)], 1024, 129), ([(Q4_K, 300)], 3840, 129), ([(Q4_K, 4800)], 8192, 257), ([(Q4_K, 300)], 768, 64), ([(Q4_K, 300)], 768, 65),
+])
+def test_launches_that_fill_the_chip_are_not_cut(ops, specs, cols, seq):
+    """A launch whose tiles fill the chip, or whose rows are short, sums a token's products in one chain along K, as a prompt of 600
+    tokens does: the same bits for the tokens that they share."""
+    import ctypes
+
+    import torch
+
+    import runnburn_b200 as r
+    rng = np.random.default_rng(cols + seq)
+    n = len(specs)
+    w = [torch.from_numpy(random_blocks(rng, t, rows, cols)).cuda() for t, rows in specs]
+    x = torch.randn(600, cols, device="cuda", generator=torch.Generator("cuda").manual_seed(seq))
+    xb = torch.empty(600 * cols, dtype=torch.int16, device="cuda")
+    out = {}
+    for tokens in (seq, 600):
+        ys = [torch.full((tokens, rows), float("nan"), device="cuda") for _, rows in specs]
+        assert r.load().rnb_b200_dev_prefill_gemm_multi(
+            n, (ctypes.c_int * n)(*[t for t, _ in specs]), (ctypes.c_void_p * n)(*[v.data_ptr() for v in w]), (ctypes.c_size_t * n)(*[rows for _, rows in specs]),
+            (ctypes.c_void_p * n)(*[y.data_ptr() for y in ys]), cols, x.data_ptr(), tokens, xb.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+        torch.cuda.synchronize()
+        assert ops.dev_error_flag() == 0
+        out[tokens] = ys
+    for a, b in zip(out[seq], out[600]):
+        assert torch.equal(a, b[:seq])
