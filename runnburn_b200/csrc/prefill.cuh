@@ -64,7 +64,7 @@ inline int launch_prefill_attention_f16kv(cudaStream_t s, const float *q, const 
     cfg.stream = s;
     const bool aligned = (((uintptr_t)k | (uintptr_t)v) & 15) == 0;
     if (!simt && tiled && aligned && group >= 1 && group <= PAT_ROWS && (group & (group - 1)) == 0 && num_heads == group * num_kv_heads &&
-        ((uintptr_t)q & 15) == 0 && ((uintptr_t)out & 15) == 0 && kv_len >= seq_len && seq_len > 0 && seq_len / (PAT_ROWS / group) < 65535 && scale > 0.f && ((uintptr_t)out_bf16 & 15) == 0) {
+        (((uintptr_t)q | (uintptr_t)out | (uintptr_t)out_bf16) & 15) == 0 && kv_len >= seq_len && seq_len > 0) {
         static bool attr_set = false;
         if (!attr_set) {
             RNB_CU(cudaFuncSetAttribute(prefill_attention_tiled_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PAT_SMEM));
@@ -74,7 +74,7 @@ inline int launch_prefill_attention_f16kv(cudaStream_t s, const float *q, const 
         PatMaps maps;
         RNB_TRY(encode_token_map(&maps.k, k, (size_t)kv_len, (size_t)num_kv_heads * HD, 0, PAT_KEYS));
         RNB_TRY(encode_token_map(&maps.v, v, (size_t)kv_len, (size_t)num_kv_heads * HD, 0, PAT_KEYS));
-        RNB_CU(launch_k(prefill_attention_tiled_kernel, dim3(num_kv_heads, (seq_len + qpc - 1) / qpc), dim3(PAT_THREADS), PAT_SMEM, s, q, maps, seq_len, kv_len,
+        RNB_CU(launch_k(prefill_attention_tiled_kernel, dim3(num_kv_heads * ((seq_len + qpc - 1) / qpc)), dim3(PAT_THREADS), PAT_SMEM, s, q, maps, seq_len, kv_len,
                         num_heads, num_kv_heads, scale, out, out_bf16, dev_error));
         if (wrote_bf16) *wrote_bf16 = out_bf16 != nullptr;
         return RNB_B200_OK;

@@ -94,8 +94,9 @@ __device__ __forceinline__ float pat_total(uint64_t a, uint64_t b) {
 }
 __device__ __forceinline__ void pat_tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// grid = (num_kv_heads, ceil(seq_len / (128 / group))): the long rows of every head come first; group = num_heads / num_kv_heads a power of two up to 128; scale > 0.
-// out_bf16 (may be null): the result rounded to bf16 there instead of f32 in `out`.
+// grid = num_kv_heads x ceil(seq_len / (128 / group)), heads fastest: the long rows of every head come first; group =
+// num_heads / num_kv_heads a power of two up to 128.  The softmax needs a positive scale (its maxima are of unscaled scores): the
+// sign, or zero, of another one goes into the queries.  out_bf16 (may be null): the result rounded to bf16 there instead of f32 in `out`.
 RNB_GLOBAL void __launch_bounds__(PAT_THREADS, 2)
 prefill_attention_tiled_kernel(const float *__restrict__ q, const __grid_constant__ PatMaps maps, int seq_len, int kv_len, int num_heads, int num_kv_heads,
                                float scale, float *__restrict__ out, uint16_t *__restrict__ out_bf16, int *__restrict__ err_flag) {
@@ -109,7 +110,7 @@ prefill_attention_tiled_kernel(const float *__restrict__ q, const __grid_constan
     volatile int *const s_failed = reinterpret_cast<volatile int *>(bars + 12);
     const uint32_t smem = smem_u32(pat_smem);
     const int group = num_heads / num_kv_heads, qpc = PAT_ROWS / group;
-    const int kv_h = blockIdx.x, i0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * qpc;   // long rows first
+    const int kv_h = (int)blockIdx.x % num_kv_heads, i0 = (((int)gridDim.x - 1 - (int)blockIdx.x) / num_kv_heads) * qpc;   // long rows first
     const int shift = kv_len - seq_len;                                              // query i sits at position shift + i
     const int n_keys = min(kv_len, shift + min(i0 + qpc, seq_len));                  // keys visible to the CTA's last query
     const int n_tiles = (n_keys + PAT_KEYS - 1) / PAT_KEYS;
@@ -143,6 +144,10 @@ prefill_attention_tiled_kernel(const float *__restrict__ q, const __grid_constan
             const int r = warp * 32 + i, qi = i0 + r / group;
             float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
             if (qi < seq_len) x = *reinterpret_cast<const float4 *>(q + ((size_t)qi * num_heads + kv_h * group + r % group) * HD + lane * 4);
+            if (!(scale > 0.f)) {
+                const float sign = scale == 0.f ? 0.f : -1.f;
+                x = make_float4(x.x * sign, x.y * sign, x.z * sign, x.w * sign);
+            }
             uint2 hi, lo;
             split_f16x2(x.x, x.y, hi.x, lo.x);
             split_f16x2(x.z, x.w, hi.y, lo.y);
@@ -159,7 +164,7 @@ prefill_attention_tiled_kernel(const float *__restrict__ q, const __grid_constan
         const bool live = qi < seq_len;
         const int pos = live ? shift + qi : kv_len - 1;   // dead rows see everything (finite numbers) and are never stored
         const uint32_t lanes = (uint32_t)(warp * 32) << 16;
-        const float sl2 = scale * 1.4426950408889634f;    // scores are kept in log2 units: exp(x) = exp2(x * log2 e)
+        const float sl2 = scale == 0.f ? 1.f : fabsf(scale) * 1.4426950408889634f;   // scores are kept in log2 units: exp(x) = exp2(x * log2 e)
         float m_ref = -INFINITY, l_run = 0.f;
         for (int t = 0; t < n_tiles && ok; t++) {
             ok = __all_sync(0xffffffffu, mbar_wait_bounded(s_full, (uint32_t)(t & 1)));

@@ -45,6 +45,28 @@ def test_prefill_attention(ops, heads, kvh, seq, kv_len, shape):
     assert np.max(np.abs(np.asarray(got).reshape(want.shape) - want)) <= 1e-4 * np.max(np.abs(want))
 
 
+@pytest.mark.parametrize("heads,kvh,seq,kv_len", [(8, 2, 33, 129), (32, 1, 5, 191)])
+def test_prefill_attention_with_any_scale(ops, heads, kvh, seq, kv_len):
+    """A scale of s with queries q and one of -s with -q are the same scores, a scale of zero is queries of zero: the same bits, and
+    a mean over the visible keys."""
+    rng = np.random.default_rng(seq)
+    q = rng.standard_normal((seq, heads, 128)).astype(np.float32)
+    k, v = (rng.standard_normal((kv_len, kvh, 128)).astype(np.float16) for _ in range(2))
+
+    def run(q, scale):
+        return np.asarray(ops.attention_prefill_flash_hd128_f16kv(q.reshape(-1), k.view(np.uint16).reshape(-1), v.view(np.uint16).reshape(-1), seq, kv_len, heads, kvh,
+                                                                  scale)).reshape(seq, heads, 128)
+
+    s = 1.0 / np.sqrt(128.0)
+    assert np.array_equal(run(q, -s), run(-q, s))
+    flat = run(q, 0.0)
+    assert np.array_equal(flat, run(0.0 * q, 1.0))
+    for got, scale in ((run(q, -s), -s), (flat, 0.0)):
+        want = reference(q, k, v, scale)
+        assert np.max(np.abs(got - want)) <= 1e-4 * np.max(np.abs(want))
+    assert ops.dev_error_flag() == 0
+
+
 @pytest.mark.parametrize("cuts", [[9], [63, 64, 65], [128, 129], [300]])
 @pytest.mark.parametrize("kind", ["window", "wide window", "one group", "latent", "latent 64 + 64"])
 def test_prompt_attention_of_mixed_stacks(kind, cuts):
