@@ -13,8 +13,8 @@
 // probabilities are at most 2^8.  Two CTAs per SM (112 KB, 256 tensor-memory columns each: 64 scores, 128 outputs, 32 + 32
 // probabilities).  Long rows are scheduled first.  Every wait is bounded.
 //
-// What bounds it: the softmax warps (tensor pipe 31 % busy).  2048 tokens of 32 / 8 heads: 108 us cold (262 with mma.sync
-// and eight warps that shared a CTA); 203 tokens behind 1000 positions through 32 layers 10.2 -> 9.4 ms.
+// What bounds it: the softmax warps.  Caches warm, 32 / 8 heads: 2048 tokens 76 us (247 with mma.sync and eight warps that shared a
+// CTA), 203 tokens behind 1000 positions 31 (65); 64 tokens of 8 / 2 heads 10.3 (7.9: the fill of tensor memory and barriers).
 #pragma once
 #include "attention.cuh"
 #include "prefill_gemm_split.cuh"
@@ -139,22 +139,28 @@ prefill_attention_tiled_kernel(const float *__restrict__ q, const __grid_constan
     bool ok = *s_failed == 0;
 
     if (warp < 4) {
-        // ---- queries as f16 hi + lo: a warp takes its 32 rows one by one, four dims per lane ----
-        for (int i = 0; i < 32 && ok; i++) {
-            const int r = warp * 32 + i, qi = i0 + r / group;
-            float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (qi < seq_len) x = *reinterpret_cast<const float4 *>(q + ((size_t)qi * num_heads + kv_h * group + r % group) * HD + lane * 4);
-            if (!(scale > 0.f)) {
-                const float sign = scale == 0.f ? 0.f : -1.f;
-                x = make_float4(x.x * sign, x.y * sign, x.z * sign, x.w * sign);
+        // ---- queries as f16 hi + lo: a warp takes its 32 rows, four dims per lane, 16 rows asked for at once (one by one the rows took
+        // 13 us, most of a short prompt's launch) ----
+        const float sign = scale > 0.f ? 1.f : scale == 0.f ? 0.f : -1.f;
+        for (int i = 0; i < 32 && ok; i += 16) {
+            float4 x[16];
+#pragma unroll
+            for (int j = 0; j < 16; j++) {
+                const int r = warp * 32 + i + j, qi = i0 + r / group;
+                x[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (qi < seq_len) x[j] = *reinterpret_cast<const float4 *>(q + ((size_t)qi * num_heads + kv_h * group + r % group) * HD + lane * 4);
             }
-            uint2 hi, lo;
-            split_f16x2(x.x, x.y, hi.x, lo.x);
-            split_f16x2(x.z, x.w, hi.y, lo.y);
-            const uint32_t at = (uint32_t)(lane >> 4) * PAT_PANEL + (uint32_t)(r >> 3) * 1024u + (uint32_t)(r & 7) * 128u + (((uint32_t)((lane & 15) >> 1) ^ (uint32_t)(r & 7)) << 4) +
-                                (uint32_t)(lane & 1) * 8u;
-            *reinterpret_cast<uint2 *>(pat_smem + at) = hi;
-            *reinterpret_cast<uint2 *>(pat_smem + 2 * PAT_PANEL + at) = lo;
+#pragma unroll
+            for (int j = 0; j < 16; j++) {
+                const int r = warp * 32 + i + j;
+                uint2 hi, lo;
+                split_f16x2(x[j].x * sign, x[j].y * sign, hi.x, lo.x);
+                split_f16x2(x[j].z * sign, x[j].w * sign, hi.y, lo.y);
+                const uint32_t at = (uint32_t)(lane >> 4) * PAT_PANEL + (uint32_t)(r >> 3) * 1024u + (uint32_t)(r & 7) * 128u +
+                                    (((uint32_t)((lane & 15) >> 1) ^ (uint32_t)(r & 7)) << 4) + (uint32_t)(lane & 1) * 8u;
+                *reinterpret_cast<uint2 *>(pat_smem + at) = hi;
+                *reinterpret_cast<uint2 *>(pat_smem + 2 * PAT_PANEL + at) = lo;
+            }
         }
         pg_proxy_fence();
         __syncwarp();
