@@ -764,8 +764,9 @@ inline int prefill_split_ks(bool q4, int tiles, size_t seq, size_t cols) {
     return (nb < 4 && seq <= 64) || (q4 && tiles >= pg_sms() && seq <= 128) ? 1 : 0;
 }
 inline int pg_pairs() { return std::max(1, pg_sms() / 2); }
-// Tokens per tile of the paired kernels (two parts, multiples of 32): the width that gives the least rounds x cost(width), of
-// those the narrowest: more pairs share the last accumulators (448 tokens, 4096 x 4096, in two tiles instead of one: 51 -> 46 us).
+// Tokens per tile of the paired kernels (two parts, multiples of 32): the width that gives the least rounds x cost(width).  In one
+// round the narrowest of those: more pairs share the accumulators' way back (448 tokens: 4096 x 4096 51 -> 48 us, 2048 x 2048 34 -> 30);
+// in several the widest, which dequantises least.
 template <class P, class F>
 inline void pg_pair_tiles(P &p, int row_pairs, int seq, F &&cost) {
     const int first = (seq + PT_MAX_TOK - 1) / PT_MAX_TOK;
@@ -773,8 +774,8 @@ inline void pg_pair_tiles(P &p, int row_pairs, int seq, F &&cost) {
     int nt = PT_MAX_TOK;
     for (int n = first; n <= 2 * first; n++) {
         const int w = std::max(((seq + n - 1) / n + 31) & ~31, 64);
-        const long c = (long)((row_pairs * ((seq + w - 1) / w) + pg_pairs() - 1) / pg_pairs()) * cost(w);
-        if (best < 0 || c <= best) best = c, nt = w;
+        const long rounds = (row_pairs * ((seq + w - 1) / w) + pg_pairs() - 1) / pg_pairs(), c = rounds * cost(w);
+        if (best < 0 || c < best || (c == best && rounds == 1)) best = c, nt = w;
     }
     p.n1 = (nt / 2 + 31) & ~31;
     p.n2 = nt - p.n1;
