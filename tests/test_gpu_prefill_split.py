@@ -57,9 +57,9 @@ def test_short_prompt_gate_up(ops, t, rows, cols, seq):
 @pytest.mark.parametrize("n", [9, 16, 17, 128, 129, 256, 257, 300])
 @pytest.mark.parametrize("design", ["dutivik", "punisun"])
 def test_prompt_products_cut_along_k(design, n):
-    """bf16 stacks whose products have 16 to 48 stages of K and few tiles (4 or 8 CTAs along K; the gate and up pair too),
-    at the edges of the token tiles, against the plain reference: every projection rounds its input to bf16, the bound
-    of the stack tests (3e-2 of the rows' scale)."""
+    """bf16 stacks whose products have 16 to 48 stages of K and few tiles (4 or 8 CTAs along K; the gate and up pair too, but for
+    257 and 300 tokens, where pairs of SMs take it), at the edges of the token tiles, against the plain reference: every
+    projection rounds its input to bf16, the bound of the stack tests (3e-2 of the rows' scale)."""
     import stack_util as su
     from hybrid_ref import Model
     if design == "dutivik":
