@@ -798,7 +798,7 @@ int LayerStack::matmul(cudaStream_t s, int n, const Mm *jobs, int n_jobs, int *e
         DenseSplit P;
         const int token_tiles = (n + DP_TOK - 1) / DP_TOK;
         P.ks = 1;
-        while (P.ks * 2 <= PS_MAX_KS && tiles * token_tiles * P.ks * 2 <= 296 && P.ks * 4 <= depth) P.ks *= 2;
+        while (P.ks * 2 <= PS_MAX_KS && tiles * token_tiles * P.ks * 2 <= 2 * pg_sms() && P.ks * 4 <= depth) P.ks *= 2;
         if (P.ks == 2 && depth < 64) P.ks = 1;
         P.nt = ((n + token_tiles - 1) / token_tiles + 15) & ~15;
         const bool split = P.ks > 1 || P.nt <= 128;
