@@ -32,9 +32,8 @@ constexpr uint32_t PG_B_BYTES = PG_ROWS * 128;   // weight tile of a stage
 __device__ __forceinline__ uint64_t pg_smem_desc(uint32_t saddr) {
     return (uint64_t)((saddr & 0x3ffffu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
-// One lane of a converged warp.  The MMAs are issued behind this and not behind `lane == 0`: their operands live in uniform
-// registers, and where the compiler cannot see that a single thread gets there it moves them there once per lane (a stage of
-// eight MMAs took 1000 cycles to issue).
+// One lane of a converged warp.  The MMAs are issued behind this and not behind `lane == 0`, where a stage of eight took 1000
+// cycles to issue (clock64 around it).
 __device__ __forceinline__ bool pg_elect() {
     uint32_t p;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
@@ -101,9 +100,6 @@ __device__ __forceinline__ uint4 pg_pair_exchange(const uint4 &mine) {
     return make_uint4(__shfl_xor_sync(0xffffffffu, mine.x, 1), __shfl_xor_sync(0xffffffffu, mine.y, 1), __shfl_xor_sync(0xffffffffu, mine.z, 1),
                       __shfl_xor_sync(0xffffffffu, mine.w, 1));
 }
-// Q6_K: group g of a block = elements 64g..64g+63 = for half n = g/2 the pair (q1,q2) if g even,
-// (q3,q4) if g odd, l = 0..31 each; y = (d*sc)*(q-32): dequant.rs:780-807.  Blocks are 210 bytes,
-// so rows are only 2-byte aligned: bytes are fetched as aligned 16-byte windows and shifted into place (pg_ldg_window).
 // f32 -> bf16 rows (activation), padded to a multiple of 8 columns by construction (cols % 256 == 0)
 RNB_GLOBAL void __launch_bounds__(256)
 f32_to_bf16_kernel(const float *__restrict__ x, uint16_t *__restrict__ y, size_t n) {
@@ -188,7 +184,7 @@ silu_mul_bf16_kernel(const float *__restrict__ gate, const float *__restrict__ u
 }
 
 // 128-byte, 64-byte aligned descriptor of the bf16 token matrix [seq][cols] (a CUtensorMap, kept
-// opaque here): boxes of 64 columns x 256 tokens, 128-byte swizzle, zero fill past the end.
+// opaque here): boxes of 64 columns x as many rows as the kernel asks for, 128-byte swizzle, zero fill past the end.
 struct alignas(64) PgTensorMap {
     unsigned long long opaque[16];
 };
@@ -243,6 +239,9 @@ __device__ __forceinline__ void pg_dequant_q4(const uint4 &hdr, const uint4 &q0,
         *reinterpret_cast<uint4 *>(row_base + (((c + 4 * h) ^ rr) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
     }
 }
+// Q6_K: group g of a block = elements 64g..64g+63 = for half n = g/2 the pair (q1,q2) if g even,
+// (q3,q4) if g odd, l = 0..31 each; y = (d*sc)*(q-32): dequant.rs:780-807.  Blocks are 210 bytes,
+// so rows are only 2-byte aligned: bytes are fetched as aligned 16-byte windows and shifted into place (pg_ldg_window).
 // Half h of the Q6_K groups of half-block n: h = 0 -> ql[64n .. 64n+31] (q1 / q3), h = 1 -> ql[64n+32 ..] (q2 / q4).
 struct PgRawQ6 {
     uint32_t ql[8], qh[4];   // qh: words 4h .. 4h+3 of the half-block's 32 bytes, the pair exchanges them when used

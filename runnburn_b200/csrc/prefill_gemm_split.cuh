@@ -66,8 +66,9 @@ __device__ __forceinline__ void ps_st_remote(uint32_t addr, uint32_t v) { asm vo
 
 // Adds the accumulators of a cluster's ks CTAs (one: its own).  A round gives every CTA up to ps_per_round chunks of
 // SUB * GROUPS tokens: the others send it theirs of those chunks, it adds them in rank order with its own and calls
-// f(chunk, count, sums).  Two cluster barriers a round, so few rounds: one or two at 256 tokens.  A worker warp holds the rows of lane quarter q and a chunk's tokens group * SUB ..; all
-// threads of the CTA come through here.  `smem` takes PS_SLOT_BYTES for the accumulators that arrive.
+// f(chunk, count, sums).  Two cluster barriers a round, so few rounds: one or two at 256 tokens.  A worker warp holds the rows of
+// lane quarter q and a chunk's tokens group * SUB ..; all threads of the CTA come through here.  `smem` takes PS_SLOT_BYTES for the
+// accumulators that arrive.
 constexpr uint32_t PS_SLOT_BYTES = 64 * 1024;
 __host__ __device__ inline int ps_per_round(int ks, uint32_t slot) { return ks > 1 ? (int)(PS_SLOT_BYTES / slot) / (ks - 1) : 1; }
 template <int SUB, int GROUPS, class F>
