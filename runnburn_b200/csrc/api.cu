@@ -45,7 +45,7 @@ const GemvTuning &gemv_tuning() {
     }();
     return t;
 }
-int encode_weight_map(GmTensorMap *out, const uint8_t *w, size_t rows, size_t row_bytes, uint32_t box_bytes, int box_rows) {
+int encode_weight_map(GmTensorMap *out, const uint8_t *w, size_t rows, size_t row_bytes, uint32_t box_bytes, int box_rows, size_t used_bytes) {
     static_assert(sizeof(GmTensorMap) == sizeof(CUtensorMap) && alignof(GmTensorMap) >= alignof(CUtensorMap), "descriptor size");
     typedef CUresult (*EncodeTiled)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
                                     const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -59,7 +59,7 @@ int encode_weight_map(GmTensorMap *out, const uint8_t *w, size_t rows, size_t ro
     }
     if (((uintptr_t)w & 15u) || (row_bytes & 15u) || (box_bytes & 15u) || box_bytes / 8 > 256 || rows == 0)
         return fail(RNB_B200_VALIDATION_FAILED, "weight matrix cannot be described for tiled copies (alignment or box width)");
-    const cuuint64_t dims[2] = {(cuuint64_t)(row_bytes / 8), (cuuint64_t)rows};
+    const cuuint64_t dims[2] = {(cuuint64_t)((used_bytes ? used_bytes + 7 : row_bytes) / 8), (cuuint64_t)rows};   // used_bytes: of a row, where rows are a part of row_bytes
     const cuuint64_t strides[1] = {(cuuint64_t)row_bytes};
     const cuuint32_t box[2] = {(cuuint32_t)(box_bytes / 8), (cuuint32_t)box_rows};
     const cuuint32_t estr[2] = {1, 1};
@@ -402,11 +402,28 @@ static int prefill_gemm_host(int type, const uint8_t *w, size_t wl, size_t rows,
     return gemv_host(type, w, wl, rows, cols, in, seq * cols, 0, seq, out, ol, nullptr, nullptr);
 }
 
+static int g_prefill_clusters[PT_MAX_KS + 1];
+int prefill_clusters(int ks) { return g_prefill_clusters[ks]; }
 int prefill_gemm_setup() {
     static bool done = false;
     if (done) return RNB_B200_OK;
-    RNB_CU(cudaFuncSetAttribute(prefill_gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PT_SMEM));
+    RNB_CU(cudaFuncSetAttribute(prefill_gemm_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PT_SMEM));
+    RNB_CU(cudaFuncSetAttribute(prefill_gemm_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PT_SMEM));
+    RNB_CU(cudaFuncSetAttribute(prefill_gemm_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PW_SMEM));
     RNB_CU(cudaFuncSetAttribute(prefill_gemm_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PS_SMEM));
+    for (int ks = 2; ks <= PT_MAX_KS; ks++) {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr = {};
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = (unsigned)(2 * ks);
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cfg.gridDim = dim3((unsigned)(2 * ks));
+        cfg.blockDim = dim3(PT_THREADS);
+        cfg.dynamicSmemBytes = PT_SMEM;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        RNB_CU(cudaOccupancyMaxActiveClusters(&g_prefill_clusters[ks], prefill_gemm_pair_kernel<true>, &cfg));
+    }
     done = true;
     return RNB_B200_OK;
 }

@@ -213,8 +213,8 @@ __device__ __forceinline__ void dg_store(void *y, size_t idx, float v) { reinter
 // Persistent: a pair walks its tiles, token tiles fastest, so that a weight matrix larger than L2 crosses DRAM once.  Warp 0
 // issues the copies (the first stages' weights before the dependency wait), warp 1 of the even CTA the MMAs, warps 2-9 read
 // the accumulators back, four per part; a part of the next tile starts when its columns are free.
-constexpr int DQ_STAGES = 4, DQ_THREADS = 320;
-constexpr uint32_t DQ_STAGE_BYTES = PT_MAX_TOK / 2 * 128 + DG_W_BYTES;
+constexpr int DQ_STAGES = 4, DQ_THREADS = 320, DQ_TOK = 512;   // DQ_TOK: most tokens of a tile
+constexpr uint32_t DQ_STAGE_BYTES = DQ_TOK / 2 * 128 + DG_W_BYTES;
 constexpr uint32_t DQ_EXCHANGE = 2 * 2 * 4 * 8 * 32 * 4;   // parts x buffers in turn x warps x tokens x rows
 constexpr size_t DQ_SMEM = (size_t)DQ_STAGES * DQ_STAGE_BYTES + DQ_EXCHANGE + 1024;
 struct DenseMapsPair {   // per job: tokens of part 1 and 2 (boxes of n1 / 2 and n2 / 2), weights, second weights

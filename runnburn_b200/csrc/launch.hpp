@@ -13,6 +13,7 @@
 #include "prefill_gemm.cuh"
 #include "prefill_gemm_pair.cuh"
 #include "prefill_gemm_split.cuh"
+#include "prefill_gemm_wide.cuh"
 #include "q8k.cuh"
 #include "state.hpp"
 
@@ -204,7 +205,7 @@ inline const KsplitTuning &ksplit_tuning() {
 // and the resident CTAs per SM the persistent grid is sized for.
 // Descriptor of a weight matrix for the integer-MMA matvec's tiled copies: [rows][row_bytes / 8] 8-byte
 // words, boxes of box_rows rows x box_bytes / 8 words, no swizzle, zeros outside the matrix.
-int encode_weight_map(GmTensorMap *out, const uint8_t *w, size_t rows, size_t row_bytes, uint32_t box_bytes, int box_rows = GM_ROWS);
+int encode_weight_map(GmTensorMap *out, const uint8_t *w, size_t rows, size_t row_bytes, uint32_t box_bytes, int box_rows = GM_ROWS, size_t used_bytes = 0);
 struct MmaTuning {
     int enabled, stages, ctas_per_sm, chunk16, tmap;
 };
@@ -736,96 +737,108 @@ inline int encode_token_map(PgTensorMap *out, const uint16_t *xb, size_t seq, si
     if (r != CUDA_SUCCESS) return fail(RNB_B200_CUDA_ERROR, "cuTensorMapEncodeTiled failed with driver code %d", (int)r);
     return RNB_B200_OK;
 }
-// CTAs along K of a launch, 0: pairs of SMs.  Four CTAs, or eight from 32 blocks of 256 columns on, while the tiles of all
-// matrices, the token tiles and the cut fill the chip at most once (two CTAs per SM); else nothing is cut, and the pairs are the
-// faster kernel, but for a few tokens of very short rows and for up to 128 tokens of more Q4_K tiles than SMs.  Rows of less
-// than 16 blocks are cut up to 128 tokens: above, their chain is short enough for the pairs.  Measured (us, cold, cut / pairs, in
-// brackets the 512-token tiles of one CTA before either kernel; rows x K):
-//   tokens               45                128               203              257              384               511
-//   4096 x 4096          28 / 42 [60]      30 / 42 [60]      38 / 44 [61]     40 / 46 [61]     44 / 49 [63]      48 / 47 [64]
-//   q + k + v, 6144      36 / 47 [81]      38 / 49 [82]      48 / 51 [83]     68 / 52 [83]     79 / 54 [84]      77 / 54 [85]
-//   10240 x 4096         44 / 42 [61]      53 / 44 [60]      71 / 46 [61]     90 / 48 [62]     102 / 50 [63]     108 / 58 [64]
-//   14336 x 4096         53 / 42 [60]      60 / 44 [60]      79 / 47 [62]     114 / 48 [62]    132 / 52 [63]     142 / 59 [65]
-//   4096 x 14336 Q6_K    52 / 136 [256]    56 / 139 [257]    67 / 143 [259]   95 / 144 [260]   106 / 147 [263]   111 / 147 [265]
-//   2048 x 8192 Q6_K     34 / 82 [152]     36 / 84 [153]     43 / 87 [154]    42 / 87 [155]    47 / 90 [157]     50 / 89 [159]
-//   2048 x 2048          24 / 27 [36]      24 / 28 [38]      32 / 30 [38]     30 / 30 [38]     32 / 33 [38]      32 / 31 [39]
-//   8192 x 2048          26 / 28 [36]      28 / 29 [37]      36 / 30 [38]     53 / 32 [38]     62 / 34 [38]      65 / 33 [40]
-//   1024 x 1024          22 / 19 [24]      22 / 20 [25]      28 / 22 [26]     28 / 22 [26]     28 / 24 [26]      30 / 22 [26]
-//   gate + up 2 x 14336  71 / 82 [120]     81 / 85 [124]     95 / 89 [128]    151 / 93 [130]   162 / 98 [133]    177 / 110 [136]   (one CTA along K)
-// What is not cut gives the same bits in every launch and on either kernel; a matrix that is cut by itself may not be in a
-// launch with others.
 inline int pg_sms() { return state().sm_count > 0 ? state().sm_count : 148; }
-inline int prefill_split_ks(bool q4, int tiles, size_t seq, size_t cols) {
-    if (seq >= (size_t)PT_MAX_TOK) return 0;
-    const int nb = (int)(cols / 256), token_tiles = (int)((seq + PS_TOK - 1) / PS_TOK);
-    int ks = nb < 4 || (nb < 16 && seq > 128) ? 1 : nb < 32 ? 4 : PS_MAX_KS;
-    while (ks >= 4 && tiles * token_tiles * ks > 2 * pg_sms()) ks /= 2;
-    if (ks >= 4) return ks;
-    return (nb < 4 && seq <= 64) || (q4 && tiles >= pg_sms() && seq <= 128) ? 1 : 0;
-}
 inline int pg_pairs() { return std::max(1, pg_sms() / 2); }
-// Tokens per tile of the paired kernels (two parts, multiples of 32): the width that gives the least rounds x cost(width).  In one
-// round the narrowest of those: more pairs share the accumulators' way back (448 tokens: 4096 x 4096 51 -> 48 us, 2048 x 2048 34 -> 30);
-// in several the widest, which dequantises least.
-template <class P, class F>
-inline void pg_pair_tiles(P &p, int row_pairs, int seq, F &&cost) {
-    const int first = (seq + PT_MAX_TOK - 1) / PT_MAX_TOK;
+int prefill_clusters(int ks);   // clusters of 2 ks CTAs that run at the same time (0: unknown)
+// Tokens of a tile and pairs along K: the least of a model of the time in ns, fitted to 1184 launches (14 shapes of 1024 to 32768
+// rows, 1024 to 14336 columns, both formats, 20 to 2048 tokens, all cuts): what it picks is 0.4 % above the fastest on
+// average, 16 % at most (2048 x 2048 at 203 tokens: 21.5 against 18.5 us).  A block of K costs its dequantisation and, above 128
+// tokens, ever more of the tensor pipe; a tile of two parts has the shallow ring; every round its fill and its way back; a cut its sum.
+inline long prefill_pair_tiles(PtParams &P, bool q4) {
+    const int row_pairs = (P.row_tiles + 1) / 2, nb = P.cols / 256, first = (P.seq + PT_TOK - 1) / PT_TOK;
+    // Launches whose tiles fill the chip, and rows of less than 16 blocks above 128 tokens, are summed in one chain along K in
+    // portions of any length: the same bits.  (2048 x 2048 at 203 tokens would take 18.5 us in two chains, 20.5 in one.)
+    const bool cut = nb >= 4 && (nb >= 16 || P.seq <= 128) && P.row_tiles * ((P.seq + 255) / 256) * 4 <= 2 * pg_sms();
     long best = -1;
-    int nt = PT_MAX_TOK;
-    for (int n = first; n <= 2 * first; n++) {
-        const int w = std::max(((seq + n - 1) / n + 31) & ~31, 64);
-        const long rounds = (row_pairs * ((seq + w - 1) / w) + pg_pairs() - 1) / pg_pairs(), c = rounds * cost(w);
-        if (best < 0 || c < best || (c == best && rounds == 1)) best = c, nt = w;
+    for (int n = first; n <= 3 * first; n++) {
+        int nt = std::max(((P.seq + n - 1) / n + 15) & ~15, 32);
+        if (nt > 256) nt = (nt + 31) & ~31;
+        const int token_tiles = (P.seq + nt - 1) / nt, tiles = row_pairs * token_tiles;
+        for (int ks = 1; ks <= (cut ? PT_MAX_KS : 1); ks++) {
+            if (ks > 1 && tiles > prefill_clusters(ks)) continue;
+            const long rounds = ks > 1 ? 1 : (tiles + pg_pairs() - 1) / pg_pairs(), blocks = rounds * ((nb + ks - 1) / ks), over = std::max(nt - 128, 0);
+            const long block = (q4 ? 1088 + over * 13 / 10 : P.skew ? 2500 : 1452 + over) + (nt <= 256 ? 0 : q4 ? 410 : 279);
+            const long ns = blocks * block + rounds * (2400 + 5 * nt) + (ks > 1 ? 126 + 15 * nt : 0);
+            if (best < 0 || ns < best) best = ns, P.nt = nt, P.ks = ks, P.token_tiles = token_tiles, P.tiles = tiles;
+        }
     }
-    p.n1 = (nt / 2 + 31) & ~31;
-    p.n2 = nt - p.n1;
-    p.token_tiles = (seq + nt - 1) / nt;
-    p.tiles = row_pairs * p.token_tiles;
+    return best;
+}
+// The same of prefill_gemm_wide_kernel: tokens of a tile, in two parts (multiples of 32)
+inline long prefill_wide_tiles(PwParams &P) {
+    const int row_pairs = (P.row_tiles + 1) / 2, nb = P.cols / 256, first = (P.seq + PW_TOK - 1) / PW_TOK;
+    long best = -1;
+    for (int n = first; n <= 2 * first; n++) {
+        const int nt = std::max(((P.seq + n - 1) / n + 31) & ~31, 64), token_tiles = (P.seq + nt - 1) / nt, tiles = row_pairs * token_tiles;
+        const long rounds = (tiles + pg_pairs() - 1) / pg_pairs(), ns = rounds * (nb * (2500 + 4 * std::max(nt - 450, 0)) + 2400 + 15 * nt);
+        if (best < 0 || ns < best) best = ns, P.n1 = (nt / 2 + 31) & ~31, P.n2 = nt - P.n1, P.token_tiles = token_tiles, P.tiles = tiles;
+    }
+    return best;
 }
 // `tiles`: row tiles of all jobs
 inline int launch_prefill_gemm_tiles(cudaStream_t s, const PgJobs &jobs, int tiles, size_t seq, size_t cols, const uint16_t *xb, int *dev_error) {
     bool q4 = true;
     for (int i = 0; i < jobs.n; i++) q4 = q4 && jobs.j[i].type == TYPE_Q4_K;
-    const int ks = prefill_split_ks(q4, tiles, seq, cols);
-    if (ks == 0) {
+    // Up to 128 tokens of rows of less than four blocks: two CTAs per SM and no cluster start faster (256 x 256 at two tokens 13 against 15 us,
+    // 20480 x 512 17.4 against 19.5; of four blocks the pairs are, 1024 x 1024 at 45 tokens 22 against 17.5).
+    if (cols >= 1024 || seq > 128) {
         PtParams P;
+        PwParams W;
+        P.seq = W.seq = (int)seq;
+        P.cols = W.cols = (int)cols;
+        P.row_tiles = W.row_tiles = tiles;
+        P.skew = 0;
+        for (int i = 0; i < jobs.n; i++)
+            if (((uintptr_t)jobs.j[i].w | (uintptr_t)jobs.j[i].w2 | row_bytes_of(jobs.j[i].type, cols)) & 15u) P.skew |= 1 << i;
+        W.direct = P.skew;
+        const bool wide = prefill_wide_tiles(W) < prefill_pair_tiles(P, q4);
         PtMaps maps;
+        PwMaps wmaps;
         memset(&maps, 0, sizeof(maps));
-        P.seq = (int)seq;
-        P.cols = (int)cols;
-        P.row_tiles = tiles;
-        P.direct = 0;
-        // a narrower tile than 450 tokens is no faster: its stages take as long as dequantising them does
-        pg_pair_tiles(P, (tiles + 1) / 2, P.seq, [](int w) { return std::max(w, 450) + 24; });
-        RNB_TRY(encode_token_map(&maps.xa, xb, seq, cols, 0, P.n1 / 2));
-        RNB_TRY(encode_token_map(&maps.xb, xb, seq, cols, 0, P.n2 / 2));
+        memset(&wmaps, 0, sizeof(wmaps));
+        if (wide) {
+            RNB_TRY(encode_token_map(&wmaps.xa, xb, seq, cols, 0, W.n1 / 2));
+            RNB_TRY(encode_token_map(&wmaps.xb, xb, seq, cols, 0, W.n2 / 2));
+        } else
+            RNB_TRY(encode_token_map(&maps.x, xb, seq, cols, 0, P.nt > 256 ? P.nt / 4 : P.nt / 2));
         for (int i = 0; i < jobs.n; i++) {
             const PgJob &j = jobs.j[i];
             const size_t rb = row_bytes_of(j.type, cols);
-            if ((((uintptr_t)j.w | (uintptr_t)j.w2 | rb) & 15u) != 0) {
-                P.direct |= 1 << i;
-                continue;
-            }
             const uint32_t box = j.type == TYPE_Q4_K ? PT_Q4_PITCH : PT_Q6_PITCH;
-            RNB_TRY(encode_weight_map(reinterpret_cast<GmTensorMap *>(&maps.w[i]), j.w, (size_t)j.rows, rb, box, PG_ROWS / 2));
-            if (j.w2) RNB_TRY(encode_weight_map(reinterpret_cast<GmTensorMap *>(&maps.w2), j.w2, (size_t)j.rows, rb, box, PG_ROWS / 2));
+            const bool skew = (P.skew >> i) & 1;
+            if (skew && wide) continue;
+            for (int m = 0; m < (j.w2 ? 2 : 1); m++) {
+                const uint8_t *w = m ? j.w2 : j.w;
+                PgTensorMap *to = wide ? (m ? &wmaps.w2 : &wmaps.w[i]) : m ? maps.w2 : maps.w[i];
+                if (!skew) RNB_TRY(encode_weight_map(reinterpret_cast<GmTensorMap *>(to), w, (size_t)j.rows, rb, box, PG_ROWS / 2));
+                for (int r = 0; skew && r < 8; r++) {
+                    // matrices of less than eight rows: the maps of those that are missing are of the first (never stored)
+                    const uint8_t *row = w + (r < j.rows ? (size_t)r * rb : 0);
+                    const size_t off = (uintptr_t)row & 15u, n = r < j.rows ? ((size_t)j.rows - r + 7) / 8 : 1;
+                    RNB_TRY(encode_weight_map(reinterpret_cast<GmTensorMap *>(to + r), row - off, n, 8 * rb, box, j.w2 ? 8 : 16, off + rb));
+                }
+            }
         }
-        RNB_CU(launch_k_cluster(prefill_gemm_pair_kernel, dim3((unsigned)(2 * std::min(P.tiles, pg_pairs()))), dim3(PT_THREADS), PT_SMEM, s, dim3(2), jobs, maps, P, dev_error));
+        if (wide) {
+            RNB_CU(launch_k_cluster(prefill_gemm_wide_kernel, dim3((unsigned)(2 * std::min(W.tiles, pg_pairs()))), dim3(PW_THREADS), PW_SMEM, s, dim3(2), jobs, wmaps, W, dev_error));
+            return RNB_B200_OK;
+        }
+        const int pairs = P.ks > 1 ? P.tiles : std::min(P.tiles, pg_pairs());
+        const dim3 grid((unsigned)(2 * P.ks * pairs)), cluster(2u * (unsigned)P.ks);
+        RNB_CU(P.ks > 1 ? launch_k_cluster(prefill_gemm_pair_kernel<true>, grid, dim3(PT_THREADS), PT_SMEM, s, cluster, jobs, maps, P, dev_error)
+                        : launch_k_cluster(prefill_gemm_pair_kernel<false>, grid, dim3(PT_THREADS), PT_SMEM, s, cluster, jobs, maps, P, dev_error));
         return RNB_B200_OK;
     }
     PgTensorMap tmap;
     PsParams P;
-    const int token_tiles = (int)((seq + PS_TOK - 1) / PS_TOK);
     P.seq = (int)seq;
     P.cols = (int)cols;
-    P.ks = ks;
-    P.nt = ((P.seq + token_tiles - 1) / token_tiles + 15) & ~15;
+    P.nt = (P.seq + 15) & ~15;
     P.stages = std::min<int>(PS_MAX_STAGES, (int)(PS_SMEM_STAGES / ((uint32_t)P.nt * 128u + PG_B_BYTES)));
     P.tmem_cols = 32;
     while ((int)P.tmem_cols < P.nt) P.tmem_cols *= 2;
     RNB_TRY(encode_token_map(&tmap, xb, seq, cols, 0, P.nt));
-    const dim3 grid((unsigned)(tiles * ks), (unsigned)token_tiles);
-    RNB_CU(launch_k_cluster(prefill_gemm_split_kernel, grid, dim3(PS_THREADS), PS_SMEM, s, dim3((unsigned)ks), jobs, tmap, P, dev_error));
+    RNB_CU(launch_k(prefill_gemm_split_kernel, dim3((unsigned)tiles), dim3(PS_THREADS), PS_SMEM, s, jobs, tmap, P, dev_error));
     return RNB_B200_OK;
 }
 inline int launch_prefill_gemm_multi(cudaStream_t s, int n, const int *types, const uint8_t *const *w, const size_t *rows, float *const *y,

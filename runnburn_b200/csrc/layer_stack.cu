@@ -737,6 +737,24 @@ uint64_t LayerStack::cache_bytes_per_pos() const {
 }
 
 // ---- matrix products ------------------------------------------------------------------------------
+// Tokens per tile of dense_gemm_pair_kernel (two parts, multiples of 32): the width that gives the least rounds x cost.  In one
+// round the narrowest of those: more pairs share the accumulators' way back; in several the widest.  A stage is bound by the
+// tensor pipe (two cycles a token) or by its copies (16 KB of weights cost as much as 256 tokens).
+static void dense_pair_tiles(DensePair &p, int row_pairs, int seq) {
+    auto cost = [](int w) { return std::max(2 * w, w + 256) + 48; };
+    const int first = (seq + DQ_TOK - 1) / DQ_TOK;
+    long best = -1;
+    int nt = DQ_TOK;
+    for (int n = first; n <= 2 * first; n++) {
+        const int w = std::max(((seq + n - 1) / n + 31) & ~31, 64);
+        const long rounds = (row_pairs * ((seq + w - 1) / w) + pg_pairs() - 1) / pg_pairs(), c = rounds * cost(w);
+        if (best < 0 || c < best || (c == best && rounds == 1)) best = c, nt = w;
+    }
+    p.n1 = (nt / 2 + 31) & ~31;
+    p.n2 = nt - p.n1;
+    p.token_tiles = (seq + nt - 1) / nt;
+    p.tiles = row_pairs * p.token_tiles;
+}
 int LayerStack::matmul(cudaStream_t s, int n, const Mm *jobs, int n_jobs, int *err) {
     if (n_jobs < 1 || n_jobs > DENSE_MAX_JOBS) return fail(RNB_B200_VALIDATION_FAILED, "stack: %d matrices in one launch", n_jobs);
     if (n <= SMALL) {
@@ -811,8 +829,7 @@ int LayerStack::matmul(cudaStream_t s, int n, const Mm *jobs, int n_jobs, int *e
             const int per = jobs[i].w2 ? DG_ROWS : 2 * DG_ROWS;
             row_pairs += (jobs[i].w->rows + per - 1) / per;
         }
-        // a stage is bound by the tensor pipe (two cycles a token) or by its copies (16 KB of weights cost as much as 256 tokens)
-        if (!split) pg_pair_tiles(Q, row_pairs, n, [](int w) { return std::max(2 * w, w + 256) + 48; });
+        if (!split) dense_pair_tiles(Q, row_pairs, n);
         tiles = 0;
         for (int i = 0; i < n_jobs; i++) {
             DenseGemmJob &j = J.j[i];

@@ -6,13 +6,11 @@
 // crates/rnb-cpu/src/quantize/dequant.rs:353-381 (Q4_K) and :780-807 (Q6_K) in f32 and rounds
 // once to bf16.
 //
-// What the two kernels share (prefill_gemm_pair.cuh: long prompts on pairs of SMs; prefill_gemm_split.cuh: short ones with K
-// cut over a cluster): the weight tile is the M operand (tensor-memory lane = weight row), the tokens the N operand.  K
-// advances 64 elements per stage (one Q4_K group, a quarter of a super-block); the operand tiles are K-major in the 128-byte
-// swizzle the MMA descriptors expect:
+// What the two kernels share (prefill_gemm_pair.cuh: pairs of SMs, weights in tensor memory; prefill_gemm_split.cuh: a few tokens of
+// short rows, weights in shared memory): the weight tile is the M operand (tensor-memory lane = weight row), the tokens the N
+// operand.  Operand tiles in shared memory are 64 elements of K, K-major in the 128-byte swizzle the MMA descriptors expect:
 //   byte offset of (row r, 16-byte chunk c) = (r / 8) * 1024 + (r % 8) * 128 + ((c ^ (r % 8)) * 16).
-// Tokens come in by tiled TMA copies (rows past the end of the batch read as zeros); a weight row's stage is dequantised by two
-// threads, each half of the 64 elements: Q4_K low or high nibbles, Q6_K the first or second 32.  Every wait is bounded; a
+// Tokens come in by tiled TMA copies (rows past the end of the batch read as zeros).  Every wait is bounded; a
 // timeout sets the error flag and all roles still meet at the final barrier, where the tensor memory is freed.
 #pragma once
 #include <cuda_bf16.h>

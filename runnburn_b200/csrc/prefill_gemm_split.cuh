@@ -1,27 +1,19 @@
-// Prefill matmul for short prompts: the same product as prefill_gemm_pair_kernel (dequantised bf16 weights x bf16 tokens,
-// f32 accumulators in tensor memory), cut so that a few hundred tokens still occupy the chip.
+// Prefill matmul of short rows (less than four blocks) for up to 128 tokens: the product of prefill_gemm_pair.cuh with two CTAs
+// of one SM each instead of a pair, weights dequantised into shared memory.  And what the cut kernels share: the sum over a cluster.
 //
-// A CTA owns 128 weight rows x up to 256 tokens and a part of K; the `ks` CTAs of a thread-block cluster share a tile
-// and add their accumulators over distributed shared memory in rank order (the same bits on every run, whichever CTA
-// adds).  A tile of all tokens per CTA leaves 32 CTAs for the 4096 rows of an output projection on 148 SMs, each with a
-// chain of 64 to 224 stages; with K cut in 8 the chain is 8 to 28 stages on 256 CTAs.
+// A CTA owns 128 weight rows x all tokens.  A stage is 64 elements of K: nt tokens x 128 bytes by one tiled TMA copy, and 128 weight
+// rows that eight warps dequantise straight into the operand tile (layouts as in prefill_gemm.cuh).  Weights do not depend on the
+// previous launch: the CTA asks L2 for its rows and dequantises its first stages before the dependency wait; only the token
+// copies and the stores come after it.  Warps 0-7 dequantise, then store; warp 8 issues the MMAs, warp 9 the token copies.  Every
+// wait is bounded; after a timeout all threads still meet at the last barriers.
 //
-// Two CTAs per SM.  A stage is 64 elements of K: nt tokens x 128 bytes by one tiled TMA copy, and 128 weight rows that
-// eight warps dequantise straight into the operand tile (layouts as in prefill_gemm.cuh).  Weights do not depend on the
-// previous launch: the CTA asks L2 for its whole part of every row and dequantises its first stages before the
-// dependency wait; only the token copies and the stores come after it.  Warps 0-7 dequantise, then reduce and store;
-// warp 8 issues the MMAs, warp 9 the token copies.  Every wait is bounded; after a timeout all threads still meet at
-// the cluster barriers.
-//
-// What bounds it: the dequantising warps' chain of a stage (about 800 cycles per SM and stage at any token count, 40 % of
-// the issue slots, tensor pipe 28 % busy at 203 tokens).  Seven matmuls of an 8B layer at 203 tokens: 226 us, with the
-// 512-token tiles 507 us; of a 1B layer at 45 tokens 84 against 252 us.
+// What bounds it: fill and drain of a launch of four to twelve stages.
 #pragma once
 #include "prefill_gemm.cuh"
 
 namespace rnb {
 
-constexpr int PS_TOK = 256;        // most tokens per CTA
+constexpr int PS_TOK = 128;        // most tokens
 constexpr int PS_THREADS = 320;
 constexpr int PS_MAX_STAGES = 5;
 constexpr uint32_t PS_SMEM_STAGES = 96 * 1024;   // operand stages; the reduction reuses them: 64 KB of slots, 32 KB of exchange
@@ -29,7 +21,7 @@ constexpr size_t PS_SMEM = PS_SMEM_STAGES + 1024;
 constexpr int PS_MAX_KS = 8;
 
 struct PsParams {
-    int seq, cols, nt, stages, ks;   // nt: tokens per CTA (multiple of 16), ks: CTAs along K (the cluster)
+    int seq, cols, nt, stages;   // nt: tokens, rounded up to a multiple of 16
     uint32_t tmem_cols;
 };
 
@@ -62,22 +54,27 @@ __device__ __forceinline__ uint32_t ps_map(uint32_t addr, int rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
     return r;
 }
+__device__ __forceinline__ void ps_st_remote4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
 __device__ __forceinline__ void ps_st_remote(uint32_t addr, uint32_t v) { asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
 
 // Adds the accumulators of a cluster's ks CTAs (one: its own).  A round gives every CTA up to ps_per_round chunks of
 // SUB * GROUPS tokens: the others send it theirs of those chunks, it adds them in rank order with its own and calls
 // f(chunk, count, sums).  Two cluster barriers a round, so few rounds: one or two at 256 tokens.  A worker warp holds the rows of
-// lane quarter q and a chunk's tokens group * SUB ..; all threads of the CTA come through here.  `smem` takes PS_SLOT_BYTES for the
-// accumulators that arrive.
+// lane quarter q and a chunk's tokens group * SUB ..; all threads of the CTA come through here.  `smem` takes BYTES for the
+// accumulators that arrive, four tokens of a row at a time (one at a time: 203 tokens of 4096 x 14336 over three pairs 56 -> 51 us).  CTA r
+// of the sum is CTA step * r + first of the cluster.
 constexpr uint32_t PS_SLOT_BYTES = 64 * 1024;
-__host__ __device__ inline int ps_per_round(int ks, uint32_t slot) { return ks > 1 ? (int)(PS_SLOT_BYTES / slot) / (ks - 1) : 1; }
-template <int SUB, int GROUPS, class F>
-__device__ __forceinline__ void ps_reduce(int ks, int kr, int n_chunks, uint8_t *smem, uint32_t tmem, bool worker, int q, int group, bool fin, F &&f) {
+__host__ __device__ inline int ps_per_round(int ks, uint32_t slot, uint32_t bytes = PS_SLOT_BYTES) { return ks > 1 ? (int)(bytes / slot) / (ks - 1) : 1; }
+template <int SUB, int GROUPS, uint32_t BYTES = PS_SLOT_BYTES, class F>
+__device__ __forceinline__ void ps_reduce(int ks, int kr, int n_chunks, uint8_t *smem, uint32_t tmem, bool worker, int q, int group, bool fin, F &&f,
+                                          int step = 1, int first = 0) {
     constexpr int CT = SUB * GROUPS;                  // tokens per chunk
-    constexpr uint32_t SLOT = CT * PG_ROWS * 4;       // one CTA's accumulators of a chunk: [token][row]
-    static_assert((PS_MAX_KS / 2 - 1) * SLOT <= PS_SLOT_BYTES, "a slot per sender");
-    const int lane = threadIdx.x & 31, M = ps_per_round(ks, SLOT);
-    const uint32_t base = smem_u32(smem), mine = (uint32_t)(group * SUB * PG_ROWS + q * 32 + lane) * 4u;
+    constexpr uint32_t SLOT = CT * PG_ROWS * 4;       // one CTA's accumulators of a chunk: [four tokens][row][token]
+    static_assert((PS_MAX_KS / 2 - 1) * SLOT <= BYTES, "a slot per sender");
+    const int lane = threadIdx.x & 31, M = ps_per_round(ks, SLOT, BYTES);
+    const uint32_t base = smem_u32(smem), mine = (uint32_t)(group * SUB * PG_ROWS + (q * 32 + lane) * 4) * 4u;
     const uint32_t lanes = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(group * SUB);
     int count = 0;
     for (int c0 = 0; c0 < n_chunks; c0 += M * ks) {
@@ -91,9 +88,10 @@ __device__ __forceinline__ void ps_reduce(int ks, int kr, int n_chunks, uint8_t 
                         if (cc >= n_chunks) break;
                         uint32_t v[SUB];
                         if (fin) ps_tmem_ld<SUB>(lanes + (uint32_t)(cc * CT), v);
-                        const uint32_t dst = ps_map(base + (uint32_t)((kr < to ? kr : kr - 1) * M + m) * SLOT + mine, to);
+                        const uint32_t dst = ps_map(base + (uint32_t)((kr < to ? kr : kr - 1) * M + m) * SLOT + mine, step * to + first);
 #pragma unroll
-                        for (int t = 0; t < SUB; t++) ps_st_remote(dst + (uint32_t)(t * PG_ROWS * 4), fin ? v[t] : 0u);
+                        for (int t = 0; t < SUB; t += 4)
+                            ps_st_remote4(dst + (uint32_t)(t * PG_ROWS * 4), fin ? v[t] : 0u, fin ? v[t + 1] : 0u, fin ? v[t + 2] : 0u, fin ? v[t + 3] : 0u);
                     }
                 }
             ps_cluster_sync();
@@ -105,27 +103,30 @@ __device__ __forceinline__ void ps_reduce(int ks, int kr, int n_chunks, uint8_t 
             if (fin) ps_tmem_ld<SUB>(lanes + (uint32_t)(cc * CT), v);
             float s[SUB];
 #pragma unroll
-            for (int t = 0; t < SUB; t++) {
-                const float own = fin ? __uint_as_float(v[t]) : 0.f;
-                const float *part = reinterpret_cast<const float *>(smem + (size_t)m * SLOT + mine) + t * PG_ROWS;
-                s[t] = kr == 0 ? own : part[0];
-                for (int r = 1; r < ks; r++) s[t] += r == kr ? own : part[(size_t)(r < kr ? r : r - 1) * M * (SLOT / 4)];
+            for (int t = 0; t < SUB; t += 4) {
+                const uint8_t *part = smem + (size_t)m * SLOT + mine + t * PG_ROWS * 4;
+                for (int r = 0; r < ks; r++) {
+                    const float4 a = r == kr ? fin ? make_float4(__uint_as_float(v[t]), __uint_as_float(v[t + 1]), __uint_as_float(v[t + 2]), __uint_as_float(v[t + 3]))
+                                                   : make_float4(0.f, 0.f, 0.f, 0.f)
+                                             : *reinterpret_cast<const float4 *>(part + (size_t)(r < kr ? r : r - 1) * M * SLOT);
+                    s[t] = r ? s[t] + a.x : a.x, s[t + 1] = r ? s[t + 1] + a.y : a.y, s[t + 2] = r ? s[t + 2] + a.z : a.z, s[t + 3] = r ? s[t + 3] + a.w : a.w;
+                }
             }
             f(cc, count++, s);
         }
     }
 }
 
-// Sums and stores a tile with eight worker warps: warp w holds tokens (w >> 2) * SUB .. of a chunk.
+// Stores a tile with eight worker warps: warp w holds tokens (w >> 2) * SUB .. of a chunk.
 template <int SUB>
-__device__ __forceinline__ void ps_finish(const PgJob &job, const PsParams &P, uint8_t *smem, uint32_t tmem, int kr, int n0, int m0, bool fin) {
+__device__ __forceinline__ void ps_finish(const PgJob &job, const PsParams &P, uint8_t *smem, uint32_t tmem, int n0, bool fin) {
     constexpr int CT = 2 * SUB;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, q = warp & 3, sub = (warp >> 2) & 1, rows = job.rows;
-    const int end = min(P.seq, m0 + P.nt), n_chunks = (end - m0 + CT - 1) / CT;
+    const int end = P.seq, n_chunks = (end + CT - 1) / CT;
     float *ex = reinterpret_cast<float *>(smem + PS_SLOT_BYTES);   // gate / up exchange, two buffers in turn
     const bool pair = job.w2 != nullptr;
-    ps_reduce<SUB, 2>(P.ks, kr, n_chunks, smem, tmem, warp < 8, q, sub, fin, [&](int cc, int j, const float (&s)[SUB]) {
-        const int tok0 = m0 + cc * CT;
+    ps_reduce<SUB, 2>(1, 0, n_chunks, smem, tmem, warp < 8, q, sub, fin, [&](int cc, int j, const float (&s)[SUB]) {
+        const int tok0 = cc * CT;
         if (pair) {
             // gate rows on lane quarters 0 and 1, the same rows of up on 2 and 3: each warp finishes half of its tokens
             float *buf = ex + (size_t)(j & 1) * (CT * PG_ROWS);
@@ -151,7 +152,7 @@ __device__ __forceinline__ void ps_finish(const PgJob &job, const PsParams &P, u
     });
 }
 
-// grid = (row tiles of all jobs x ks, token tiles), cluster (ks, 1, 1); 320 threads; dynamic shared memory PS_SMEM.
+// grid = row tiles of all jobs; 320 threads; dynamic shared memory PS_SMEM.
 RNB_GLOBAL void __launch_bounds__(PS_THREADS, 2)
 prefill_gemm_split_kernel(const __grid_constant__ PgJobs jobs, const __grid_constant__ PgTensorMap tmap_x, const PsParams P, int *__restrict__ err_flag) {
     extern __shared__ __align__(1024) uint8_t pg_smem_raw[];
@@ -161,7 +162,7 @@ prefill_gemm_split_kernel(const __grid_constant__ PgJobs jobs, const __grid_cons
     pdl_launch_dependents();
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(pg_smem_raw) + 1023) & ~(uintptr_t)1023);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int tile = (int)blockIdx.x / P.ks, kr = (int)blockIdx.x - tile * P.ks;
+    const int tile = (int)blockIdx.x;
     int jsel = 0;
     for (int i = 1; i < jobs.n; i++)
         if (tile >= jobs.j[i].tile0) jsel = i;
@@ -169,8 +170,8 @@ prefill_gemm_split_kernel(const __grid_constant__ PgJobs jobs, const __grid_cons
     const int rows = job.rows, S = P.stages;
     const bool pair = job.w2 != nullptr, q4 = job.type == TYPE_Q4_K;
     const uint32_t BLK = q4 ? Q4K_BYTES : Q6K_BYTES, x_bytes = (uint32_t)P.nt * 128u, stage_bytes = x_bytes + PG_B_BYTES;
-    const int n0 = (tile - job.tile0) * (pair ? PG_ROWS / 2 : PG_ROWS), m0 = blockIdx.y * P.nt;
-    const int nb = P.cols >> 8, b0 = nb * kr / P.ks, b1 = nb * (kr + 1) / P.ks, KT = (b1 - b0) * 4;   // this CTA's blocks of K
+    const int n0 = (tile - job.tile0) * (pair ? PG_ROWS / 2 : PG_ROWS);
+    const int nb = P.cols >> 8, KT = nb * 4;
     if (tid == 0) {
         for (int s = 0; s < S; s++) {
             mbar_init(&full[s], 9);    // one arrival per dequantising warp + the thread that issues the token copies
@@ -188,8 +189,8 @@ prefill_gemm_split_kernel(const __grid_constant__ PgJobs jobs, const __grid_cons
         const size_t rb = (size_t)nb * BLK;
         // rows past the end repeat the last one (never stored)
         const uint8_t *wr = (pair ? (row < PG_ROWS / 2 ? job.w : job.w2) + (size_t)min(n0 + (row & (PG_ROWS / 2 - 1)), rows - 1) * rb
-                                  : job.w + (size_t)min(n0 + row, rows - 1) * rb) + (size_t)b0 * BLK;
-        for (uint32_t o = 128u * (uint32_t)h; o < (uint32_t)(b1 - b0) * BLK; o += 256u) asm volatile("prefetch.global.L2 [%0];" ::"l"(wr + o));
+                                  : job.w + (size_t)min(n0 + row, rows - 1) * rb);
+        for (uint32_t o = 128u * (uint32_t)h; o < (uint32_t)nb * BLK; o += 256u) asm volatile("prefetch.global.L2 [%0];" ::"l"(wr + o));
         uint8_t *const brow = smem + x_bytes + (row >> 3) * 1024 + rr * 128;
         int s = 0;
         uint32_t phase = 0;
@@ -210,9 +211,9 @@ prefill_gemm_split_kernel(const __grid_constant__ PgJobs jobs, const __grid_cons
                 for (int g = 0; g < 4; g++) qq[g] = ldg_nc_u4(blk + 16 + 32 * g + 16 * h);
             };
             load(wr, hh, qc);
-            for (int b = b0; b < b1 && ok; b++) {
+            for (int b = 0; b < nb && ok; b++) {
                 wr += BLK;
-                if (b + 1 < b1) load(wr, hn, qn);
+                if (b + 1 < nb) load(wr, hn, qn);
                 const uint32_t ox = __shfl_xor_sync(0xffffffffu, hh.x, 1), oy = __shfl_xor_sync(0xffffffffu, hh.y, 1);
                 const uint4 hdr = h ? make_uint4(ox, oy, hh.x, hh.y) : make_uint4(hh.x, hh.y, ox, oy);
 #pragma unroll
@@ -230,8 +231,8 @@ prefill_gemm_split_kernel(const __grid_constant__ PgJobs jobs, const __grid_cons
         } else {
             PgRawQ6 cur, nxt;
             pg_load_q6(cur, wr, 0, h);
-            for (int hb = 0; hb < 2 * (b1 - b0) && ok; hb++) {   // half blocks of 128 elements, two stages each
-                if (hb + 1 < 2 * (b1 - b0)) pg_load_q6(nxt, wr + (size_t)((hb + 1) >> 1) * BLK, (hb + 1) & 1, h);
+            for (int hb = 0; hb < 2 * nb && ok; hb++) {   // half blocks of 128 elements, two stages each
+                if (hb + 1 < 2 * nb) pg_load_q6(nxt, wr + (size_t)((hb + 1) >> 1) * BLK, (hb + 1) & 1, h);
 #pragma unroll
                 for (int g = 0; g < 2; g++) {
                     if (ok) ok = begin();
@@ -275,7 +276,7 @@ prefill_gemm_split_kernel(const __grid_constant__ PgJobs jobs, const __grid_cons
             ok = mbar_wait_bounded(&empty[s], phase ^ 1u);
             if (!ok) break;
             mbar_arrive_expect_tx(&full[s], x_bytes);
-            pg_tma_2d(smem_u32(smem + (uint32_t)s * stage_bytes), &tmap_x, (b0 * 4 + kt) * PG_K, m0, &full[s]);
+            pg_tma_2d(smem_u32(smem + (uint32_t)s * stage_bytes), &tmap_x, kt * PG_K, 0, &full[s]);
             issued = kt + 1;
             if (++s == S) s = 0, phase ^= 1u;
         }
@@ -289,9 +290,7 @@ prefill_gemm_split_kernel(const __grid_constant__ PgJobs jobs, const __grid_cons
     if (!fin) s_failed = 1;
     pg_fence_after();
     const uint32_t tmem = tmem_slot;
-    if (P.ks > 1) ps_cluster_sync();   // every CTA's MMAs have read their stages: the slots may be written
-    if (P.ks > 4) ps_finish<8>(job, P, smem, tmem, kr, n0, m0, fin);
-    else ps_finish<16>(job, P, smem, tmem, kr, n0, m0, fin);
+    ps_finish<16>(job, P, smem, tmem, n0, fin);
     pg_fence_before();
     __syncthreads();
     if (warp == 8) {
