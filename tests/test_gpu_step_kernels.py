@@ -1,0 +1,57 @@
+"""Kernels of a decode step at the sizes where their splits end, bit for bit against the oracle: attention in position order (an
+eighth of the positions per CTA, groups of 16, slabs of 512 positions; heads of a cluster on one or two KV heads) and the
+matvec of rows that bulk copies cannot fetch."""
+import numpy as np
+import pytest
+
+import oracle as orc
+from synth import Q4_K, Q6_K, llama_description, random_blocks
+from test_gpu_ops import bits_equal, ops  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("kv_len", [1, 7, 8, 9, 15, 16, 17, 63, 65, 127, 255, 300, 496, 511, 512])
+@pytest.mark.parametrize("heads,kvh", [(4, 2), (3, 3), (2, 2), (1, 1), (8, 1)])
+def test_attention_in_position_order(ops, heads, kvh, kv_len):
+    rng = np.random.default_rng(heads * 1000 + kv_len)
+    q = (rng.standard_normal(heads * 128) * 3).astype(np.float32)
+    k, v = (orc.f32_to_f16_bits(rng.standard_normal(kv_len * kvh * 128)) for _ in range(2))
+    scale = 1.0 / np.sqrt(128.0)
+    assert np.array_equal(ops.attention_decode_hd128(q, k, v, kv_len, heads, kvh, scale), orc.attention_decode(q, k, v, heads, kvh, 128, kv_len, scale))
+
+
+def test_attention_in_position_order_past_a_slab():
+    """A limit of 1100 positions: the second and third slab of values, in a decoder's step."""
+    import runnburn_b200 as r
+    desc = llama_description(seed=5, n_layer=1, hidden=256, n_head=2, n_kv_head=1, n_ff=512, vocab=512)
+    n = 1100
+    dec = r.Decoder(r.ModelConfig(max_ctx=n, **desc["cfg"]))
+    dec.set_exact_attention_max(n)
+    dec.load_description(desc)
+    ref = orc.Model(desc, n)
+    for pos, tok in enumerate(np.random.default_rng(1).integers(0, 512, n).tolist()):
+        want = pos in (511, 512, 527, 1023, 1024, n - 1)
+        got = dec.step(tok, pos, want_logits=want)
+        ref_logits = ref.decode(tok, pos)
+        if want:
+            assert np.array_equal(got[1], ref_logits), pos
+    dec.close()
+    ref.close()
+
+
+@pytest.mark.parametrize("t,blocks", [(Q6_K, n) for n in (1, 2, 3, 5, 7, 9, 11, 15, 17)] + [(Q4_K, 1), (Q4_K, 9)])
+@pytest.mark.parametrize("rows", [1, 4, 5, 1027])
+def test_matvec_rows_at_any_even_address(ops, t, blocks, rows):
+    rng = np.random.default_rng(rows * 100 + blocks)
+    cols = 256 * blocks
+    w, x = random_blocks(rng, t, rows, cols), rng.standard_normal(cols).astype(np.float32)
+    want = orc.gemv(t, w, x, rows, cols)
+    assert bits_equal(ops.gemv(t, w, rows, cols, x), want)
+    ops.clear_q4k_cache()
+    for start in (1, 2, 6):
+        backing = np.zeros(w.size + 64, np.uint8)
+        backing[start:start + w.size] = w
+        ops.prewarm_q4k_weights([backing])
+        assert bits_equal(ops.gemv(t, backing[start:start + w.size], rows, cols, x), want), start
+        ops.clear_q4k_cache()
