@@ -834,35 +834,54 @@ flash_decode_reduce_q8k_wide_kernel(const float *__restrict__ partials, int n_ch
 // 2^(k/32) * P(r) in binary64 (a 32-entry table of 2^(i/32) and a cubic in r) and rounds once to
 // f32.  The same evaluation here agrees with it on every input up to the binary64 rounding of
 // intermediate steps, which is 2^29 times finer than an f32 ulp.
+//
+// Two heads (a Q8_K block of the output) belong to a cluster of eight CTAs.  A CTA computes the scores of an eighth of the
+// positions for both heads and hands them to the four CTAs of each head; a CTA then takes the softmax of its head, which needs all
+// scores, and 32 of the head's output dims: products by all threads, sums over the positions by one warp.  Values travel into
+// shared memory while the softmax runs.
+//
+// What bounds it: a chain of latencies (launch, one round trip for keys, three cluster barriers, 1000 cycles each) and the two sums
+// in position order, four to six cycles a position each.  In the step of 16 heads on 8 KV heads: 6.5 us at 100 positions, 11.5 at 345
+// (two heads per CTA, without a cluster: 7.4 and 22.3).
 // ---------------------------------------------------------------------------------------------
-constexpr int AX_THREADS = 512;       // two heads per CTA
-constexpr int AX_MAX_LEN = 4096;      // scores of both heads: 2 * 4 bytes * 4096 positions = 32 KB
-constexpr int AX_STAGE_BYTES = 32768; // staged K or V rows: 128 positions of one KV head, or 64 of two
-constexpr int AX_STAGE_VECS = AX_STAGE_BYTES / 16 / AX_THREADS;   // 16-byte loads per thread per tile
-inline size_t ax_smem_bytes(int max_len) { return (size_t)AX_STAGE_BYTES + (size_t)max_len * 2 * sizeof(float); }
+constexpr int AX_CTAS = 8, AX_THREADS = 256;
+constexpr int AX_MAX_LEN = 4096;      // scores of a head: 16 KB
+constexpr int AX_SLAB = 512;          // positions of V at a time, 32 dims each
+// pitches: of a position's values (80 bytes), of a dim's products (516): four threads, eight threads apart in the banks
+constexpr int AX_ROW = 80, AX_COL = AX_SLAB + 4;
+constexpr uint32_t AX_PROD = AX_SLAB * AX_ROW, AX_SCORES = AX_PROD + 32 * AX_COL * 4;
+inline size_t ax_smem_bytes(int max_len) { return (size_t)AX_SCORES + (size_t)(max_len + 16) * sizeof(float); }   // reads run ahead by a group of 16
 
-// One tile of K or V rows into registers (16-byte loads, all in flight together), then into the
-// staging buffer.  `shared_kv`: both heads of the CTA read the same KV head, the tile is 128
-// positions of it; otherwise 64 positions of each head's KV head (slot = head).
-struct AxTile {
-    uint4 r[AX_STAGE_VECS];
-};
-__device__ __forceinline__ void ax_fetch(AxTile &t, const uint16_t *__restrict__ base, size_t kv_dim, size_t off0, size_t off1, bool shared_kv,
-                                         int pos0, int kv_len, int tid) {
+__device__ __forceinline__ void ax_copy16(void *dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+// positions pos0.. of 32 dims (64 bytes a position) into the slab
+__device__ __forceinline__ void ax_fetch_values(uint8_t *slab, const uint16_t *__restrict__ v, size_t kv_dim, int pos0, int n, int tid) {
+    for (int i = tid; i < 4 * n; i += AX_THREADS) ax_copy16(slab + AX_ROW * (i >> 2) + 16 * (i & 3), v + (size_t)(pos0 + (i >> 2)) * kv_dim + 8 * (i & 3));
+}
+// start + x[0] + x[1] + ... in order; the next sixteen on their way while these are added
+__device__ __forceinline__ float ax_sum(const float *x, int n, float start) {
+    float4 next[4];
 #pragma unroll
-    for (int i = 0; i < AX_STAGE_VECS; i++) {
-        const int idx = tid + AX_THREADS * i;
-        const int slot = shared_kv ? 0 : idx >> 10, p = shared_kv ? idx >> 4 : (idx & 1023) >> 4, seg = idx & 15;
-        t.r[i] = make_uint4(0, 0, 0, 0);
-        if (pos0 + p < kv_len) t.r[i] = *reinterpret_cast<const uint4 *>(base + (size_t)(pos0 + p) * kv_dim + (slot ? off1 : off0) + seg * 8);
+    for (int u = 0; u < 4; u++) next[u] = *reinterpret_cast<const float4 *>(x + 4 * u);   // past the end: not used
+    int j = 0;
+    for (; j + 16 <= n; j += 16) {
+        float4 p[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) p[u] = next[u];
+        if (j + 32 <= n) {
+#pragma unroll
+            for (int u = 0; u < 4; u++) next[u] = *reinterpret_cast<const float4 *>(x + j + 16 + 4 * u);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) start = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(start, p[u].x), p[u].y), p[u].z), p[u].w);
     }
+    for (; j < n; j++) start = __fadd_rn(start, x[j]);
+    return start;
 }
-__device__ __forceinline__ void ax_store(const AxTile &t, uint16_t *stage, int tid) {
-#pragma unroll
-    for (int i = 0; i < AX_STAGE_VECS; i++) *reinterpret_cast<uint4 *>(stage + (size_t)(tid + AX_THREADS * i) * 8) = t.r[i];
-}
+__device__ __forceinline__ void ax_values_landed() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// grid = ceil(num_heads / 2); dynamic shared memory = ax_smem_bytes(max_len).  Writes `out`
+// grid = AX_CTAS x ceil(num_heads / 2), cluster (AX_CTAS, 1, 1); dynamic shared memory = ax_smem_bytes(max_len).  Writes `out`
 // ([num_heads][128] f32) and/or the Q8_K blocks of the output (`xq_out`, needs an even head
 // count: two heads are one 256-element block).  K and V must be 16-byte aligned.  A context
 // longer than max_len raises the error flag and writes nothing.
@@ -871,156 +890,138 @@ attention_decode_exact_kernel(const float *__restrict__ q, const uint16_t *__res
                               const int *__restrict__ kv_len_dev, int kv_len_host, int max_len, int num_heads, int num_kv_heads,
                               float scale, float *__restrict__ out, uint8_t *__restrict__ xq_out, int *__restrict__ err_flag) {
     pdl_launch_dependents();
-    pdl_wait();
     extern __shared__ __align__(16) uint8_t s_dyn[];
-    uint16_t *stage = reinterpret_cast<uint16_t *>(s_dyn);                    // [slot][position][128]
-    float *s_score = reinterpret_cast<float *>(s_dyn + AX_STAGE_BYTES);       // [2][max_len]
+    uint8_t *const slab = s_dyn;                                              // [position][32 dims]
+    float *const prod = reinterpret_cast<float *>(s_dyn + AX_PROD);           // [32 dims][position]
+    float *const sc = reinterpret_cast<float *>(s_dyn + AX_SCORES);           // [max_len]
     __shared__ unsigned long long s_tab[32];
-    __shared__ float s_red[2][8];
-    __shared__ float s_inv[2];
+    __shared__ float s_red[AX_THREADS / 32];
+    __shared__ float s_inv;
     __shared__ __align__(16) float s_o[2 * HD];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int kv_len = kv_len_dev ? *kv_len_dev + kv_len_host : kv_len_host;
-    if (kv_len < 1 || kv_len > max_len) {
-        if (tid == 0 && err_flag) atomicExch(err_flag, DEV_ERR_BAD_JOB);
-        return;
-    }
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rank = (int)blockIdx.x % AX_CTAS;
     if (tid < 32) s_tab[tid] = c_exp2_tab32[tid];
     const int group = num_heads / num_kv_heads;
     const size_t kv_dim = (size_t)num_kv_heads * HD;
-    const int h0 = blockIdx.x * 2, h1 = min(h0 + 1, num_heads - 1);           // an odd head count repeats the last head
+    const int h0 = ((int)blockIdx.x / AX_CTAS) * 2, h1 = min(h0 + 1, num_heads - 1);   // an odd head count repeats the last head
     const size_t off0 = (size_t)(h0 / group) * HD, off1 = (size_t)(h1 / group) * HD;
     const bool shared_kv = off0 == off1;
-    const int tile_pos = shared_kv ? 128 : 64;
-    const int n_tiles = (kv_len + tile_pos - 1) / tile_pos;
+    const int hs = rank >> 2, d0 = (rank & 3) * 32;                           // this CTA's head, its output dims
+    asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
+    pdl_wait();
+    const int kv_len = kv_len_dev ? *kv_len_dev + kv_len_host : kv_len_host;
+    if (kv_len < 1 || kv_len > max_len) {
+        if (tid == 0 && err_flag) atomicExch(err_flag, DEV_ERR_BAD_JOB);
+        asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+        return;
+    }
+    const uint16_t *const vh = v + (hs ? off1 : off0) + d0;
+    ax_fetch_values(slab, vh, kv_dim, 0, min(kv_len, AX_SLAB), tid);
 
-    // pass 1: scores.  Half-warp (16 lanes) per position, lane l owns dims 16 i + l.
+    // pass 1: scores.  Half-warp (16 lanes) per position, lane l owns dims 16 i + l; four positions' rows in flight.
     {
-        const int l16 = lane & 15, hw = tid >> 4;                             // 32 half-warps
-        // the two halves of a warp can run different trip counts: shuffles name the own half only
-        const unsigned hmask = (lane & 16) ? 0xffff0000u : 0x0000ffffu;
-        // shared KV head: every half-warp serves both heads of its positions; else 16 half-warps per head
-        const int slot = shared_kv ? 0 : hw >> 4, p_first = shared_kv ? hw : hw & 15, p_step = shared_kv ? 32 : 16;
-        const int ha = shared_kv ? h0 : (slot ? h1 : h0), hb = shared_kv ? h1 : ha;
+        const int l16 = lane & 15, hw = tid >> 4, per = (kv_len + AX_CTAS - 1) / AX_CTAS, first = rank * per, last = min(kv_len, first + per);
         float qa[8], qb[8];
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-            qa[i] = q[(size_t)ha * HD + 16 * i + l16];
-            qb[i] = q[(size_t)hb * HD + 16 * i + l16];
+            qa[i] = q[(size_t)h0 * HD + 16 * i + l16];
+            qb[i] = q[(size_t)h1 * HD + 16 * i + l16];
         }
-        AxTile t;
-        ax_fetch(t, k, kv_dim, off0, off1, shared_kv, 0, kv_len, tid);
-        for (int ti = 0; ti < n_tiles; ti++) {
-            const int pos0 = ti * tile_pos, n_here = min(tile_pos, kv_len - pos0);
-            __syncthreads();
-            ax_store(t, stage, tid);
-            __syncthreads();
-            if (ti + 1 < n_tiles) ax_fetch(t, k, kv_dim, off0, off1, shared_kv, pos0 + tile_pos, kv_len, tid);
-            for (int p = p_first; p < n_here; p += p_step) {
-                const uint16_t *row = stage + ((size_t)slot * 64 + p) * HD + l16;
+        // lanes 0-3 hand the first head's score to CTAs 0-3, lanes 4-7 the second's to CTAs 4-7
+        const uint32_t to = ps_map(smem_u32(sc), l16 & 7);
+        bool others = false;
+        auto wait_for_others = [&]() {   // every CTA of the cluster runs: its memory may be written
+            if (!others) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+            others = true;
+        };
+        for (int b = first; b < last; b += 4 * (AX_THREADS / 16)) {   // the same trips for all threads
+            const int j0 = b + hw;
+            uint16_t ka[4][8], kb[4][8];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const int j = min(j0 + u * (AX_THREADS / 16), last - 1);
+                const uint16_t *row = k + (size_t)j * kv_dim + l16;
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    ka[u][i] = row[off0 + 16 * i];
+                    kb[u][i] = shared_kv ? ka[u][i] : row[off1 + 16 * i];
+                }
+            }
+            wait_for_others();
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const int j = j0 + u * (AX_THREADS / 16);
+                if (b + u * (AX_THREADS / 16) >= last) break;
                 float acc0 = 0.0f, acc1 = 0.0f;
 #pragma unroll
                 for (int i = 0; i < 8; i++) {
-                    const float kf = __half2float(__ushort_as_half(row[16 * i]));
-                    acc0 = __fadd_rn(acc0, __fmul_rn(qa[i], kf));
-                    acc1 = __fadd_rn(acc1, __fmul_rn(qb[i], kf));
+                    acc0 = __fadd_rn(acc0, __fmul_rn(qa[i], __half2float(__ushort_as_half(ka[u][i]))));
+                    acc1 = __fadd_rn(acc1, __fmul_rn(qb[i], __half2float(__ushort_as_half(kb[u][i]))));
                 }
                 // lanes l and l + 8 are the reference's two accumulators; then lo + hi, movehdup, movehl
 #pragma unroll
                 for (int o = 8; o >= 4; o >>= 1) {
-                    acc0 = __fadd_rn(acc0, __shfl_xor_sync(hmask, acc0, o));
-                    acc1 = __fadd_rn(acc1, __shfl_xor_sync(hmask, acc1, o));
+                    acc0 = __fadd_rn(acc0, __shfl_xor_sync(0xffffffffu, acc0, o));
+                    acc1 = __fadd_rn(acc1, __shfl_xor_sync(0xffffffffu, acc1, o));
                 }
-                acc0 = __fadd_rn(acc0, __shfl_xor_sync(hmask, acc0, 1));
-                acc1 = __fadd_rn(acc1, __shfl_xor_sync(hmask, acc1, 1));
-                acc0 = __fadd_rn(acc0, __shfl_xor_sync(hmask, acc0, 2));
-                acc1 = __fadd_rn(acc1, __shfl_xor_sync(hmask, acc1, 2));
-                if (l16 == 0) {
-                    if (shared_kv) {
-                        s_score[pos0 + p] = __fmul_rn(acc0, scale);
-                        s_score[max_len + pos0 + p] = __fmul_rn(acc1, scale);
-                    } else {
-                        s_score[(size_t)slot * max_len + pos0 + p] = __fmul_rn(acc0, scale);
-                    }
-                }
+                acc0 = __fadd_rn(acc0, __shfl_xor_sync(0xffffffffu, acc0, 1));
+                acc1 = __fadd_rn(acc1, __shfl_xor_sync(0xffffffffu, acc1, 1));
+                acc0 = __fadd_rn(acc0, __shfl_xor_sync(0xffffffffu, acc0, 2));
+                acc1 = __fadd_rn(acc1, __shfl_xor_sync(0xffffffffu, acc1, 2));
+                if (l16 < AX_CTAS && j < last) ps_st_remote(to + 4u * (uint32_t)j, __float_as_uint(__fmul_rn(l16 < 4 ? acc0 : acc1, scale)));
             }
         }
+        wait_for_others();
     }
-    __syncthreads();
-    const int hs = warp >> 3, th = tid & 255;                                 // head slot, thread within the head
-    const int h = h0 + hs;
-    const bool live = h < num_heads;
-    float *sc = s_score + (size_t)hs * max_len;
-    // V rows of the first tile travel while the softmax runs
-    AxTile tv;
-    ax_fetch(tv, v, kv_dim, off0, off1, shared_kv, 0, kv_len, tid);
+    __syncwarp();
+    ps_cluster_sync();
     // pass 2: max
     float m = -INFINITY;
-    for (int j = th; j < kv_len; j += 256) m = fmaxf(m, sc[j]);
+    for (int j = tid; j < kv_len; j += AX_THREADS) m = fmaxf(m, sc[j]);
     m = warp_max(m);
-    if (lane == 0) s_red[hs][warp & 7] = m;
+    if (lane == 0) s_red[warp] = m;
     __syncthreads();
-    float M = s_red[hs][0];
+    float M = s_red[0];
 #pragma unroll
-    for (int i = 1; i < 8; i++) M = fmaxf(M, s_red[hs][i]);
-    // pass 3: exponentials in parallel, their sum in position order by one thread per head
-    for (int j = th; j < kv_len; j += 256) sc[j] = expf_libm_smem(__fsub_rn(sc[j], M), s_tab);
+    for (int i = 1; i < AX_THREADS / 32; i++) M = fmaxf(M, s_red[i]);
+    // pass 3: exponentials in parallel, their sum in position order by one thread
+    for (int j = tid; j < kv_len; j += AX_THREADS) sc[j] = expf_libm_smem(__fsub_rn(sc[j], M), s_tab);
     __syncthreads();
-    if (th == 0) {
-        float sum = 0.0f;
-        int j = 0;
-        for (; j + 32 <= kv_len; j += 32) {
-            float4 p[8];
-#pragma unroll
-            for (int u = 0; u < 8; u++) p[u] = *reinterpret_cast<const float4 *>(sc + j + 4 * u);
-#pragma unroll
-            for (int u = 0; u < 8; u++) sum = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sum, p[u].x), p[u].y), p[u].z), p[u].w);
-        }
-        for (; j < kv_len; j++) sum = __fadd_rn(sum, sc[j]);
-        s_inv[hs] = sum > 0.0f ? __fdiv_rn(1.0f, sum) : 0.0f;
+    if (tid == 0) {
+        const float sum = ax_sum(sc, kv_len, 0.0f);
+        s_inv = sum > 0.0f ? __fdiv_rn(1.0f, sum) : 0.0f;
     }
     __syncthreads();
-    // pass 4: weights in parallel, then one thread per output dim walks the positions in order
-    {
-        const float inv = s_inv[hs];
-        for (int j = th; j < kv_len; j += 256) sc[j] = __fmul_rn(sc[j], inv);
-    }
+    // pass 4: weights times values in parallel, their sum in position order by one thread per output dim
+    const float inv = s_inv;
     float o = 0.0f;
-    const int v_slot = shared_kv ? 0 : hs;
-    for (int ti = 0; ti < n_tiles; ti++) {
-        const int pos0 = ti * tile_pos, n_here = min(tile_pos, kv_len - pos0);
-        __syncthreads();                                                      // weights written / previous tile consumed
-        ax_store(tv, stage, tid);
-        __syncthreads();
-        if (ti + 1 < n_tiles) ax_fetch(tv, v, kv_dim, off0, off1, shared_kv, pos0 + tile_pos, kv_len, tid);
-        if (th < HD) {
-            const uint16_t *col = stage + (size_t)v_slot * 64 * HD + th;
-            const float *w = sc + pos0;
-            int p = 0;
-            for (; p + 8 <= n_here; p += 8) {
-                float x[8], wt[8];
-#pragma unroll
-                for (int u = 0; u < 8; u++) {
-                    x[u] = __half2float(__ushort_as_half(col[(size_t)(p + u) * HD]));
-                    wt[u] = w[p + u];
-                }
-#pragma unroll
-                for (int u = 0; u < 8; u++) o = __fadd_rn(o, __fmul_rn(x[u], wt[u]));
-            }
-            for (; p < n_here; p++) o = __fadd_rn(o, __fmul_rn(__half2float(__ushort_as_half(col[(size_t)p * HD])), w[p]));
+    for (int pos0 = 0; pos0 < kv_len; pos0 += AX_SLAB) {
+        const int n = min(AX_SLAB, kv_len - pos0);
+        if (pos0 > 0) ax_fetch_values(slab, vh, kv_dim, pos0, n, tid);
+        ax_values_landed();
+        __syncthreads();                                                      // values landed; the products before these have been read
+        for (int p = lane; p < n; p += 32) {                                  // four dims of a position
+            const uint2 x = *reinterpret_cast<const uint2 *>(slab + AX_ROW * p + 8 * warp);
+            const float w = __fmul_rn(sc[pos0 + p], inv);
+            const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&x.x)), c = __half22float2(*reinterpret_cast<const __half2 *>(&x.y));
+            float *to = prod + 4 * warp * AX_COL + p;
+            to[0] = __fmul_rn(a.x, w), to[AX_COL] = __fmul_rn(a.y, w), to[2 * AX_COL] = __fmul_rn(c.x, w), to[3 * AX_COL] = __fmul_rn(c.y, w);
         }
+        __syncthreads();
+        if (warp == 0) o = ax_sum(prod + lane * AX_COL, n, o);
     }
-    if (th < HD) {
-        if (live && out) out[(size_t)h * HD + th] = o;
-        s_o[hs * HD + th] = live ? o : 0.0f;
+    const int h = h0 + hs;
+    const bool live = h < num_heads;
+    if (warp == 0) {
+        if (live && out) out[(size_t)h * HD + d0 + lane] = o;
+        if (xq_out) ps_st_remote(ps_map(smem_u32(s_o + hs * HD + d0 + lane), 0), __float_as_uint(live ? o : 0.0f));
     }
     if (!xq_out) return;
-    __syncthreads();
-    if (tid < 32) {
+    ps_cluster_sync();
+    if (rank == 0 && tid < 32) {
         const float4 v0 = *reinterpret_cast<const float4 *>(s_o + lane * 8), v1 = *reinterpret_cast<const float4 *>(s_o + lane * 8 + 4);
         const float vals[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
         Q8kDevView dv = q8k_dev_view(xq_out, num_heads * HD);
-        const int b = blockIdx.x;
+        const int b = (int)blockIdx.x / AX_CTAS;
         q8k_quantize_block_warp(vals, lane, dv.qs + b * 256, dv.d + b, dv.bsum16 + b * 16, nullptr);
     }
 }

@@ -697,7 +697,7 @@ inline int launch_attention_decode_exact(cudaStream_t s, const float *q, const u
     if (xq_out && num_heads % 2) return fail(RNB_B200_VALIDATION_FAILED, "exact attention: Q8_K output needs an even head count");
     if (((uintptr_t)k | (uintptr_t)v) & 15u) return fail(RNB_B200_VALIDATION_FAILED, "exact attention: K and V must be 16-byte aligned");
     RNB_TRY(attention_exact_setup());
-    RNB_CU(launch_k(attention_decode_exact_kernel, dim3((num_heads + 1) / 2), dim3(AX_THREADS), ax_smem_bytes(max_len), s, q, k, v,
+    RNB_CU(launch_k_cluster(attention_decode_exact_kernel, dim3(AX_CTAS * ((num_heads + 1) / 2)), dim3(AX_THREADS), ax_smem_bytes(max_len), s, dim3(AX_CTAS), q, k, v,
                     kv_len_dev, kv_len_host, max_len, num_heads, num_kv_heads, scale, out, xq_out, dev_error));
     return RNB_B200_OK;
 }

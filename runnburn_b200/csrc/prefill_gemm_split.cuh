@@ -46,19 +46,6 @@ __device__ __forceinline__ void ps_tmem_ld(uint32_t taddr, uint32_t (&v)[N]) {
                      : "r"(taddr));
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
-__device__ __forceinline__ void ps_cluster_sync() {
-    asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t ps_map(uint32_t addr, int rank) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ void ps_st_remote4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-    asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
-__device__ __forceinline__ void ps_st_remote(uint32_t addr, uint32_t v) { asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
-
 // Adds the accumulators of a cluster's ks CTAs (one: its own).  A round gives every CTA up to ps_per_round chunks of
 // SUB * GROUPS tokens: the others send it theirs of those chunks, it adds them in rank order with its own and calls
 // f(chunk, count, sums).  Two cluster barriers a round, so few rounds: one or two at 256 tokens.  A worker warp holds the rows of
