@@ -1,6 +1,6 @@
 """Kernels of a decode step at the sizes where their splits end, bit for bit against the oracle: attention in position order (an
 eighth of the positions per CTA, groups of 16, slabs of 512 positions; heads of a cluster on one or two KV heads) and the
-matvec of rows that bulk copies cannot fetch."""
+matvec of rows that bulk copies cannot fetch; and the merge of up to 512 chunks of a context, within the bounds of that path."""
 import numpy as np
 import pytest
 
@@ -55,3 +55,22 @@ def test_matvec_rows_at_any_even_address(ops, t, blocks, rows):
         ops.prewarm_q4k_weights([backing])
         assert bits_equal(ops.gemv(t, backing[start:start + w.size], rows, cols, x), want), start
         ops.clear_q4k_cache()
+
+
+@pytest.mark.parametrize("max_ctx,heads,kvh", [(40, 2, 1), (160, 4, 2), (3000, 2, 2), (16384, 4, 2), (16384, 2, 1)])
+def test_chunks_of_a_context_merge(max_ctx, heads, kvh):
+    """2, 5, 94, 296 and 512 chunks, most of them empty or ragged: more than a warp has on the way ahead, more than the threads.
+    Bounds: those of the decoder's tests for this path."""
+    import runnburn_b200 as r
+    from synth import max_err_vs_norm
+    from test_gpu_decoder import LOGIT_TOL
+    desc = llama_description(seed=heads, n_layer=1, hidden=256, n_head=heads, n_kv_head=kvh, n_ff=512, vocab=512)
+    dec = r.Decoder(r.ModelConfig(max_ctx=max_ctx, **desc["cfg"]))
+    dec.set_exact_attention_max(0)
+    dec.load_description(desc)
+    ref = orc.Model(desc, 160)
+    for pos, tok in enumerate(np.random.default_rng(2).integers(0, 512, min(max_ctx, 150)).tolist()):
+        got = dec.step(tok, pos, want_logits=True)[1]
+        assert max_err_vs_norm(got, ref.decode(tok, pos)) <= LOGIT_TOL, pos
+    dec.close()
+    ref.close()
