@@ -295,11 +295,29 @@ int State::check_dev_error() {
 }
 
 // D2H of results through pinned staging, then synchronise and surface device error flags.
+// A result and the error flag into pinned memory by a kernel of the chain, 16 bytes a thread.
+RNB_GLOBAL void __launch_bounds__(256)
+deliver_kernel(const uint8_t *__restrict__ src, uint8_t *host, size_t n, const int *err, int *host_err) {
+    pdl_wait();
+    const size_t i = ((size_t)blockIdx.x * 256 + threadIdx.x) * 16;
+    if (i + 16 <= n) *reinterpret_cast<uint4 *>(host + i) = *reinterpret_cast<const uint4 *>(src + i);
+    else
+        for (size_t k = i; k < n; k++) host[k] = src[k];
+    if (i == 0) *host_err = *err;
+}
+// Up to this size a kernel moves data between pinned memory and the device instead of a copy: 16 KB of a matvec's input and result took
+// three copies and gaps between them, 20 of 42 us.  Larger ones are faster by the copy engine.
+constexpr size_t DIRECT_BYTES = 128 * 1024;
 static int finish_to_host(State &st, const void *dev_src, void *host_dst, size_t n) {
     RNB_TRY(st.pin_out.ensure(n + 16));
-    RNB_CU(cudaMemcpyAsync(st.pin_out.p, dev_src, n, cudaMemcpyDeviceToHost, st.stream));
     int *flag = reinterpret_cast<int *>(st.pin_out.as<uint8_t>() + ((n + 3) & ~(size_t)3));
-    RNB_CU(cudaMemcpyAsync(flag, st.dev_error, sizeof(int), cudaMemcpyDeviceToHost, st.stream));
+    if (n > 0 && n <= DIRECT_BYTES && ((uintptr_t)dev_src & 15u) == 0) {
+        RNB_CU(launch_k(deliver_kernel, dim3((unsigned)((n + 4095) / 4096)), dim3(256), 0, st.stream, (const uint8_t *)dev_src, st.pin_out.as<uint8_t>(), n,
+                        (const int *)st.dev_error, flag));
+    } else {
+        RNB_CU(cudaMemcpyAsync(st.pin_out.p, dev_src, n, cudaMemcpyDeviceToHost, st.stream));
+        RNB_CU(cudaMemcpyAsync(flag, st.dev_error, sizeof(int), cudaMemcpyDeviceToHost, st.stream));
+    }
     RNB_CU(cudaStreamSynchronize(st.stream));
     st.ctr.d2h_bytes += n;
     if (*flag != 0) {
@@ -351,9 +369,16 @@ static int gemv_host(int type, const uint8_t *weights, size_t weights_len, size_
     const uint8_t *w_dev = nullptr;
     RNB_TRY(st.resident_ptr(weights, weights_len, false, &w_dev));
     const float *x_dev = reinterpret_cast<const float *>(input_dev);
-    if (!input_dev) {
-        RNB_TRY(st.in_f32.ensure(cols * seq * sizeof(float)));
-        RNB_TRY(st.h2d(st.in_f32.p, input, cols * seq * sizeof(float), st.pin_in));
+    const size_t in_bytes = cols * seq * sizeof(float);
+    if (!input_dev && type != TYPE_Q8_0 && in_bytes <= DIRECT_BYTES) {
+        // the quantisation reads the staged input where it is
+        RNB_TRY(st.pin_in.ensure(in_bytes));
+        memcpy(st.pin_in.p, input, in_bytes);
+        st.ctr.h2d_bytes += in_bytes;
+        x_dev = st.pin_in.as<float>();
+    } else if (!input_dev) {
+        RNB_TRY(st.in_f32.ensure(in_bytes));
+        RNB_TRY(st.h2d(st.in_f32.p, input, in_bytes, st.pin_in));
         x_dev = st.in_f32.as<float>();
     }
     const void *act = x_dev;

@@ -132,7 +132,7 @@ __device__ __forceinline__ void gr_run(const GemvJob *__restrict__ job, const Gs
                                        uint8_t *smem, uint64_t *full, int *__restrict__ dev_error) {
     constexpr uint32_t BLK = TYPE == TYPE_Q4_K ? Q4K_BYTES : Q6K_BYTES;
     const int tid = threadIdx.x, lane = tid & 31;
-    const int R = P.rows_per_cta, cols = P.cols, nb = cols >> 8, CB = P.chunk_blocks, S = P.n_stages, n_parts = job->n_parts;
+    const int cols = P.cols, nb = cols >> 8, CB = P.chunk_blocks, S = P.n_stages, n_parts = job->n_parts;
     const uint32_t row_stride = P.row_stride, act_off = P.act_off, slot_bytes = P.slot_bytes;
     const uint32_t rb = (uint32_t)nb * BLK;
     const int n_chunks = (nb + CB - 1) / CB;
