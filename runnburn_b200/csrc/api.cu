@@ -297,7 +297,7 @@ int State::check_dev_error() {
 // D2H of results through pinned staging, then synchronise and surface device error flags.
 // A result and the error flag into pinned memory by a kernel of the chain, 16 bytes a thread.
 RNB_GLOBAL void __launch_bounds__(256)
-deliver_kernel(const uint8_t *__restrict__ src, uint8_t *host, size_t n, const int *err, int *host_err) {
+deliver_kernel(const uint8_t *src, uint8_t *host, size_t n, const int *err, int *host_err) {
     pdl_wait();
     const size_t i = ((size_t)blockIdx.x * 256 + threadIdx.x) * 16;
     if (i + 16 <= n) *reinterpret_cast<uint4 *>(host + i) = *reinterpret_cast<const uint4 *>(src + i);

@@ -736,7 +736,7 @@ flash_decode_reduce_kernel(const float *__restrict__ partials, int n_chunks,
 // threads per block, the maxima first: 7.1.
 constexpr int FDR_CTAS = 8, FDR_THREADS = 256, FDR_AHEAD = 10;
 RNB_GLOBAL void __launch_bounds__(FDR_THREADS)
-flash_decode_reduce_q8k_cluster_kernel(const float *__restrict__ partials, int n_chunks, int num_heads, uint8_t *__restrict__ xq_out) {
+flash_decode_reduce_q8k_cluster_kernel(const float *partials, int n_chunks, int num_heads, uint8_t *xq_out) {   // no __restrict__: loads stay behind the wait
     pdl_launch_dependents();
     asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
     pdl_wait();
@@ -837,7 +837,7 @@ __device__ __forceinline__ void ax_copy16(void *dst, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
 // positions pos0.. of 32 dims (64 bytes a position) into the slab
-__device__ __forceinline__ void ax_fetch_values(uint8_t *slab, const uint16_t *__restrict__ v, size_t kv_dim, int pos0, int n, int tid) {
+__device__ __forceinline__ void ax_fetch_values(uint8_t *slab, const uint16_t *v, size_t kv_dim, int pos0, int n, int tid) {
     for (int i = tid; i < 4 * n; i += AX_THREADS) ax_copy16(slab + AX_ROW * (i >> 2) + 16 * (i & 3), v + (size_t)(pos0 + (i >> 2)) * kv_dim + 8 * (i & 3));
 }
 // start + x[0] + x[1] + ... in order; the next sixteen on their way while these are added
@@ -865,11 +865,11 @@ __device__ __forceinline__ void ax_values_landed() { asm volatile("cp.async.wait
 // grid = AX_CTAS x ceil(num_heads / 2), cluster (AX_CTAS, 1, 1); dynamic shared memory = ax_smem_bytes(max_len).  Writes `out`
 // ([num_heads][128] f32) and/or the Q8_K blocks of the output (`xq_out`, needs an even head
 // count: two heads are one 256-element block).  K and V must be 16-byte aligned.  A context
-// longer than max_len raises the error flag and writes nothing.
+// longer than max_len raises the error flag and writes nothing.  (No __restrict__ on what the launch before writes: loads of memory that
+// nobody writes during a kernel may be moved ahead of the dependency wait.)
 RNB_GLOBAL void __launch_bounds__(AX_THREADS)
-attention_decode_exact_kernel(const float *__restrict__ q, const uint16_t *__restrict__ k, const uint16_t *__restrict__ v,
-                              const int *__restrict__ kv_len_dev, int kv_len_host, int max_len, int num_heads, int num_kv_heads,
-                              float scale, float *__restrict__ out, uint8_t *__restrict__ xq_out, int *__restrict__ err_flag) {
+attention_decode_exact_kernel(const float *q, const uint16_t *k, const uint16_t *v, const int *kv_len_dev, int kv_len_host, int max_len, int num_heads,
+                              int num_kv_heads, float scale, float *out, uint8_t *xq_out, int *err_flag) {
     pdl_launch_dependents();
     extern __shared__ __align__(16) uint8_t s_dyn[];
     uint8_t *const slab = s_dyn;                                              // [position][32 dims]

@@ -74,3 +74,17 @@ def test_chunks_of_a_context_merge(max_ctx, heads, kvh):
         assert max_err_vs_norm(got, ref.decode(tok, pos)) <= LOGIT_TOL, pos
     dec.close()
     ref.close()
+
+
+def test_steps_repeat_their_bits():
+    """Token and position of a step are in place before any launch of it starts: 300 steps of a latent attention layer with a key
+    that dominates, ten times over on one decoder, bit for bit (a layer that read the position too early left out the
+    newest key in about one step of a thousand)."""
+    import stack_util as su
+    cfg = su.config([su.latent(heads=2, dim=16, vdim=16, rot_dim=4, kv_rank=32, base=1e6, ff=0)], width=64, vocab=32, residual_mult=1.0)
+    dec = su.decoder(cfg, su.weights(cfg, 11), "float32")
+    toks = np.random.default_rng(0).integers(0, 32, 230)
+    first = su.feed(dec, toks, [200] + [1] * 30)
+    for _ in range(10):
+        assert np.array_equal(su.feed(dec, toks, [200] + [1] * 30), first)
+    dec.close()
