@@ -926,7 +926,9 @@ int LayerStack::boundary(cudaStream_t s, int n, StackScratch &b, int &cur, const
     const int threads = std::max(32, std::min(n <= SMALL ? 1024 : 512, (want + 31) / 32 * 32));
     const size_t smem = (size_t)cfg.width * 4 * (shift ? 2 : 1);
     const dim3 grid((unsigned)((n + a.rows_per_cta - 1) / a.rows_per_cta)), block((unsigned)threads);
-    if (narrow(n)) {
+    if (n == 1 && v4 && cfg.width <= RN_STEP_WIDTH && !narrow(n)) {
+        RNB_CU(launch_k(residual_norm_step_kernel, dim3(1), block, 0, s, a));
+    } else if (narrow(n)) {
         if (v4) RNB_CU(launch_k(residual_norm_kernel<bf16, 4>, grid, block, smem, s, a));
         else RNB_CU(launch_k(residual_norm_kernel<bf16, 1>, grid, block, smem, s, a));
     } else {
