@@ -22,12 +22,12 @@ constexpr int HD = 128;
 // rope_table: [max_pos][2][64] (cos then sin) indexed by position when table_by_pos != 0,
 // else a single row.  Position = *pos_dev (optional device scalar) + pos_offset.
 RNB_GLOBAL void __launch_bounds__(64)
-rope_kv_append_kernel(float *__restrict__ q, const float *__restrict__ k,
-                      const float *__restrict__ v, const float *__restrict__ rope_table,
-                      const int *__restrict__ pos_dev, int pos_offset, int table_by_pos,
-                      int num_heads, int num_kv_heads, int neox, uint16_t *__restrict__ k_cache,
-                      uint16_t *__restrict__ v_cache, uint16_t *__restrict__ k_row_out,
-                      uint16_t *__restrict__ v_row_out) {
+rope_kv_append_kernel(float *q, const float *k,
+                      const float *v, const float *__restrict__ rope_table,
+                      const int *pos_dev, int pos_offset, int table_by_pos,
+                      int num_heads, int num_kv_heads, int neox, uint16_t *k_cache,
+                      uint16_t *v_cache, uint16_t *k_row_out,
+                      uint16_t *v_row_out) {
     pdl_launch_dependents();
     pdl_wait();
     // gridDim.y > 1: a batch of consecutive tokens (prefill), token t = blockIdx.y at position base + t,
@@ -85,8 +85,8 @@ rope_kv_append_kernel(float *__restrict__ q, const float *__restrict__ k,
 // thread (g = tid / 64, i = tid % 64) owns rotation pair i of heads g, g + 4, ... - the cos/sin of
 // the pair is read once.  Same arithmetic and rounding as rope_kv_append_kernel.
 RNB_GLOBAL void __launch_bounds__(256)
-rope_kv_append_tokens_kernel(float *__restrict__ q, const float *__restrict__ k, const float *__restrict__ v, const float *__restrict__ rope_table,
-                             int pos0, int num_heads, int num_kv_heads, int neox, uint16_t *__restrict__ k_cache, uint16_t *__restrict__ v_cache) {
+rope_kv_append_tokens_kernel(float *q, const float *k, const float *v, const float *__restrict__ rope_table,
+                             int pos0, int num_heads, int num_kv_heads, int neox, uint16_t *k_cache, uint16_t *v_cache) {
     pdl_launch_dependents();
     pdl_wait();
     const int t = blockIdx.x, pos = pos0 + t, i = threadIdx.x & 63, g = threadIdx.x >> 6;
@@ -113,7 +113,7 @@ rope_kv_append_tokens_kernel(float *__restrict__ q, const float *__restrict__ k,
 }
 
 // Plain f32 -> f16 row append (no RoPE) for callers that rotate elsewhere.
-RNB_GLOBAL void kv_append_f16_kernel(const float *__restrict__ src, uint16_t *__restrict__ dst,
+RNB_GLOBAL void kv_append_f16_kernel(const float *src, uint16_t *dst,
                                      size_t n) {
     pdl_launch_dependents();
     pdl_wait();
@@ -134,26 +134,24 @@ constexpr int FD_MAX_CHUNKS = 1024;   // merge kernels keep one rescale factor p
 
 // four consecutive K/V elements as f32, from an f16 cache (decode) or f32 tensors (prefill API)
 __device__ __forceinline__ float4 kv_load4(const uint16_t *p) {
-    const uint2 b = ldg_nc_u2(p);
+    const uint2 b = *reinterpret_cast<const uint2 *>(p);
     const float2 lo = __half22float2(*reinterpret_cast<const __half2 *>(&b.x));
     const float2 hi = __half22float2(*reinterpret_cast<const __half2 *>(&b.y));
     return make_float4(lo.x, lo.y, hi.x, hi.y);
 }
 __device__ __forceinline__ float4 kv_load4(const float *p) {
-    const uint4 b = ldg_nc_u4(p);
-    return make_float4(__uint_as_float(b.x), __uint_as_float(b.y), __uint_as_float(b.z),
-                       __uint_as_float(b.w));
+    return *reinterpret_cast<const float4 *>(p);
 }
 
 // G = query heads handled per pass (<= group size).  When `direct_out` is given the merged,
 // normalised result is written there ([head][128]) instead of a partial record.
 template <int G, typename KVT>
-__device__ __forceinline__ void fd_process(const float *__restrict__ q, const KVT *__restrict__ k,
-                                           const KVT *__restrict__ v, int kv_h, int head0,
+__device__ __forceinline__ void fd_process(const float *q, const KVT *k,
+                                           const KVT *v, int kv_h, int head0,
                                            int heads_here, size_t kv_dim, int p_begin, int p_end,
                                            float scale, int n_chunks, int chunk,
-                                           float *__restrict__ partials, float *s_acc, float *s_ml,
-                                           float *__restrict__ direct_out = nullptr) {
+                                           float *partials, float *s_acc, float *s_ml,
+                                           float *direct_out = nullptr) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float qr[G][4], acc[G][4], m[G], l[G];
 #pragma unroll
@@ -237,10 +235,10 @@ __device__ __forceinline__ void fd_process(const float *__restrict__ q, const KV
 }
 
 RNB_GLOBAL void __launch_bounds__(FD_THREADS)
-flash_decode_partials_kernel(const float *__restrict__ q, const uint16_t *__restrict__ k,
-                             const uint16_t *__restrict__ v, const int *__restrict__ kv_len_dev,
+flash_decode_partials_kernel(const float *q, const uint16_t *k,
+                             const uint16_t *v, const int *kv_len_dev,
                              int kv_len_host, int num_heads, int num_kv_heads, float scale,
-                             float *__restrict__ partials) {
+                             float *partials) {
     pdl_launch_dependents();
     pdl_wait();
     __shared__ float s_acc[(FD_THREADS / 32) * 4 * HD];
@@ -327,9 +325,9 @@ struct FdMerge {
                          // cluster's CTA b merges heads 2b, 2b + 1 of the group after a cluster barrier
 };
 template <bool PREFILL>
-__device__ __forceinline__ void fdm_body(const float *__restrict__ q, const uint16_t *__restrict__ k, const uint16_t *__restrict__ v,
-                                         const int *__restrict__ kv_len_dev, int kv_len_host, int seq_len, int num_heads, int num_kv_heads,
-                                         float scale, float *__restrict__ partials, float *__restrict__ out, int *__restrict__ err_flag,
+__device__ __forceinline__ void fdm_body(const float *q, const uint16_t *k, const uint16_t *v,
+                                         const int *kv_len_dev, int kv_len_host, int seq_len, int num_heads, int num_kv_heads,
+                                         float scale, float *partials, float *out, int *err_flag,
                                          const FdMerge merge = FdMerge{nullptr, nullptr, nullptr, 0}) {
     pdl_launch_dependents();
     pdl_wait();
@@ -657,16 +655,16 @@ __device__ __forceinline__ void fdm_body(const float *__restrict__ q, const uint
 }
 
 RNB_GLOBAL void __launch_bounds__(FDM_THREADS, 4)
-flash_decode_mma_kernel(const float *__restrict__ q, const uint16_t *__restrict__ k,
-                        const uint16_t *__restrict__ v, const int *__restrict__ kv_len_dev,
+flash_decode_mma_kernel(const float *q, const uint16_t *k,
+                        const uint16_t *v, const int *kv_len_dev,
                         int kv_len_host, int num_heads, int num_kv_heads, float scale,
-                        float *__restrict__ partials, int *__restrict__ err_flag, const FdMerge merge) {
+                        float *partials, int *err_flag, const FdMerge merge) {
     fdm_body<false>(q, k, v, kv_len_dev, kv_len_host, 1, num_heads, num_kv_heads, scale, partials, nullptr, err_flag, merge);
 }
 // Causal prefill attention on the same machinery: grid (kv heads, ceil(seq / queries per CTA)).
 RNB_GLOBAL void __launch_bounds__(FDM_THREADS, 4)
-prefill_attention_mma_kernel(const float *__restrict__ q, const uint16_t *__restrict__ k, const uint16_t *__restrict__ v, int seq_len,
-                             int kv_len, int num_heads, int num_kv_heads, float scale, float *__restrict__ out, int *__restrict__ err_flag) {
+prefill_attention_mma_kernel(const float *q, const uint16_t *k, const uint16_t *v, int seq_len,
+                             int kv_len, int num_heads, int num_kv_heads, float scale, float *out, int *err_flag) {
     fdm_body<true>(q, k, v, nullptr, kv_len, seq_len, num_heads, num_kv_heads, scale, nullptr, out, err_flag);
 }
 
@@ -675,8 +673,8 @@ prefill_attention_mma_kernel(const float *__restrict__ q, const uint16_t *__rest
 // dimension d over the chunks c = g, g + 4, ...; the four groups are added at the end.  A head
 // sharded onto one GPU of eight has hundreds of chunks: a serial walk would take tens of us.
 RNB_GLOBAL void __launch_bounds__(4 * HD)
-flash_decode_reduce_kernel(const float *__restrict__ partials, int n_chunks,
-                           float *__restrict__ out, const PeerOut po = PeerOut{}) {
+flash_decode_reduce_kernel(const float *partials, int n_chunks,
+                           float *out, const PeerOut po = PeerOut{}) {
     pdl_launch_dependents();
     pdl_wait();
     __shared__ float s_f[FD_MAX_CHUNKS];
@@ -736,7 +734,7 @@ flash_decode_reduce_kernel(const float *__restrict__ partials, int n_chunks,
 // threads per block, the maxima first: 7.1.
 constexpr int FDR_CTAS = 8, FDR_THREADS = 256, FDR_AHEAD = 10;
 RNB_GLOBAL void __launch_bounds__(FDR_THREADS)
-flash_decode_reduce_q8k_cluster_kernel(const float *partials, int n_chunks, int num_heads, uint8_t *xq_out) {   // no __restrict__: loads stay behind the wait
+flash_decode_reduce_q8k_cluster_kernel(const float *partials, int n_chunks, int num_heads, uint8_t *xq_out) {
     pdl_launch_dependents();
     asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
     pdl_wait();
@@ -865,8 +863,7 @@ __device__ __forceinline__ void ax_values_landed() { asm volatile("cp.async.wait
 // grid = AX_CTAS x ceil(num_heads / 2), cluster (AX_CTAS, 1, 1); dynamic shared memory = ax_smem_bytes(max_len).  Writes `out`
 // ([num_heads][128] f32) and/or the Q8_K blocks of the output (`xq_out`, needs an even head
 // count: two heads are one 256-element block).  K and V must be 16-byte aligned.  A context
-// longer than max_len raises the error flag and writes nothing.  (No __restrict__ on what the launch before writes: loads of memory that
-// nobody writes during a kernel may be moved ahead of the dependency wait.)
+// longer than max_len raises the error flag and writes nothing.
 RNB_GLOBAL void __launch_bounds__(AX_THREADS)
 attention_decode_exact_kernel(const float *q, const uint16_t *k, const uint16_t *v, const int *kv_len_dev, int kv_len_host, int max_len, int num_heads,
                               int num_kv_heads, float scale, float *out, uint8_t *xq_out, int *err_flag) {

@@ -14,8 +14,8 @@ constexpr int AW_MAX_CHUNKS = 256;
 // partials: [head][chunk][HD + 2] = unnormalised output, running max, running sum
 template <int HD_>
 RNB_GLOBAL void __launch_bounds__(AW_THREADS)
-attention_wide_partials_kernel(const float *__restrict__ q, const uint16_t *__restrict__ k, const uint16_t *__restrict__ v, int kv_len,
-                               int num_heads, int num_kv_heads, float scale, float *__restrict__ partials) {
+attention_wide_partials_kernel(const float *q, const uint16_t *k, const uint16_t *v, int kv_len,
+                               int num_heads, int num_kv_heads, float scale, float *partials) {
     constexpr int PER = HD_ / 32;   // dims per lane: 8 (hd256) or 16 (hd512), contiguous
     static_assert(PER % 8 == 0, "a lane reads whole 16-byte groups of f16");
     pdl_launch_dependents();
@@ -90,7 +90,7 @@ attention_wide_partials_kernel(const float *__restrict__ q, const uint16_t *__re
 
 template <int HD_>
 RNB_GLOBAL void __launch_bounds__(HD_ / 2)
-attention_wide_merge_kernel(const float *__restrict__ partials, int n_chunks, float *__restrict__ out) {
+attention_wide_merge_kernel(const float *partials, int n_chunks, float *out) {
     pdl_launch_dependents();
     pdl_wait();
     const int head = blockIdx.x;

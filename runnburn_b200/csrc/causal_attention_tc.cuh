@@ -29,7 +29,7 @@ constexpr uint32_t CT_IDESC_O = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) 
 // grid = (heads, ceil(tokens / 128)), PAT_THREADS threads.  KP: panels of 64 elements of a key; pos0: the first query's position.
 template <int KP>
 RNB_GLOBAL void __launch_bounds__(PAT_THREADS, 2)
-causal_attention_tc_kernel(const __grid_constant__ CausalAttentionArgs a, const __grid_constant__ CausalAttentionMaps maps, int pos0, int *__restrict__ err_flag) {
+causal_attention_tc_kernel(const __grid_constant__ CausalAttentionArgs a, const __grid_constant__ CausalAttentionMaps maps, int pos0, int *err_flag) {
     extern __shared__ __align__(1024) uint8_t ct_mem[];
     constexpr int NV = ct_v_slots(KP);
     pdl_launch_dependents();

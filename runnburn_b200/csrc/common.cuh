@@ -125,11 +125,19 @@ __device__ __forceinline__ void ps_st_remote(uint32_t addr, uint32_t v) { asm vo
 
 // Programmatic dependent launch: let the next kernel in the stream start its prologue, and
 // wait for the previous kernel's memory to be visible.
+//
+// The wait orders only loads that the compiler has to keep behind it.  What a kernel is told that nobody writes
+// while it runs (const __restrict__ parameters, __ldg, ld.global.nc) may be loaded ahead of the wait, and read-only
+// loads are not coherent with a launch that is still writing.  So those forms are for weights, tables
+// and descriptors; activations, caches, positions, tokens, job tables that a kernel fills, partial results and counters
+// are reached through plain pointers.  (A latent attention whose position was loaded ahead left out the newest key
+// in about one step of a thousand.)
 __device__ __forceinline__ void pdl_launch_dependents() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// Weights only (see above).
 __device__ __forceinline__ uint4 ldg_nc_u4(const void *p) {
     uint4 v;
     asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];"

@@ -224,7 +224,7 @@ struct DensePair {
     int n1, n2, token_tiles, tiles;   // n1, n2: multiples of 32, at most 256; tiles: pairs of row tiles of all jobs x token tiles
 };
 RNB_GLOBAL void __launch_bounds__(DQ_THREADS, 1)
-dense_gemm_pair_kernel(const __grid_constant__ DenseGemmJobs jobs, const __grid_constant__ DenseMapsPair maps, const DensePair P, int *__restrict__ err_flag) {
+dense_gemm_pair_kernel(const __grid_constant__ DenseGemmJobs jobs, const __grid_constant__ DenseMapsPair maps, const DensePair P, int *err_flag) {
     extern __shared__ __align__(1024) uint8_t dg_smem_raw[];
     __shared__ __align__(8) uint64_t full[DQ_STAGES], empty[DQ_STAGES], acc_full, acc_free[2];
     __shared__ uint32_t tmem_slot;
@@ -428,7 +428,7 @@ struct DenseSplit {
     uint32_t tmem_cols;
 };
 RNB_GLOBAL void __launch_bounds__(DP_THREADS)
-dense_gemm_split_kernel(const __grid_constant__ DenseGemmJobs jobs, const __grid_constant__ DenseMaps maps, const DenseSplit P, int *__restrict__ err_flag) {
+dense_gemm_split_kernel(const __grid_constant__ DenseGemmJobs jobs, const __grid_constant__ DenseMaps maps, const DenseSplit P, int *err_flag) {
     extern __shared__ __align__(1024) uint8_t dg_smem_raw[];
     __shared__ __align__(8) uint64_t full[DP_MAX_STAGES], empty[DP_MAX_STAGES], done_bar;
     __shared__ uint32_t tmem_slot;

@@ -97,8 +97,8 @@ __device__ __forceinline__ Q4kTerms q4k_block_terms(const uint8_t *blk, int t, c
     if (valid) {
         const uint4 hdr = *reinterpret_cast<const uint4 *>(blk);
         const uint4 q = *reinterpret_cast<const uint4 *>(blk + 16 + 16 * t);
-        const uint4 alo = ldg_nc_u4(xq + 64 * g + 16 * h);
-        const uint4 ahi = ldg_nc_u4(xq + 64 * g + 32 + 16 * h);
+        const uint4 alo = *reinterpret_cast<const uint4 *>(xq + 64 * g + 16 * h);
+        const uint4 ahi = *reinterpret_cast<const uint4 *>(xq + 64 * g + 32 + 16 * h);
         // 6-bit scale/min unpack (get_scale_min_k4) for all 8 sub-blocks at once
         const uint32_t sc03 = hdr.y & 0x3f3f3f3fu;
         const uint32_t mn03 = hdr.z & 0x3f3f3f3fu;
@@ -115,7 +115,7 @@ __device__ __forceinline__ Q4kTerms q4k_block_terms(const uint8_t *blk, int t, c
         const int k = t & 3;
         const uint32_t mnw = k < 2 ? mn03 : mn47;
         const int mn_a = (mnw >> (16 * (k & 1))) & 0xff, mn_b = (mnw >> (16 * (k & 1) + 8)) & 0xff;
-        const uint2 bs = ldg_nc_u2(bsum16 + 4 * k);  // four consecutive i16, 8-byte aligned
+        const uint2 bs = *reinterpret_cast<const uint2 *>(bsum16 + 4 * k);  // four consecutive i16, 8-byte aligned
         const int b32a = (short)((short)(bs.x & 0xffff) + (short)(bs.x >> 16));
         const int b32b = (short)((short)(bs.y & 0xffff) + (short)(bs.y >> 16));
         r.min_prod = mn_a * b32a + mn_b * b32b;
@@ -146,7 +146,8 @@ __device__ __forceinline__ void q6k_block_terms(uint32_t blk, int t, const int8_
         const uint2 qlb = lds8_unaligned(blk + 64 * n + 32 + 8 * m);
         const uint2 qh = lds8_unaligned(blk + 128 + 32 * n + 8 * m);
         const int8_t *xa = xq + 128 * n + 8 * m;
-        const uint2 a0 = ldg_nc_u2(xa), a1 = ldg_nc_u2(xa + 32), a2 = ldg_nc_u2(xa + 64), a3 = ldg_nc_u2(xa + 96);
+        const uint2 a0 = *reinterpret_cast<const uint2 *>(xa), a1 = *reinterpret_cast<const uint2 *>(xa + 32), a2 = *reinterpret_cast<const uint2 *>(xa + 64),
+                    a3 = *reinterpret_cast<const uint2 *>(xa + 96);
         const uint32_t sc = blk + 192 + 8 * n + (m >> 1);
         int s0, s1, s2, s3, sa, sb, dh;
         asm volatile("ld.shared.s8 %0, [%1];" : "=r"(s0) : "r"(sc));
@@ -168,7 +169,7 @@ __device__ __forceinline__ void q6k_block_terms(uint32_t blk, int t, const int8_
             if (w) u1 = acc;
             else u0 = acc;
         }
-        const uint32_t bs = __ldg(reinterpret_cast<const uint32_t *>(bsum16 + 2 * l));
+        const uint32_t bs = *reinterpret_cast<const uint32_t *>(bsum16 + 2 * l);
         corr = 32 * ((int)(short)(bs & 0xffff) * sa + (int)(short)(bs >> 16) * sb);
         d = __fmul_rn(yd, f16_bits_to_f32((uint32_t)dh));
     }
@@ -210,9 +211,9 @@ __device__ __forceinline__ void q8_0_block_terms(uint32_t blk, const float *x, b
 // (tile bytes rounded up to 16, plus 16 bytes of slack for the unaligned readers).
 // `dynamic_table`: the job table itself is written by the previous kernel (routed experts), so
 // it may only be read after the dependency wait.
-__device__ __forceinline__ void gemv_tile_body(const GemvJob *__restrict__ jobs, int n_jobs,
+__device__ __forceinline__ void gemv_tile_body(const GemvJob *jobs, int n_jobs,
                                                int cols, uint32_t part_stride,
-                                               int *__restrict__ dev_error, int dynamic_table) {
+                                               int *dev_error, int dynamic_table) {
     if (dynamic_table) pdl_wait();
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ __align__(8) uint64_t bar;
@@ -285,7 +286,7 @@ __device__ __forceinline__ void gemv_tile_body(const GemvJob *__restrict__ jobs,
                     const int b = b0 + bsub;
                     const bool valid = b < nb;
                     const int bc = valid ? b : b0;
-                    const Q4kTerms tm = q4k_block_terms(rowp + bc * Q4K_BYTES, t, qs + bc * 256, __ldg(xd + bc), bs + bc * 16, valid);
+                    const Q4kTerms tm = q4k_block_terms(rowp + bc * Q4K_BYTES, t, qs + bc * 256, xd[bc], bs + bc * 16, valid);
                     const int nvalid = min(4, nb - b0);
 #pragma unroll
                     for (int bb = 0; bb < 4; bb++) {
@@ -321,7 +322,7 @@ __device__ __forceinline__ void gemv_tile_body(const GemvJob *__restrict__ jobs,
                     const int bc = valid ? b : b0;
                     int lsum;
                     float dmine;
-                    q6k_block_terms(rows32 + bc * Q6K_BYTES, t, qs + bc * 256, __ldg(xd + bc), bs + bc * 16, valid, lsum, dmine);
+                    q6k_block_terms(rows32 + bc * Q6K_BYTES, t, qs + bc * 256, xd[bc], bs + bc * 16, valid, lsum, dmine);
                     const int nvalid = min(4, nb - b0);
 #pragma unroll
                     for (int bb = 0; bb < 4; bb++) {
@@ -354,7 +355,7 @@ __device__ __forceinline__ void gemv_tile_body(const GemvJob *__restrict__ jobs,
                 dot = a;
             }
             // expert_out *= route weight; out += expert_out (moe_view/fanout.rs:301-303, moe_view.rs:416-423)
-            if (job->parts[p].scale) dot = __fmul_rn(dot, __ldg(job->parts[p].scale));
+            if (job->parts[p].scale) dot = __fmul_rn(dot, *job->parts[p].scale);
             acc = n_parts == 1 ? dot : __fadd_rn(acc, dot);
         }
         if (lane == 0) {
@@ -366,22 +367,22 @@ __device__ __forceinline__ void gemv_tile_body(const GemvJob *__restrict__ jobs,
 
 // Job table in global memory (multi-matrix launches: q/k/v, gate/up, routed experts).
 RNB_GLOBAL void __launch_bounds__(GEMV_THREADS)
-gemv_tile_kernel(const GemvJob *__restrict__ jobs, int n_jobs, int cols, uint32_t part_stride,
-                 int *__restrict__ dev_error, int dynamic_table) {
+gemv_tile_kernel(const GemvJob *jobs, int n_jobs, int cols, uint32_t part_stride,
+                 int *dev_error, int dynamic_table) {
     gemv_tile_body(jobs, n_jobs, cols, part_stride, dev_error, dynamic_table);
 }
 // Single job passed by value in kernel-parameter space (no table upload).
 RNB_GLOBAL void __launch_bounds__(GEMV_THREADS)
 gemv_tile_kernel_1(const __grid_constant__ GemvJob job, int cols, uint32_t part_stride,
-                   int *__restrict__ dev_error) {
+                   int *dev_error) {
     gemv_tile_body(&job, 1, cols, part_stride, dev_error, 0);
 }
 
 // LM-head epilogue: greedy argmax with the reference CPU sampler's tie rule (the LAST of equal
 // maxima, crates/rnb-llm/src/sampler/greedy.rs:4-11).  Single CTA.
 RNB_GLOBAL void __launch_bounds__(1024)
-argmax_last_kernel(const float *__restrict__ x, int n, uint32_t *__restrict__ idx_out,
-                   float *__restrict__ val_out) {
+argmax_last_kernel(const float *x, int n, uint32_t *idx_out,
+                   float *val_out) {
     pdl_launch_dependents();
     pdl_wait();
     __shared__ float sv[32];
@@ -423,7 +424,7 @@ argmax_last_kernel(const float *__restrict__ x, int n, uint32_t *__restrict__ id
 // Two-stage form for long vectors (the 128k-entry logits): stage 1 leaves one (value, index)
 // candidate per CTA of 1024 threads x 4 elements, stage 2 is argmax_last_pairs_kernel.
 RNB_GLOBAL void __launch_bounds__(1024)
-argmax_last_partial_kernel(const float *__restrict__ x, int n, float *__restrict__ vals, uint32_t *__restrict__ idxs) {
+argmax_last_partial_kernel(const float *x, int n, float *vals, uint32_t *idxs) {
     pdl_launch_dependents();
     pdl_wait();
     __shared__ float sv[32];
@@ -464,8 +465,8 @@ argmax_last_partial_kernel(const float *__restrict__ x, int n, float *__restrict
 }
 // one warp: last index of the maximum among n (value, index) candidates
 RNB_GLOBAL void __launch_bounds__(32)
-argmax_last_pairs_kernel(const float *__restrict__ vals, const uint32_t *__restrict__ idxs, int n, uint32_t *__restrict__ idx_out,
-                         float *__restrict__ val_out) {
+argmax_last_pairs_kernel(const float *vals, const uint32_t *idxs, int n, uint32_t *idx_out,
+                         float *val_out) {
     pdl_launch_dependents();
     pdl_wait();
     float best = -INFINITY;

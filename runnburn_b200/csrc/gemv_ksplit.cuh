@@ -28,7 +28,7 @@ __host__ __device__ constexpr uint32_t gk_smem(int stages) { return (uint32_t)st
 
 // grid = ceil(rows / 4); 128 threads; dynamic shared memory gk_smem(S).  cols % 2048 == 0, operands 16-byte aligned.
 RNB_GLOBAL void __launch_bounds__(GK_THREADS)
-gemv_ksplit_q6k_kernel(const __grid_constant__ GemvJob job, int cols, int S, int *__restrict__ dev_error) {
+gemv_ksplit_q6k_kernel(const __grid_constant__ GemvJob job, int cols, int S, int *dev_error) {
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ __align__(8) uint64_t full[GK_MAX_STAGES];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -117,7 +117,7 @@ gemv_ksplit_q6k_kernel(const __grid_constant__ GemvJob job, int cols, int S, int
         v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 4));
         v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 2));
         v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 1));
-        if (job.parts[0].scale) v = __fmul_rn(v, __ldg(job.parts[0].scale));
+        if (job.parts[0].scale) v = __fmul_rn(v, *job.parts[0].scale);
         const int cr = lane >> 3;
         if ((lane & 7) == 0 && cr < nrows) {
             const size_t o = (size_t)row0 + cr;

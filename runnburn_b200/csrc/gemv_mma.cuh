@@ -340,7 +340,7 @@ struct GmCursor {
     int tile, part, chunk;
     int jsel, row0, nrows, type, n_parts;
 };
-__device__ __forceinline__ bool gm_locate(const GemvJob *__restrict__ jobs, int n_jobs, GmCursor &c) {
+__device__ __forceinline__ bool gm_locate(const GemvJob *jobs, int n_jobs, GmCursor &c) {
     int t0 = 0;
     for (int i = 0; i < n_jobs; i++) {
         const int rows = jobs[i].rows, nt = (rows + GM_ROWS - 1) / GM_ROWS;
@@ -357,7 +357,7 @@ __device__ __forceinline__ bool gm_locate(const GemvJob *__restrict__ jobs, int 
     return false;
 }
 // advances to the next item; returns false when the CTA's tiles are exhausted
-__device__ __forceinline__ bool gm_next(const GemvJob *__restrict__ jobs, int n_jobs, int n_chunks, int n_tiles, int tile_step, GmCursor &c) {
+__device__ __forceinline__ bool gm_next(const GemvJob *jobs, int n_jobs, int n_chunks, int n_tiles, int tile_step, GmCursor &c) {
     if (++c.chunk < n_chunks) return true;
     c.chunk = 0;
     if (++c.part < c.n_parts) return true;
@@ -370,7 +370,7 @@ __device__ __forceinline__ bool gm_next(const GemvJob *__restrict__ jobs, int n_
 // PEER: the instantiation whose epilogue also stores the rows into the peers' buffers (sharded decode);
 // the single-GPU instantiation carries none of that code.
 template <bool PEER>
-__device__ __forceinline__ void gemv_mma_body(const GemvJob *__restrict__ jobs, int n_jobs, const GmParams &P, int *__restrict__ dev_error,
+__device__ __forceinline__ void gemv_mma_body(const GemvJob *jobs, int n_jobs, const GmParams &P, int *dev_error,
                                               const GpTail &tail, const GmTmaps *__restrict__ tmaps) {
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ __align__(8) uint64_t full[GM_MAX_STAGES], empty[GM_MAX_STAGES], pfull[2], pempty[2];
@@ -630,7 +630,7 @@ __device__ __forceinline__ void gemv_mma_body(const GemvJob *__restrict__ jobs, 
             const float m13 = __fadd_rn(accm[1], __shfl_xor_sync(0xffffffffu, accm[1], 1));
             if (q4) dot = __fadd_rn(dot, __fadd_rn(m02, m13));
             const GemvJob &job = jobs[cur.jsel];
-            if (job.parts[cur.part].scale) dot = __fmul_rn(dot, __ldg(job.parts[cur.part].scale));
+            if (job.parts[cur.part].scale) dot = __fmul_rn(dot, *job.parts[cur.part].scale);
             acc_total = cur.n_parts == 1 ? dot : __fadd_rn(acc_total, dot);
 #pragma unroll
             for (int k = 0; k < 4; k++) acc[k] = 0.f;
@@ -696,19 +696,19 @@ __device__ __forceinline__ void gemv_mma_body(const GemvJob *__restrict__ jobs, 
 }
 
 RNB_GLOBAL void __launch_bounds__(GM_THREADS, GM_MIN_CTAS)
-gemv_mma_kernel(const GemvJob *__restrict__ jobs, int n_jobs, const GmParams P, int *__restrict__ dev_error) {
+gemv_mma_kernel(const GemvJob *jobs, int n_jobs, const GmParams P, int *dev_error) {
     GpTail none;
     none.kind = 0;
     none.peer.peers = nullptr;
     gemv_mma_body<false>(jobs, n_jobs, P, dev_error, none, nullptr);
 }
 RNB_GLOBAL void __launch_bounds__(GM_THREADS, GM_MIN_CTAS)
-gemv_mma_kernel_1(const __grid_constant__ GemvJobPack jobs, int n_jobs, const GmParams P, int *__restrict__ dev_error,
+gemv_mma_kernel_1(const __grid_constant__ GemvJobPack jobs, int n_jobs, const GmParams P, int *dev_error,
                   const __grid_constant__ GpTail tail, const __grid_constant__ GmTmaps tmaps) {
     gemv_mma_body<false>(jobs.j, n_jobs, P, dev_error, tail, &tmaps);
 }
 RNB_GLOBAL void __launch_bounds__(GM_THREADS, GM_MIN_CTAS)
-gemv_mma_kernel_1_peer(const __grid_constant__ GemvJobPack jobs, int n_jobs, const GmParams P, int *__restrict__ dev_error,
+gemv_mma_kernel_1_peer(const __grid_constant__ GemvJobPack jobs, int n_jobs, const GmParams P, int *dev_error,
                        const __grid_constant__ GpTail tail, const __grid_constant__ GmTmaps tmaps) {
     gemv_mma_body<true>(jobs.j, n_jobs, P, dev_error, tail, &tmaps);
 }

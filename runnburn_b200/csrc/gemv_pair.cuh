@@ -95,7 +95,7 @@ __device__ __forceinline__ void gp_q4k_block(const uint8_t *blk, const uint8_t *
 // DYN: the expert-gathered instantiation (virtual rows, ids read after the wait on the previous kernel, tails 1 with
 // per-expert vectors and 3); the dense instantiation carries none of that code.
 template <bool DYN>
-__device__ __forceinline__ void gemv_pair_body(const GemvJobPack &jobs, int n_jobs, const GpParams &P, int *__restrict__ dev_error, const GpTail &tail) {
+__device__ __forceinline__ void gemv_pair_body(const GemvJobPack &jobs, int n_jobs, const GpParams &P, int *dev_error, const GpTail &tail) {
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ __align__(8) uint64_t full[GP_MAX_STAGES];
     const int lane = threadIdx.x, r = lane >> 1, h = lane & 1;
@@ -192,7 +192,7 @@ __device__ __forceinline__ void gemv_pair_body(const GemvJobPack &jobs, int n_jo
     const float x0 = __fadd_rn(A.m[0], __shfl_xor_sync(0xffffffffu, A.m[0], 1));
     const float x1 = __fadd_rn(A.m[1], __shfl_xor_sync(0xffffffffu, A.m[1], 1));
     float dot = __fadd_rn(hs, __fadd_rn(x0, x1));
-    if (job.parts[0].scale) dot = __fmul_rn(dot, __ldg(job.parts[0].scale));
+    if (job.parts[0].scale) dot = __fmul_rn(dot, *job.parts[0].scale);
     if (r < nrows && h == 0) {
         const size_t o = (size_t)row0 + r;
         job.y[o] = job.residual ? __fadd_rn(job.residual[o], dot) : dot;
@@ -250,12 +250,12 @@ __device__ __forceinline__ void gemv_pair_body(const GemvJobPack &jobs, int n_jo
     }
 }
 RNB_GLOBAL void __launch_bounds__(32)
-gemv_pair_q4k_kernel(const __grid_constant__ GemvJobPack jobs, int n_jobs, const GpParams P, int *__restrict__ dev_error,
+gemv_pair_q4k_kernel(const __grid_constant__ GemvJobPack jobs, int n_jobs, const GpParams P, int *dev_error,
                      const __grid_constant__ GpTail tail) {
     gemv_pair_body<false>(jobs, n_jobs, P, dev_error, tail);
 }
 RNB_GLOBAL void __launch_bounds__(32)
-gemv_pair_q4k_dyn_kernel(const __grid_constant__ GemvJobPack jobs, int n_jobs, const GpParams P, int *__restrict__ dev_error,
+gemv_pair_q4k_dyn_kernel(const __grid_constant__ GemvJobPack jobs, int n_jobs, const GpParams P, int *dev_error,
                          const __grid_constant__ GpTail tail) {
     gemv_pair_body<true>(jobs, n_jobs, P, dev_error, tail);
 }

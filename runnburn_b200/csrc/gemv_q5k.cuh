@@ -22,7 +22,7 @@ constexpr int G5_WARPS = 4;
 
 // xq: Q8K-dev layout of the activation (qs[cols] | bsum16[cols/16] | d[cols/256]); seq tokens, xq_stride bytes apart
 RNB_GLOBAL void __launch_bounds__(G5_WARPS * 32)
-gemv_q5k_kernel(const uint8_t *__restrict__ w, const uint8_t *__restrict__ xq, size_t xq_stride, float *__restrict__ y, int rows, int cols, int seq) {
+gemv_q5k_kernel(const uint8_t *__restrict__ w, const uint8_t *xq, size_t xq_stride, float *y, int rows, int cols, int seq) {
     pdl_launch_dependents();
     pdl_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -105,7 +105,7 @@ gemv_q5k_kernel(const uint8_t *__restrict__ w, const uint8_t *__restrict__ xq, s
 constexpr int TYPE_Q2_K = 10;
 constexpr int Q2K_BYTES = 84;
 RNB_GLOBAL void __launch_bounds__(G5_WARPS * 32)
-gemv_q2k_kernel(const uint8_t *__restrict__ w, const uint8_t *__restrict__ xq, size_t xq_stride, float *__restrict__ y, int rows, int cols, int seq) {
+gemv_q2k_kernel(const uint8_t *__restrict__ w, const uint8_t *xq, size_t xq_stride, float *y, int rows, int cols, int seq) {
     pdl_launch_dependents();
     pdl_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -174,7 +174,7 @@ __device__ __forceinline__ uint32_t ld32_a2(const uint8_t *p) {   // 4 bytes fro
     return (uint32_t)h[0] | ((uint32_t)h[1] << 16);
 }
 RNB_GLOBAL void __launch_bounds__(G5_WARPS * 32)
-gemv_q3k_kernel(const uint8_t *__restrict__ w, const uint8_t *__restrict__ xq, size_t xq_stride, float *__restrict__ y, int rows, int cols, int seq) {
+gemv_q3k_kernel(const uint8_t *__restrict__ w, const uint8_t *xq, size_t xq_stride, float *y, int rows, int cols, int seq) {
     pdl_launch_dependents();
     pdl_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;

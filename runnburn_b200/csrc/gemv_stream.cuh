@@ -128,8 +128,8 @@ __device__ __forceinline__ Q4kStep gr_q4k_step(const uint8_t *blk, const uint8_t
 }
 
 template <int TYPE>
-__device__ __forceinline__ void gr_run(const GemvJob *__restrict__ job, const GsParams &P, const int row0, const int nrows,
-                                       uint8_t *smem, uint64_t *full, int *__restrict__ dev_error) {
+__device__ __forceinline__ void gr_run(const GemvJob *job, const GsParams &P, const int row0, const int nrows,
+                                       uint8_t *smem, uint64_t *full, int *dev_error) {
     constexpr uint32_t BLK = TYPE == TYPE_Q4_K ? Q4K_BYTES : Q6K_BYTES;
     const int tid = threadIdx.x, lane = tid & 31;
     const int cols = P.cols, nb = cols >> 8, CB = P.chunk_blocks, S = P.n_stages, n_parts = job->n_parts;
@@ -249,13 +249,13 @@ __device__ __forceinline__ void gr_run(const GemvJob *__restrict__ job, const Gs
             if (nblk == GS_MAX_CHUNK) {
 #pragma unroll
                 for (int j = 0; j < GS_MAX_CHUNK; j++) {
-                    const Q4kStep st = gr_q4k_step(rowp + j * Q4K_BYTES, act + j * 256, bs16 + j * 16, __ldg(xd + j), t);
+                    const Q4kStep st = gr_q4k_step(rowp + j * Q4K_BYTES, act + j * 256, bs16 + j * 16, xd[j], t);
                     lane_acc = __fmaf_rn(st.d, (float)st.lane_sum, lane_acc);
                     min_acc = __fmaf_rn(st.dmin, (float)st.min_prod, min_acc);
                 }
             } else {
                 for (int j = 0; j < nblk; j++) {
-                    const Q4kStep st = gr_q4k_step(rowp + j * Q4K_BYTES, act + j * 256, bs16 + j * 16, __ldg(xd + j), t);
+                    const Q4kStep st = gr_q4k_step(rowp + j * Q4K_BYTES, act + j * 256, bs16 + j * 16, xd[j], t);
                     lane_acc = __fmaf_rn(st.d, (float)st.lane_sum, lane_acc);
                     min_acc = __fmaf_rn(st.dmin, (float)st.min_prod, min_acc);
                 }
@@ -269,15 +269,15 @@ __device__ __forceinline__ void gr_run(const GemvJob *__restrict__ job, const Gs
                 const uint32_t dh0 = *reinterpret_cast<const uint16_t *>(b0 + 208), dh1 = *reinterpret_cast<const uint16_t *>(b1 + 208);
                 const int ls0 = gs_q6k_lanes<0>(b0, act + j * 256, bs16 + j * 16, 0.f, t, true, &dd);
                 const int ls1 = gs_q6k_lanes<2>(b1, act + (j + 1) * 256, bs16 + (j + 1) * 16, 0.f, t, true, &dd);
-                lane_acc = __fmaf_rn(__fmul_rn(__ldg(xd + j), f16_bits_to_f32(dh0)), (float)ls0, lane_acc);
-                lane_acc = __fmaf_rn(__fmul_rn(__ldg(xd + j + 1), f16_bits_to_f32(dh1)), (float)ls1, lane_acc);
+                lane_acc = __fmaf_rn(__fmul_rn(xd[j], f16_bits_to_f32(dh0)), (float)ls0, lane_acc);
+                lane_acc = __fmaf_rn(__fmul_rn(xd[j + 1], f16_bits_to_f32(dh1)), (float)ls1, lane_acc);
             }
             if (nblk & 1) {
                 const int j = nblk - 1;
                 const uint8_t *b0 = rowp + j * Q6K_BYTES;
                 const uint32_t dh0 = *reinterpret_cast<const uint16_t *>(b0 + 208);
                 const int ls0 = gs_q6k_lanes<0>(b0, act + j * 256, bs16 + j * 16, 0.f, t, true, &dd);
-                lane_acc = __fmaf_rn(__fmul_rn(__ldg(xd + j), f16_bits_to_f32(dh0)), (float)ls0, lane_acc);
+                lane_acc = __fmaf_rn(__fmul_rn(xd[j], f16_bits_to_f32(dh0)), (float)ls0, lane_acc);
             }
         }
         __syncthreads();  // slot consumed by every group
@@ -300,7 +300,7 @@ __device__ __forceinline__ void gr_run(const GemvJob *__restrict__ job, const Gs
                 hs = __fadd_rn(hs, __shfl_xor_sync(0xffffffffu, hs, 4));
                 dot = hs;
             }
-            if (job->parts[p].scale) dot = __fmul_rn(dot, __ldg(job->parts[p].scale));
+            if (job->parts[p].scale) dot = __fmul_rn(dot, *job->parts[p].scale);
             acc_total = n_parts == 1 ? dot : __fadd_rn(acc_total, dot);
             lane_acc = 0.f;
             min_acc = 0.f;
@@ -335,8 +335,8 @@ __device__ __forceinline__ void gr_run(const GemvJob *__restrict__ job, const Gs
     else job->epi_cache[(size_t)pos * job->epi_kv_dim + o] = __half_as_ushort(__float2half_rn(outv));
 }
 
-__device__ __forceinline__ void gemv_stream_body(const GemvJob *__restrict__ jobs, int n_jobs, const GsParams &P,
-                                                   int *__restrict__ dev_error) {
+__device__ __forceinline__ void gemv_stream_body(const GemvJob *jobs, int n_jobs, const GsParams &P,
+                                                   int *dev_error) {
     if (P.dynamic_table) pdl_wait();
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ __align__(8) uint64_t full[GS_MAX_STAGES];
@@ -364,7 +364,7 @@ __device__ __forceinline__ void gemv_stream_body(const GemvJob *__restrict__ job
     else gr_run<TYPE_Q6_K>(job, P, row0, nrows, smem, full, dev_error);
 }
 RNB_GLOBAL void __launch_bounds__(128)
-gemv_stream_kernel(const GemvJob *__restrict__ jobs, int n_jobs, const GsParams P, int *__restrict__ dev_error) {
+gemv_stream_kernel(const GemvJob *jobs, int n_jobs, const GsParams P, int *dev_error) {
     gemv_stream_body(jobs, n_jobs, P, dev_error);
 }
 // Static job tables travel as a kernel parameter (constant bank): no dependent global loads
@@ -374,7 +374,7 @@ struct GemvJobPack {
     GemvJob j[GS_PACK];
 };
 RNB_GLOBAL void __launch_bounds__(128)
-gemv_stream_kernel_1(const __grid_constant__ GemvJobPack jobs, int n_jobs, const GsParams P, int *__restrict__ dev_error) {
+gemv_stream_kernel_1(const __grid_constant__ GemvJobPack jobs, int n_jobs, const GsParams P, int *dev_error) {
     gemv_stream_body(jobs.j, n_jobs, P, dev_error);
 }
 

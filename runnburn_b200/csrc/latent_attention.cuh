@@ -29,8 +29,8 @@ __device__ __forceinline__ void latent_append_row(const float *y, const float *w
 // grid = tokens
 template <class CT>
 RNB_GLOBAL void __launch_bounds__(128)
-latent_append_kernel(const float *__restrict__ y, const float *__restrict__ w, float eps, const LatentDims d, const Rotation rot, const int *__restrict__ pos0,
-                     CT *__restrict__ cache) {
+latent_append_kernel(const float *y, const float *__restrict__ w, float eps, const LatentDims d, const Rotation rot, const int *pos0,
+                     CT *cache) {
     __shared__ float red[32];
     pdl_launch_dependents();
     pdl_wait();
@@ -140,8 +140,8 @@ __host__ __device__ __forceinline__ int latent_part_ld(int rank) { return ((rank
 // floats) holds the unnormalised latent sum (rank), the maximum and the sum of the weights.
 template <class CT, int NQ>
 RNB_GLOBAL void __launch_bounds__(128)
-latent_attend_kernel(const float *__restrict__ qf, const CT *__restrict__ cache, const LatentDims d, float scale, const int *__restrict__ pos0,
-                     float *__restrict__ part) {
+latent_attend_kernel(const float *qf, const CT *cache, const LatentDims d, float scale, const int *pos0,
+                     float *part) {
     __shared__ float s_o[4][32 * NQ], s_m[4], s_l[4];
     pdl_launch_dependents();
     pdl_wait();
@@ -194,8 +194,8 @@ latent_attend_kernel(const float *__restrict__ qf, const CT *__restrict__ cache,
 constexpr int LO_THREADS = 512;
 template <class HT>
 RNB_GLOBAL void __launch_bounds__(LO_THREADS)
-latent_output_kernel(const float *__restrict__ part, const bf16 *__restrict__ uv, const LatentDims d, int max_chunks, const int *__restrict__ pos0, int rows_per_cta,
-                     HT *__restrict__ act, int lda, float mul) {
+latent_output_kernel(const float *part, const bf16 *__restrict__ uv, const LatentDims d, int max_chunks, const int *pos0, int rows_per_cta,
+                     HT *act, int lda, float mul) {
     extern __shared__ __align__(16) float lo_smem[];
     __shared__ float s_inv;
     pdl_launch_dependents();
@@ -278,8 +278,8 @@ __host__ __device__ inline LatentMmaSmem latent_mma_smem(const LatentDims &d) {
 }
 template <int NT>
 RNB_GLOBAL void __launch_bounds__(LM_THREADS)
-latent_attend_mma_kernel(const bf16 *__restrict__ qf, const bf16 *__restrict__ cache, const LatentDims d, float scale, const int *__restrict__ pos0,
-                         float *__restrict__ part) {
+latent_attend_mma_kernel(const bf16 *qf, const bf16 *cache, const LatentDims d, float scale, const int *pos0,
+                         float *part) {
     extern __shared__ __align__(128) uint8_t lm_smem[];
     pdl_launch_dependents();
     pdl_wait();

@@ -25,7 +25,7 @@ __device__ __forceinline__ void prefetch_l2(const void *p, size_t bytes, int tid
 
 // grid = tokens.  x and (when kept for later passes) emb: [tokens][width] f32
 RNB_GLOBAL void __launch_bounds__(256)
-dense_embed_kernel(const bf16 *__restrict__ table, const uint32_t *__restrict__ token, int width, float scale, float *__restrict__ x, float *__restrict__ emb) {
+dense_embed_kernel(const bf16 *__restrict__ table, const uint32_t *token, int width, float scale, float *x, float *emb) {
     pdl_launch_dependents();
     pdl_wait();
     const size_t row = (size_t)token[blockIdx.x] * width, o = (size_t)blockIdx.x * width;
@@ -240,8 +240,8 @@ residual_norm_step_kernel(const __grid_constant__ ResidualNormArgs a) {
 // rows null: row blockIdx.x itself.  grid = rows, dynamic shared memory none.
 template <class HT>
 RNB_GLOBAL void __launch_bounds__(512)
-norm_rows_kernel(const float *__restrict__ x, const int *__restrict__ rows, const float *__restrict__ w, const float *__restrict__ b, float eps, int width,
-                 HT *__restrict__ h) {
+norm_rows_kernel(const float *x, const int *rows, const float *__restrict__ w, const float *__restrict__ b, float eps, int width,
+                 HT *h) {
     __shared__ float red[32];
     pdl_launch_dependents();
     pdl_wait();

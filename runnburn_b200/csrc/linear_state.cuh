@@ -161,7 +161,7 @@ linear_state_chunk_kernel(const __grid_constant__ LinearChunkArgs a) {
 // elements of a channel's row; the contributions of eight chunks are in flight at a time.
 template <int V>
 RNB_GLOBAL void __launch_bounds__(256)
-linear_state_scan_kernel(const float *__restrict__ state, float *starts, const float *__restrict__ decays, const float *__restrict__ decay, int heads, int dim,
+linear_state_scan_kernel(const float *state, float *starts, const float *decays, const float *__restrict__ decay, int heads, int dim,
                          int vdim, int chunk, int n_chunks) {
     pdl_launch_dependents();
     pdl_wait();
@@ -194,8 +194,8 @@ linear_state_scan_kernel(const float *__restrict__ state, float *starts, const f
 // Decays from their low-rank input: out[t][c] = decay_of(sum_j w2[c][j] f(z[t][j]) + w0[c]); f: tanh for DECAY_EXP, else none.
 // grid = (ceil(channels / 128), ceil(tokens / 16)), 128 threads; dynamic shared memory 16 * rank floats.
 RNB_GLOBAL void __launch_bounds__(128)
-decay_rows_kernel(const float *__restrict__ z, const bf16 *__restrict__ w2, const float *__restrict__ w0, int tokens, int rank, int channels, int kind,
-                  float inv_tau, float *__restrict__ out) {
+decay_rows_kernel(const float *z, const bf16 *__restrict__ w2, const float *__restrict__ w0, int tokens, int rank, int channels, int kind,
+                  float inv_tau, float *out) {
     extern __shared__ __align__(16) float dr_smem[];   // [rank][16]
     pdl_launch_dependents();
     pdl_wait();
@@ -231,7 +231,7 @@ decay_rows_kernel(const float *__restrict__ z, const bf16 *__restrict__ w2, cons
 // z [tokens][rank] f32 -> [f(z) rounded to bf16 | what the rounding left] [tokens][2 rank], f = tanh or none: against
 // [w2 | w2] the tensor-core matmul gives w2 f(z) to about f32 accuracy.
 RNB_GLOBAL void __launch_bounds__(256)
-split_rows_kernel(const float *__restrict__ z, int rank, size_t n, int kind, bf16 *__restrict__ out) {
+split_rows_kernel(const float *z, int rank, size_t n, int kind, bf16 *out) {
     pdl_launch_dependents();
     pdl_wait();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;

@@ -13,7 +13,7 @@ namespace rnb {
 // logits are what makes the selected expert ids identical.  hidden % 16 == 0.
 // The loads of a batch of steps are issued together (the chain of FMAs is latency-bound on its
 // loads otherwise).  Any number of experts per CTA (blockDim / 16).
-__device__ __forceinline__ void router_logits_body(const float *__restrict__ w, const float *__restrict__ h, int n_expert,
+__device__ __forceinline__ void router_logits_body(const float *__restrict__ w, const float *h, int n_expert,
                                                    int hidden, float *logits) {
     pdl_launch_dependents();
     // WB steps of router weights per batch (elements j, j + 16, ...) are in registers before they are needed: the
@@ -54,8 +54,8 @@ __device__ __forceinline__ void router_logits_body(const float *__restrict__ w, 
     if (live && j == 0) logits[e] = acc;
 }
 RNB_GLOBAL void __launch_bounds__(128)
-router_logits_kernel(const float *__restrict__ w, const float *__restrict__ h, int n_expert,
-                     int hidden, float *__restrict__ logits) {
+router_logits_kernel(const float *__restrict__ w, const float *h, int n_expert,
+                     int hidden, float *logits) {
     router_logits_body(w, h, n_expert, hidden, logits);
 }
 
@@ -66,7 +66,7 @@ router_logits_kernel(const float *__restrict__ w, const float *__restrict__ h, i
 // One warp per token; n_expert <= 1024, top_k <= 32.  exp is libm's expf (expf_libm), as the CPU's routing.
 // Returns the id this lane selected (lane r holds rank r; other lanes return 0).
 __device__ __forceinline__ uint32_t moe_route_topk_warp(const float *logits, int token, int n_expert, int top_k,
-                                                        uint32_t *__restrict__ ids_out, float *__restrict__ weights_out) {
+                                                        uint32_t *ids_out, float *weights_out) {
     const int lane = threadIdx.x;
     const float *lg = logits + (size_t)token * n_expert;
     uint32_t *ids = ids_out + (size_t)token * top_k;
@@ -130,8 +130,8 @@ __device__ __forceinline__ uint32_t moe_route_topk_warp(const float *logits, int
     return my_id;
 }
 RNB_GLOBAL void __launch_bounds__(32)
-moe_route_topk_kernel(const float *__restrict__ logits, int n_expert, int top_k,
-                      uint32_t *__restrict__ ids_out, float *__restrict__ weights_out) {
+moe_route_topk_kernel(const float *logits, int n_expert, int top_k,
+                      uint32_t *ids_out, float *weights_out) {
     pdl_launch_dependents();
     pdl_wait();
     moe_route_topk_warp(logits, (int)blockIdx.x, n_expert, top_k, ids_out, weights_out);
@@ -144,8 +144,8 @@ struct MoeLayerPtrs {
     const uint8_t *gate_base, *up_base, *down_base;
     size_t gate_stride, down_stride;
 };
-__device__ __forceinline__ void moe_fill_jobs_warp(size_t id, const float *__restrict__ weights, int top_k,
-                                                   const MoeLayerPtrs &lp, GemvJob *__restrict__ gate_up_jobs, GemvJob *__restrict__ down_job) {
+__device__ __forceinline__ void moe_fill_jobs_warp(size_t id, const float *weights, int top_k,
+                                                   const MoeLayerPtrs &lp, GemvJob *gate_up_jobs, GemvJob *down_job) {
     const int e = threadIdx.x;
     if (e >= top_k) return;
     gate_up_jobs[e].parts[0].w = lp.gate_base + id * lp.gate_stride;
@@ -157,9 +157,9 @@ __device__ __forceinline__ void moe_fill_jobs_warp(size_t id, const float *__res
 // experts' logits each; the CTA that finishes last (a counter that it re-arms) selects the experts
 // and points the expert-gathered matvecs at them.
 RNB_GLOBAL void __launch_bounds__(32)
-router_route_fill_kernel(const float *__restrict__ w, const float *__restrict__ h, int n_expert, int hidden, float *logits,
-                         int top_k, uint32_t *__restrict__ ids_out, float *__restrict__ weights_out, MoeLayerPtrs lp,
-                         GemvJob *__restrict__ gate_up_jobs, GemvJob *__restrict__ down_job, int *__restrict__ counter) {
+router_route_fill_kernel(const float *__restrict__ w, const float *h, int n_expert, int hidden, float *logits,
+                         int top_k, uint32_t *ids_out, float *weights_out, MoeLayerPtrs lp,
+                         GemvJob *gate_up_jobs, GemvJob *down_job, int *counter) {
     router_logits_body(w, h, n_expert, hidden, logits);
     __threadfence();   // this CTA's logits are visible device-wide before the CTA is counted
     __syncwarp();

@@ -12,9 +12,9 @@ namespace rnb {
 // keys 0..(kv_len - seq_len + i).  q/out f32 [seq][heads][128]; k, v [kv_len][kv_heads][128].
 template <typename KVT>
 RNB_GLOBAL void __launch_bounds__(FD_THREADS)
-prefill_attention_kernel(const float *__restrict__ q, const KVT *__restrict__ k,
-                         const KVT *__restrict__ v, int seq_len, int kv_len, int num_heads,
-                         int num_kv_heads, float scale, float *__restrict__ out) {
+prefill_attention_kernel(const float *q, const KVT *k,
+                         const KVT *v, int seq_len, int kv_len, int num_heads,
+                         int num_kv_heads, float scale, float *out) {
     pdl_launch_dependents();
     pdl_wait();
     __shared__ float s_acc[(FD_THREADS / 32) * 4 * HD];

@@ -98,8 +98,8 @@ __device__ __forceinline__ void pat_tmem_st_wait() { asm volatile("tcgen05.wait:
 // num_heads / num_kv_heads a power of two up to 128.  The softmax needs a positive scale (its maxima are of unscaled scores): the
 // sign, or zero, of another one goes into the queries.  out_bf16 (may be null): the result rounded to bf16 there instead of f32 in `out`.
 RNB_GLOBAL void __launch_bounds__(PAT_THREADS, 2)
-prefill_attention_tiled_kernel(const float *__restrict__ q, const __grid_constant__ PatMaps maps, int seq_len, int kv_len, int num_heads, int num_kv_heads,
-                               float scale, float *__restrict__ out, uint16_t *__restrict__ out_bf16, int *__restrict__ err_flag) {
+prefill_attention_tiled_kernel(const float *q, const __grid_constant__ PatMaps maps, int seq_len, int kv_len, int num_heads, int num_kv_heads,
+                               float scale, float *out, uint16_t *out_bf16, int *err_flag) {
     extern __shared__ __align__(1024) uint8_t pat_smem[];
     pdl_launch_dependents();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;

@@ -100,7 +100,7 @@ __device__ __forceinline__ uint4 pg_pair_exchange(const uint4 &mine) {
 }
 // f32 -> bf16 rows (activation), padded to a multiple of 8 columns by construction (cols % 256 == 0)
 RNB_GLOBAL void __launch_bounds__(256)
-f32_to_bf16_kernel(const float *__restrict__ x, uint16_t *__restrict__ y, size_t n) {
+f32_to_bf16_kernel(const float *x, uint16_t *y, size_t n) {
     pdl_launch_dependents();
     pdl_wait();
     const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 8;
@@ -115,8 +115,8 @@ f32_to_bf16_kernel(const float *__restrict__ x, uint16_t *__restrict__ y, size_t
 // token; hidden % 256 == 0.  A row of up to 16 elements per thread stays in registers between the sum and the output.
 template <int THREADS>
 RNB_GLOBAL void __launch_bounds__(THREADS)
-add_rmsnorm_bf16_kernel(float *__restrict__ x, const float *__restrict__ t, const float *__restrict__ w, float eps, int hidden,
-                        uint16_t *__restrict__ out) {
+add_rmsnorm_bf16_kernel(float *x, const float *t, const float *__restrict__ w, float eps, int hidden,
+                        uint16_t *out) {
     constexpr int KEEP = 4;
     pdl_launch_dependents();
     pdl_wait();
@@ -164,7 +164,7 @@ add_rmsnorm_bf16_kernel(float *__restrict__ x, const float *__restrict__ t, cons
 // silu_mul_q8k_kernel) written straight as the bf16 token matrix of the down
 // matmul: the f32 value is rounded to bf16 exactly as f32_to_bf16_kernel would round it.
 RNB_GLOBAL void __launch_bounds__(256)
-silu_mul_bf16_kernel(const float *__restrict__ gate, const float *__restrict__ up, uint16_t *__restrict__ y, size_t n) {
+silu_mul_bf16_kernel(const float *gate, const float *up, uint16_t *y, size_t n) {
     pdl_launch_dependents();
     pdl_wait();
     const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 8;

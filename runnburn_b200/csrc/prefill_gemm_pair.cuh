@@ -302,7 +302,7 @@ __device__ __forceinline__ void pt_store(const PgJob &job, int r, int tok0, int 
 // CUT: ks > 1, a cluster per tile.  grid = 2 x ks x pairs, cluster (2 ks, 1, 1).  PT_THREADS threads; dynamic shared memory PT_SMEM.
 template <bool CUT>
 RNB_GLOBAL void __launch_bounds__(PT_THREADS, 1)
-prefill_gemm_pair_kernel(const __grid_constant__ PgJobs jobs, const __grid_constant__ PtMaps maps, const PtParams P, int *__restrict__ err_flag) {
+prefill_gemm_pair_kernel(const __grid_constant__ PgJobs jobs, const __grid_constant__ PtMaps maps, const PtParams P, int *err_flag) {
     extern __shared__ __align__(1024) uint8_t pg_smem_raw[];
     // weights written (both CTAs' warps), tokens landed (both CTAs' copies), stage free; blocks landed, read; accumulators complete, read
     __shared__ __align__(8) uint64_t w_full[PT_STAGES], full[PT_STAGES], empty[PT_STAGES], raw_full[PT_RAWS], raw_empty[PT_RAWS], acc_full, acc_free;

@@ -141,7 +141,7 @@ __device__ __forceinline__ void ps_finish(const PgJob &job, const PsParams &P, u
 
 // grid = row tiles of all jobs; 320 threads; dynamic shared memory PS_SMEM.
 RNB_GLOBAL void __launch_bounds__(PS_THREADS, 2)
-prefill_gemm_split_kernel(const __grid_constant__ PgJobs jobs, const __grid_constant__ PgTensorMap tmap_x, const PsParams P, int *__restrict__ err_flag) {
+prefill_gemm_split_kernel(const __grid_constant__ PgJobs jobs, const __grid_constant__ PgTensorMap tmap_x, const PsParams P, int *err_flag) {
     extern __shared__ __align__(1024) uint8_t pg_smem_raw[];
     __shared__ __align__(8) uint64_t full[PS_MAX_STAGES], empty[PS_MAX_STAGES], done_bar;
     __shared__ uint32_t tmem_slot;

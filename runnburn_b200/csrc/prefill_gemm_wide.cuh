@@ -42,7 +42,7 @@ struct PwMaps {   // tokens of the two parts (boxes of n1 / 2 and n2 / 2), block
 
 // grid = 2 x pairs, cluster (2, 1, 1); PW_THREADS threads; dynamic shared memory PW_SMEM.
 RNB_GLOBAL void __launch_bounds__(PW_THREADS, 1)
-prefill_gemm_wide_kernel(const __grid_constant__ PgJobs jobs, const __grid_constant__ PwMaps maps, const PwParams P, int *__restrict__ err_flag) {
+prefill_gemm_wide_kernel(const __grid_constant__ PgJobs jobs, const __grid_constant__ PwMaps maps, const PwParams P, int *err_flag) {
     extern __shared__ __align__(1024) uint8_t pg_smem_raw[];
     __shared__ __align__(8) uint64_t full[PW_STAGES], empty[PW_STAGES], raw_full, raw_empty, acc_full, acc_free;
     __shared__ uint32_t tmem_slot;

@@ -80,7 +80,7 @@ __device__ __forceinline__ Q8kDevView q8k_dev_view(uint8_t *base, int cols) {
 // x: [seq][cols] f32.  dev_out: [seq] device-layout vectors (stride q8k_dev_bytes(cols)), may
 // be null.  ref_out: [seq][cols/256] reference 292-byte blocks, may be null.
 RNB_GLOBAL void __launch_bounds__(128)
-quantize_q8k_kernel(const float *__restrict__ x, int cols, int seq, uint8_t *dev_out,
+quantize_q8k_kernel(const float *x, int cols, int seq, uint8_t *dev_out,
                     uint8_t *ref_out) {
     pdl_launch_dependents();
     pdl_wait();
@@ -104,8 +104,8 @@ quantize_q8k_kernel(const float *__restrict__ x, int cols, int seq, uint8_t *dev
 // result.  One CTA per token.  `h_out` (f32 normalised vector) is optional.
 template <int THREADS>
 RNB_GLOBAL void __launch_bounds__(THREADS)
-rmsnorm_q8k_kernel(const float *__restrict__ x, const float *__restrict__ w, float eps, int hidden,
-                   float *__restrict__ h_out, uint8_t *__restrict__ xq_out) {
+rmsnorm_q8k_kernel(const float *x, const float *__restrict__ w, float eps, int hidden,
+                   float *h_out, uint8_t *xq_out) {
     pdl_launch_dependents();
     pdl_wait();
     __shared__ double red[THREADS / 32];
@@ -155,7 +155,7 @@ rmsnorm_q8k_kernel(const float *__restrict__ x, const float *__restrict__ w, flo
 constexpr int RQ_THREADS = 256, RQ_AHEAD = 4;
 RNB_GLOBAL void __launch_bounds__(RQ_THREADS)
 rmsnorm_q8k_blocks_kernel(const float *x, const float *__restrict__ w, float eps, int hidden,
-                          float *__restrict__ h_out, uint8_t *__restrict__ xq_out, const PeerWait pw = PeerWait{}) {
+                          float *h_out, uint8_t *xq_out, const PeerWait pw = PeerWait{}) {
     pdl_launch_dependents();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, b = blockIdx.x;
     // the norm weights do not depend on the previous kernel
@@ -209,8 +209,8 @@ rmsnorm_q8k_blocks_kernel(const float *x, const float *__restrict__ w, float eps
 // fused with Q8_K quantisation.  exp is libm's expf evaluated as the C library does (expf_libm),
 // so the value fed to the quantiser has the CPU's bits.
 RNB_GLOBAL void __launch_bounds__(128)
-silu_mul_q8k_kernel(const float *__restrict__ gate, const float *__restrict__ up, int n, int seq,
-                    float *__restrict__ act_out, uint8_t *__restrict__ xq_out) {
+silu_mul_q8k_kernel(const float *gate, const float *up, int n, int seq,
+                    float *act_out, uint8_t *xq_out) {
     pdl_launch_dependents();
     pdl_wait();
     const int nb = n / 256;

@@ -88,3 +88,42 @@ def test_steps_repeat_their_bits():
     for _ in range(10):
         assert np.array_equal(su.feed(dec, toks, [200] + [1] * 30), first)
     dec.close()
+
+
+def _step_models():
+    import runnburn_b200 as r
+    import stack_util as su
+    from synth import moe_description
+
+    def dense(exact, describe=llama_description):
+        desc = describe(seed=3)
+        dec = r.Decoder(r.ModelConfig(max_ctx=256, **desc["cfg"]))
+        dec.set_exact_attention_max(256 if exact else 0)
+        dec.load_description(desc)
+        return dec
+
+    def stack(cfg):
+        return su.decoder(cfg, su.weights(cfg, 5), "float32")
+
+    mixed = su.config([su.wkv(), su.retention(), su.latent()], residual_mult=1.0)
+    return {"exact": lambda: dense(True), "flash": lambda: dense(False), "experts": lambda: dense(False, moe_description),
+            "punisun": lambda: stack(mixed), "dutivik": lambda: stack(su.dutivik([su.parallel(), su.gla()]))}
+
+
+@pytest.mark.parametrize("model", ["exact", "flash", "experts", "punisun", "dutivik"])
+def test_chained_steps_repeat_the_bits_of_host_steps(model):
+    """60 steps with one launch starting behind the other, fifteen times over: the logits at the end are those of steps that the host
+    waits for, bit for bit, for every kind of layer (no launch reads what the one before has yet to write)."""
+    dec = _step_models()[model]()
+    prompt, steps = np.random.default_rng(4).integers(0, 90, 20).tolist(), 60
+    token = dec.prefill(prompt, 0)
+    for pos in range(20, 20 + steps):
+        token, logits = dec.step(token, pos, want_logits=True)
+    for _ in range(15):
+        dec.prefill(prompt, 0)
+        dec.step_dev(20, True)
+        for _ in range(steps - 1):
+            dec.step_dev(-1, True)
+        dec.sync()
+        assert np.array_equal(dec.read_logits(), logits)
+    dec.close()
