@@ -566,14 +566,14 @@ __device__ __forceinline__ void fdm_body(const float *q, const uint16_t *k, cons
             if (hA + e < group) {
                 const float *base = partials + (size_t)head * n_chunks * FD_PART_STRIDE;
                 float M = -INFINITY;
-                for (int c = 0; c < n_chunks; c++) M = fmaxf(M, __ldcg(base + (size_t)c * FD_PART_STRIDE + HD));
+                for (int c = 0; c < n_chunks; c++) M = fmaxf(M, ld_l2(base + (size_t)c * FD_PART_STRIDE + HD));
                 float a = 0.f, L = 0.f;
 #pragma unroll 4
                 for (int c = 0; c < n_chunks; c++) {
-                    const float mc = __ldcg(base + (size_t)c * FD_PART_STRIDE + HD);
+                    const float mc = ld_l2(base + (size_t)c * FD_PART_STRIDE + HD);
                     const float f = mc == -INFINITY ? 0.f : expf(mc - M);
-                    L += __ldcg(base + (size_t)c * FD_PART_STRIDE + HD + 1) * f;
-                    a += __ldcg(base + (size_t)c * FD_PART_STRIDE + tid) * f;
+                    L += ld_l2(base + (size_t)c * FD_PART_STRIDE + HD + 1) * f;
+                    a += ld_l2(base + (size_t)c * FD_PART_STRIDE + tid) * f;
                 }
                 o_val = L > 0.f ? a / L : 0.f;
                 if (merge.out) merge.out[(size_t)head * HD + tid] = o_val;
@@ -610,14 +610,14 @@ __device__ __forceinline__ void fdm_body(const float *q, const uint16_t *k, cons
             const int head = kv_h * group + g0 + hh;
             const float *base = partials + (size_t)head * n_chunks * FD_PART_STRIDE;
             float m = -INFINITY;
-            for (int c = lane; c < n_chunks; c += 32) m = fmaxf(m, __ldcg(base + (size_t)c * FD_PART_STRIDE + HD));
+            for (int c = lane; c < n_chunks; c += 32) m = fmaxf(m, ld_l2(base + (size_t)c * FD_PART_STRIDE + HD));
             const float M = warp_max(m);
             float l = 0.f;
             for (int c = lane; c < n_chunks; c += 32) {
-                const float mc = __ldcg(base + (size_t)c * FD_PART_STRIDE + HD);
+                const float mc = ld_l2(base + (size_t)c * FD_PART_STRIDE + HD);
                 const float f = mc == -INFINITY ? 0.f : expf(mc - M);
                 my_f[c] = f;
-                l += __ldcg(base + (size_t)c * FD_PART_STRIDE + HD + 1) * f;
+                l += ld_l2(base + (size_t)c * FD_PART_STRIDE + HD + 1) * f;
             }
             const float L = warp_sum(l);
             __syncwarp();
@@ -626,7 +626,7 @@ __device__ __forceinline__ void fdm_body(const float *q, const uint16_t *k, cons
             for (int c = 0; c < n_chunks; c++) {
                 // records are 130 floats apart: 8-byte alignment is all that holds for every chunk
                 const float2 *rp = reinterpret_cast<const float2 *>(base + (size_t)c * FD_PART_STRIDE) + 2 * lane;
-                const float2 r0 = __ldcg(rp), r1 = __ldcg(rp + 1);
+                const float2 r0 = ld_l2(rp), r1 = ld_l2(rp + 1);
                 const float f = my_f[c];
                 a.x += r0.x * f;
                 a.y += r0.y * f;

@@ -321,8 +321,8 @@ static __device__ __noinline__ void gm_silu_tail(const GpTail &tail, int blk, in
     if (!last) return;
     __threadfence();
     const size_t off = (size_t)blk * 256 + lane * 8;
-    const float4 g0 = __ldcg(reinterpret_cast<const float4 *>(tail.gate + off)), g1 = __ldcg(reinterpret_cast<const float4 *>(tail.gate + off + 4));
-    const float4 u0 = __ldcg(reinterpret_cast<const float4 *>(tail.up + off)), u1 = __ldcg(reinterpret_cast<const float4 *>(tail.up + off + 4));
+    const float4 g0 = ld_l2(reinterpret_cast<const float4 *>(tail.gate + off)), g1 = ld_l2(reinterpret_cast<const float4 *>(tail.gate + off + 4));
+    const float4 u0 = ld_l2(reinterpret_cast<const float4 *>(tail.up + off)), u1 = ld_l2(reinterpret_cast<const float4 *>(tail.up + off + 4));
     const float gv[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w}, uv[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
     float v[8];
 #pragma unroll

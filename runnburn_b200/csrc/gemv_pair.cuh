@@ -151,7 +151,7 @@ __device__ __forceinline__ void gemv_pair_body(const GemvJobPack &jobs, int n_jo
         // the ids come from an earlier kernel: nothing can be fetched before the wait
         pdl_wait();
         const int e = row0 / job.dyn_rows;
-        const uint32_t id = __ldcg(job.dyn_ids + e);
+        const uint32_t id = ld_l2(job.dyn_ids + e);
         w = job.parts[0].w + ((size_t)id * (size_t)job.dyn_rows + (size_t)(row0 - e * job.dyn_rows)) * rb;
         x += (size_t)e * job.dyn_x_stride;
     }
@@ -207,8 +207,8 @@ __device__ __forceinline__ void gemv_pair_body(const GemvJobPack &jobs, int n_jo
         if (!last) return;
         __threadfence();
         const size_t off = (size_t)blk * 256 + lane * 8;
-        const float4 g0 = __ldcg(reinterpret_cast<const float4 *>(tail.gate + off)), g1 = __ldcg(reinterpret_cast<const float4 *>(tail.gate + off + 4));
-        const float4 u0 = __ldcg(reinterpret_cast<const float4 *>(tail.up + off)), u1 = __ldcg(reinterpret_cast<const float4 *>(tail.up + off + 4));
+        const float4 g0 = ld_l2(reinterpret_cast<const float4 *>(tail.gate + off)), g1 = ld_l2(reinterpret_cast<const float4 *>(tail.gate + off + 4));
+        const float4 u0 = ld_l2(reinterpret_cast<const float4 *>(tail.up + off)), u1 = ld_l2(reinterpret_cast<const float4 *>(tail.up + off + 4));
         const float gv[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w}, uv[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
         float v[8];
 #pragma unroll
@@ -243,8 +243,8 @@ __device__ __forceinline__ void gemv_pair_body(const GemvJobPack &jobs, int n_jo
         if (lane < RPT && lrow0 + lane < tail.n) {
             const size_t o = (size_t)lrow0 + lane;
             float acc = 0.f;
-            for (int k = 0; k < tail.sum_k; k++) acc = __fadd_rn(acc, __fmul_rn(__ldcg(tail.gate + (size_t)k * tail.n + o), __ldcg(tail.up + k)));
-            tail.sum_out[o] = tail.sum_res ? __fadd_rn(__ldcg(tail.sum_res + o), acc) : acc;
+            for (int k = 0; k < tail.sum_k; k++) acc = __fadd_rn(acc, __fmul_rn(ld_l2(tail.gate + (size_t)k * tail.n + o), ld_l2(tail.up + k)));
+            tail.sum_out[o] = tail.sum_res ? __fadd_rn(ld_l2(tail.sum_res + o), acc) : acc;
         }
         if (lane == 0) tail.counters[ctr] = 0;
     }

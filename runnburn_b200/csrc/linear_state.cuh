@@ -593,13 +593,13 @@ __device__ __forceinline__ void head_norm_gate_rows(const float *o, const float 
         const float *x = o + ((size_t)t * heads + h) * vdim;
         float ss = 0.f;
         for (int i = lane; i < vdim; i += 32) {
-            const float v = __ldcg(x + i);
+            const float v = ld_l2(x + i);
             ss = fmaf(v, v, ss);
         }
         const float r = mul / sqrtf(warp_sum(ss) / (float)vdim + eps);
         const float *gt = g + (size_t)t * ldg + (size_t)h * vdim;
         float *at = act + (size_t)t * lda + (size_t)h * vdim;
-        for (int i = lane; i < vdim; i += 32) at[i] = __ldcg(x + i) * r * (norm ? norm[(size_t)h * norm_head + i] : 1.0f) * silu_f32(gt[i]);
+        for (int i = lane; i < vdim; i += 32) at[i] = ld_l2(x + i) * r * (norm ? norm[(size_t)h * norm_head + i] : 1.0f) * silu_f32(gt[i]);
     }
 }
 struct LinearStepArgs {

@@ -82,7 +82,7 @@ __device__ __forceinline__ uint32_t moe_route_topk_warp(const float *logits, int
     float cv[RC];
     if (cached) {
 #pragma unroll
-        for (int s = 0; s < RC; s++) cv[s] = lane + 32 * s < n_expert ? __ldcg(lg + lane + 32 * s) : 0.0f;
+        for (int s = 0; s < RC; s++) cv[s] = lane + 32 * s < n_expert ? ld_l2(lg + lane + 32 * s) : 0.0f;
     }
     for (int r = 0; r < sel; r++) {
         float best = -INFINITY;
@@ -99,7 +99,7 @@ __device__ __forceinline__ uint32_t moe_route_topk_warp(const float *logits, int
         } else {
             for (int s = 0, e = lane; e < n_expert; s++, e += 32) {
                 if (taken & (1u << s)) continue;
-                const float v = __ldcg(lg + e);   // may have been written by other CTAs of the same launch
+                const float v = ld_l2(lg + e);   // may have been written by other CTAs of the same launch
                 if (bi == 0x7fffffff || v > best) {  // ascending e: strict > keeps the lowest id
                     best = v;
                     bi = e;

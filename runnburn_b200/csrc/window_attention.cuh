@@ -421,8 +421,8 @@ __device__ __forceinline__ void attention_step_block(const WindowAttentionArgs &
 #pragma unroll
         for (int i = 0; i < 2; i++) {
             const int c = lane + 32 * i;
-            mc[i] = c < active ? __ldcg(part + c * pl + rep * vdim + j) : -INFINITY;
-            lc[i] = c < active ? __ldcg(part + c * pl + rep * (vdim + 1) + j) : 0.f;
+            mc[i] = c < active ? ld_l2(part + c * pl + rep * vdim + j) : -INFINITY;
+            lc[i] = c < active ? ld_l2(part + c * pl + rep * (vdim + 1) + j) : 0.f;
             m = fmaxf(m, mc[i]);
         }
         m = warp_max(m);
@@ -440,7 +440,7 @@ __device__ __forceinline__ void attention_step_block(const WindowAttentionArgs &
         const int j = i / vdim;
         float o = 0.f;
 #pragma unroll 8
-        for (int c = 0; c < active; c++) o = fmaf(ss[j * AS_KEYS + c], __ldcg(part + c * pl + i), o);
+        for (int c = 0; c < active; c++) o = fmaf(ss[j * AS_KEYS + c], ld_l2(part + c * pl + i), o);
         act[(size_t)(g * rep + j) * vdim + i % vdim] = from_f32<AT>(o * s_l[j]);
     }
 }

@@ -55,3 +55,9 @@ def test_read_only_loads_are_of_weights(path):
         assert "ld.global.nc" not in text
     found = {a for call in ("__ldg", "ldg_nc_u2", "ldg_nc_u4") for a in arguments(text, call)}
     assert found <= READ_ONLY_LOADS.get(path.name, set()), found
+
+
+@pytest.mark.parametrize("path", FILES, ids=lambda p: p.name)
+def test_loads_from_l2_keep_their_place(path):
+    """ld_l2 stays behind waits and fences; the built-in promises nothing of the kind."""
+    assert not re.search(r"__ldc[gas]\(", code(path))
