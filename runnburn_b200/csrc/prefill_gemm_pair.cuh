@@ -212,7 +212,7 @@ __device__ __forceinline__ void pt_dequant_q6(const uint8_t *blk, int g, uint32_
 }
 // The same where all rows of a warp have their block at 4 K + 2 odd bytes behind a 16-byte boundary (base): which words are needed
 // is known.  An element's six bits in a byte become f16 of 1024 + q by one permutation for two; d times that less what is too
-// much, and its product with the scale, are exact in f32, as they are above.
+// much, and its product with the scale, are exact in f32, as they are above.  d is finite: else that difference is NaN for every q.
 template <int K, class F>
 __device__ __forceinline__ void pt_dequant_q6_at(const uint8_t *base, uint32_t odd, int g, uint32_t (&o)[32], F &&read) {
     const int n = g >> 1;
@@ -420,8 +420,10 @@ prefill_gemm_pair_kernel(const __grid_constant__ PgJobs jobs, const __grid_const
                         __syncwarp();
                         if (lane == 0) pg_arrive(&raw_empty[rs]);
                     };
+                    // an infinite scale of a Q6_K block (the look for one costs 0.7 % of a 203-token prompt)
+                    auto beyond = [&]() { return (*reinterpret_cast<const uint16_t *>(at + rs * PT_RAW_BYTES + (shift & 15u) + 208) & 0x7c00u) == 0x7c00u; };
                     if (q4) pt_dequant_q4(at + rs * PT_RAW_BYTES, grp, o, read);
-                    else if (skew) pt_dequant_q6(at + rs * PT_RAW_BYTES + (shift & 15u), grp, o, read);
+                    else if (skew || __any_sync(0xffffffffu, beyond())) pt_dequant_q6(at + rs * PT_RAW_BYTES + (shift & 15u), grp, o, read);
                     else {
                         const uint8_t *base = at + rs * PT_RAW_BYTES;
                         const uint32_t odd = (shift >> 1) & 1u;

@@ -10,7 +10,7 @@ import numpy as np
 import pytest
 
 import oracle as orc
-from synth import Q4_K, Q6_K
+from synth import Q4_K, Q6_K, random_blocks
 from test_gpu_prefill_gemm import bf16_round, ops  # noqa: F401
 from test_gpu_prefill_pair import off, weights
 
@@ -55,3 +55,43 @@ def test_gate_and_up_in_tensor_memory(ops, t, rows, cols, seq):
     bound = 1e-4 * (1.1 * sg * np.abs(u) + np.abs(g) * su) + 2.0 ** -8 * np.abs(want) + 1e-30
     got = act.float().cpu().numpy()
     assert np.all(np.abs(got - want) <= bound)
+
+
+@pytest.mark.parametrize("t,cols,seq", [(Q6_K, 2048, 45), (Q6_K, 1280, 45), (Q6_K, 2048, 300), (Q4_K, 2048, 45), (Q6_K, 768, 45)])
+def test_a_block_with_an_infinite_scale(ops, t, cols, seq):
+    """Its elements are infinities of their signs, 0 x infinity where a quant or a sub-block scale is zero: rows of one sign give that
+    infinity, rows of both and rows with a zero give NaN, and the other rows stay as they are."""
+    rng = np.random.default_rng(cols + seq)
+    rows, nb = 130, cols // 256
+    w = random_blocks(rng, t, rows, cols).reshape(rows, nb, -1)
+    x = np.abs(rng.standard_normal((seq, cols))).astype(np.float32) + 0.5
+    d = slice(208, 210) if t == Q6_K else slice(0, 2)
+
+    def block(row, scale, quant, zeros=()):
+        b = w[row, 1]
+        if t == Q6_K:
+            q = np.full(256, quant)
+            q[list(zeros)] = 32
+            part, l = q.reshape(2, 4, 32), np.arange(32)
+            for n in range(2):
+                b[64 * n + l] = (part[n, 0] & 15) | ((part[n, 2] & 15) << 4)
+                b[64 * n + 32 + l] = (part[n, 1] & 15) | ((part[n, 3] & 15) << 4)
+                b[128 + 32 * n + l] = sum((part[n, i] >> 4) << (2 * i) for i in range(4))
+            b[192:208] = 3
+        else:
+            b[4:16], b[2:4] = 0x11, 0
+            b[16:] = 0x55 if not zeros else 0x50
+        b[d] = np.frombuffer(np.float16(scale).tobytes(), np.uint8)
+
+    block(3, np.inf, 40)
+    block(64, -np.inf, 63)
+    block(77, np.inf, 41, zeros=(5, 200))
+    if t == Q6_K:
+        block(129, np.inf, 7)
+    fn = ops.q4k_bf16_gemm_batch if t == Q4_K else ops.q6k_bf16_gemm_batch
+    got = fn(np.ascontiguousarray(w).reshape(-1), rows, cols, x).reshape(seq, rows)
+    assert np.all(got[:, 3] == np.inf) and np.all(got[:, 64] == -np.inf) and np.all(np.isnan(got[:, 77]))
+    if t == Q6_K:
+        assert np.all(got[:, 129] == -np.inf)
+    rest = [r for r in range(rows) if r not in (3, 64, 77, 129)]
+    assert off(got[:, rest], t, np.ascontiguousarray(w[rest]).reshape(-1), len(rest), cols, x) <= 1e-4
