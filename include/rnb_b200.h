@@ -713,6 +713,11 @@ int rnb_b200_dev_prefill_gemm_multi(int n, const int *types, const uint8_t *cons
 int rnb_b200_dev_prefill_gemm_silu(int type, const uint8_t *gate_dev, const uint8_t *up_dev,
                                    size_t rows, size_t cols, const float *x_dev, size_t seq,
                                    uint16_t *xb_dev, uint16_t *act_dev, void *stream);
+/* The kernel that a prefill matmul of these matrices takes, for tests: 0 rows of less than four blocks and up to 128 tokens,
+ * 1 weights in tensor memory, 2 weights in shared memory with tiles of up to 512 tokens; the tokens of a tile; the portions
+ * that K is cut into.  w2_dev: the up matrix of gate + up (n = 1), else null.  Addresses count for their alignment alone. */
+int rnb_b200_dev_prefill_gemm_plan(int n, const int *types, const uint8_t *const *w_dev, const uint8_t *w2_dev,
+                                   const size_t *rows, size_t cols, size_t seq, int *kernel, int *tokens, int *cuts);
 int rnb_b200_dev_flash_decode(const float *q_dev, const uint16_t *k_dev, const uint16_t *v_dev,
                               size_t kv_len, size_t num_heads, size_t num_kv_heads, float scale,
                               float *partials_dev, size_t partials_bytes, int n_chunks,

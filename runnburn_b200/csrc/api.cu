@@ -294,7 +294,6 @@ int State::check_dev_error() {
     return RNB_B200_OK;
 }
 
-// D2H of results through pinned staging, then synchronise and surface device error flags.
 // A result and the error flag into pinned memory by a kernel of the chain, 16 bytes a thread.
 RNB_GLOBAL void __launch_bounds__(256)
 deliver_kernel(const uint8_t *src, uint8_t *host, size_t n, const int *err, int *host_err) {
@@ -308,6 +307,7 @@ deliver_kernel(const uint8_t *src, uint8_t *host, size_t n, const int *err, int 
 // Up to this size a kernel moves data between pinned memory and the device instead of a copy: 16 KB of a matvec's input and result took
 // three copies and gaps between them, 20 of 42 us.  Larger ones are faster by the copy engine.
 constexpr size_t DIRECT_BYTES = 128 * 1024;
+// D2H of results through pinned staging, then synchronise and surface device error flags.
 static int finish_to_host(State &st, const void *dev_src, void *host_dst, size_t n) {
     RNB_TRY(st.pin_out.ensure(n + 16));
     int *flag = reinterpret_cast<int *>(st.pin_out.as<uint8_t>() + ((n + 3) & ~(size_t)3));
@@ -760,6 +760,31 @@ int rnb_b200_dev_prefill_gemm_multi(int n, const int *types, const uint8_t *cons
     Locked L;
     RNB_TRY(L.st.open());
     return launch_prefill_gemm_multi((cudaStream_t)stream, n, types, w_dev, rows, y_dev, cols, x_dev, seq, xb_dev, L.st.dev_error);
+}
+
+int rnb_b200_dev_prefill_gemm_plan(int n, const int *types, const uint8_t *const *w_dev, const uint8_t *w2_dev, const size_t *rows, size_t cols, size_t seq,
+                                   int *kernel, int *tokens, int *cuts) {
+    if (!types || !w_dev || !rows || !kernel || !tokens || !cuts) return fail(RNB_B200_VALIDATION_FAILED, "null pointer argument");
+    if (n < 1 || n > PG_MAX_JOBS || (w2_dev && n != 1) || cols == 0 || cols % 256 != 0 || seq == 0) return fail(RNB_B200_VALIDATION_FAILED, "prefill plan: bad shape");
+    PgJobs jobs;
+    memset(&jobs, 0, sizeof(jobs));
+    jobs.n = n;
+    jobs.j[0].w2 = w2_dev;
+    int tiles = 0;
+    for (int i = 0; i < n; i++) {
+        const size_t per = w2_dev ? PG_ROWS / 2 : PG_ROWS;
+        jobs.j[i].w = w_dev[i];
+        jobs.j[i].type = types[i];
+        tiles += (int)((rows[i] + per - 1) / per);
+    }
+    Locked L;
+    RNB_TRY(L.st.open());
+    RNB_TRY(prefill_gemm_setup());
+    const PrefillPlan plan = prefill_plan(jobs, tiles, seq, cols);
+    *kernel = plan.kernel;
+    *tokens = plan.kernel == PREFILL_WIDE ? plan.W.n1 + plan.W.n2 : plan.kernel == PREFILL_PAIR ? plan.P.nt : (int)((seq + 15) & ~(size_t)15);
+    *cuts = plan.kernel == PREFILL_PAIR ? plan.P.ks : 1;
+    return RNB_B200_OK;
 }
 
 int rnb_b200_dev_prefill_gemm_silu(int type, const uint8_t *gate_dev, const uint8_t *up_dev, size_t rows, size_t cols, const float *x_dev, size_t seq,

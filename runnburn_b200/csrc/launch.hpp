@@ -777,23 +777,39 @@ inline long prefill_wide_tiles(PwParams &P) {
     }
     return best;
 }
+// The kernel of a launch and its tiles
+enum PrefillKernel { PREFILL_SPLIT, PREFILL_PAIR, PREFILL_WIDE };
+struct PrefillPlan {
+    PrefillKernel kernel;
+    PtParams P;
+    PwParams W;
+};
 // `tiles`: row tiles of all jobs
-inline int launch_prefill_gemm_tiles(cudaStream_t s, const PgJobs &jobs, int tiles, size_t seq, size_t cols, const uint16_t *xb, int *dev_error) {
-    bool q4 = true;
-    for (int i = 0; i < jobs.n; i++) q4 = q4 && jobs.j[i].type == TYPE_Q4_K;
+inline PrefillPlan prefill_plan(const PgJobs &jobs, int tiles, size_t seq, size_t cols) {
+    PrefillPlan plan = {};
     // Up to 128 tokens of rows of less than four blocks: two CTAs per SM and no cluster start faster (256 x 256 at two tokens 13 against 15 us,
     // 20480 x 512 17.4 against 19.5; of four blocks the pairs are, 1024 x 1024 at 45 tokens 22 against 17.5).
-    if (cols >= 1024 || seq > 128) {
-        PtParams P;
-        PwParams W;
-        P.seq = W.seq = (int)seq;
-        P.cols = W.cols = (int)cols;
-        P.row_tiles = W.row_tiles = tiles;
-        P.skew = 0;
-        for (int i = 0; i < jobs.n; i++)
-            if (((uintptr_t)jobs.j[i].w | (uintptr_t)jobs.j[i].w2 | row_bytes_of(jobs.j[i].type, cols)) & 15u) P.skew |= 1 << i;
-        W.direct = P.skew;
-        const bool wide = prefill_wide_tiles(W) < prefill_pair_tiles(P, q4);
+    if (cols < 1024 && seq <= 128) return plan;
+    PtParams &P = plan.P;
+    PwParams &W = plan.W;
+    bool q4 = true;
+    P.seq = W.seq = (int)seq;
+    P.cols = W.cols = (int)cols;
+    P.row_tiles = W.row_tiles = tiles;
+    for (int i = 0; i < jobs.n; i++) {
+        q4 = q4 && jobs.j[i].type == TYPE_Q4_K;
+        if (((uintptr_t)jobs.j[i].w | (uintptr_t)jobs.j[i].w2 | row_bytes_of(jobs.j[i].type, cols)) & 15u) P.skew |= 1 << i;
+    }
+    W.direct = P.skew;
+    plan.kernel = prefill_wide_tiles(W) < prefill_pair_tiles(P, q4) ? PREFILL_WIDE : PREFILL_PAIR;
+    return plan;
+}
+inline int launch_prefill_gemm_tiles(cudaStream_t s, const PgJobs &jobs, int tiles, size_t seq, size_t cols, const uint16_t *xb, int *dev_error) {
+    const PrefillPlan plan = prefill_plan(jobs, tiles, seq, cols);
+    if (plan.kernel != PREFILL_SPLIT) {
+        const PtParams &P = plan.P;
+        const PwParams &W = plan.W;
+        const bool wide = plan.kernel == PREFILL_WIDE;
         PtMaps maps;
         PwMaps wmaps;
         memset(&maps, 0, sizeof(maps));
