@@ -766,13 +766,16 @@ inline long prefill_pair_tiles(PtParams &P, bool q4) {
     }
     return best;
 }
-// The same of prefill_gemm_wide_kernel: tokens of a tile, in two parts (multiples of 32)
-inline long prefill_wide_tiles(PwParams &P) {
+// The same of prefill_gemm_wide_kernel: tokens of a tile, in two parts (multiples of 32).  What takes tiled copies has constants by format, so
+// that it is taken where it is the faster one while every SM is at work and the clock is down: Q4_K 8192 x 8192 at 850 tokens 98.8 -> 92.6 us,
+// 11008 x 4096 at 1300 102.4 -> 96.5, Q6_K 14336 x 4096 at 1024 115.5 -> 108.8 against one set for all.
+inline long prefill_wide_tiles(PwParams &P, bool q4) {
     const int row_pairs = (P.row_tiles + 1) / 2, nb = P.cols / 256, first = (P.seq + PW_TOK - 1) / PW_TOK;
     long best = -1;
     for (int n = first; n <= 2 * first; n++) {
         const int nt = std::max(((P.seq + n - 1) / n + 31) & ~31, 64), token_tiles = (P.seq + nt - 1) / nt, tiles = row_pairs * token_tiles;
-        const long rounds = (tiles + pg_pairs() - 1) / pg_pairs(), ns = rounds * (nb * (2500 + 4 * std::max(nt - 450, 0)) + 2400 + 15 * nt);
+        const long rounds = (tiles + pg_pairs() - 1) / pg_pairs(), over = std::max(nt - 450, 0);
+        const long block = P.direct ? 2500 + 4 * over : q4 ? 2250 + 4 * over : 2625 + 3 * over, ns = rounds * (nb * block + 2400 + (P.direct ? 15 : 10) * nt);
         if (best < 0 || ns < best) best = ns, P.n1 = (nt / 2 + 31) & ~31, P.n2 = nt - P.n1, P.token_tiles = token_tiles, P.tiles = tiles;
     }
     return best;
@@ -801,7 +804,7 @@ inline PrefillPlan prefill_plan(const PgJobs &jobs, int tiles, size_t seq, size_
         if (((uintptr_t)jobs.j[i].w | (uintptr_t)jobs.j[i].w2 | row_bytes_of(jobs.j[i].type, cols)) & 15u) P.skew |= 1 << i;
     }
     W.direct = P.skew;
-    plan.kernel = prefill_wide_tiles(W) < prefill_pair_tiles(P, q4) ? PREFILL_WIDE : PREFILL_PAIR;
+    plan.kernel = prefill_wide_tiles(W, q4) < prefill_pair_tiles(P, q4) ? PREFILL_WIDE : PREFILL_PAIR;
     return plan;
 }
 inline int launch_prefill_gemm_tiles(cudaStream_t s, const PgJobs &jobs, int tiles, size_t seq, size_t cols, const uint16_t *xb, int *dev_error) {

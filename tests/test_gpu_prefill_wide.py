@@ -61,6 +61,12 @@ def test_matrices_of_both_formats(ops, types, rows):
     multiply(ops, types, rows, 2048, 1153, sum(rows))
 
 
+@pytest.mark.parametrize("rows,cols,seq", [(4990, 4096, 1300)])
+def test_one_matrix_of_four_bits(ops, rows, cols, seq):
+    """An odd number of row tiles; the last tile of tokens holds 404 of 448."""
+    multiply(ops, (Q4_K,), (rows,), cols, seq, rows)
+
+
 def test_gate_and_up(ops):
     import torch
 
@@ -85,7 +91,9 @@ def test_gate_and_up(ops):
 
 @pytest.mark.parametrize("t,rows,cols,seq,want", [
     (Q6_K, 256, 256, 2, SPLIT), (Q6_K, 256, 768, 128, SPLIT), (Q6_K, 256, 768, 129, PAIR), (Q6_K, 256, 1024, 2, PAIR),   # rows of less than four blocks, 128 tokens
-    (Q4_K, 9472, 4096, 1024, PAIR), (Q6_K, 9472, 4096, 300, PAIR),
+    (Q6_K, 9472, 4096, 300, PAIR),
+    (Q4_K, 8192, 8192, 850, WIDE), (Q4_K, 11008, 4096, 1300, WIDE), (Q6_K, 14336, 4096, 1024, WIDE),   # where this kernel is the faster one by 6 %
+    (Q4_K, 28672, 4096, 2048, PAIR), (Q6_K, 4096, 14336, 203, PAIR),
 ])
 def test_the_kernel_of_a_launch(ops, t, rows, cols, seq, want):
     import torch
