@@ -304,8 +304,9 @@ deliver_kernel(const uint8_t *src, uint8_t *host, size_t n, const int *err, int 
         for (size_t k = i; k < n; k++) host[k] = src[k];
     if (i == 0) *host_err = *err;
 }
-// Up to this size a kernel moves data between pinned memory and the device instead of a copy: 16 KB of a matvec's input and result took
-// three copies and gaps between them, 20 of 42 us.  Larger ones are faster by the copy engine.
+// Up to this size a kernel moves data between pinned memory and the device instead of a copy.  Whole calls, us, copies / kernel, Q4_K of 256
+// columns: a result of 16 KB 32.7 / 25.2, 128 KB 47.6 / 34.7, 256 KB 54.5 / 42.5, 512 KB 69.4 / 60.5; an input of 16 KB 103.3 / 92.5, 128 KB
+// 603 / 590, 256 KB 1158 / 1153, 512 KB 2501 / 2514.  The line is where the gain on an input falls under 2 %, not where copies win.
 constexpr size_t DIRECT_BYTES = 128 * 1024;
 // D2H of results through pinned staging, then synchronise and surface device error flags.
 static int finish_to_host(State &st, const void *dev_src, void *host_dst, size_t n) {

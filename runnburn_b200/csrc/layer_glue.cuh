@@ -141,7 +141,7 @@ residual_norm_kernel(const __grid_constant__ ResidualNormArgs a) {
                     const Vec mu = *reinterpret_cast<const Vec *>(a.mu + (size_t)s * D + i);
                     HVec o;
 #pragma unroll
-                    for (int e = 0; e < V; e++) o.v[e] = from_f32<HT>(c.v[e] + (p.v[e] - c.v[e]) * mu.v[e]);
+                    for (int e = 0; e < V; e++) o.v[e] = from_f32<HT>(fmaf(p.v[e] - c.v[e], mu.v[e], c.v[e]));
                     *reinterpret_cast<HVec *>(h + (size_t)s * a.tokens * D + row + i) = o;
                 }
             } else {

@@ -127,3 +127,41 @@ def test_chained_steps_repeat_the_bits_of_host_steps(model):
         dec.sync()
         assert np.array_equal(dec.read_logits(), logits)
     dec.close()
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("width", [124, 2044, 2048, 4092, 4096, 4097, 4100])
+def test_norms_of_one_token(width, dtype):
+    """Steps at the widths where the norm of one token ends (4096, multiples of 4, whole warps): root-mean-square norms with token shift
+    and an embedding that is added again, and layer norms with a bias; against the plain reference, bounds of the stacks' tests."""
+    import hybrid_ref as ref
+    import stack_util as su
+    for cfg in (su.config([su.wkv(heads=2, ff=0), su.retention(heads=1)], width=width, vocab=31, loop={"start": 0, "stop": 2, "times": 2}),
+                su.dutivik([su.gla(heads=2), su.parallel(ff=0)], width=width, vocab=31)):
+        w = su.weights(cfg, 3)
+        toks = su.tokens(cfg, 12)
+        dec = su.decoder(cfg, w, dtype)
+        assert not su.bad(su.feed(dec, toks, [3] + [1] * 9), ref.Model(cfg, w).forward(toks), dtype)
+        dec.close()
+
+
+@pytest.mark.parametrize("rows", [1, 3, 5, 1021, 32764, 32767, 32768, 32769])
+def test_results_up_to_and_past_the_direct_limit(ops, rows):
+    """A result of 128 KB is written to the host by a kernel, a larger one by a copy; whole 16 bytes and ends of every size."""
+    rng = np.random.default_rng(rows)
+    w, x = random_blocks(rng, Q4_K, rows, 256), rng.standard_normal(256).astype(np.float32)
+    assert bits_equal(ops.q4k_gemv(w, rows, 256, x), orc.gemv(Q4_K, w, x, rows, 256))
+    ops.clear_q4k_cache()
+
+
+@pytest.mark.parametrize("t", [Q4_K, Q6_K])
+@pytest.mark.parametrize("seq", [1, 127, 128, 129])
+def test_inputs_up_to_and_past_the_direct_limit(ops, t, seq):
+    """128 tokens of 256 values are read where they are staged, 129 are copied first; and one call behind the other does not see the last one's."""
+    rng = np.random.default_rng(seq)
+    w = random_blocks(rng, t, 20, 256)
+    fn = ops.q4k_gemv_batch if t == Q4_K else ops.q6k_gemv_batch
+    for _ in range(3):
+        x = rng.standard_normal((seq, 256)).astype(np.float32)
+        assert bits_equal(fn(w, 20, 256, x).reshape(seq, 20), np.stack([orc.gemv(t, w, x[i], 20, 256) for i in range(seq)]))
+    ops.clear_q4k_cache()
