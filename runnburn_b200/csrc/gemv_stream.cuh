@@ -158,8 +158,8 @@ __device__ __forceinline__ void gr_run(const GemvJob *job, const GsParams &P, co
         }
     };
     // Rows that bulk copies cannot fetch (their bytes start at any even address: Q6_K of a number of blocks that is not a multiple
-    // of eight): a row's eight threads take it in aligned words, sixteen in flight each, shifted into place.  It was byte by byte behind the
-    // dependency wait: in the step of a small model 512 rows of 4 blocks took 27 us, now 3.8, the 2 blocks of a vocabulary of 2048 15.6, now 2.3.
+    // of eight): a row's eight threads take it in aligned words, sixteen in flight each, shifted into place.  In the step of a small model 512
+    // rows of 4 blocks take 3.8 us, byte by byte behind the dependency wait 27; the 2 blocks of a vocabulary of 2048 2.3 and 15.6.
     auto fetch_row = [&](int p, int c, uint8_t *slot) {
         const int r = tid >> 3, nblk = min(CB, nb - c * CB);
         if (r >= nrows) return;

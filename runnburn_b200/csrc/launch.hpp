@@ -742,10 +742,12 @@ inline int encode_token_map(PgTensorMap *out, const uint16_t *xb, size_t seq, si
 inline int pg_sms() { return state().sm_count > 0 ? state().sm_count : 148; }
 inline int pg_pairs() { return std::max(1, pg_sms() / 2); }
 int prefill_clusters(int ks);   // clusters of 2 ks CTAs that run at the same time (0: unknown)
-// Tokens of a tile and pairs along K: the least of a model of the time in ns, fitted to 1184 launches (14 shapes of 1024 to 32768
-// rows, 1024 to 14336 columns, both formats, 20 to 2048 tokens, all cuts): what it picks is 0.4 % above the fastest on
-// average, 16 % at most (2048 x 2048 at 203 tokens: 21.5 against 18.5 us).  A block of K costs its dequantisation and, above 128
-// tokens, ever more of the tensor pipe; a tile of two parts has the shallow ring; every round its fill and its way back; a cut its sum.
+// Tokens of a tile and pairs along K: the least of a model of the time in ns, a least-squares fit to 1184 launches timed one by one
+// (14 shapes of 1024 to 32768 rows, 1024 to 14336 columns, both formats, 20 to 2048 tokens, all cuts).  A block of K costs its
+// dequantisation and, above 128 tokens, ever more of the tensor pipe; a tile of two parts has the shallow ring; every round its fill and its
+// way back; a cut its sum.  Measured again with prefill_wide_tiles on 800 launches that follow each other (20 shapes, 2 to 3000 tokens):
+// what the two pick is 0.9 % above the fastest of all candidates on average, over 5 % in 50 of them, 30 % at most (skewed Q6_K of
+// 4096 x 11008 at 1300 tokens: 165 against 127 us).
 inline long prefill_pair_tiles(PtParams &P, bool q4) {
     const int row_pairs = (P.row_tiles + 1) / 2, nb = P.cols / 256, first = (P.seq + PT_TOK - 1) / PT_TOK;
     // Launches whose tiles fill the chip, and rows of less than 16 blocks above 128 tokens, are summed in one chain along K in

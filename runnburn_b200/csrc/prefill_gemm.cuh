@@ -6,8 +6,8 @@
 // crates/rnb-cpu/src/quantize/dequant.rs:353-381 (Q4_K) and :780-807 (Q6_K) in f32 and rounds
 // once to bf16.
 //
-// What the two kernels share (prefill_gemm_pair.cuh: pairs of SMs, weights in tensor memory; prefill_gemm_split.cuh: a few tokens of
-// short rows, weights in shared memory): the weight tile is the M operand (tensor-memory lane = weight row), the tokens the N
+// What the three kernels share (prefill_gemm_pair.cuh: pairs of SMs, weights in tensor memory; prefill_gemm_wide.cuh: pairs of SMs, tiles of
+// up to 512 tokens, weights in shared memory; prefill_gemm_split.cuh: a few tokens of short rows, the same): the weight tile is the M operand (tensor-memory lane = weight row), the tokens the N
 // operand.  Operand tiles in shared memory are 64 elements of K, K-major in the 128-byte swizzle the MMA descriptors expect:
 //   byte offset of (row r, 16-byte chunk c) = (r / 8) * 1024 + (r % 8) * 128 + ((c ^ (r % 8)) * 16).
 // Tokens come in by tiled TMA copies (rows past the end of the batch read as zeros).  Every wait is bounded; a

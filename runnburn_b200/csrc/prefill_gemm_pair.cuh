@@ -4,9 +4,10 @@
 // A pair of CTAs multiplies 256 weight rows x up to 256 tokens: each CTA dequantises its own 128 rows, brings in half of the
 // tokens, and holds its rows' accumulators in the first 256 columns of its tensor memory.  The other 256 columns are a ring of
 // weights, two blocks of K deep (64 elements = 32 columns): a thread dequantises the 64 elements of a row in registers and
-// writes them to the row's lane.  Tiles of up to 384 tokens (two MMAs, a ring of one block) dequantise less where the chip stays full.  Weights as an operand in shared memory had every stage behind a proxy fence and, in the odd
-// CTA, behind a release across the cluster; tensor memory needs neither (tcgen05.wait::st, a tcgen05 fence and a relaxed
-// arrival at the even CTA's barrier), and what the dequantising warps cost is their instructions.
+// writes them to the row's lane.  Tiles of up to 384 tokens (two MMAs, a ring of one block) dequantise less where the chip stays
+// full.  Weights as an operand in shared memory have every stage behind a proxy fence and, in the odd CTA, behind a release across the
+// cluster (prefill_gemm_wide.cuh); tensor memory needs neither (tcgen05.wait::st, a tcgen05 fence and a relaxed arrival at the even
+// CTA's barrier), and what the dequantising warps cost is their instructions.
 //
 // Blocks of 256 elements of the 128 rows come into shared memory as they are, by tiled copies, up to three ahead; a group of
 // four warps (128 rows) takes one of a block's four stages.  Both CTAs' token copies count on the even CTA's barriers.  One
@@ -18,14 +19,15 @@
 // in rank order (the same bits on every run).
 //
 // Warps 0-15 dequantise and store, warp 16 of the even CTA issues the MMAs, warp 17 of each CTA the token copies, warp 18 those
-// of the weights.  The MMAs wait for half a block at a time: with a wait a stage their loop took 2900 cycles a block, more than the rest.
+// of the weights.  The MMAs wait for half a block at a time: with a wait a stage their loop takes 2900 cycles a block, more than the rest.
 // Every wait is bounded; after a timeout all threads still meet at the cluster barrier.
 //
-// What bounds it: the issue slots of the dequantising warps (360 instructions a block and warp of Q4_K, 460 of Q6_K; a block takes
-// 1.07 and 1.43 us), from about 200 tokens a tile on the tensor pipe.  Measured with 203 / 512 / 2048 tokens, us, cold, with the
-// conversion of the tokens to bf16 (weights in shared memory before): gate + up 28672 x 4096 60 / 110 / 345 (91 / 116 / 382), down
-// 4096 x 14336 Q6_K 50 / 69 / 198 (69 / 150 / 198), q + k + v 32 / 44 / 89 (48 / 56 / 106), o 26 / 32 / 69 (40 / 48 / 69): gate + up
-// without the conversion 1460 TFLOP/s, 0.86 of the measured 1701.
+// What bounds it: the issue slots of the dequantising warps (Q4_K 407 to 424 warp instructions a block and warp, the way back of the
+// tile included; a block takes 1.1 us, 1.23 with every SM at work, of Q6_K 1.45 and 1.6), from about 200 tokens a tile on the tensor pipe.
+// Measured with 203 / 511 / 2048 tokens, us, cold, with the conversion of the tokens to bf16 (weights in shared memory before): gate + up
+// 28672 x 4096 60 / 110 / 335 (89 / 114 / 372), down 4096 x 14336 Q6_K 50 / 71 / 190 (68 / 116 / 191), q + k + v 32 / 44 / 89 (48 / 54 / 103), o
+// 26 / 32 / 69 (40 / 48 / 69).  ncu, 2048 tokens: gate + up 354 us = 1357 TFLOP/s = 0.82 of the measured 1658, tensor pipe 80 % and issue
+// slots 67 % of the active cycles; o 65 and 56 %, q + k + v 70 and 46 %.
 #pragma once
 #include "prefill_gemm.cuh"
 #include "prefill_gemm_split.cuh"
@@ -49,8 +51,9 @@ struct PtParams {
     int row_tiles, token_tiles, tiles; // tiles: pairs of row tiles x token tiles
     int skew;                          // bit i: job i's rows start at any even address (Q6_K)
 };
-// Tokens (boxes of half a part of a tile: up to 256 tokens are one part, more are two); blocks of each job's rows, and of the second matrix of a pair: boxes of 64 rows.  Skewed rows have a map for
-// every eighth row (they lie a multiple of 16 bytes apart), from the 16-byte boundary before its first byte: boxes of 16, 8 in a pair.
+// Tokens (boxes of half a part of a tile: up to 256 tokens are one part, more are two); blocks of each job's rows, and of the second
+// matrix of a pair: boxes of 64 rows.  Skewed rows have a map for every eighth row (they lie a multiple of 16 bytes apart), from the 16-byte
+// boundary before its first byte: boxes of 16, 8 in a pair.
 struct PtMaps {
     PgTensorMap x, w[PG_MAX_JOBS][8], w2[8];
 };

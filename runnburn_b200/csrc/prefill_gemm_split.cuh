@@ -13,7 +13,6 @@
 
 namespace rnb {
 
-constexpr int PS_TOK = 128;        // most tokens
 constexpr int PS_THREADS = 320;
 constexpr int PS_MAX_STAGES = 5;
 constexpr uint32_t PS_SMEM_STAGES = 96 * 1024;   // operand stages; the reduction reuses them: 64 KB of slots, 32 KB of exchange

@@ -1,9 +1,8 @@
 """Prefill matmul with the weights in tensor memory: tiles of one part (up to 256 tokens) and of two, K cut over two to four pairs
-of SMs, rows that start at any even address (less than eight of them, in a pair of matrices too), and a launch whose tiles of
-512 tokens go to the kernel with the weights in shared memory.
+of SMs, rows that start at any even address (less than eight of them, in a pair of matrices too), and blocks whose scale is infinite.
 
 Bound: f32 accumulation only, 1e-4 of a dot product's scale sqrt(sum (x w)^2), as for the other prompt kernels; silu(gate) * up is
-rounded to bf16 once more, half a unit in the last place (2^-9), on products that are off by that bound."""
+rounded to bf16 once more, half a unit in the last place (2^-8 at most), on products that are off by that bound."""
 import ctypes
 
 import numpy as np
